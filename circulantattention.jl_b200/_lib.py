@@ -7,6 +7,8 @@ raises, and every op raises on non-CUDA tensors.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
@@ -44,7 +46,7 @@ def _load():
         raise ImportError(
             f"{LIB_PATH} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'` "
             "(nvcc, sm_100a). There is no CPU or PyTorch fallback.")
-    return C.CDLL(LIB_PATH)
+    return C.CDLL(LIB_PATH, mode=C.RTLD_GLOBAL)      # global: the host extension resolves the ca_* symbols from it
 
 
 lib = _load()
@@ -97,6 +99,23 @@ for _name, (_res, _args) in PROTOTYPES.items():
     _fn = getattr(lib, _name)
     _fn.restype = _res
     _fn.argtypes = _args
+
+
+def _load_host():
+    """The native host path (csrc/host.cpp): allocation, descriptors and autograd nodes around the C ABI."""
+    path = os.path.join(PKG_DIR, "_circatt_host.so")
+    if not os.path.exists(path):
+        raise ImportError(f"{path} is missing: build it with `python -c 'import __graft_entry__ as g; g.build()'`")
+    import torch  # noqa: F401  (loads the libraries the extension links against)
+    loader = importlib.machinery.ExtensionFileLoader("_circatt_host", path)
+    spec = importlib.util.spec_from_file_location("_circatt_host", path, loader=loader)
+    mod = importlib.util.module_from_spec(spec)
+    loader.exec_module(mod)
+    mod.set_error_class(CircAttError)
+    return mod
+
+
+host = _load_host()
 
 
 def last_error() -> str:

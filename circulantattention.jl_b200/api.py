@@ -2,10 +2,10 @@
 
 Names, argument meaning and error behaviour follow the reference; Julia's `!`
 suffix becomes a trailing underscore, `⊗` is `otimes` and `⨷` is `Otimes`.
-Dense arrays are Julia-shaped column-major tensors (see `jl`).  Gradients are
-attached with `torch.autograd.Function`s that play the role of the reference's
-ChainRules rrules (src/rrules.jl); every forward and pullback is one or more
-calls into the C ABI.
+Dense arrays are Julia-shaped column-major tensors (see `jl`).  Gradients come
+from the autograd nodes of the native host path (csrc/host.cpp), which play the role
+of the reference's ChainRules rrules (src/rrules.jl); every forward and pullback is
+one or more calls into the C ABI.
 """
 from __future__ import annotations
 
@@ -15,7 +15,7 @@ from typing import Optional
 import torch
 
 from . import jl, ops
-from ._lib import CA_DISTANCE, CA_DOT, CA_ENTMAX15, CA_SOFTMAX
+from ._lib import CA_DISTANCE, CA_DOT, CA_ENTMAX15, CA_SOFTMAX, host
 
 
 # ----------------------------------------------------------------- similarity types
@@ -155,7 +155,7 @@ class Circulant:
             raise AssertionError("only batch dims of a Circulant can be repeated")
         breps = tuple(reps[2:]) + (1,) * (len(self.batch) - len(reps[2:]))
         c = jl.ones(breps, torch.float32, self.nzVal.device)
-        return Circulant._from_nz(_ScaleFn.apply(c, self.nzVal), self.kernel_length, self.spatial_size)
+        return Circulant._from_nz(host.scale_batch(c, self.nzVal), self.kernel_length, self.spatial_size)
 
     # -- algebra (src/array.jl:66-85, 179-189)
     def _same(self, other):
@@ -165,11 +165,11 @@ class Circulant:
 
     def __add__(self, other):
         self._same(other)
-        return Circulant._from_nz(_AxpbyFn.apply(self.nzVal, other.nzVal, 1.0, 1.0), self.kernel_length, self.spatial_size)
+        return Circulant._from_nz(host.axpby(self.nzVal, other.nzVal, 1.0, 1.0), self.kernel_length, self.spatial_size)
 
     def __sub__(self, other):
         self._same(other)
-        return Circulant._from_nz(_AxpbyFn.apply(self.nzVal, other.nzVal, 1.0, -1.0), self.kernel_length, self.spatial_size)
+        return Circulant._from_nz(host.axpby(self.nzVal, other.nzVal, 1.0, -1.0), self.kernel_length, self.spatial_size)
 
     def __neg__(self):
         return -1 * self
@@ -180,7 +180,7 @@ class Circulant:
     def __rmul__(self, c):
         if isinstance(c, torch.Tensor) and c.ndim > 0:
             return scale(c, self)                                        # src/array.jl:189
-        return Circulant._from_nz(_AxpbyFn.apply(self.nzVal, None, float(c), 0.0), self.kernel_length, self.spatial_size)
+        return Circulant._from_nz(host.axpby(self.nzVal, None, float(c), 0.0), self.kernel_length, self.spatial_size)
 
     def __eq__(self, other):                                             # src/array.jl:103-117
         if not isinstance(other, Circulant):
@@ -217,146 +217,6 @@ def spatial_dims(A):
     return len(A.spatial_size)
 
 
-# ----------------------------------------------------------------- autograd glue
-class _AxpbyFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, y, alpha, beta):
-        ctx.ab = (alpha, beta, y is not None)
-        return ops.axpby(alpha, x, beta, y)
-
-    @staticmethod
-    def backward(ctx, g):
-        alpha, beta, has_y = ctx.ab
-        gx = ops.axpby(alpha, g) if ctx.needs_input_grad[0] else None
-        gy = ops.axpby(beta, g) if has_y and ctx.needs_input_grad[1] else None
-        return gx, gy, None, None
-
-
-class _ScaleFn(torch.autograd.Function):
-    """scale(c, A) and its pullback (src/array.jl:179-186, src/rrules.jl:97-114)."""
-
-    @staticmethod
-    def forward(ctx, c, nz):
-        ctx.save_for_backward(c, nz)
-        return ops.scale_batch(c, nz)
-
-    @staticmethod
-    def backward(ctx, dB):
-        c, nz = ctx.saved_tensors
-        dc = dA = None
-        nb = max(c.ndim, nz.ndim - 1)
-        cs = tuple(c.shape) + (1,) * (nb - c.ndim)
-        as_ = tuple(nz.shape[1:]) + (1,) * (nb - (nz.ndim - 1))
-        if ctx.needs_input_grad[0]:
-            full = ops.dot_batch(dB, nz)                                  # (o1, o2): per-slice sum dB*A
-            full = jl.reshape(full, (1,) + tuple(full.shape))
-            s1 = cs[0] == 1 and full.shape[1] > 1
-            s2 = len(cs) > 1 and cs[1] == 1 and full.ndim > 2 and full.shape[2] > 1
-            red = ops.sum_batch(full, s1, s2) if (s1 or s2) else full
-            dc = jl.reshape(red, tuple(c.shape))
-        if ctx.needs_input_grad[1]:
-            full = ops.scale_batch(c, dB)
-            s1 = as_[0] == 1 and full.shape[1] > 1
-            s2 = len(as_) > 1 and as_[1] == 1 and full.ndim > 2 and full.shape[2] > 1
-            red = ops.sum_batch(full, s1, s2) if (s1 or s2) else full
-            dA = jl.reshape(red, tuple(nz.shape))
-        return dc, dA
-
-
-class _SimilarityFn(torch.autograd.Function):
-    """circulant_similarity and its rrules (src/similarity.jl:138-142, src/rrules.jl:1-32)."""
-
-    @staticmethod
-    def forward(ctx, x, y, kind, ws):
-        ctx.save_for_backward(x, y)
-        ctx.cfg = (kind, ws)
-        return ops.similarity(kind, x, y, ws)
-
-    @staticmethod
-    def backward(ctx, dS):
-        x, y = ctx.saved_tensors
-        kind, ws = ctx.cfg
-        dx, dy = ops.similarity_bwd(kind, x, y, ws, dS)
-        return dx, dy, None, None
-
-
-class _NormalizeFn(torch.autograd.Function):
-    """NNlib.softmax(::Circulant) and its rrule (src/similarity.jl:113-126, src/rrules.jl:42-56)."""
-
-    @staticmethod
-    def forward(ctx, nz, spatial, ws, normalizer):
-        p = ops.row_normalize(nz, spatial, ws, normalizer)
-        ctx.save_for_backward(p)
-        ctx.cfg = (spatial, ws, normalizer)
-        return p
-
-    @staticmethod
-    def backward(ctx, dp):
-        (p,) = ctx.saved_tensors
-        spatial, ws, normalizer = ctx.cfg
-        return ops.row_normalize_bwd(p, dp, spatial, ws, normalizer), None, None, None
-
-
-class _ApplyFn(torch.autograd.Function):
-    """A ⊗ x / Aᵀ ⊗ x and their rrules (src/attention.jl:53-80, src/rrules.jl:58-88)."""
-
-    @staticmethod
-    def forward(ctx, nz, x, ws, transpose):
-        ctx.save_for_backward(nz, x)
-        ctx.cfg = (ws, transpose)
-        return ops.apply(jl.reshape(nz, (nz.shape[0], -1)), x, ws, transpose)
-
-    @staticmethod
-    def backward(ctx, dc):
-        nz, x = ctx.saved_tensors
-        ws, transpose = ctx.cfg
-        ua = nz.numel() // nz.shape[0]
-        if ua != x.shape[-1]:
-            raise NotImplementedError("pullback of a batch-broadcast apply is not defined by the reference")
-        dA = db = None
-        if ctx.needs_input_grad[0]:
-            d = ops.similarity(CA_DOT, dc, x, ws) if not transpose else ops.similarity(CA_DOT, x, dc, ws)
-            dA = jl.reshape(d, tuple(nz.shape))
-        if ctx.needs_input_grad[1]:
-            db = ops.apply(jl.reshape(nz, (nz.shape[0], -1)), dc, ws, not transpose)
-        return dA, db, None, None
-
-
-class _AttentionFn(torch.autograd.Function):
-    """Fused circulant_(mh_)attention with a direct pullback equal to the composition of the reference's
-    rrules (src/rrules.jl:1-72).  The head split (src/attention.jl:44, a reshape) happens inside, so the
-    autograd graph holds one node for the whole call instead of one per reshape."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, kind, ws, normalizer, want_A, scale=None, nheads=1):
-        qr, kr, vr = (splitheads(t, nheads) for t in (q, k, v)) if nheads != 1 else (q, k, v)
-        # the forward's workspace (the packed copy of k and v) is kept for the pullback, like the
-        # intermediates the reference's pullback closures capture (src/rrules.jl:44-55)
-        y, nz, stats, fws = ops.attention_fwd(kind, normalizer, qr, kr, vr, ws, want_A, scale=scale, keep_workspace=True)
-        ctx.set_materialize_grads(False)      # an unused A must arrive as None, not as zeros, in backward
-        ctx.save_for_backward(qr, kr, vr, y, stats, nz if want_A else None)
-        ctx.fws = fws if normalizer == 0 else None
-        ctx.cfg = (kind, ws, normalizer, want_A, scale, nheads, tuple(q.shape))
-        yo = jl.reshape(y, tuple(q.shape)) if nheads != 1 else y
-        return (yo, nz) if want_A else (yo, None)
-
-    @staticmethod
-    def backward(ctx, dy, dnz):
-        q, k, v, y, stats, nz = ctx.saved_tensors
-        kind, ws, normalizer, want_A, scale, nheads, shape = ctx.cfg
-        if dy is None:
-            dy = jl.zeros(y.shape, y.dtype, y.device)
-        elif nheads != 1:
-            dy = splitheads(dy, nheads)
-        # the saved A (when the forward materialised it) spares the operator-chain backward a recomputation
-        dq, dk, dv = ops.attention_bwd(kind, normalizer, q, k, v, y, dy, stats, ws, nz=nz, dA=dnz, scale=scale,
-                                       fwd_workspace=ctx.fws)
-        ctx.fws = None
-        if nheads != 1:
-            dq, dk, dv = (jl.reshape(t, shape) for t in (dq, dk, dv))
-        return dq, dk, dv, None, None, None, None, None, None
-
-
 # ----------------------------------------------------------------- L2: similarity / adjacency
 def _kind(simfun):
     if not isinstance(simfun, AbstractSimilarity):
@@ -373,8 +233,7 @@ def circulant_similarity(simfun, x, y, W: int) -> Circulant:
     """src/similarity.jl:138-142.  Returns a Circulant of size (Np, Np, 1, B)."""
     _check_odd(W)
     _check_xy(x, y)
-    nz = _SimilarityFn.apply(x, y, _kind(simfun), int(W))
-    nz = jl.reshape(nz, (nz.shape[0], 1, x.shape[-1]))
+    nz = host.similarity(x, y, _kind(simfun), int(W), 1)
     return Circulant._from_nz(nz, int(W), tuple(x.shape[:-2]))
 
 
@@ -391,7 +250,7 @@ def circulant_similarity_(A: Circulant, simfun, x, y) -> Circulant:
 
 def softmax(A: Circulant, normalizer=SOFTMAX) -> Circulant:
     """NNlib.softmax(A::Circulant): row-wise (src/similarity.jl:113-126)."""
-    p = _NormalizeFn.apply(A.nzVal, A.spatial_size, A.kernel_length, normalizer)
+    p = host.normalize(A.nzVal, A.spatial_size, A.kernel_length, normalizer)
     return Circulant._from_nz(p, A.kernel_length, A.spatial_size)
 
 
@@ -434,12 +293,10 @@ def _fused(simfun, q, k, v, W, nheads, normalizer, return_A):
     _check_odd(W)
     if not (q.shape == k.shape == v.shape and q.dtype == k.dtype == v.dtype):
         raise TypeError("q, k, v must have the same element type and size")
-    B = q.shape[-1]
     assert q.shape[-2] % nheads == 0, f"channels ({q.shape[-2]}) must be divisible by nheads ({nheads})"
-    y, nz = _AttentionFn.apply(q, k, v, _kind(simfun), int(W), normalizer, bool(return_A), None, int(nheads))
+    y, nz = host.attention(q, k, v, _kind(simfun), int(W), normalizer, bool(return_A), None, int(nheads))
     if not return_A:
         return y, None
-    nz = jl.reshape(nz, (nz.shape[0], nheads, B))
     return y, Circulant._from_nz(nz, int(W), tuple(q.shape[:-2]))
 
 
@@ -482,23 +339,22 @@ def circulant_mh_adjacency(simfun, x, y, W: int, nheads: int, normalizer=SOFTMAX
         _check_xy(x, y)
         assert x.shape[-2] % nheads == 0, f"channels ({x.shape[-2]}) must be divisible by nheads ({nheads})"
         return LazyAdjacency([(1, simfun, x, y, normalizer)], W, nheads, tuple(x.shape[:-2]), x.shape[-1], True)
-    xr, yr = splitheads(x, nheads), splitheads(y, nheads)
-    A = circulant_adjacency(simfun, xr, yr, W, normalizer)
-    return _circulant_reshape(A, nheads, x.shape[-1])
+    _check_odd(W)
+    _check_xy(x, y)
+    assert x.shape[-2] % nheads == 0, f"channels ({x.shape[-2]}) must be divisible by nheads ({nheads})"
+    nz = host.similarity(x, y, _kind(simfun), int(W), int(nheads))
+    return softmax(Circulant._from_nz(nz, int(W), tuple(x.shape[:-2])), normalizer)
 
 
-def _circulant_reshape(A: Circulant, *batch) -> Circulant:
-    """src/array.jl:58-60 (its rrule, src/rrules.jl:34-40, is autograd's reshape)."""
-    return A.reshape(A.shape[0], A.shape[1], *batch)
-
-
-def _apply(A: Circulant, x, transpose):
+def _apply(A: Circulant, x, transpose, nheads=1):
+    """A or A^T applied to x (spatial..., C, B) of `nheads` heads (src/attention.jl:44: splitting heads is a reshape)."""
     N = x.ndim
     assert spatial_dims(A) == N - 2, \
         f"spatial-dims ({spatial_dims(A)} of A must match spatial dims of x ({N - 2})"
     assert tuple(x.shape[:-2]) == A.spatial_size, \
         f"spatial size {A.spatial_size} of A must match that of x {tuple(x.shape[:-2])}"
-    return _ApplyFn.apply(A.nzVal, x, A.kernel_length, transpose)
+    assert x.shape[-2] % nheads == 0, f"channels ({x.shape[-2]}) must be divisible by nheads ({nheads})"
+    return host.apply(A.nzVal, x, A.kernel_length, transpose, nheads)
 
 
 def otimes(A: Circulant, x):
@@ -526,6 +382,11 @@ def circulant_transposed_attention_(y, A: Circulant, x):
     return y
 
 
+def _mh_apply(A: Circulant, x, transpose):
+    y = _apply(A, x, transpose, A.size(3))
+    return y if y.shape == x.shape else jl.reshape(y, tuple(x.shape))
+
+
 def Otimes(A: Circulant, x):
     """y = A ⨷ x: multi-head apply, nheads = size(A, 3) (src/attention.jl:89-94)."""
     if isinstance(A, LazyAdjacency):
@@ -534,16 +395,14 @@ def Otimes(A: Circulant, x):
         return A.apply(x)
     if A.ndim != 4:
         raise TypeError("A ⨷ x needs a 4-dimensional Circulant (Np, Np, nheads, B)")
-    xr = splitheads(x, A.size(3))
-    return jl.reshape(otimes(A, xr), tuple(x.shape))
+    return _mh_apply(A, x, False)
 
 
 def circulant_mh_transposed_attention(A: Circulant, x):
     """src/attention.jl:98-103."""
     if A.ndim != 4:
         raise TypeError("needs a 4-dimensional Circulant (Np, Np, nheads, B)")
-    xr = splitheads(x, A.size(3))
-    return jl.reshape(circulant_transposed_attention(A, xr), tuple(x.shape))
+    return _mh_apply(A, x, True)
 
 
 def mix_otimes(terms, x):
@@ -647,7 +506,7 @@ class LazyAdjacency:
         out = None
         for c, simfun, a, b, normalizer in self.terms:
             ar, br = (splitheads(t, self.nheads) for t in (a, b)) if self.mh else (a, b)
-            y, _ = _AttentionFn.apply(ar, br, xr, _kind(simfun), self.kernel_length, normalizer, False, 1.0)
+            y, _ = host.attention(ar, br, xr, _kind(simfun), self.kernel_length, normalizer, False, 1.0, 1)
             cu = self._units_coeff(c, y)
             y = y * cu if not (isinstance(cu, (int, float)) and cu == 1) else y
             out = y if out is None else out + y
@@ -701,7 +560,7 @@ def batched_mul(A, B):
     Ac = A.parent if transpose else A
     Ar = Ac.reshape(Ac.shape[0], Ac.shape[1], -1)
     x = jl.reshape(B, Ac.spatial_size + tuple(B.shape[1:]))
-    y = _ApplyFn.apply(Ar.nzVal, x, Ac.kernel_length, transpose)
+    y = host.apply(Ar.nzVal, x, Ac.kernel_length, transpose, 1)
     return jl.reshape(y, (B.shape[0],) + tuple(y.shape[len(Ac.spatial_size):]))
 
 
@@ -720,7 +579,7 @@ def scale(c, A: Circulant) -> Circulant:
     if c.ndim != A.ndim:
         raise TypeError(f"scale needs c and A with the same number of dims ({c.ndim} vs {A.ndim})")
     cb = jl.reshape(c, tuple(c.shape[2:]))
-    return Circulant._from_nz(_ScaleFn.apply(cb, A.nzVal), A.kernel_length, A.spatial_size)
+    return Circulant._from_nz(host.scale_batch(cb, A.nzVal), A.kernel_length, A.spatial_size)
 
 
 def dot(X: Circulant, Y: Circulant):

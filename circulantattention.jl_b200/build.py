@@ -4,6 +4,7 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
@@ -11,6 +12,10 @@ OUT = os.path.join(PKG_DIR, "libcircatt_b200.so")
 SOURCES = ["api.cu", "tiled.cu", "static_scratch.cu", "comm.cu", "line.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--use_fast_math", "-Xcompiler", "-fPIC"]
+
+
+HOST_SRC = os.path.join(CSRC, "host.cpp")
+HOST_OUT = os.path.join(PKG_DIR, "_circatt_host.so")
 
 
 def _nvcc():
@@ -21,7 +26,7 @@ def _stale():
     if not os.path.exists(OUT):
         return True
     t = os.path.getmtime(OUT)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".h"))]
     deps.append(os.path.join(PKG_DIR, "..", "include", "circatt_b200.h"))
     return any(os.path.getmtime(d) > t for d in deps)
 
@@ -37,7 +42,35 @@ def _obj_stale(src_path: str, obj: str) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _host_command():
+    """g++ on the host extension; the ca_* symbols stay undefined and come from the library loaded before it."""
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], cuda]
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"] + ["-I" + d for d in include] +
+            [HOST_SRC, "-o", HOST_OUT, "-L" + os.path.join(root, "lib"), "-lc10", "-ltorch", "-ltorch_cpu", "-lc10_cuda",
+             "-ltorch_python"])
+
+
+def _host_stale():
+    if not os.path.exists(HOST_OUT):
+        return True
+    t = os.path.getmtime(HOST_OUT)
+    return any(os.path.getmtime(d) > t for d in (HOST_SRC, os.path.join(PKG_DIR, "..", "include", "circatt_b200.h")))
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    host = subprocess.Popen(_host_command()) if force or _host_stale() else None
+    try:
+        return _build_library(force, verbose)
+    finally:
+        if host is not None and host.wait() != 0:
+            raise RuntimeError("g++ failed on host.cpp")
+
+
+def _build_library(force, verbose):
     if not force and not _stale():
         return OUT
     objs = []

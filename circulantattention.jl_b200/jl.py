@@ -11,6 +11,8 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+from ._lib import host
+
 
 def _rev(n):
     return tuple(range(n - 1, -1, -1))
@@ -72,18 +74,4 @@ def to_numpy(t: torch.Tensor) -> np.ndarray:
 
 def reshape(t: torch.Tensor, *shape) -> torch.Tensor:
     """Julia `reshape` (column-major): a view when `t` is column-major."""
-    shape = list(shape[0]) if len(shape) == 1 and isinstance(shape[0], (tuple, list)) else list(shape)
-    n = t.numel()
-    if shape.count(-1) == 1:
-        known = int(np.prod([s for s in shape if s != -1])) if len(shape) > 1 else 1
-        shape[shape.index(-1)] = n // max(known, 1)
-    t = colmajor(t)
-    if not (torch.is_grad_enabled() and t.requires_grad):
-        # nothing to differentiate through: one strided view of the same column-major memory
-        strides, acc = [], 1
-        for n_ in shape:
-            strides.append(acc)
-            acc *= n_
-        return t.as_strided(tuple(shape), tuple(strides), t.storage_offset())
-    flat = t.permute(_rev(t.ndim)).reshape(tuple(reversed(shape)))
-    return flat.permute(_rev(len(shape)))
+    return host.reshape(t, list(shape[0]) if len(shape) == 1 and isinstance(shape[0], (tuple, list)) else list(shape))

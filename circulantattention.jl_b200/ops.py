@@ -1,16 +1,17 @@
 """Thin tensor-level wrappers over the C ABI: shape bookkeeping, output
 allocation (the caller owns every buffer, as CUDA.jl's pool does on the Julia
-side) and the ctypes calls.  No arithmetic happens here."""
+side) and the ctypes calls.  No arithmetic happens here.  The public API takes the
+native route of csrc/host.cpp; the attention wrappers here serve callers that drive
+the stages themselves (the band split, the benchmark)."""
 from __future__ import annotations
 
 import math
-import threading
 from dataclasses import dataclass
 
 import torch
 
 from . import _lib, jl
-from ._lib import CA_BF16, CA_C64, CA_F32, ca_desc, check, lib, ptr  # noqa: F401  (re-exported: parallel.py uses ops.lib / ops.check)
+from ._lib import CA_BF16, CA_C64, CA_F32, ca_desc, check, host, lib, ptr  # noqa: F401  (re-exported: parallel.py uses ops.lib / ops.check)
 
 
 @dataclass(frozen=True)
@@ -73,6 +74,7 @@ def enable_nvtx(flag: bool = True) -> bool:
     """NVTX ranges ("circatt.fwd", "circatt.bwd", "circatt.halo") around the library's calls, for timeline
     profilers; off by default (a range costs two host calls).  Returns the previous setting."""
     old, _NVTX[0] = _NVTX[0], bool(flag)
+    host.enable_nvtx(bool(flag))
     return old
 
 
@@ -129,81 +131,28 @@ def structure(spatial, ws, batch, device):
     return rowptr, colval
 
 
-def _operator_workspace(d, device):
-    """Scratch of ca_operator_workspace() bytes, or None when the shape runs on the generic kernels."""
-    n = lib.ca_operator_workspace(d)
-    return torch.empty(n, dtype=torch.uint8, device=device) if n else None
-
-
+# ------------------------------------------------------------------ operators on values (native: csrc/host.cpp)
 def similarity(kind, x, y, ws, scale=1.0):
-    require_cuda(x, y)
-    x, y = _dense_ok(x), _dense_ok(y)
-    m = meta_of(x, ws)
-    nz = jl.empty((m.Np * m.K, m.units), torch.float32, x.device)
-    d = m.desc(similarity=kind, scale=scale)
-    with _on_device(x.device):
-        ws_buf = _operator_workspace(d, x.device)
-        check(lib.ca_similarity(d, ptr(x), ptr(y), ptr(nz), ptr(ws_buf), _stream()))
-    return nz
+    """Scaled scores (Np*K, units) of head-split (spatial..., c, units) tensors."""
+    return host.similarity_raw(kind, x, y, ws, scale)
 
 
 def similarity_bwd(kind, x, y, ws, dS, scale=1.0):
-    x, y = _dense_ok(x), _dense_ok(y)
-    dS = jl.colmajor(dS)
-    m = meta_of(x, ws)
-    dx, dy = jl.empty(x.shape, x.dtype, x.device), jl.empty(y.shape, y.dtype, y.device)
-    d = m.desc(similarity=kind, scale=scale)
-    with _on_device(x.device):
-        ws_buf = _operator_workspace(d, x.device)
-        check(lib.ca_similarity_bwd(d, ptr(x), ptr(y), ptr(dS), ptr(dx), ptr(dy), ptr(ws_buf), _stream()))
-    return dx, dy
-
-
-def _nz_meta(spatial, ws, units):
-    return Meta(tuple(spatial), 1, int(units), int(ws), False)
+    return host.similarity_bwd_raw(kind, x, y, ws, dS, scale)
 
 
 def row_normalize(nz, spatial, ws, normalizer, out=None, want_stats=False):
-    require_cuda(nz)
-    nz = jl.colmajor(nz)
-    units = nz.numel() // nz.shape[0]
-    m = _nz_meta(spatial, ws, units)
-    out = jl.empty(nz.shape, torch.float32, nz.device) if out is None else out
-    stats = jl.empty((m.Np, units), torch.float32, nz.device) if want_stats else None
-    with _on_device(nz.device):
-        check(lib.ca_row_normalize(m.desc(normalizer=normalizer), ptr(nz), ptr(out), ptr(stats), _stream()))
-    return (out, stats) if want_stats else out
+    p, stats = host.normalize_raw(nz, list(spatial), ws, normalizer, out, want_stats)
+    return (p, stats) if want_stats else p
 
 
 def row_normalize_bwd(p, dp, spatial, ws, normalizer):
-    p, dp = jl.colmajor(p), jl.colmajor(dp)
-    units = p.numel() // p.shape[0]
-    m = _nz_meta(spatial, ws, units)
-    ds = jl.empty(p.shape, torch.float32, p.device)
-    with _on_device(p.device):
-        check(lib.ca_row_normalize_bwd(m.desc(normalizer=normalizer), ptr(p), ptr(dp), ptr(ds), _stream()))
-    return ds
+    return host.normalize_bwd_raw(p, dp, list(spatial), ws, normalizer)
 
 
 def apply(nz, v, ws, transpose=False, out=None):
     """A (x) v or A^T (x) v.  nz: (Np*K, ua); v: (spatial..., c, uv); ua, uv broadcast."""
-    require_cuda(nz, v)
-    nz, v = jl.colmajor(nz), _dense_ok(v)
-    m = meta_of(v, ws)
-    ua = nz.numel() // nz.shape[0]
-    units = max(ua, m.units)
-    if ua not in (1, units) or m.units not in (1, units):
-        raise AssertionError(f"batch dims of A ({ua}) and of x ({m.units}) do not broadcast")
-    if nz.shape[0] != m.Np * m.K:
-        raise AssertionError(f"A has {nz.shape[0]} stored entries per batch, x needs {m.Np * m.K}")
-    if out is None:
-        out = jl.empty(tuple(v.shape[:-1]) + (units,), v.dtype, v.device)
-    d = m.desc(units=units)
-    with _on_device(v.device):
-        ws_buf = _operator_workspace(d, v.device)
-        check(lib.ca_apply(d, ptr(nz), ptr(v), ptr(out), int(transpose), int(ua == 1 and units > 1),
-                           int(m.units == 1 and units > 1), ptr(ws_buf), _stream()))
-    return out
+    return host.apply_raw(nz, v, ws, bool(transpose), 1, out)
 
 
 # Transient scratch per (device, stream, purpose): grown on demand and reused by later calls on the
@@ -229,31 +178,20 @@ def release_scratch():
 
 
 # ------------------------------------------------------------------ device-side failure reporting
-_STATUS = {}
-_REGISTERED = threading.local()
-
-
 def _status_word(device):
-    """The int32 on `device` in which kernels flag a wait that ran out; registered with the library for
-    the calling host thread (the registration is per thread, so it is redone when the thread last
-    registered another device's word)."""
-    w = _STATUS.get(device.index)
-    if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=device)
-        _STATUS[device.index] = w
-    if getattr(_REGISTERED, "index", None) != device.index:
-        check(lib.ca_status_word(ptr(w)))
-        _REGISTERED.index = device.index
-    return w
+    """The int32 on `device` in which kernels flag a wait that ran out; registered with the library for the
+    calling host thread."""
+    return host.status_word(torch.cuda.current_device() if device.index is None else device.index)
 
 
 def check_status(device=None):
     """Synchronising check: raises if a kernel of this library gave up a bounded device-side wait since the
     last check on `device` (its tile then holds NaN).  Call it where the program synchronises anyway."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    w = _STATUS.get(device.index)
-    if w is None:
+    index = torch.cuda.current_device() if device.index is None else device.index
+    if not host.has_status_word(index):
         return
+    w = host.status_word(index)
     flag = int(w.item())
     if flag:
         w.zero_()
@@ -319,87 +257,31 @@ def entmax_scratch_limit(nbytes: int = -1) -> int:
     return int(lib.ca_entmax_scratch_limit(int(nbytes)))
 
 
-# ------------------------------------------------------------------ algebra
+# ------------------------------------------------------------------ algebra (native: csrc/host.cpp)
 def axpby(alpha, x, beta=0.0, y=None):
-    require_cuda(x, y)
-    x = jl.colmajor(x)
-    y = jl.colmajor(y) if y is not None else None
-    out = jl.empty(x.shape, torch.float32, x.device)
-    with _on_device(x.device):
-        check(lib.ca_axpby(x.numel(), float(alpha), ptr(x), float(beta), ptr(y), ptr(out), _stream()))
-    return out
-
-
-def _b12(batch):
-    batch = tuple(batch)
-    if len(batch) > 2:
-        raise NotImplementedError("at most two batch dims (heads, batch) are supported")
-    return (batch + (1, 1))[:2]
+    return host.axpby_raw(float(alpha), x, float(beta), y)
 
 
 def scale_batch(c, nz):
     """nz (inner, a...) times c (c...) with Julia-style extent-1 broadcasting."""
-    require_cuda(c, nz)
-    c, nz = jl.colmajor(c), jl.colmajor(nz)
-    a1, a2 = _b12(nz.shape[1:])
-    c1, c2 = _b12(c.shape)
-    o1, o2 = max(a1, c1), max(a2, c2)
-    nb = max(nz.ndim - 1, c.ndim)
-    out = jl.empty((nz.shape[0],) + (o1, o2)[:nb], torch.float32, nz.device)
-    with _on_device(nz.device):
-        check(lib.ca_scale_batch(nz.shape[0], o1, o2, ptr(nz), a1, a2, ptr(c), c1, c2, ptr(out), _stream()))
-    return out
+    return host.scale_batch_raw(c, nz)
 
 
 def dot_batch(x, y=None):
     """per-slice sum_n x*y (y None: sum of x); x, y: (inner, b...) broadcasting -> (b...)"""
-    require_cuda(x, y)
-    x = jl.colmajor(x)
-    x1, x2 = _b12(x.shape[1:])
-    if y is not None:
-        y = jl.colmajor(y)
-        y1, y2 = _b12(y.shape[1:])
-    else:
-        y1 = y2 = 1
-    o1, o2 = max(x1, y1), max(x2, y2)
-    nb = max(x.ndim, y.ndim if y is not None else 0) - 1
-    out = jl.empty((o1, o2)[:nb] if nb else (1,), torch.float32, x.device)
-    with _on_device(x.device):
-        check(lib.ca_dot_batch(x.shape[0], o1, o2, ptr(x), x1, x2, ptr(y), y1, y2, ptr(out), _stream()))
-    return out
+    return host.dot_batch(x, y)
 
 
 def sum_batch(nz, sum1, sum2):
-    require_cuda(nz)
-    nz = jl.colmajor(nz)
-    b1, b2 = _b12(nz.shape[1:])
-    o = (1 if sum1 else b1, 1 if sum2 else b2)[:nz.ndim - 1]
-    out = jl.empty((nz.shape[0],) + o, torch.float32, nz.device)
-    with _on_device(nz.device):
-        check(lib.ca_sum_batch(nz.shape[0], b1, b2, int(sum1), int(sum2), ptr(nz), ptr(out), _stream()))
-    return out
+    return host.sum_batch(nz, bool(sum1), bool(sum2))
 
 
 def sum_rows(nz, spatial, ws):
-    require_cuda(nz)
-    nz = jl.colmajor(nz)
-    units = nz.numel() // nz.shape[0]
-    m = _nz_meta(spatial, ws, units)
-    out = jl.empty((m.Np, 1) + tuple(nz.shape[1:]), torch.float32, nz.device)
-    with _on_device(nz.device):
-        check(lib.ca_sum_rows(m.desc(), ptr(nz), ptr(out), _stream()))
-    return out
+    return host.sum_axis(nz, list(spatial), ws, True)
 
 
 def sum_cols(nz, spatial, ws):
-    require_cuda(nz)
-    nz = jl.colmajor(nz)
-    units = nz.numel() // nz.shape[0]
-    m = _nz_meta(spatial, ws, units)
-    out = jl.empty((1, m.Np) + tuple(nz.shape[1:]), torch.float32, nz.device)
-    with _on_device(nz.device):
-        check(lib.ca_sum_cols(m.desc(), ptr(nz), ptr(out), _stream()))
-    return out
+    return host.sum_axis(nz, list(spatial), ws, False)
 
 
 # ------------------------------------------------------------------ backward stages (band split)
