@@ -161,8 +161,7 @@ static int launch_row_normalize(int64_t rows, int K, int entmax, const float* s,
         else if (K <= 512) row_entmax15_reg_kernel<16><<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
         else row_entmax15_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
     }
-    else CA_ROW_SHAPE(K, (row_softmax_reg_kernel<G, R><<<(unsigned)((rows * G + 255) / 256), 256, 0, st>>>(rows, K, s, p, stats)),
-                      (row_softmax_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats)));
+    else row_softmax_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
     CA_CHECK_LAUNCH("row normalize kernel");
     return CA_OK;
 }
@@ -171,8 +170,7 @@ static int launch_row_normalize_bwd(int64_t rows, int K, int entmax, const float
                                     cudaStream_t st) {
     const int64_t blocks = (rows * 32 + 255) / 256;
     if (blocks > INT32_MAX) { set_error("too many rows"); return CA_ERR_TOO_LARGE; }
-    CA_ROW_SHAPE(K, (row_normalize_bwd_reg_kernel<G, R><<<(unsigned)((rows * G + 255) / 256), 256, 0, st>>>(rows, K, entmax, p, dp, ds)),
-                 (row_normalize_bwd_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, entmax, p, dp, ds)));
+    row_normalize_bwd_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, entmax, p, dp, ds);
     CA_CHECK_LAUNCH("row normalize pullback kernel");
     return CA_OK;
 }
@@ -356,7 +354,6 @@ size_t ca_attention_fwd_workspace(const ca_desc* d, int32_t want_nz) {
     }
     if (composed_path(d, g)) return (want_nz ? 0 : score_bytes(g)) + tiled_operator_workspace(g);
     const bool band = g.Wk != g.W;
-    if (tc_route(g)) return tc_fwd_workspace(g, want_nz != 0);
     return (want_nz && band) ? 0 : tiled_fwd_workspace(g);
 }
 
@@ -409,9 +406,6 @@ int ca_attention_fwd(const ca_desc* d, const void* q, const void* k, const void*
         return launch_apply(g, sbuf, (const float*)v, nullptr, (float*)y, 1.f, 0, 0, 0, st);
     }
 
-    if (workspace && tc_route(g))
-        return tc_attention_fwd(g, d->scale, dist, (const float*)q, (const float*)k, (const float*)v, (float*)y, nz, stats,
-                                workspace, st);
     if (workspace) {
         rc = tiled_attention_fwd(g, d->scale, dist, (const float*)q, (const float*)k, (const float*)v,
                                  (float*)y, nz, stats, workspace, st);
@@ -434,7 +428,7 @@ size_t ca_attention_bwd_workspace(const ca_desc* d, int32_t with_dA) {
     Geo g;
     if (make_geo(d, &g, false)) return 0;
     // D, then the larger of the two scratch layouts the shape can take (fused tiled kernels; operator chain)
-    const size_t fused = tc_route(g) && d->normalizer == CA_SOFTMAX ? tc_bwd_workspace(g) : tiled_bwd_workspace(g);
+    const size_t fused = tiled_bwd_workspace(g);
     const size_t chain = composed_path(d, g, true, with_dA != 0) ? 2 * score_bytes(g) + tiled_operator_workspace(g) : 0;
     return d_bytes(g) + (fused > chain ? fused : chain);
 }
@@ -600,10 +594,6 @@ int ca_attention_bwd(const ca_desc* d, const void* q, const void* k, const void*
     }
     if (d->normalizer == CA_SOFTMAX && !dA) {
         if (!q || !k || !v || !y || !dy || !stats || !dq || !dk || !dv) { set_error("a required pointer is NULL"); return CA_ERR_NULL; }
-        if (tc_route(g))
-            return tc_attention_bwd(g, d->scale, d->similarity == CA_DISTANCE, (const float*)q, (const float*)k,
-                                    (const float*)v, (const float*)y, (const float*)dy, stats, D, (float*)dq, (float*)dk,
-                                    (float*)dv, (char*)workspace + d_bytes(g), fwd_workspace, as_stream(stream));
         rc = tiled_attention_bwd(g, d->scale, d->similarity == CA_DISTANCE, (const float*)q, (const float*)k,
                                  (const float*)v, (const float*)y, (const float*)dy, stats, D, (float*)dq,
                                  (float*)dk, (float*)dv, (char*)workspace + d_bytes(g), fwd_workspace, as_stream(stream));
@@ -674,8 +664,7 @@ int ca_sum_rows(const ca_desc* d, const float* nz, float* out, void* stream) {
     if (!nz || !out) { set_error("nz/out is NULL"); return CA_ERR_NULL; }
     const int64_t rows = (int64_t)g.Np * g.units;
     if ((rows * 32 + 255) / 256 > INT32_MAX) { set_error("too many rows"); return CA_ERR_TOO_LARGE; }
-    CA_ROW_SHAPE(g.K, (sum_rows_reg_kernel<G, R><<<(unsigned)(((rows + 1) / 2 * G + 255) / 256), 256, 0, as_stream(stream)>>>(rows, g.K, nz, out)),
-                 (sum_rows_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, as_stream(stream)>>>(rows, g.K, nz, out)));
+    sum_rows_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, as_stream(stream)>>>(rows, g.K, nz, out);
     CA_CHECK_LAUNCH("row sum kernel");
     return CA_OK;
 }

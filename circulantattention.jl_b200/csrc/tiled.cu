@@ -37,10 +37,314 @@
 // Small grids.  When the grid would not fill the GPU, the column stages of a
 // tile are split between two groups of warps of the same CTA (each with its own
 // copy pipeline) whose partial results are merged through shared memory.
-#include "tile_common.cuh"
+#include "tiled.cuh"
+#include "tma.cuh"
+#include <cuda_bf16.h>
+#include <stdlib.h>
+#include <algorithm>
+#include <type_traits>
+#include <mutex>
+#include <atomic>
 
 namespace ca {
 namespace {
+
+// Two-channel arithmetic: a channel pair lives in two ordinary registers and a pair operation is
+// two scalar FMAs.  (Packed fma.rn.f32x2 was measured slower here: a dot product or an outer
+// product has two fresh 64-bit operands per instruction, which the register file does not deliver
+// at the packed rate.)
+struct u64 { float x, y; };
+__device__ __forceinline__ u64 pack2(float a, float b) { return u64{a, b}; }
+__device__ __forceinline__ void unpack2(u64 v, float& a, float& b) { a = v.x; b = v.y; }
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { return u64{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) { return u64{a.x * b.x, a.y * b.y}; }
+__device__ __forceinline__ u64 add2(u64 a, u64 b) { return u64{a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ u64 zero2() { return u64{0.f, 0.f}; }
+__device__ __forceinline__ void lds128(uint32_t addr, u64& lo, u64& hi) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(lo.x), "=f"(lo.y), "=f"(hi.x), "=f"(hi.y) : "r"(addr));
+}
+__device__ __forceinline__ float hsum2(u64 v) {
+    float a, b;
+    unpack2(v, a, b);
+    return a + b;
+}
+
+// Sum of a per-lane partial over the NS lanes that share a pixel (NS = 1: nothing to do).
+template <int NS>
+__device__ __forceinline__ float lane_sum(float x) {
+#pragma unroll
+    for (int m = 1; m < NS; m <<= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
+    return x;
+}
+
+struct TileArgs {
+    Geo g;
+    float scale;
+    int TH;                 // rows per CTA
+    int roff;               // p' - p: first window row inside a stage buffer
+    int stage_bytes;        // bytes of one stage buffer (multiple of 1024)
+    int nsplit;             // 1 or 2 groups of warps sharing the stages of a tile
+    int which;              // half of the packed pair a single-tensor kernel streams (0 or 1)
+    int iter;               // entmax threshold search: number of the step (late steps fall back to Newton)
+    int row_bytes;          // bytes of one packed pixel row: 144 per 16-channel slab
+    int nstages;            // copy stages in flight per part: 2 or 3 (kStages)
+    const float* c0;        // centre tensors (reference layout)
+    const float* c1;
+    const float* cs0;       // centre scalars (dq kernel: stats, D)
+    const float* cs1;
+    float* o0;              // outputs
+    float* o1;
+    float* ostats;
+    int* status;            // nullable device word of the caller: bit 0 is set when a stage wait ran out
+    uint32_t wait_tries;    // polls before a stage wait gives up
+};
+
+constexpr int kStages = 3;
+constexpr uint32_t kWaitTries = 1u << 20;
+constexpr int kEntmaxFwdSteps = 16;            // launches of the entmax threshold step (settled blocks leave at once)
+
+// Number of CTAs that gave up waiting for a stage copy (stays 0 in a healthy run).
+__device__ int g_stage_timeouts = 0;
+
+constexpr int kRowFloats = 36;                 // 16 + 16 + 4 padding
+constexpr int kRowBytes = kRowFloats * 4;      // 144
+constexpr int kRunChunk = 32;                  // window rows whose entries of A are staged at a time
+constexpr int kSingleFloats = 20;              // single-tensor rows: 16 + 4 padding (80 bytes, also conflict free)
+
+// Units with 16*NS real channels ("slabs" of 16) pack a pixel row as 36*NS words: the first
+// tensor's channels, then the second's, then 4*NS words of padding.  Inside a tensor's part the
+// order is [4-channel chunk][slab][4]: chunk c of slab s sits 16*(c*NS + s) bytes in, so the NS
+// lanes that share a pixel read consecutive 16-byte pieces, and the row stride (144*NS bytes:
+// 16, 32 or 64 bytes past a multiple of 128) spreads the 8/NS pixels of a 128-bit load phase over
+// distinct bank groups.  NS = 1 is the plain channel order.
+// 16-channel slab `slab` of tensor `which` of the pixel row at shared-space byte address `a0`.
+template <int NS>
+__device__ __forceinline__ void lds_slab16(uint32_t a0, int which, int slab, u64 (&v)[8]) {
+    const uint32_t b = a0 + which * (64 * NS) + slab * 16;
+    lds128(b, v[0], v[1]);
+    lds128(b + 16 * NS, v[2], v[3]);
+    lds128(b + 32 * NS, v[4], v[5]);
+    lds128(b + 48 * NS, v[6], v[7]);
+}
+
+// Global offset of real channel cc of unit u at pixel pix (npix pixels per plane, NCR real
+// channels per unit).
+template <int CPE, int NCR = 16>
+__device__ __forceinline__ int64_t goff(int u, int cc, int npix, int pix) {
+    if (CPE == 1) return ((int64_t)u * NCR + cc) * npix + pix;
+    return (((int64_t)u * (NCR / 2) + (cc >> 1)) * npix + pix) * 2 + (cc & 1);
+}
+
+// Window radius along w: p for 2-D windows, 0 for a folded 1-D signal (wsw == 1), whose window
+// runs along h only and continues into the neighbouring columns through the packed halo rows.
+__device__ __forceinline__ int radius_w(const Geo& g) { return (g.wsw - 1) >> 1; }
+
+__device__ __forceinline__ int stage_column(const Geo& g, int w0, int s) {
+    int kc = (w0 - radius_w(g) + s + g.wk_off) % g.Wk;
+    return kc < 0 ? kc + g.Wk : kc;
+}
+
+// Rotation of the sorted run of a CSR row: the entry of window offset d sits at (d + p + rot) mod ws,
+// where the row's pixel has coordinate x on the window axis of length X (src/circulant.jl:11-15).
+__device__ __forceinline__ int run_rot(int x, int X, int p, int ws) {
+    return x < p ? x - p + ws : (x >= X - p ? x - p - X + ws : 0);
+}
+// Coordinate and length of the window axis for pixel (h, w): the image row in 2-D, the linear
+// index in a folded 1-D signal.
+__device__ __forceinline__ int axis_coord(const Geo& g, int h, int w) { return g.wsw == 1 ? h + g.H * w : h; }
+__device__ __forceinline__ int axis_len(const Geo& g) { return g.wsw == 1 ? g.Np : g.H; }
+
+template <int NQ>
+__device__ __forceinline__ int stage_mask(int s, int p) {
+    int mask = 0;
+#pragma unroll
+    for (int r = 0; r < NQ; ++r)
+        if (s >= r && s <= r + 2 * p) mask |= 1 << r;
+    return mask;
+}
+
+// Barrier of one group of warps (ids 1 and 2; id 0 stays the CTA-wide barrier).
+__device__ __forceinline__ void part_sync(int part, int nthreads) {
+    if (part == 0) asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
+    else asm volatile("bar.sync 2, %0;" ::"r"(nthreads) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Stage pipeline of one group of warps ("part").  Thread 0 of the part is the
+// producer: it arms the stage's mbarrier with the byte count and issues the
+// TMA boxes; every consumer wait is bounded.
+// ---------------------------------------------------------------------------
+template <bool NSC>
+struct StagePipe {
+    uint64_t* full;          // kStages barriers of this part
+    unsigned char* base;     // kStages stage buffers of this part
+    const CUtensorMap* mv;
+    const CUtensorMap* msc;
+    int ROWS, stage_bytes, row_bytes, u, h0, w0;
+
+    __device__ __forceinline__ unsigned char* vec(int buf) const { return base + (size_t)buf * stage_bytes; }
+    __device__ __forceinline__ int sstride() const { return (ROWS * 4 + 127) & ~127; }
+    __device__ __forceinline__ int vbytes() const { return (ROWS * row_bytes + 127) & ~127; }
+    __device__ __forceinline__ float* sc0(int buf) const { return reinterpret_cast<float*>(vec(buf) + vbytes()); }
+    __device__ __forceinline__ float* sc1(int buf) const { return reinterpret_cast<float*>(vec(buf) + vbytes() + sstride()); }
+
+    __device__ __forceinline__ void issue(const Geo& g, int s, int buf) const {
+        const int kc = stage_column(g, w0, s);
+        mbar_arrive_expect_tx(&full[buf], (uint32_t)(ROWS * row_bytes + (NSC ? ROWS * 8 : 0)));
+        tma_load_4d(vec(buf), mv, 0, h0, kc, u, &full[buf]);
+        if (NSC) {
+            tma_load_3d(sc0(buf), msc, h0, kc, 2 * u, &full[buf]);
+            tma_load_3d(sc1(buf), msc, h0, kc, 2 * u + 1, &full[buf]);
+        }
+    }
+};
+
+// Declares the pipeline of this thread's part and starts the first copies.
+// Needs in scope: a (TileArgs), g, ROWS, u, h0, w0, NSTAGES (stages of the tile), mv, msc.
+#define CA_PIPE_PROLOGUE(NSCV)                                                                       \
+    extern __shared__ unsigned char smem_raw[];                                                      \
+    __shared__ __align__(8) uint64_t full_bar[2 * kStages];                                          \
+    __shared__ int s_err;                                                                            \
+    const int PT = blockDim.x / a.nsplit;          /* threads per part */                            \
+    const int part = threadIdx.x / PT;                                                               \
+    const int lt = threadIdx.x - part * PT;                                                          \
+    const int s_begin = part * (NSTAGES / a.nsplit);                                                      \
+    const int s_end = (part + 1 == a.nsplit) ? NSTAGES : (part + 1) * (NSTAGES / a.nsplit);                    \
+    unsigned char* smem_al = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);            \
+    StagePipe<NSCV> pipe;                                                                            \
+    pipe.full = full_bar + part * kStages;                                                           \
+    pipe.base = smem_al + (size_t)part * a.nstages * a.stage_bytes;                                  \
+    pipe.mv = &mv; pipe.msc = &msc;                                                                  \
+    pipe.ROWS = ROWS; pipe.stage_bytes = a.stage_bytes; pipe.row_bytes = a.row_bytes;                \
+    pipe.u = u; pipe.h0 = h0; pipe.w0 = w0;                                                          \
+    if (threadIdx.x == 0) {                                                                          \
+        for (int i = 0; i < 2 * kStages; ++i) mbar_init(&full_bar[i], 1);                            \
+        s_err = 0;                                                                                   \
+        mbar_fence_init();                                                                           \
+    }                                                                                                \
+    __syncthreads();                                                                                 \
+    if (lt == 0)                                                                                     \
+        for (int i = 0; i < a.nstages && s_begin + i < s_end; ++i) pipe.issue(g, s_begin + i, i);
+
+// Consumer loop over the stages of this part: bounded wait, BODY, recycle the buffer.
+#define CA_PIPE_LOOP(...)                                                                            \
+    for (int s = s_begin; s < s_end; ++s) {                                                          \
+        const int it = s - s_begin;                                                                  \
+        const int buf = it % a.nstages;                                                              \
+        if (!mbar_wait(&pipe.full[buf], (uint32_t)((it / a.nstages) & 1), a.wait_tries)) s_err = 1;  \
+        __VA_ARGS__                                                                                  \
+        part_sync(part, PT);                                                                         \
+        if (s_err) break;                                                                            \
+        if (lt == 0 && s + a.nstages < s_end) pipe.issue(g, s + a.nstages, buf);                     \
+    }                                                                                                \
+    __syncthreads();                                                                                 \
+    /* A wait that ran out: the CTA stops computing, reports (device counter, caller's status word)  \
+       and poisons what it still stores with NaN, so that the failure cannot pass for a result. */   \
+    float ca_poison = 0.f;                                                                           \
+    if (s_err) {                                                                                     \
+        /* give copies still in flight a bounded chance to land before the CTA exits */              \
+        if (lt == 0)                                                                                 \
+            for (int i = 0; i < a.nstages; ++i) mbar_wait(&pipe.full[i], 0, 1u << 12);               \
+        if (threadIdx.x == 0) {                                                                      \
+            atomicAdd(&g_stage_timeouts, 1);                                                         \
+            if (a.status) atomicOr(a.status, 1);                                                     \
+        }                                                                                            \
+        ca_poison = __int_as_float(0x7fc00000);                                                      \
+    }
+
+// One real element of a dense tensor stored as Float32 or bfloat16 (element offset `off`).
+// BF is a compile-time flag so that a batch of loads stays a batch of independent loads; callers
+// branch once on Geo::bf16 around the whole batch.
+template <bool BF>
+__device__ __forceinline__ float ld_real(const float* base, int64_t off) {
+    if (BF) {
+        const unsigned short h = __ldg(reinterpret_cast<const unsigned short*>(base) + off);
+        return __uint_as_float((unsigned)h << 16);
+    }
+    return __ldg(base + off);
+}
+template <bool BF>
+__device__ __forceinline__ void st_real(float* base, int64_t off, float v) {
+    if (BF) reinterpret_cast<__nv_bfloat16*>(base)[off] = __float2bfloat16_rn(v);
+    else base[off] = v;
+}
+
+// Runs the statements once with `constexpr bool BF` (bfloat16 storage) and `constexpr int NCRV`
+// (8 or 16 real channels per unit) set from the geometry: one uniform branch around a whole
+// epilogue instead of one per element.  Needs CPE and g in scope.
+#define CA_OUT_DISPATCH_NCR(NCRVAL, ...)               \
+    if (CPE == 1 && g.bf16) {                          \
+        constexpr bool BF = true;                      \
+        constexpr int NCRV = NCRVAL;                   \
+        __VA_ARGS__                                    \
+    } else {                                           \
+        constexpr bool BF = false;                     \
+        constexpr int NCRV = NCRVAL;                   \
+        __VA_ARGS__                                    \
+    }
+#define CA_BF_DISPATCH(...)                            \
+    if (g.cr == 8) {                                   \
+        CA_OUT_DISPATCH_NCR(8, __VA_ARGS__)            \
+    } else {                                           \
+        CA_OUT_DISPATCH_NCR(16, __VA_ARGS__)           \
+    }
+
+// Loads the 16-channel vectors of the NQ centre pixels of this thread, times `mul`.
+template <int CPE, int NQ, int NCR, bool BF>
+__device__ __forceinline__ void load_centre_impl(const float* src, const Geo& g, int u, int h, int w0, bool active,
+                                                 float mul, u64 (&dst)[NQ][8], int ch0) {
+#pragma unroll
+    for (int r = 0; r < NQ; ++r) {
+        const bool ok = active && (w0 + r < g.W);
+        const int pix = h + g.H * (w0 + r);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float x = 0.f, y = 0.f;
+            if (ok && (NCR >= 16 || 2 * i < NCR)) {         // units narrower than a slab are zero-extended
+                if (CPE == 1) {
+                    x = ld_real<BF>(src, goff<1, NCR>(u, ch0 + 2 * i, g.Np, pix));
+                    y = ld_real<BF>(src, goff<1, NCR>(u, ch0 + 2 * i + 1, g.Np, pix));
+                } else {
+                    const float2 t = __ldg(reinterpret_cast<const float2*>(src + goff<2, NCR>(u, ch0 + 2 * i, g.Np, pix)));
+                    x = t.x;
+                    y = t.y;
+                }
+            }
+            dst[r][i] = pack2(x * mul, y * mul);
+        }
+    }
+}
+
+template <int CPE, int NQ, int NCR = 16>
+__device__ __forceinline__ void load_centre(const float* src, const Geo& g, int u, int h, int w0, bool active,
+                                            float mul, u64 (&dst)[NQ][8], int ch0 = 0) {
+    if (NCR == 16 && g.cr == 8) {
+        // a kernel compiled for one 16-channel slab running on 8-channel units: zero-extended
+        if (CPE == 1 && g.bf16) load_centre_impl<CPE, NQ, 8, true>(src, g, u, h, w0, active, mul, dst, ch0);
+        else load_centre_impl<CPE, NQ, 8, false>(src, g, u, h, w0, active, mul, dst, ch0);
+        return;
+    }
+    if (CPE == 1 && g.bf16) load_centre_impl<CPE, NQ, NCR, true>(src, g, u, h, w0, active, mul, dst, ch0);
+    else load_centre_impl<CPE, NQ, NCR, false>(src, g, u, h, w0, active, mul, dst, ch0);
+}
+
+template <int CPE, int NCR = 16, bool BF = false>
+__device__ __forceinline__ void store_centre(float* dst, const Geo& g, int u, int h, int w0, bool active, int r,
+                                             int i, float x, float y, int ch0 = 0) {
+    if (!(active && (w0 + r < g.W))) return;
+    if (NCR < 16 && 2 * i >= NCR) return;
+    const int pix = h + g.H * (w0 + r);
+    if (CPE == 1) {
+        st_real<BF>(dst, goff<1, NCR>(u, ch0 + 2 * i, g.Np, pix), x);
+        st_real<BF>(dst, goff<1, NCR>(u, ch0 + 2 * i + 1, g.Np, pix), y);
+    } else {
+        *reinterpret_cast<float2*>(dst + goff<2, NCR>(u, ch0 + 2 * i, g.Np, pix)) = make_float2(x, y);
+    }
+}
+
+// MASK != 0: all centre pixels pair with this stage (compile time);
+// MASK == 0: the set is the run-time `rm` (warp-uniform branches).
+#define CA_ON(r) ((MASK != 0) || ((rm >> (r)) & 1))
 
 // =====================================================================
 // Forward
@@ -213,7 +517,7 @@ __device__ __forceinline__ void fwd_init_max(uint32_t rowbase, int init, float s
     if ((mask) == (FULL)) { constexpr int MK = (FULL); CALL; }      \
     else { constexpr int MK = 0; CALL; }
 
-// NCRT = real channels per unit the kernel is compiled for: 16 (narrower units are zero-extended),
+// NCRT = real channels per unit the kernel is compiled for: 16 (also runs 8-channel units, zero-extended),
 // 32 or 64 (NS = 2 or 4 lanes per pixel, one 16-channel slab each; launched without a stage split).
 template <int DC, bool DIST, int CPE, bool EXACT, int NQ, int NCRT = 16>
 __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) fwd_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
@@ -312,21 +616,417 @@ __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) fwd_tiled_kernel(TileA
             }
         }
     }
-    CA_OUT_DISPATCH(
-        _Pragma("unroll")
+    if (NS == 1) {
+        CA_BF_DISPATCH(
+            _Pragma("unroll")
+            for (int r = 0; r < NQ; ++r) {
+                const float inv = 1.f / l[r] + ca_poison;
+                _Pragma("unroll")
+                for (int i = 0; i < 8; ++i) {
+                    float x, y;
+                    unpack2(acc[r][i], x, y);
+                    store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, x * inv, y * inv);
+                }
+            })
+    } else {
+#pragma unroll
         for (int r = 0; r < NQ; ++r) {
             const float inv = 1.f / l[r] + ca_poison;
-            _Pragma("unroll")
+#pragma unroll
             for (int i = 0; i < 8; ++i) {
                 float x, y;
                 unpack2(acc[r][i], x, y);
-                store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, x * inv, y * inv, 16 * slab);
+                store_centre<CPE, NCRT>(a.o0, g, u, h, w0, active, r, i, x * inv, y * inv, 16 * slab);
             }
-        })
+        }
+    }
 #pragma unroll
     for (int r = 0; r < NQ; ++r)
-        if (a.ostats && active && slab == 0 && has_pixel(g, h, w0 + r))
+        if (a.ostats && active && slab == 0 && w0 + r < g.W)
             a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = (log2f(l[r]) - nm[r]) * kLn2 + ca_poison;
+}
+
+// =====================================================================
+// A in CSR order.  Second sweep over the same packed (k|v) stages: with the
+// saved log-sum-exp the normalised entry is P = 2^(q.k - L) directly; without
+// row statistics (cs0 == NULL) the kernel writes the scaled scores themselves,
+// which is the stand-alone similarity operator.  A thread
+// produces, per stage, the ws entries of one (row, window column) run, which
+// are contiguous in the row's CSR segment; a warp stages its 32 rows x ws run
+// in shared memory and writes it out with consecutive lanes on consecutive
+// addresses, so the 4*K*heads bytes per pixel leave the SM in full sectors.
+// =====================================================================
+// NCRT = real channels per unit: 8 (zero-extended to one slab), 16, 32 or 64.
+template <bool DIST, int CPE, int NCRT>
+__global__ void __launch_bounds__(128, 3) emit_a_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+                                                              const __grid_constant__ CUtensorMap msc) {
+    constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;             // 16-channel slabs = lanes per pixel
+    constexpr int RW = 32 / NS;                                // pixel rows per warp
+    const Geo& g = a.g;
+    const int RB = a.row_bytes;                                // packed row: pair (144*NS) or single tensor (80*NS)
+    const int ROWS = a.TH + 2 * (g.p + a.roff);
+    const int pw = radius_w(g);
+    const int w0 = blockIdx.x * 4, h0 = blockIdx.y * a.TH, u = blockIdx.z;
+    const int NSTAGES = g.wsw + min(3, g.W - 1 - w0);          // no stages for centre columns past the image
+    const float sl2 = a.scale * kLog2e;
+    CA_PIPE_PROLOGUE(false)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slab = lane % NS, lrow = lane / NS;              // this lane's channel slab and row inside the warp
+    const int lr = (lt >> 5) * RW + lrow, h = h0 + lr;         // row inside the tile, image row
+    const bool active = h < g.H;
+    // per-warp staging tile [4][RW][CH] after the stage buffers: the entries of CH = min(ws, 32)
+    // consecutive window rows at a time, then the run rotations of the warp's rows [4][RW]
+    const int CH = min(g.ws, kRunChunk);
+    const int CHS = CH | 1;                                    // odd row stride: conflict-free column access
+    const int nslots = g.wsw == 1 ? 1 : 4;                     // folded 1-D: a stage pairs with one centre column
+    float* tile = reinterpret_cast<float*>(smem_al + (size_t)a.nsplit * a.nstages * a.stage_bytes) +
+                  (size_t)warp * (nslots * RW * CHS + 4 * RW + RW * CH);     // tile, rotations, offset table
+    int* rots = reinterpret_cast<int*>(tile + nslots * RW * CHS);
+    // 2-D windows that fit one piece: the destination offset of every tile element is the same
+    // for all stages and centre columns (row*K + sorted position) and comes from a table
+    const bool tabled = g.ws <= kRunChunk && g.wsw != 1;
+    int* etab = rots + 4 * RW;
+    const int hw0 = h0 + (lt >> 5) * RW;                       // first image row of this warp
+    for (int i = lane; i < 4 * RW; i += 32)
+        rots[i] = run_rot(axis_coord(g, hw0 + i % RW, w0 + i / RW), axis_len(g), g.p, g.ws);
+    if (tabled)
+        for (int idx = lane; idx < RW * g.ws; idx += 32) {
+            const int row = idx / g.ws, e = idx - row * g.ws;
+            int posh = e + run_rot(hw0 + row, g.H, g.p, g.ws);
+            posh -= (posh >= g.ws) ? g.ws : 0;
+            etab[idx] = row * g.K + posh;
+        }
+    __syncwarp();
+
+    const bool raw = a.cs0 == nullptr;
+    u64 q[4][8];
+    load_centre<CPE, 4, NCRT>(a.c0, g, u, h, w0, active, sl2, q, 16 * slab);
+    u64 nL2[4];
+    float bq[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const bool ok = active && (w0 + r < g.W) && slab == 0;   // the row statistic enters the lane sum once
+        nL2[r] = pack2((ok && !raw) ? -__ldg(a.cs0 + (int64_t)u * g.Np + h + g.H * (w0 + r)) * kLog2e : 0.f, 0.f);
+        bq[r] = 0.f;
+        if (DIST) {
+            u64 n = zero2();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) n = fma2(q[r][i], q[r][i], n);
+            bq[r] = -0.5f * hsum2(n) / sl2;
+        }
+    }
+    const int64_t warp_row0 = (int64_t)u * g.Np + hw0;
+    const int rows_here = min(RW, g.H - hw0);
+
+    CA_PIPE_LOOP({
+        const int mask = stage_mask<4>(s, pw);
+        const uint32_t rowbase = smem_u32(pipe.vec(buf)) + (lr + a.roff) * RB;
+        for (int d0 = 0; d0 < g.ws; d0 += CH) {
+            const int len = min(CH, g.ws - d0);                // window rows d0 .. d0 + len - 1
+            // FULL: the dot products of all four centre columns run interleaved (the columns that do
+            // not pair with this stage are computed too and dropped: cheaper than four serial chains);
+            // otherwise only the paired columns are computed (folded 1-D: one column per stage)
+            auto sweep = [&](auto full_tag) {
+                constexpr bool FULL = decltype(full_tag)::value;
+                u64 kn[8];                                 // the next window row's vector, fetched one row ahead
+                lds_slab16<NS>(rowbase + d0 * RB, 0, slab, kn);
+#pragma unroll 2
+                for (int e = 0; e < len; ++e) {
+                    u64 k2[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) k2[i] = kn[i];
+                    if (e + 1 < len) lds_slab16<NS>(rowbase + (d0 + e + 1) * RB, 0, slab, kn);
+                    float bk = 0.f;
+                    if (DIST) {
+                        u64 n = zero2();
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) n = fma2(k2[i], k2[i], n);
+                        bk = -0.5f * sl2 * hsum2(n);
+                    }
+                    u64 t[4];
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        t[r] = nL2[r];
+                        if (DIST) t[r] = add2(t[r], pack2(bq[r] + bk, 0.f));
+                    }
+                    if (FULL) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+#pragma unroll
+                            for (int r = 0; r < 4; ++r) t[r] = fma2(q[r][i], k2[i], t[r]);
+                    } else {
+#pragma unroll
+                        for (int r = 0; r < 4; ++r)
+                            if ((mask >> r) & 1) {
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) t[r] = fma2(q[r][i], k2[i], t[r]);
+                            }
+                    }
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        if (!((mask >> r) & 1)) continue;
+                        float sc = hsum2(t[r]);
+#pragma unroll
+                        for (int m = 1; m < NS; m <<= 1) sc += __shfl_xor_sync(0xffffffffu, sc, m);
+                        if (slab == 0) tile[((nslots == 1 ? 0 : r) * RW + lrow) * CHS + e] = raw ? sc * kLn2 : fast_exp2(sc);
+                    }
+                }
+            };
+            if (mask == 15 || g.wsw != 1) sweep(std::true_type{});
+            else sweep(std::false_type{});
+            __syncwarp();
+            // write this piece of the runs of the stage: row j, positions posw*ws + (d + rot_j) mod ws
+#pragma unroll 1
+            for (int r = 0; r < 4; ++r) {
+                if (!((mask >> r) & 1) || w0 + r >= g.W) continue;
+                const int posw = axis_pos(s - pw - r, w0 + r, g.W, pw, g.wsw);
+                float* dst = a.o0 + ((warp_row0 + (int64_t)g.H * (w0 + r)) * g.K + posw * g.ws);
+                const float* src = tile + (nslots == 1 ? 0 : r) * RW * CHS;
+                const int n = rows_here * len;
+                if (tabled) {                                      // CHS == len == ws: tile index == idx
+#pragma unroll 4
+                    for (int idx = lane; idx < n; idx += 32) dst[etab[idx]] = src[idx];
+                    continue;
+                }
+                int row = lane / len, e = lane - row * len;        // element idx = row*len + e
+                const int drow = 32 / len, de = 32 - drow * len;
+                for (int idx = lane; idx < n; idx += 32) {
+                    int posh = d0 + e + rots[r * RW + row];
+                    posh -= (posh >= g.ws) ? g.ws : 0;
+                    dst[(int64_t)row * g.K + posh] = src[row * CHS + e];
+                    row += drow;
+                    e += de;
+                    if (e >= len) { e -= len; ++row; }
+                }
+            }
+            __syncwarp();
+        }
+    })
+}
+
+// =====================================================================
+// A (x) V and A^T (x) V from stored values.  The dense operand is streamed as
+// packed column stages exactly like the keys of the forward; the values of A
+// that pair with a stage are, for every centre column r, one run of ws
+// consecutive entries per CSR row (window column fixed, window rows varying),
+// which a warp copies into shared memory before the stage's FMAs:
+//   plain     : rows = the warp's own 32 pixels, run at posw(s - p - r; w0 + r);
+//   transposed: rows = the 32 + 2p pixels of the streamed column around the warp
+//               (by window symmetry A[j, i] sits in row j at offset i - j), run at
+//               posw(r + p - s; streamed column).
+// out = alpha * (sum_e a_e v_e - (sum_e a_e) * centre) with centre optional: the
+// second term is the Distance similarity pullback.
+// =====================================================================
+// Four-byte asynchronous copy global -> shared (the runs of A are only 4-byte aligned).
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+template <int CPE, bool TRANS, int NCRT>
+__global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+                                                             const __grid_constant__ CUtensorMap msc) {
+    constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;             // 16-channel slabs = lanes per pixel
+    constexpr int RW = 32 / NS;                                // pixel rows per warp
+    const Geo& g = a.g;
+    const int RB = a.row_bytes;                                // packed row: pair (144*NS) or single tensor (80*NS)
+    const int ROWS = a.TH + 2 * (g.p + a.roff);
+    const int pw = radius_w(g);
+    const bool fold = g.wsw == 1;                              // folded 1-D signal: rows continue into neighbour columns
+    const int w0 = blockIdx.x * 4, h0 = blockIdx.y * a.TH, u = blockIdx.z;
+    const int NSTAGES = g.wsw + min(3, g.W - 1 - w0);          // no stages for centre columns past the image
+    CA_PIPE_PROLOGUE(false)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slab = lane % NS, lrow = lane / NS;              // this lane's channel slab and row inside the warp
+    const int lr = (lt >> 5) * RW + lrow, h = h0 + lr;         // row inside the tile, image row
+    const bool active = h < g.H;
+    // Values of A are staged for CH = min(ws, 32) window rows at a time, per centre column r in
+    // slot r (one shared slot when folded: a stage then pairs with a single column), as
+    // [tile row][CHS] with tile row = warp row (plain) or warp row + row inside the chunk
+    // (transposed: the CSR row of the streamed pixel).  Two buffers per warp: the next piece is
+    // copied while the current one is used.
+    const int CH = min(g.ws, kRunChunk), CHS = CH | 1;
+    const int TRW = RW + (TRANS ? CH - 1 : 0);
+    const int nslots = fold ? 1 : 4;
+    const int buf_floats = nslots * TRW * CHS;
+    const int nch = (g.ws + CH - 1) / CH;                      // pieces per stage
+    // 2-D windows that fit one piece: source and tile offsets of every staged element are the same
+    // for all stages and centre columns up to the column base; they come from two tables
+    const bool tabled = nch == 1 && !fold;
+    float* wbase = reinterpret_cast<float*>(smem_al + (size_t)a.nstages * a.stage_bytes) +
+                   (size_t)warp * (2 * buf_floats + (tabled ? 2 * RW * CH : 0));
+    const int hw0 = h0 + (lt >> 5) * RW;                       // first image row of this warp
+    const float* nzu = a.cs0 + (int64_t)u * g.Np * g.K;
+    const int rows_here = hw0 >= g.H ? 0 : min(RW, g.H - hw0);
+    const int X = axis_len(g);
+    int* tsrc = reinterpret_cast<int*>(wbase + 2 * buf_floats);
+    int* tdst = tsrc + RW * CH;
+    if (tabled) {
+        for (int idx = lane; idx < RW * g.ws; idx += 32) {
+            const int wr = idx / g.ws, e = idx - wr * g.ws;
+            if (!TRANS) {
+                int posh = e + run_rot(hw0 + wr, g.H, g.p, g.ws);
+                posh -= (posh >= g.ws) ? g.ws : 0;
+                tsrc[idx] = (hw0 + wr) * g.K + posh;
+                tdst[idx] = wr * CHS + e;
+            } else {
+                const int tr = wr + e;
+                int hj = (hw0 + tr - g.p) % g.H;
+                hj += (hj < 0) ? g.H : 0;
+                tsrc[idx] = hj * g.K + axis_pos(g.p - e, hj, g.H, g.p, g.ws);
+                tdst[idx] = tr * CHS + e;
+            }
+        }
+        __syncwarp();
+    }
+
+    // starts the copies for piece c of stage s into buffer tb
+    auto fetch_piece = [&](int s, int c, int tb) {
+        const int mask = stage_mask<4>(s, pw);
+        const int wc = stage_column(g, w0, s);
+        const int d0 = c * CH, len = min(CH, g.ws - d0);
+        float* tbuf = wbase + tb * buf_floats;
+        if (hw0 >= g.H) { cp_async_commit(); return; }                 // warp past the image: nothing to stage
+        const int row0 = lane / len, e0 = lane - row0 * len;           // first element of this lane
+        const int drow = 32 / len, de = 32 - drow * len;               // step of 32 elements
+#pragma unroll 1
+        for (int r = 0; r < 4; ++r) {
+            if (!((mask >> r) & 1) || w0 + r >= g.W) continue;
+            float* dst = tbuf + (fold ? 0 : r) * TRW * CHS;
+            if (tabled) {
+                const int posw = TRANS ? axis_pos(r + pw - s, wc, g.W, pw, g.wsw)
+                                       : axis_pos(s - pw - r, w0 + r, g.W, pw, g.wsw);
+                const float* src = nzu + (int64_t)g.H * (TRANS ? wc : w0 + r) * g.K + posw * g.ws;
+                const int n = (TRANS ? RW : rows_here) * g.ws;
+#pragma unroll 4
+                for (int idx = lane; idx < n; idx += 32) cp_async4(dst + tdst[idx], src + tsrc[idx]);
+            } else if (!TRANS) {
+                const int posw = axis_pos(s - pw - r, w0 + r, g.W, pw, g.wsw);
+                const float* src = nzu + ((int64_t)g.H * (w0 + r) + hw0) * g.K + posw * g.ws;
+                const int n = rows_here * len;
+                int row = row0, e = e0;                                    // element idx = row*len + e
+                for (int idx = lane; idx < n; idx += 32) {
+                    int posh = d0 + e + run_rot(axis_coord(g, hw0 + row, w0 + r), X, g.p, g.ws);
+                    posh -= (posh >= g.ws) ? g.ws : 0;
+                    cp_async4(dst + row * CHS + e, src + (int64_t)row * g.K + posh);
+                    row += drow;
+                    e += de;
+                    if (e >= len) { e -= len; ++row; }
+                }
+            } else {
+                // entry (tile row tr, e) belongs to warp row tr - e: the CSR row of the streamed pixel
+                // (column wc, image row hw0 + d0 + tr - p), at the position of offset p - (d0 + e)
+                const int posw = axis_pos(r + pw - s, wc, g.W, pw, g.wsw);
+                const int n = RW * len;
+                int wr = row0, e = e0;                                     // warp row, row inside the chunk
+                for (int idx = lane; idx < n; idx += 32) {
+                    const int tr = wr + e;
+                    int hj = hw0 + d0 + tr - g.p;
+                    int64_t rowidx;                                         // CSR row inside the unit
+                    int x;
+                    if (fold) {
+                        x = (g.H * wc + hj) % X;
+                        x += (x < 0) ? X : 0;
+                        rowidx = x;
+                    } else {
+                        hj += (hj < 0) ? g.H : 0;                          // here ws > 32, so H > 32 > the tile's
+                        hj -= (hj >= g.H) ? g.H : 0;                       // overhang: two subtractions suffice
+                        hj -= (hj >= g.H) ? g.H : 0;
+                        x = hj;
+                        rowidx = hj + (int64_t)g.H * wc;
+                    }
+                    const int posh = axis_pos(g.p - d0 - e, x, X, g.p, g.ws);
+                    cp_async4(dst + tr * CHS + e, nzu + rowidx * g.K + posw * g.ws + posh);
+                    wr += drow;
+                    e += de;
+                    if (e >= len) { e -= len; ++wr; }
+                }
+            }
+        }
+        cp_async_commit();
+    };
+
+    u64 acc[4][8];
+    float asum[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        asum[r] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[r][i] = zero2();
+    }
+    fetch_piece(s_begin, 0, 0);
+    int piece = 0;                                             // pieces consumed so far (buffer = piece & 1)
+
+    CA_PIPE_LOOP({
+        const int mask = stage_mask<4>(s, pw);
+        const uint32_t rowbase = smem_u32(pipe.vec(buf)) + (lr + a.roff) * RB;
+        for (int c = 0; c < nch; ++c, ++piece) {
+            const int d0 = c * CH, len = min(CH, g.ws - d0);
+            if (c + 1 < nch) {
+                fetch_piece(s, c + 1, (piece + 1) & 1);
+                cp_async_wait<1>();
+            } else if (s + 1 < s_end) {
+                fetch_piece(s + 1, 0, (piece + 1) & 1);
+                cp_async_wait<1>();
+            } else {
+                cp_async_wait<0>();
+            }
+            __syncwarp();
+            const float* tile = wbase + (piece & 1) * buf_floats;
+            // operands of window row d0 + e: the streamed vector and the four values of A, fetched
+            // one row ahead of the FMAs that use them
+            auto fetch_row = [&](int e, u64 (&vv)[8], float (&aa)[4]) {
+                lds_slab16<NS>(rowbase + (d0 + e) * RB, a.which, slab, vv);
+                const float* ap = tile + (lrow + (TRANS ? e : 0)) * CHS + e;
+#pragma unroll
+                for (int r = 0; r < 4; ++r) aa[r] = ((mask >> r) & 1) ? ap[(fold ? 0 : r) * TRW * CHS] : 0.f;
+            };
+            u64 vn[8];
+            float an[4];
+            fetch_row(0, vn, an);
+#pragma unroll 2
+            for (int e = 0; e < len; ++e) {
+                u64 v2[8];
+                float av[4];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v2[i] = vn[i];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) av[r] = an[r];
+                if (e + 1 < len) fetch_row(e + 1, vn, an);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    if ((mask >> r) & 1) {
+                        asum[r] += av[r];
+                        const u64 a2 = pack2(av[r], av[r]);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[r][i] = fma2(a2, v2[i], acc[r][i]);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    })
+
+    if (a.c0) {
+        u64 ctr[4][8];
+        load_centre<CPE, 4, NCRT>(a.c0, g, u, h, w0, active, 1.f, ctr, 16 * slab);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const u64 ns = pack2(-asum[r], -asum[r]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[r][i] = fma2(ns, ctr[r][i], acc[r][i]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float x, y;
+            unpack2(acc[r][i], x, y);
+            store_centre<CPE, NCRT>(a.o0, g, u, h, w0, active, r, i, a.scale * x + ca_poison, a.scale * y + ca_poison, 16 * slab);
+        }
 }
 
 // =====================================================================
@@ -428,7 +1128,7 @@ __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dq_tiled_kernel(TileAr
 #pragma unroll
         for (int r = 0; r < NQ; ++r) {
             settled[r] = true;
-            if (hh < g.H && has_pixel(g, hh, w0 + r)) settled[r] = __ldg(a.cs1 + (int64_t)u * g.Np + hh + g.H * (w0 + r)) != 0.f;
+            if (hh < g.H && w0 + r < g.W) settled[r] = __ldg(a.cs1 + (int64_t)u * g.Np + hh + g.H * (w0 + r)) != 0.f;
             mine = mine && settled[r];
         }
         if (__syncthreads_and(mine)) return;
@@ -452,7 +1152,7 @@ __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dq_tiled_kernel(TileAr
     float bq[NQ], sumds[NQ], aux[NQ], ex[NQ][3];
 #pragma unroll
     for (int r = 0; r < NQ; ++r) {
-        const bool ok = active && (has_pixel(g, h, w0 + r)) && slab == 0;       // row scalars enter the lane sums once
+        const bool ok = active && (w0 + r < g.W) && slab == 0;       // row scalars enter the lane sums once
         const int64_t o = (int64_t)u * g.Np + h + g.H * (w0 + r);
         nL2[r] = pack2((ok && MODE != 3) ? -__ldg(a.cs0 + o) * (MODE ? 1.f : kLog2e) : 0.f, 0.f);
         nD2[r] = pack2((ok && MODE <= 1) ? -__ldg(a.cs1 + o) : 0.f, 0.f);
@@ -482,7 +1182,7 @@ __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dq_tiled_kernel(TileAr
         // first threshold of the search: tau >= max - 1 always
 #pragma unroll
         for (int r = 0; r < NQ; ++r)
-            if (active && slab == 0 && has_pixel(g, h, w0 + r))
+            if (active && slab == 0 && w0 + r < g.W)
                 a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = aux[r] - 1.f + ca_poison;
         return;
     }
@@ -491,7 +1191,7 @@ __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dq_tiled_kernel(TileAr
         // the same support and the step was short against the distances it was computed from
 #pragma unroll
         for (int r = 0; r < NQ; ++r)
-            if (active && slab == 0 && has_pixel(g, h, w0 + r) && !settled[r]) {
+            if (active && slab == 0 && w0 + r < g.W && !settled[r]) {
                 const int64_t o = (int64_t)u * g.Np + h + g.H * (w0 + r);
                 const float n = ex[r][0], sa = sumds[r], sb = aux[r];
                 float d = 0.f;
@@ -513,7 +1213,7 @@ __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dq_tiled_kernel(TileAr
         // pre-pass of the entmax pullback: D = sum g*dP / sum g per query row (launched without a stage split)
 #pragma unroll
         for (int r = 0; r < NQ; ++r)
-            if (active && slab == 0 && has_pixel(g, h, w0 + r))
+            if (active && slab == 0 && w0 + r < g.W)
                 a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = (sumds[r] > 0.f ? aux[r] / sumds[r] : 0.f) + ca_poison;
         return;
     }
@@ -544,24 +1244,39 @@ __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dq_tiled_kernel(TileAr
     }
     // dq = scale * (sum ds*k - [distance] sum(ds) * q);  q registers hold q*scale*log2(e) (entmax: q*scale/2)
     const float qfac = MODE ? 2.f : kLn2;
-    CA_OUT_DISPATCH(
-        _Pragma("unroll")
-        for (int r = 0; r < NQ; ++r) {
+    if (NS == 1) {
+        CA_BF_DISPATCH(
             _Pragma("unroll")
+            for (int r = 0; r < NQ; ++r) {
+                _Pragma("unroll")
+                for (int i = 0; i < 8; ++i) {
+                    float x, y, qx, qy;
+                    unpack2(dq[r][i], x, y);
+                    unpack2(q[r][i], qx, qy);
+                    if (MODE == 5) {
+                        x += ca_poison;
+                        y += ca_poison;
+                    } else {
+                        x = a.scale * x - (DIST ? sumds[r] * qx * qfac : 0.f) + ca_poison;
+                        y = a.scale * y - (DIST ? sumds[r] * qy * qfac : 0.f) + ca_poison;
+                    }
+                    store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, x, y);
+                }
+            })
+    } else {
+#pragma unroll
+        for (int r = 0; r < NQ; ++r) {
+#pragma unroll
             for (int i = 0; i < 8; ++i) {
                 float x, y, qx, qy;
                 unpack2(dq[r][i], x, y);
                 unpack2(q[r][i], qx, qy);
-                if (MODE == 5) {
-                    x += ca_poison;
-                    y += ca_poison;
-                } else {
-                    x = a.scale * x - (DIST ? sumds[r] * qx * qfac : 0.f) + ca_poison;
-                    y = a.scale * y - (DIST ? sumds[r] * qy * qfac : 0.f) + ca_poison;
-                }
-                store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, x, y, 16 * slab);
+                x = a.scale * x - (DIST ? sumds[r] * qx * qfac : 0.f) + ca_poison;
+                y = a.scale * y - (DIST ? sumds[r] * qy * qfac : 0.f) + ca_poison;
+                store_centre<CPE, NCRT>(a.o0, g, u, h, w0, active, r, i, x, y, 16 * slab);
             }
-        })
+        }
+    }
 }
 
 // =====================================================================
@@ -697,10 +1412,26 @@ __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dkdv_tiled_kernel(Tile
         }
     }
     // dk = scale * (sum ds*q - [distance] sum(ds) * k);  k registers hold k*scale*log2(e)
-    CA_OUT_DISPATCH(
-        _Pragma("unroll")
-        for (int r = 0; r < NQ; ++r) {
+    if (NS == 1) {
+        CA_BF_DISPATCH(
             _Pragma("unroll")
+            for (int r = 0; r < NQ; ++r) {
+                _Pragma("unroll")
+                for (int i = 0; i < 8; ++i) {
+                    float x, y, kx, ky, vx, vy;
+                    unpack2(dk[r][i], x, y);
+                    unpack2(k[r][i], kx, ky);
+                    unpack2(dv[r][i], vx, vy);
+                    x = a.scale * x - (DIST ? sumds[r] * kx * (ENT ? 2.f : kLn2) : 0.f) + ca_poison;
+                    y = a.scale * y - (DIST ? sumds[r] * ky * (ENT ? 2.f : kLn2) : 0.f) + ca_poison;
+                    store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, x, y);
+                    store_centre<CPE, NCRV, BF>(a.o1, g, u, h, w0, active, r, i, vx + ca_poison, vy + ca_poison);
+                }
+            })
+    } else {
+#pragma unroll
+        for (int r = 0; r < NQ; ++r) {
+#pragma unroll
             for (int i = 0; i < 8; ++i) {
                 float x, y, kx, ky, vx, vy;
                 unpack2(dk[r][i], x, y);
@@ -708,10 +1439,540 @@ __global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dkdv_tiled_kernel(Tile
                 unpack2(dv[r][i], vx, vy);
                 x = a.scale * x - (DIST ? sumds[r] * kx * (ENT ? 2.f : kLn2) : 0.f) + ca_poison;
                 y = a.scale * y - (DIST ? sumds[r] * ky * (ENT ? 2.f : kLn2) : 0.f) + ca_poison;
-                store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, x, y, 16 * slab);
-                store_centre<CPE, NCRV, BF>(a.o1, g, u, h, w0, active, r, i, vx + ca_poison, vy + ca_poison, 16 * slab);
+                store_centre<CPE, NCRT>(a.o0, g, u, h, w0, active, r, i, x, y, 16 * slab);
+                store_centre<CPE, NCRT>(a.o1, g, u, h, w0, active, r, i, vx + ca_poison, vy + ca_poison, 16 * slab);
             }
-        })
+        }
+    }
+}
+
+// =====================================================================
+// Pack kernel: two tensors in the reference layout -> [unit][column][row'][32]
+// with the circular halo along h unrolled, plus (optionally) the two scalar
+// planes [2*unit + {0: stats*log2(e), 1: D}][column][row'].
+// One thread per (row', column, unit, tensor) plus one per (row', column, unit) for the planes.
+// =====================================================================
+struct PackArgs {
+    Geo g;
+    int pp;                 // p' (even)
+    int Hp;                 // padded rows per column: roundup4(H + 2p')
+    int npairs;             // 1 or 2 tensor pairs
+    int single;             // 1: rows hold one tensor (src[0]) in 20 words per slab instead of a pair in 36
+    const float* src[4];    // pair j = (src[2j], src[2j+1])
+    float* dst[2];
+    float* planes;          // nullable
+    const float* stats;     // with planes
+    float stat_mul;         // plane 0 = stats * stat_mul: log2(e) for the softmax log-sum-exp, 1 for the entmax tau
+    const float* Din;       // with planes: D given ...
+    const float* y;         // ... or computed as dy . y
+    const float* dy;
+    float* Dout;            // nullable: D in the reference layout (interior rows)
+};
+
+template <int CPE, int NCRT, bool BF>
+__device__ __forceinline__ void pack_body(const PackArgs& a) {
+    constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
+    constexpr int NCR = NCRT;
+    const Geo& g = a.g;
+    const int rr = blockIdx.x * blockDim.x + threadIdx.x;
+    const int w = blockIdx.y;
+    // z slot: one per tensor copy and unit, plus one slot for the scalar planes
+    const int nt = a.single ? 1 : 2;                      // tensors per packed row
+    const int slots = nt * a.npairs + (a.planes ? 1 : 0);
+    const int u = blockIdx.z / slots, slot = blockIdx.z % slots;
+    if (rr >= a.Hp) return;
+    const bool real_row = rr < g.H + 2 * a.pp;
+    // source pixel of packed row rr: the halo rows wrap inside the column (2-D) or continue into the
+    // neighbouring columns of a folded 1-D signal
+    int pix = 0;
+    if (real_row) {
+        if (g.wsw == 1) {
+            pix = (g.H * w + rr - a.pp) % g.Npk;
+            if (pix < 0) pix += g.Npk;
+        } else {
+            pix = (rr - a.pp + g.H) % g.H + g.H * w;
+        }
+    }
+    const int64_t orow = ((int64_t)u * g.Wk + w) * a.Hp + rr;
+    if (slot < nt * a.npairs) {
+        const int pair = slot / nt, t = slot % nt;
+        const float* src = a.src[2 * pair + t];
+        const int row_floats = (a.single ? kSingleFloats : kRowFloats) * NS;
+        float4* dp = reinterpret_cast<float4*>(a.dst[pair] + orow * row_floats) + 4 * NS * t;
+        // chunk-major: the NS slabs of a 4-channel chunk are adjacent, so each pass writes 16*NS
+        // contiguous bytes
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            float4 vals[NS];
+#pragma unroll
+            for (int sl = 0; sl < NS; ++sl) {
+                const int cc = 16 * sl + 4 * c;
+                if (!real_row || cc >= NCR) {             // padding rows; channels past a narrow unit
+                    vals[sl] = make_float4(0.f, 0.f, 0.f, 0.f);
+                } else if (CPE == 1) {
+                    const int64_t o = goff<1, NCR>(u, cc, g.Npk, pix);
+                    vals[sl] = make_float4(ld_real<BF>(src, o), ld_real<BF>(src, o + g.Npk),
+                                           ld_real<BF>(src, o + 2 * (int64_t)g.Npk),
+                                           ld_real<BF>(src, o + 3 * (int64_t)g.Npk));
+                } else {
+                    const float2 lo = __ldg(reinterpret_cast<const float2*>(src + goff<2, NCR>(u, cc, g.Npk, pix)));
+                    const float2 hi = __ldg(reinterpret_cast<const float2*>(src + goff<2, NCR>(u, cc + 2, g.Npk, pix)));
+                    vals[sl] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                }
+            }
+#pragma unroll
+            for (int sl = 0; sl < NS; ++sl) dp[c * NS + sl] = vals[sl];
+        }
+        if (t == nt - 1) {
+#pragma unroll
+            for (int sl = 0; sl < NS; ++sl) dp[4 * NS + sl] = make_float4(0.f, 0.f, 0.f, 0.f);    // padding
+        }
+        return;
+    }
+    float L = 0.f, D = 0.f;
+    if (real_row) {
+        const int64_t so = (int64_t)u * g.Npk + pix;
+        L = __ldg(a.stats + so) * a.stat_mul;
+        if (a.Din) {
+            D = __ldg(a.Din + so);
+        } else {
+            constexpr int NC = NCR;                             // D = dy . y over all real channels of the unit
+            float dyv[NC], yv[NC];
+#pragma unroll
+            for (int cc = 0; cc < NC; ++cc) {
+                const int64_t o = goff<CPE, NCR>(u, cc, g.Npk, pix);
+                dyv[cc] = ld_real<BF>(a.dy, o);
+                yv[cc] = ld_real<BF>(a.y, o);
+            }
+#pragma unroll
+            for (int cc = 0; cc < NC; ++cc) D = fmaf(dyv[cc], yv[cc], D);
+            if (a.Dout && rr >= a.pp && rr < a.pp + g.H) a.Dout[so] = D;
+        }
+    }
+    const int64_t plane = (int64_t)g.Wk * a.Hp;
+    a.planes[(2 * (int64_t)u) * plane + (int64_t)w * a.Hp + rr] = L;
+    a.planes[(2 * (int64_t)u + 1) * plane + (int64_t)w * a.Hp + rr] = D;
+}
+
+template <int CPE, int NCRT>
+__global__ void __launch_bounds__(128) pack_kernel(PackArgs a) {
+    if (CPE == 1 && a.g.bf16) pack_body<CPE, NCRT, true>(a);
+    else pack_body<CPE, NCRT, false>(a);
+}
+
+// Pair packing for one-slab units (8 or 16 real channels) through shared memory: a block gathers 128
+// packed rows of one (column, unit, pair) -- every thread the 2 x NCR channel values of its row, 32
+// independent coalesced loads -- into a [128][36] tile, and the block writes the tile out as one contiguous
+// run of 16-byte stores (consecutive lanes on consecutive addresses: full sectors), where the direct form
+// above writes 64-byte pieces 144 bytes apart.  z slots: one per pair and unit, plus one for the planes.
+template <int CPE, int NCRT, bool BF>
+__device__ __forceinline__ void pack_rows_body(const PackArgs& a, float (*tile)[kRowFloats]) {
+    const Geo& g = a.g;
+    const int rr0 = blockIdx.x * 128, rr = rr0 + threadIdx.x;
+    const int w = blockIdx.y;
+    const int slots = a.npairs + (a.planes ? 1 : 0);
+    const int u = blockIdx.z / slots, slot = blockIdx.z % slots;
+    const bool in_rows = rr < a.Hp;
+    const bool real_row = in_rows && rr < g.H + 2 * a.pp;
+    int pix = 0;
+    if (real_row) {
+        if (g.wsw == 1) {
+            pix = (g.H * w + rr - a.pp) % g.Npk;
+            if (pix < 0) pix += g.Npk;
+        } else {
+            pix = (rr - a.pp + g.H) % g.H + g.H * w;
+        }
+    }
+    if (slot < a.npairs) {
+        float4 vals[8];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const float* src = a.src[2 * slot + t];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int cc = 4 * c;
+                if (!real_row || cc >= NCRT) {
+                    vals[4 * t + c] = make_float4(0.f, 0.f, 0.f, 0.f);
+                } else if (CPE == 1) {
+                    const int64_t o = goff<1, NCRT>(u, cc, g.Npk, pix);
+                    vals[4 * t + c] = make_float4(ld_real<BF>(src, o), ld_real<BF>(src, o + g.Npk),
+                                                  ld_real<BF>(src, o + 2 * (int64_t)g.Npk),
+                                                  ld_real<BF>(src, o + 3 * (int64_t)g.Npk));
+                } else {
+                    const float2 lo = __ldg(reinterpret_cast<const float2*>(src + goff<2, NCRT>(u, cc, g.Npk, pix)));
+                    const float2 hi = __ldg(reinterpret_cast<const float2*>(src + goff<2, NCRT>(u, cc + 2, g.Npk, pix)));
+                    vals[4 * t + c] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                }
+            }
+        }
+        float4* trow = reinterpret_cast<float4*>(tile[threadIdx.x]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) trow[i] = vals[i];
+        trow[8] = make_float4(0.f, 0.f, 0.f, 0.f);                       // padding words
+        __syncthreads();
+        const int nrows = min(128, a.Hp - rr0);
+        float4* out = reinterpret_cast<float4*>(a.dst[slot] + (((int64_t)u * g.Wk + w) * a.Hp + rr0) * kRowFloats);
+        const float4* tin = reinterpret_cast<const float4*>(&tile[0][0]);
+        for (int i = threadIdx.x; i < nrows * (kRowFloats / 4); i += 128) out[i] = tin[i];
+        return;
+    }
+    if (!in_rows) return;
+    float L = 0.f, D = 0.f;
+    if (real_row) {
+        const int64_t so = (int64_t)u * g.Npk + pix;
+        L = __ldg(a.stats + so) * a.stat_mul;
+        if (a.Din) {
+            D = __ldg(a.Din + so);
+        } else {
+            float dyv[NCRT], yv[NCRT];
+#pragma unroll
+            for (int cc = 0; cc < NCRT; ++cc) {
+                const int64_t o = goff<CPE, NCRT>(u, cc, g.Npk, pix);
+                dyv[cc] = ld_real<BF>(a.dy, o);
+                yv[cc] = ld_real<BF>(a.y, o);
+            }
+#pragma unroll
+            for (int cc = 0; cc < NCRT; ++cc) D = fmaf(dyv[cc], yv[cc], D);
+            if (a.Dout && rr >= a.pp && rr < a.pp + g.H) a.Dout[so] = D;
+        }
+    }
+    const int64_t plane = (int64_t)g.Wk * a.Hp;
+    a.planes[(2 * (int64_t)u) * plane + (int64_t)w * a.Hp + rr] = L;
+    a.planes[(2 * (int64_t)u + 1) * plane + (int64_t)w * a.Hp + rr] = D;
+}
+
+template <int CPE, int NCRT>
+__global__ void __launch_bounds__(128) pack_rows_kernel(PackArgs a) {
+    __shared__ __align__(16) float tile[128][kRowFloats];
+    if (CPE == 1 && a.g.bf16) pack_rows_body<CPE, NCRT, true>(a, tile);
+    else pack_rows_body<CPE, NCRT, false>(a, tile);
+}
+
+// The same for units of NS = 2 or 4 slabs (32 / 64 real channels), Float32 or ComplexF32: a block gathers 128 / NS
+// packed rows, thread (row, slab) the two 16-channel slabs of its row and slab (consecutive lanes on consecutive
+// rows: coalesced planar loads), into a [128 / NS][36 * NS] tile in the packed order [tensor][4-channel chunk]
+// [slab][4], and writes the tile out as one contiguous run.  The direct form writes 16 * NS-byte pieces 144 * NS
+// bytes apart.  In the planes slot the NS threads of a row share the dy . y sum through the tile.
+template <int CPE, int NCRT>
+__global__ void __launch_bounds__(128) pack_rows_wide_kernel(PackArgs a) {
+    constexpr int NS = NCRT / 16, RB = 128 / NS, RF = kRowFloats * NS;
+    __shared__ __align__(16) float tile[RB][RF];
+    const Geo& g = a.g;
+    const int rl = threadIdx.x % RB, slab = threadIdx.x / RB;
+    const int rr0 = blockIdx.x * RB, rr = rr0 + rl;
+    const int w = blockIdx.y;
+    const int slots = a.npairs + (a.planes ? 1 : 0);
+    const int u = blockIdx.z / slots, slot = blockIdx.z % slots;
+    const bool in_rows = rr < a.Hp;
+    const bool real_row = in_rows && rr < g.H + 2 * a.pp;
+    int pix = 0;
+    if (real_row) {
+        if (g.wsw == 1) {
+            pix = (g.H * w + rr - a.pp) % g.Npk;
+            if (pix < 0) pix += g.Npk;
+        } else {
+            pix = (rr - a.pp + g.H) % g.H + g.H * w;
+        }
+    }
+    if (slot < a.npairs) {
+        float4* trow = reinterpret_cast<float4*>(tile[rl]);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const float* src = a.src[2 * slot + t];
+            float4 vals[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int cc = 16 * slab + 4 * c;
+                if (!real_row) {
+                    vals[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+                } else if (CPE == 1) {
+                    const int64_t o = goff<1, NCRT>(u, cc, g.Npk, pix);
+                    vals[c] = make_float4(__ldg(src + o), __ldg(src + o + g.Npk), __ldg(src + o + 2 * (int64_t)g.Npk),
+                                          __ldg(src + o + 3 * (int64_t)g.Npk));
+                } else {
+                    const float2 lo = __ldg(reinterpret_cast<const float2*>(src + goff<2, NCRT>(u, cc, g.Npk, pix)));
+                    const float2 hi = __ldg(reinterpret_cast<const float2*>(src + goff<2, NCRT>(u, cc + 2, g.Npk, pix)));
+                    vals[c] = make_float4(lo.x, lo.y, hi.x, hi.y);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) trow[t * (4 * NS) + c * NS + slab] = vals[c];
+        }
+        trow[8 * NS + slab] = make_float4(0.f, 0.f, 0.f, 0.f);                 // padding words
+        __syncthreads();
+        const int nrows = min(RB, a.Hp - rr0);
+        float4* out = reinterpret_cast<float4*>(a.dst[slot] + (((int64_t)u * g.Wk + w) * a.Hp + rr0) * RF);
+        const float4* tin = reinterpret_cast<const float4*>(&tile[0][0]);
+        for (int i = threadIdx.x; i < nrows * (RF / 4); i += 128) out[i] = tin[i];
+        return;
+    }
+    // scalar planes: L and D = dy . y (or the given D); every thread sums its slab's 16 channels
+    float part = 0.f;
+    if (real_row && !a.Din) {
+        float dyv[16], yv[16];
+#pragma unroll
+        for (int cc = 0; cc < 16; ++cc) {
+            const int64_t o = goff<CPE, NCRT>(u, 16 * slab + cc, g.Npk, pix);
+            dyv[cc] = __ldg(a.dy + o);
+            yv[cc] = __ldg(a.y + o);
+        }
+#pragma unroll
+        for (int cc = 0; cc < 16; ++cc) part = fmaf(dyv[cc], yv[cc], part);
+    }
+    tile[rl][slab] = part;
+    __syncthreads();
+    if (slab != 0 || !in_rows) return;
+    float L = 0.f, D = 0.f;
+    if (real_row) {
+        const int64_t so = (int64_t)u * g.Npk + pix;
+        L = __ldg(a.stats + so) * a.stat_mul;
+        if (a.Din) {
+            D = __ldg(a.Din + so);
+        } else {
+#pragma unroll
+            for (int sl = 0; sl < NS; ++sl) D += tile[rl][sl];
+            if (a.Dout && rr >= a.pp && rr < a.pp + g.H) a.Dout[so] = D;
+        }
+    }
+    const int64_t plane = (int64_t)g.Wk * a.Hp;
+    a.planes[(2 * (int64_t)u) * plane + (int64_t)w * a.Hp + rr] = L;
+    a.planes[(2 * (int64_t)u + 1) * plane + (int64_t)w * a.Hp + rr] = D;
+}
+
+// ---------------------------------------------------------------- host side
+struct Padded {
+    int pp, Hp;
+    size_t pair_floats;     // one packed tensor pair
+    size_t single_floats;   // one packed single tensor
+    size_t plane_floats;    // both scalar planes
+};
+
+int slabs_of(const Geo& g) { return g.cr <= 16 ? 1 : g.cr / 16; }
+
+Padded padded_of(const Geo& g) {
+    Padded P;
+    P.pp = (g.p + 1) & ~1;
+    P.Hp = (g.H + 2 * P.pp + 3) & ~3;
+    P.pair_floats = (size_t)g.units * g.Wk * P.Hp * kRowFloats * slabs_of(g);
+    P.single_floats = (size_t)g.units * g.Wk * P.Hp * kSingleFloats * slabs_of(g);
+    P.plane_floats = (size_t)2 * g.units * g.Wk * P.Hp;
+    return P;
+}
+
+bool tiled_shape_ok(const Geo& g) {
+    // 16 real channels per unit, 8 zero-extended to 16 (half of the FMAs are then spent on zeros), or 32 / 64
+    // (2 / 4 lanes per pixel; Float32 storage only)
+    const bool chan = g.cr == 16 || g.cr == 8 || ((g.cr == 32 || g.cr == 64) && !g.bf16);
+    return chan && (g.wsw == g.ws || g.wsw == 1) && g.ws >= 3 && g.H >= 16 && g.ws <= (g.wsw == 1 ? 127 : 63);
+}
+
+// The stand-alone operator kernels also take 8 (zero-extended), 32 or 64 real channels per unit
+// (2 or 4 lanes per pixel for the wide ones).
+bool tiled_operator_ok(const Geo& g) {
+    return (g.cr == 8 || g.cr == 16 || g.cr == 32 || g.cr == 64) && (g.wsw == g.ws || g.wsw == 1) && g.ws >= 3 &&
+           g.H >= 16 && g.ws <= (g.wsw == 1 ? 127 : 63) && g.Wk == g.W;
+}
+
+// The geometry the tiled kernels run on.  2-D problems are taken as they are.  A 1-D signal of
+// length N (H = N, W = 1) is folded column-major into an Hf x (N / Hf) image: pixel n = h + Hf*w keeps
+// its address, its window is the rows h-p..h+p of its own column, and the halo rows of the packed
+// columns continue into the neighbouring columns (the pack kernel fills them by linear index), so
+// the 2-D kernels run unchanged with a window that is one column wide.
+bool fold_geo(const Geo& in, Geo* out) {
+    *out = in;
+    if (in.wsw == in.ws) return true;                      // 2-D
+    if (in.wsw != 1 || in.Wk != in.W) return false;
+    if (in.W != 1) return true;                            // already folded
+    for (int hf : {128, 96, 64, 48, 32, 16}) {
+        if (in.H % hf == 0 && in.H / hf >= 1) {
+            out->H = hf;
+            out->W = out->Wk = in.H / hf;
+            return true;
+        }
+    }
+    return false;
+}
+
+// Launch-shape overrides for tuning sessions.  Compiled out of the shipped library (the build
+// never defines CA_TUNING): no launch reads the environment.
+#ifdef CA_TUNING
+int tune_int(const char* name, int dflt) {
+    const char* v = getenv(name);
+    return v && *v ? atoi(v) : dflt;
+}
+#else
+inline int tune_int(const char*, int dflt) { return dflt; }
+#endif
+
+int launch_pack(const PackArgs& a, cudaStream_t st) {
+    dim3 grid((a.Hp + 127) / 128, a.g.Wk, a.g.units * ((a.single ? 1 : 2) * a.npairs + (a.planes ? 1 : 0)));
+    const int cr = a.g.cr;
+    // beyond the grid limits (very long folded 1-D signals, very many units) the generic kernels run
+    if (grid.y > 65535u || grid.z > 65535u) return CA_ERR_UNSUPPORTED;
+    if (!a.single && cr <= 16) {
+        // one-slab pairs: the shared-memory form (one z slot per pair instead of one per tensor)
+        dim3 grid2(grid.x, grid.y, a.g.units * (a.npairs + (a.planes ? 1 : 0)));
+        if (a.g.cpe == 1) {
+            if (cr == 8) pack_rows_kernel<1, 8><<<grid2, 128, 0, st>>>(a);
+            else pack_rows_kernel<1, 16><<<grid2, 128, 0, st>>>(a);
+        } else {
+            if (cr == 8) pack_rows_kernel<2, 8><<<grid2, 128, 0, st>>>(a);
+            else pack_rows_kernel<2, 16><<<grid2, 128, 0, st>>>(a);
+        }
+        CA_CHECK_LAUNCH("pack kernel");
+        return CA_OK;
+    }
+    if (!a.single && (cr == 32 || cr == 64) && !a.g.bf16) {
+        // wide pairs: the shared-memory form with 128 / NS rows per block
+        const int rb = 128 / (cr / 16);
+        dim3 grid2((a.Hp + rb - 1) / rb, grid.y, a.g.units * (a.npairs + (a.planes ? 1 : 0)));
+        if (a.g.cpe == 1) {
+            if (cr == 32) pack_rows_wide_kernel<1, 32><<<grid2, 128, 0, st>>>(a);
+            else pack_rows_wide_kernel<1, 64><<<grid2, 128, 0, st>>>(a);
+        } else {
+            if (cr == 32) pack_rows_wide_kernel<2, 32><<<grid2, 128, 0, st>>>(a);
+            else pack_rows_wide_kernel<2, 64><<<grid2, 128, 0, st>>>(a);
+        }
+        CA_CHECK_LAUNCH("pack kernel");
+        return CA_OK;
+    }
+#define CA_PACK(CPEV)                                                        \
+    do {                                                                     \
+        if (cr == 8) pack_kernel<CPEV, 8><<<grid, 128, 0, st>>>(a);          \
+        else if (cr == 16) pack_kernel<CPEV, 16><<<grid, 128, 0, st>>>(a);   \
+        else if (cr == 32) pack_kernel<CPEV, 32><<<grid, 128, 0, st>>>(a);   \
+        else pack_kernel<CPEV, 64><<<grid, 128, 0, st>>>(a);                 \
+    } while (0)
+    if (a.g.cpe == 1) CA_PACK(1);
+    else CA_PACK(2);
+#undef CA_PACK
+    CA_CHECK_LAUNCH("pack kernel");
+    return CA_OK;
+}
+
+struct Launch {
+    TileArgs a;
+    CUtensorMap mv, msc;
+    dim3 grid;
+    int threads;
+    size_t smem;
+};
+
+// SM count of the current device (cached per device ordinal).
+int sm_count() {
+    static std::atomic<int> cache[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = cache[dev].load(std::memory_order_relaxed);
+    if (!n) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        cache[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+// Fills the launch geometry and the tensor maps of the packed pair (and of the
+// scalar planes when given).  `nq` centre pixels per thread, `xch_floats` per
+// thread for the merge of a split tile.  CTAs have at most 128 threads: four
+// warps of rows, or two warps of rows times two stage groups on small grids.
+int prepare(const Geo& g, const Padded& P, int nq, int xch_floats, const char* env_warps, const float* pair,
+            const float* planes, Launch* L, bool allow_split = true, int max_warps = 4, int ns = 1,
+            bool single = false, int stages = kStages) {
+    const int rw = 32 / ns;                             // pixel rows per warp (ns lanes share a pixel)
+    const int rf = (single ? kSingleFloats : kRowFloats) * ns, rb = rf * 4;
+    int warps = (g.H + rw - 1) / rw;
+    if (warps > max_warps) warps = max_warps;
+    const long cols = (g.W + nq - 1) / nq;
+    const long ctas4 = cols * ((g.H + rw * warps - 1) / (rw * warps)) * g.units;
+    int nsplit = (ctas4 * warps < 6L * sm_count()) ? 2 : 1;
+    nsplit = tune_int("CIRCATT_SPLIT", nsplit);
+    if (!allow_split) nsplit = 1;
+    if (nsplit == 2 && warps > 2) warps = 2;
+    warps = tune_int(env_warps, warps);
+    if (warps * nsplit > 4) warps = 4 / nsplit;
+    TileArgs& a = L->a;
+    a.g = g;
+    a.status = status_word();
+    a.wait_tries = kWaitTries;
+    a.TH = rw * warps;
+    a.roff = P.pp - g.p;
+    a.nsplit = nsplit;
+    a.row_bytes = rb;
+    const int ROWS = a.TH + 2 * P.pp;
+    if (ROWS > 256) { set_error("tile of %d rows exceeds the TMA box limit", ROWS); return CA_ERR_UNSUPPORTED; }
+    const int sstride = (ROWS * 4 + 127) & ~127;
+    const int vbytes = (ROWS * rb + 127) & ~127;
+    a.stage_bytes = (vbytes + (planes ? 2 * sstride : 0) + 1023) & ~1023;
+    L->grid = dim3((unsigned)cols, (g.H + a.TH - 1) / a.TH, g.units);
+    L->threads = 32 * warps * nsplit;
+    a.nstages = stages;
+    size_t smem = (size_t)nsplit * stages * a.stage_bytes;
+    const size_t xch = (size_t)xch_floats * 32 * warps * sizeof(float);
+    if (nsplit == 2 && xch > smem) smem = xch;
+    L->smem = smem + 1024;
+    if (L->smem > 220 * 1024) return CA_ERR_UNSUPPORTED;     // window too large for the stage ring: generic kernels
+    const uint64_t dims[4] = {(uint64_t)rf, (uint64_t)P.Hp, (uint64_t)g.Wk, (uint64_t)g.units};
+    const uint64_t strides[3] = {(uint64_t)rb, (uint64_t)P.Hp * rb, (uint64_t)P.Hp * rb * g.Wk};
+    const uint32_t box[4] = {(uint32_t)rf, (uint32_t)ROWS, 1, 1};
+    int rc;
+    if ((rc = encode_tensor_map(&L->mv, pair, 4, dims, strides, box, false))) return rc;
+    if (planes) {
+        const uint64_t sdims[3] = {(uint64_t)P.Hp, (uint64_t)g.Wk, (uint64_t)2 * g.units};
+        const uint64_t sstr[2] = {(uint64_t)P.Hp * 4, (uint64_t)P.Hp * 4 * g.Wk};
+        const uint32_t sbox[3] = {(uint32_t)ROWS, 1, 1};
+        if ((rc = encode_tensor_map(&L->msc, planes, 3, sdims, sstr, sbox, false))) return rc;
+    } else {
+        L->msc = L->mv;
+    }
+    return CA_OK;
+}
+
+template <typename K>
+int set_smem(K kernel, size_t bytes) {
+    if (bytes > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(shared memory)");
+    }
+    return CA_OK;
+}
+
+#define CA_LAUNCH_TILED(KERNEL, L, st)                                                \
+    do {                                                                              \
+        int rc__ = set_smem(KERNEL, (L).smem);                                        \
+        if (rc__) return rc__;                                                        \
+        KERNEL<<<(L).grid, (L).threads, (L).smem, st>>>((L).a, (L).mv, (L).msc);      \
+        count_tiled_launch();                                                         \
+    } while (0)
+
+#define CA_DIST_CPE(KERNEL_T, dist, cpe, L, st)                                       \
+    do {                                                                              \
+        if ((cpe) == 1) {                                                             \
+            if (dist) CA_LAUNCH_TILED((KERNEL_T<true, 1>), L, st);                    \
+            else CA_LAUNCH_TILED((KERNEL_T<false, 1>), L, st);                        \
+        } else {                                                                      \
+            if (dist) CA_LAUNCH_TILED((KERNEL_T<true, 2>), L, st);                    \
+            else CA_LAUNCH_TILED((KERNEL_T<false, 2>), L, st);                        \
+        }                                                                             \
+    } while (0)
+
+#define CA_DIST_CPE_NQ(KERNEL_T, dist, cpe, NQV, XV, NCRV_, L, st)                    \
+    do {                                                                              \
+        if ((cpe) == 1) {                                                             \
+            if (dist) CA_LAUNCH_TILED((KERNEL_T<true, 1, NQV, XV, NCRV_>), L, st);    \
+            else CA_LAUNCH_TILED((KERNEL_T<false, 1, NQV, XV, NCRV_>), L, st);        \
+        } else {                                                                      \
+            if (dist) CA_LAUNCH_TILED((KERNEL_T<true, 2, NQV, XV, NCRV_>), L, st);    \
+            else CA_LAUNCH_TILED((KERNEL_T<false, 2, NQV, XV, NCRV_>), L, st);        \
+        }                                                                             \
+    } while (0)
+
+// Centre pixels per thread.  Large problems use the widest tile the registers allow (least
+// shared-memory traffic per FMA); problems too small to fill the GPU use narrower tiles, which
+// means more, shorter-lived warps.
+int pick_nq(const Geo& g, int wide, int narrow, const char* env) {
+    const long tasks = ((long)(g.W + wide - 1) / wide) * ((g.H + 31) / 32) * g.units;     // warps at the wide tile
+    const int nq = tasks < 12L * sm_count() ? narrow : wide;
+    return tune_int(env, nq);
 }
 
 // mode 0: softmax; 1: entmax; 2: entmax pre-pass (writes D, needs no D and no dq).  The entmax
@@ -725,7 +1986,7 @@ int run_dq(const Geo& g, const Padded& P, float scale, int dist, const float* q,
     // two query columns per thread measured faster than four at every size for the softmax dq sweep of one-slab
     // units (160 registers, three blocks per SM, against 255 and two)
     const int nq = mode ? 4 : (ns > 1 ? (g.ws <= 9 ? 2 : 4) : tune_int("CIRCATT_DQ_NQ", 2));
-    int rc = prepare(g, P, nq, 17 * nq, "CIRCATT_DQ_WARPS", kv, nullptr, &L, mode == 0 && ns == 1 ? 2 : 1, 4, ns);
+    int rc = prepare(g, P, nq, 17 * nq, "CIRCATT_DQ_WARPS", kv, nullptr, &L, mode == 0 && ns == 1, 4, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.c1 = dy; L.a.cs0 = stats; L.a.cs1 = D; L.a.o0 = dq; L.a.ostats = Dout;
     if (ns == 2 && nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 32, L, st);
@@ -746,7 +2007,7 @@ int run_entmax_fwd_sweep(const Geo& g, const Padded& P, float scale, int dist, c
                          float* tau, float* settled, float* y, int mode, int iter, cudaStream_t st) {
     Launch L{};
     if (slabs_of(g) > 1) return CA_ERR_UNSUPPORTED;
-    int rc = prepare(g, P, 4, 17 * 4, "CIRCATT_DQ_WARPS", kv, nullptr, &L, 1, 4, 1);
+    int rc = prepare(g, P, 4, 17 * 4, "CIRCATT_DQ_WARPS", kv, nullptr, &L, false, 4, 1);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.cs0 = tau; L.a.cs1 = settled; L.a.o0 = y; L.a.o1 = settled; L.a.ostats = tau;
     L.a.iter = iter;
@@ -763,7 +2024,7 @@ int run_dkdv(const Geo& g, const Padded& P, float scale, int dist, const float* 
     const int ns = slabs_of(g);
     if (ns > 1 && entmax) return CA_ERR_UNSUPPORTED;
     const int nq = 3;
-    int rc = prepare(g, P, nq, 33 * nq, "CIRCATT_DKDV_WARPS", qdy, planes, &L, ns == 1 ? 2 : 1, 4, ns);
+    int rc = prepare(g, P, nq, 33 * nq, "CIRCATT_DKDV_WARPS", qdy, planes, &L, ns == 1, 4, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = k; L.a.c1 = v; L.a.o0 = dk; L.a.o1 = dv;
     if (ns == 2) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 32, L, st);
@@ -775,6 +2036,38 @@ int run_dkdv(const Geo& g, const Padded& P, float scale, int dist, const float* 
 }
 
 }  // namespace
+
+// ---------------------------------------------------------------- tensor maps
+int encode_tensor_map(CUtensorMap* map, const float* base, int rank, const uint64_t* dims,
+                      const uint64_t* strides_bytes, const uint32_t* box, bool swizzle128) {
+    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static EncodeFn fn = nullptr;
+    if (!fn) {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q);
+        if (e != cudaSuccess || !sym) {
+            set_error("cuTensorMapEncodeTiled is not available from the driver");
+            return CA_ERR_CUDA;
+        }
+        fn = reinterpret_cast<EncodeFn>(sym);
+    }
+    cuuint64_t gdims[5], gstr[4];
+    cuuint32_t gbox[5], estr[5];
+    for (int i = 0; i < rank; ++i) { gdims[i] = dims[i]; gbox[i] = box[i]; estr[i] = 1; }
+    for (int i = 0; i + 1 < rank; ++i) gstr[i] = strides_bytes[i];
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<float*>(base), gdims, gstr,
+                    gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+        return CA_ERR_CUDA;
+    }
+    return CA_OK;
+}
 
 // ---------------------------------------------------------------- entry points of this file
 size_t tiled_fwd_workspace(const Geo& gin) {
@@ -800,6 +2093,15 @@ size_t tiled_bwd_workspace(const Geo& gin) {
     return (2 * P.pair_floats + P.plane_floats) * sizeof(float);
 }
 
+int tiled_stage_timeouts(int* count) {
+    cudaError_t e = cudaMemcpyFromSymbol(count, g_stage_timeouts, sizeof(int));
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyFromSymbol(stage timeouts)");
+    return CA_OK;
+}
+
+int tiled_emit_a(const Geo& g, float scale, int dist, const float* q, const float* stats, float* nz,
+                 void* workspace, cudaStream_t st, bool single = false);
+
 int tiled_attention_fwd(const Geo& gin, float scale, int dist, const float* q, const float* k, const float* v,
                         float* y, float* nz, float* stats, void* workspace, cudaStream_t st) {
     Geo g;
@@ -819,7 +2121,7 @@ int tiled_attention_fwd(const Geo& gin, float scale, int dist, const float* q, c
     // four columns per thread, or two when the grid is small or the window is short (with ws <= 9 most
     // stages of a four-column tile pair with only some of its columns: measured 18 % faster at ws 7)
     const int nq = g.ws <= 9 ? tune_int("CIRCATT_FWD_NQ", 2) : (ns > 1 ? 4 : pick_nq(g, 4, 2, "CIRCATT_FWD_NQ"));
-    if ((rc = prepare(g, P, nq, 18 * nq, "CIRCATT_FWD_WARPS", kv, nullptr, &L, ns == 1 ? 2 : 1, 4, ns))) return rc;
+    if ((rc = prepare(g, P, nq, 18 * nq, "CIRCATT_FWD_WARPS", kv, nullptr, &L, ns == 1, 4, ns))) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.o0 = y; L.a.ostats = stats;
 #define CA_FWD2(DCV, EX, NQV, NCRV_)                                                            \
     do {                                                                                 \
@@ -856,6 +2158,55 @@ int tiled_attention_fwd(const Geo& gin, float scale, int dist, const float* q, c
 #undef CA_FWD
     CA_CHECK_LAUNCH("tiled forward kernel");
     if (nz) return tiled_emit_a(g, scale, dist, q, stats, nz, workspace, st);
+    return CA_OK;
+}
+
+// A's values in CSR order from q, the packed (k|v) pair left in `workspace` by
+// tiled_attention_fwd, and the row statistics.
+int tiled_emit_a(const Geo& g, float scale, int dist, const float* q, const float* stats, float* nz,
+                 void* workspace, cudaStream_t st, bool single) {
+    if (!tiled_operator_ok(g)) return CA_ERR_UNSUPPORTED;
+    const Padded P = padded_of(g);
+    const int ns = slabs_of(g);
+    Launch L{};
+    // three copy stages, or two when that lets one more CTA reside on an SM
+    const int ch = std::min(g.ws, kRunChunk), nslots = g.wsw == 1 ? 1 : 4;
+    int rc = CA_OK;
+    auto setup = [&](int stages) {
+        L = Launch{};
+        rc = prepare(g, P, 4, 0, "CIRCATT_FWD_WARPS", static_cast<const float*>(workspace), nullptr, &L, true, 4, ns,
+                     single, stages);
+        // per warp: staging tile, run rotations, offset table
+        if (!rc) L.smem += (size_t)L.threads / 32 * (32 / ns) * (nslots * (ch + 1) + 4 + ch) * sizeof(float);
+        return rc;
+    };
+    if (setup(kStages)) return rc;
+    {
+        const size_t per_sm = 227 * 1024, with3 = L.smem + 1024;          // + the driver's per-CTA reservation
+        const size_t with2 = with3 - (size_t)L.a.nsplit * L.a.stage_bytes;
+        const int want = tune_int("CIRCATT_EMIT_STAGES", 0);
+        // the kernel's registers allow three CTAs per SM at most
+        if (want == 2 || (want == 0 && std::min<size_t>(3, per_sm / with2) > std::min<size_t>(3, per_sm / with3)))
+            if (setup(2)) return rc;
+    }
+    if (L.smem > 200 * 1024) return CA_ERR_UNSUPPORTED;
+#define CA_EMIT(NSV)                                                                  \
+    do {                                                                              \
+        if (g.cpe == 1) {                                                             \
+            if (dist) CA_LAUNCH_TILED((emit_a_tiled_kernel<true, 1, NSV>), L, st);    \
+            else CA_LAUNCH_TILED((emit_a_tiled_kernel<false, 1, NSV>), L, st);        \
+        } else {                                                                      \
+            if (dist) CA_LAUNCH_TILED((emit_a_tiled_kernel<true, 2, NSV>), L, st);    \
+            else CA_LAUNCH_TILED((emit_a_tiled_kernel<false, 2, NSV>), L, st);        \
+        }                                                                             \
+    } while (0)
+    L.a.scale = scale; L.a.c0 = q; L.a.cs0 = stats; L.a.o0 = nz;
+    if (g.cr == 8) CA_EMIT(8);
+    else if (g.cr == 16) CA_EMIT(16);
+    else if (g.cr == 32) CA_EMIT(32);
+    else CA_EMIT(64);
+#undef CA_EMIT
+    CA_CHECK_LAUNCH("tiled A kernel");
     return CA_OK;
 }
 
@@ -1031,6 +2382,142 @@ int tiled_attention_fwd_entmax(const Geo& gin, float scale, int dist, const floa
     for (int it = 0; it < kEntmaxFwdSteps; ++it)
         if ((rc = run_entmax_fwd_sweep(g, P, scale, dist, q, kv, stats, settled, nullptr, 4, it, st))) return rc;
     return run_entmax_fwd_sweep(g, P, scale, dist, q, kv, stats, settled, y, 5, 0, st);
+}
+
+// ---------------------------------------------------------------- stand-alone operators
+size_t tiled_operator_workspace(const Geo& gin) {
+    Geo g;
+    if (!fold_geo(gin, &g)) return 0;
+    if (!tiled_operator_ok(g)) return 0;
+    return padded_of(g).single_floats * sizeof(float);
+}
+
+// Packs one tensor as single-tensor rows.
+static int pack_single(const Geo& g, const Padded& P, const float* src, float* dst, cudaStream_t st) {
+    PackArgs pa{};
+    pa.g = g; pa.pp = P.pp; pa.Hp = P.Hp; pa.npairs = 1; pa.single = 1;
+    pa.src[0] = src; pa.dst[0] = dst;
+    return launch_pack(pa, st);
+}
+
+// Scaled similarity scores in CSR order: x indexes the row pixel, y the column pixel.
+int tiled_similarity(const Geo& gin, float scale, int dist, const float* x, const float* y, float* nz,
+                     void* workspace, cudaStream_t st) {
+    Geo g;
+    if (!fold_geo(gin, &g)) return CA_ERR_UNSUPPORTED;
+    if (!workspace || !tiled_operator_workspace(g)) return CA_ERR_UNSUPPORTED;
+    int rc = pack_single(g, padded_of(g), y, static_cast<float*>(workspace), st);
+    if (rc) return rc;
+    return tiled_emit_a(g, scale, dist, x, nullptr, nz, workspace, st, true);
+}
+
+static int run_apply(const Geo& g, const Padded& P, const float* nz, const float* packed,
+                     const float* centre, float* out, float alpha, int transposed, cudaStream_t st) {
+    Launch L{};
+    const int ns = slabs_of(g);
+    // 2-D, one slab: two warps of rows per CTA (smaller stages, more CTAs per SM); otherwise four
+    int rc = prepare(g, P, 4, 0, "CIRCATT_APPLY_WARPS", packed, nullptr, &L, false, (ns == 1 && g.wsw != 1) ? 2 : 4, ns, true);
+    if (rc) return rc;
+    const int ch = std::min(g.ws, kRunChunk), chs = ch | 1;
+    const int trw = 32 / ns + (transposed ? ch - 1 : 0);
+    // per warp: two buffers and, for single-piece 2-D windows, the two offset tables
+    const bool tabled = g.ws <= kRunChunk && g.wsw != 1;
+    L.smem += (size_t)L.threads / 32 * (2 * (g.wsw == 1 ? 1 : 4) * trw * chs + (tabled ? 2 * (32 / ns) * ch : 0)) * sizeof(float);
+    if (L.smem > 200 * 1024) {
+        set_error("tiled apply: window %d with %d channels per unit needs %zu bytes of shared memory", g.ws, g.cr, L.smem);
+        return CA_ERR_UNSUPPORTED;
+    }
+    L.a.scale = alpha; L.a.which = 0; L.a.c0 = centre; L.a.cs0 = nz; L.a.o0 = out;
+#define CA_APPLY(NSV)                                                                     \
+    do {                                                                                  \
+        if (g.cpe == 1) {                                                                 \
+            if (transposed) CA_LAUNCH_TILED((apply_tiled_kernel<1, true, NSV>), L, st);   \
+            else CA_LAUNCH_TILED((apply_tiled_kernel<1, false, NSV>), L, st);             \
+        } else {                                                                          \
+            if (transposed) CA_LAUNCH_TILED((apply_tiled_kernel<2, true, NSV>), L, st);   \
+            else CA_LAUNCH_TILED((apply_tiled_kernel<2, false, NSV>), L, st);             \
+        }                                                                                 \
+    } while (0)
+    if (g.cr == 8) CA_APPLY(8);
+    else if (g.cr == 16) CA_APPLY(16);
+    else if (g.cr == 32) CA_APPLY(32);
+    else CA_APPLY(64);
+#undef CA_APPLY
+    CA_CHECK_LAUNCH("tiled apply kernel");
+    return CA_OK;
+}
+
+// out = alpha * (A (x) v) or alpha * (A^T (x) v) from the values of A in CSR order.
+int tiled_apply(const Geo& gin, const float* nz, const float* v, float* out, float alpha, int transposed,
+                void* workspace, cudaStream_t st) {
+    Geo g;
+    if (!fold_geo(gin, &g)) return CA_ERR_UNSUPPORTED;
+    if (!workspace || !tiled_operator_workspace(g)) return CA_ERR_UNSUPPORTED;
+    const Padded P = padded_of(g);
+    float* packed = static_cast<float*>(workspace);
+    int rc = pack_single(g, P, v, packed, st);
+    if (rc) return rc;
+    return run_apply(g, P, nz, packed, nullptr, out, alpha, transposed, st);
+}
+
+// Pullback of the similarity: dx[j] = scale * sum_i dS[j,i] y[i], dy[i] = scale * sum_j dS[j,i] x[j]
+// (Distance: minus the sum of the dS involved times the pixel's own vector).
+int tiled_similarity_bwd(const Geo& gin, float scale, int dist, const float* x, const float* y, const float* dS,
+                         float* dx, float* dy, void* workspace, cudaStream_t st) {
+    Geo g;
+    if (!fold_geo(gin, &g)) return CA_ERR_UNSUPPORTED;
+    if (!workspace || !tiled_operator_workspace(g)) return CA_ERR_UNSUPPORTED;
+    const Padded P = padded_of(g);
+    float* packed = static_cast<float*>(workspace);
+    int rc;
+    if (dx) {
+        if ((rc = pack_single(g, P, y, packed, st))) return rc;
+        if ((rc = run_apply(g, P, dS, packed, dist ? x : nullptr, dx, scale, 0, st))) return rc;
+    }
+    if (dy) {
+        if ((rc = pack_single(g, P, x, packed, st))) return rc;
+        if ((rc = run_apply(g, P, dS, packed, dist ? y : nullptr, dy, scale, 1, st))) return rc;
+    }
+    return CA_OK;
+}
+
+
+// ---------------------------------------------------------------- bounded-wait self test
+// One CTA arms a stage barrier with more bytes than the single bulk copy it issues delivers, so the
+// barrier never completes; the wait must run out after `tries` polls, the CTA must report through the
+// same counter and status word as the tiled kernels and return.  Nothing faults and nothing spins
+// without a limit; the copy itself lands (the thread polls its destination, again with a limit).
+__device__ __align__(16) float g_probe_src[8] = {1.f, 2.f, 3.f, 4.f, 5.f, 6.f, 7.f, 8.f};
+
+__global__ void __launch_bounds__(32) stage_timeout_probe_kernel(uint32_t tries, int* status, int* out) {
+    __shared__ __align__(16) float dst[8];
+    __shared__ __align__(8) uint64_t bar;
+    if (threadIdx.x == 0) {
+        dst[7] = 0.f;
+        mbar_init(&bar, 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        mbar_arrive_expect_tx(&bar, 64);                      // 64 bytes expected ...
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 32, [%2];"
+                     ::"r"(smem_u32(dst)), "l"(g_probe_src), "r"(smem_u32(&bar)) : "memory");   // ... 32 delivered
+        ok = mbar_wait(&bar, 0, tries);
+        // the copy in flight gets a bounded chance to land before the CTA (and its shared memory) goes away
+        for (uint32_t i = 0; i < (1u << 16) && *reinterpret_cast<volatile float*>(&dst[7]) != 8.f; ++i) {}
+        if (!ok) {
+            atomicAdd(&g_stage_timeouts, 1);
+            if (status) atomicOr(status, 1);
+        }
+        if (out) *out = ok ? 0 : 1;
+    }
+}
+
+int tiled_probe_stage_timeout(uint32_t tries, int* out, cudaStream_t st) {
+    stage_timeout_probe_kernel<<<1, 32, 0, st>>>(tries, status_word(), out);
+    CA_CHECK_LAUNCH("stage timeout probe kernel");
+    return CA_OK;
 }
 
 }  // namespace ca

@@ -37,25 +37,11 @@ int tiled_stage_timeouts(int* count);
 // Launches the one-CTA self test of the bounded stage wait (`out`: nullable device int, 1 = the wait ran out).
 int tiled_probe_stage_timeout(uint32_t tries, int* out, cudaStream_t st);
 
-// 2-D softmax attention on the tensor cores (tensor.cu), for the problems that tc_route() accepts.  The forward's workspace
-// serves the backward of the same problem as `fwd_workspace`.
-bool tc_route(const Geo& g);
-size_t tc_fwd_workspace(const Geo& g, bool want_nz);
-size_t tc_bwd_workspace(const Geo& g);          // whole backward (without D)
-int tc_attention_fwd(const Geo& g, float scale, int dist, const float* q, const float* k, const float* v, float* y,
-                     float* nz, float* stats, void* workspace, cudaStream_t st);
-int tc_attention_bwd(const Geo& g, float scale, int dist, const float* q, const float* k, const float* v, const float* y,
-                     const float* dy, const float* stats, float* D, float* dq, float* dk, float* dv, void* workspace,
-                     const void* fwd_workspace, cudaStream_t st);
-
 // Stand-alone operators on the tiled kernels.  `workspace` holds one packed
 // tensor pair (tiled_operator_workspace bytes, 0 when the shape is not covered).
 size_t tiled_operator_workspace(const Geo& g);
 int tiled_similarity(const Geo& g, float scale, int dist, const float* x, const float* y, float* nz,
                      void* workspace, cudaStream_t st);
-// The normalised entries exp(score - stats) in CSR order.
-int tiled_weights(const Geo& g, float scale, int dist, const float* x, const float* y, const float* stats, float* nz,
-                  void* workspace, cudaStream_t st);
 int tiled_apply(const Geo& g, const float* nz, const float* v, float* out, float alpha, int transposed,
                 void* workspace, cudaStream_t st);
 int tiled_similarity_bwd(const Geo& g, float scale, int dist, const float* x, const float* y, const float* dS,
