@@ -161,7 +161,8 @@ static int launch_row_normalize(int64_t rows, int K, int entmax, const float* s,
         else if (K <= 512) row_entmax15_reg_kernel<16><<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
         else row_entmax15_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
     }
-    else row_softmax_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
+    else CA_ROW_SHAPE(K, (row_softmax_reg_kernel<G, R><<<(unsigned)((rows * G + 255) / 256), 256, 0, st>>>(rows, K, s, p, stats)),
+                      (row_softmax_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats)));
     CA_CHECK_LAUNCH("row normalize kernel");
     return CA_OK;
 }
@@ -170,7 +171,8 @@ static int launch_row_normalize_bwd(int64_t rows, int K, int entmax, const float
                                     cudaStream_t st) {
     const int64_t blocks = (rows * 32 + 255) / 256;
     if (blocks > INT32_MAX) { set_error("too many rows"); return CA_ERR_TOO_LARGE; }
-    row_normalize_bwd_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, entmax, p, dp, ds);
+    CA_ROW_SHAPE(K, (row_normalize_bwd_reg_kernel<G, R><<<(unsigned)((rows * G + 255) / 256), 256, 0, st>>>(rows, K, entmax, p, dp, ds)),
+                 (row_normalize_bwd_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, entmax, p, dp, ds)));
     CA_CHECK_LAUNCH("row normalize pullback kernel");
     return CA_OK;
 }
@@ -664,7 +666,8 @@ int ca_sum_rows(const ca_desc* d, const float* nz, float* out, void* stream) {
     if (!nz || !out) { set_error("nz/out is NULL"); return CA_ERR_NULL; }
     const int64_t rows = (int64_t)g.Np * g.units;
     if ((rows * 32 + 255) / 256 > INT32_MAX) { set_error("too many rows"); return CA_ERR_TOO_LARGE; }
-    sum_rows_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, as_stream(stream)>>>(rows, g.K, nz, out);
+    CA_ROW_SHAPE(g.K, (sum_rows_reg_kernel<G, R><<<(unsigned)(((rows + 1) / 2 * G + 255) / 256), 256, 0, as_stream(stream)>>>(rows, g.K, nz, out)),
+                 (sum_rows_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, as_stream(stream)>>>(rows, g.K, nz, out)));
     CA_CHECK_LAUNCH("row sum kernel");
     return CA_OK;
 }
