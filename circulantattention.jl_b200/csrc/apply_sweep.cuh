@@ -1,0 +1,343 @@
+// A (x) V and A^T (x) V on the tiled kernels (compiled by apply_exact.cu and apply_any.cu).
+#include "tile_common.cuh"
+
+namespace ca {
+namespace {
+
+// =====================================================================
+// A (x) V and A^T (x) V from stored values.  The dense operand is streamed as
+// packed column stages exactly like the keys of the forward; the values of A
+// that pair with a stage are, for every centre column r, one run of ws
+// consecutive entries per CSR row (window column fixed, window rows varying),
+// which a warp copies into shared memory before the FMAs that use them:
+//   plain     : the runs of the warp's own rows; lane wr uses entry (e + rotation) of its row at step e;
+//   transposed: the runs of the streamed column's rows hw0 - p .. hw0 + RW - 1 + p; lane wr uses the entry of the
+//               opposite offset of row wr + e (window symmetry: A[j, i] sits in row j at offset i - j).
+// out = alpha * (sum_e a_e v_e - (sum_e a_e) * centre) with centre optional: the
+// second term is the Distance similarity pullback.
+//
+// Staging.  Runs are copied as aligned 16-byte pieces, eight lanes per row.  The misalignment of a run grows by K
+// (odd) modulo four words per row, so a row pitch of 4*C + K % 4 words (C pieces per run) puts the run of row t at
+// word t * pitch + a exactly, a = misalignment of row 0: source and destination of a lane's pieces advance by
+// constants (4 rows each), and the odd pitch makes the lanes' reads conflict free.  (Four-byte copies of
+// single entries took 36 instructions per copy with their address arithmetic: 95 us at 128 x 96 x 64 x 2, ws 15,
+// 4 heads, 41 % of the issue slots busy.)
+//
+// Bound: reading A (4 bytes per entry) and, next to it, 16 FMAs per entry and slab.  One thread per pixel row of
+// four columns is only 768 warps at that size, five per SM, so up to four warps of a CTA share the stages of a tile.
+// FMAs are packed (an outer product: 61 against 50 TFLOP/s in registers).  Measured times stand at run_apply().
+// =====================================================================
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// acc += (a, a) * v on a channel pair as one packed FMA (outer products run at the packed rate: the coefficient pair
+// is reused by consecutive instructions).
+__device__ __forceinline__ void fma_outer(uint64_t& acc, uint64_t a2, uint64_t v) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a2), "l"(v));
+}
+__device__ __forceinline__ uint64_t dup2(float a) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ u64 split2(uint64_t v) {
+    u64 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void lds128p(uint32_t addr, uint64_t& lo, uint64_t& hi) {
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(addr));
+}
+__device__ __forceinline__ float lds32(uint32_t addr) {
+    float x;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(addr));
+    return x;
+}
+
+// 16-byte pieces that cover a run of ws words at any misalignment, and the row pitch in words.  Rows that wrap around
+// an axis whose length is no multiple of four change their misalignment, which takes one more piece of room.
+__host__ __device__ inline int run_pieces(int ws) { return (ws + 6) / 4; }
+__host__ __device__ inline int run_pitch(const Geo& g, bool loose) { return 4 * run_pieces(g.ws) + (loose ? 4 : 0) + (g.K & 3); }
+// Words of one warp's run area: nslots centre columns of `rows` rows.
+__host__ __device__ inline int run_area(const Geo& g, int rows, int nslots, bool loose) { return nslots * ((rows * run_pitch(g, loose) + 8) & ~3); }
+
+// Position of the entry that lane pixel n (coordinate on the window axis of length X) needs from the row of the streamed
+// pixel n - p + e, inside that row's run: the sorted columns of a border row start at the front of the axis, where
+// column n is the n-th entry, and end at its back, where it is the (X - n)-th from the end.
+__device__ __forceinline__ int transposed_pos(int n, int e, int X, int p, int ws) { return max(min(2 * p - e, n), n - X + ws); }
+
+template <int CPE, bool TRANS, int NCRT>
+__global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+                                                             const __grid_constant__ CUtensorMap msc) {
+    constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;             // 16-channel slabs = lanes per pixel
+    constexpr int RW = 32 / NS;                                // pixel rows per warp
+    constexpr int RB = kSingleFloats * 4 * NS;                 // bytes of a packed row of a single tensor
+    const Geo& g = a.g;
+    const int ROWS = a.TH + 2 * (g.p + a.roff);
+    const int pw = radius_w(g), p2 = TRANS ? g.p : 0;
+    const bool fold = g.wsw == 1;                              // folded 1-D signal: rows continue into neighbour columns
+    const int w0 = blockIdx.x * 4, h0 = blockIdx.y * a.TH, u = blockIdx.z;
+    const int NSTAGES = g.wsw + min(3, g.W - 1 - w0);          // no stages for centre columns past the image
+    CA_PIPE_PROLOGUE(false, 4)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slab = lane % NS, lrow = lane / NS;              // this lane's channel slab and row inside the warp
+    const int lr = (lt >> 5) * RW + lrow, h = h0 + lr;         // row inside the tile, image row
+    const bool active = h < g.H;
+    const int X = axis_len(g);
+    const bool loose = TRANS && (X & 3);
+    const int SR = run_pitch(g, loose), C = run_pieces(g.ws);
+    const int NR = RW + (TRANS ? g.ws - 1 : 0);                // staged rows per centre column
+    const int slot_words = run_area(g, NR, 1, loose), buf_words = (fold ? 1 : 4) * slot_words;
+    const uint32_t wbase = smem_u32(smem_al) + (uint32_t)a.nsplit * a.nstages * a.stage_bytes + (uint32_t)warp * a.nbuf * buf_words * 4;
+    const int hw0 = h0 + (lt >> 5) * RW;                       // first image row of this warp
+    const int xs = hw0 - p2;                                   // first staged row (plain: the warp's own)
+    const bool wraps = TRANS && (fold || xs < 0 || xs + NR > g.H);   // a staged row may lie past an end of the axis
+    const float* nzw = a.cs0 + ((int64_t)u * g.Np + xs) * g.K;
+    const int64_t colstep = (int64_t)g.H * g.K;                // words between the same rows of neighbouring columns
+    const float* own = nzw + colstep * w0;                     // plain: centre column 0
+
+    // starts the copies of the runs of stage s into buffer tb; returns the misalignments of staged row 0, two bits per
+    // centre column
+    const int wr0 = lane >> 3, j0 = lane & 7;
+    const int64_t step = 4 * (int64_t)g.K;
+    auto fetch_runs = [&](int s, int tb) {
+        const int mask = stage_mask<4>(s, pw), wc = stage_column(g, w0, s);
+        // staged rows that some pixel of the image needs: the rest of a ragged tile is not copied
+        const int hc = kAnyC && fold ? min(g.H, g.Np - g.H * (w0 + s)) : g.H;
+        const int nrows = hw0 >= hc ? 0 : min(NR, hc - hw0 + 2 * p2);
+        const float* col = TRANS ? nzw + colstep * wc : own;
+        int mis4 = 0;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int posw = TRANS ? axis_pos(r + pw - s, wc, g.W, pw, g.wsw) : axis_pos(s - pw - r, w0 + r, g.W, pw, g.wsw);
+            const float* row0 = col + posw * g.ws;             // run of staged row 0
+            if (!TRANS) col += colstep;
+            if (!((mask >> r) & 1) || w0 + r >= g.W) continue;
+            const int ar = (int)((uintptr_t)row0 >> 2) & 3;
+            mis4 |= ar << (2 * r);
+            const uint32_t slot = wbase + (uint32_t)(tb * buf_words + (fold ? 0 : r) * slot_words) * 4;
+            for (int j = j0; j < C; j += 8) {
+                const int mis = (ar + wr0 * g.K) & 3;          // the same for every fourth row
+                const float* src = row0 + (wr0 * g.K - mis + 4 * j);
+                uint32_t dst = slot + (((wr0 * SR + ar) & ~3) + 4 * j) * 4;
+                const uint32_t dstep = 16 * SR;
+                if (loose && wraps) {
+                    // rows past an end of an axis whose length is no multiple of four: another misalignment
+                    for (int t = wr0; t < nrows; t += 4) {
+                        const int x = xs + t + (fold ? g.H * wc : 0), dx = wrap_axis(x, X) - x;
+                        const int q = t * SR + ((ar + dx * g.K) & 3), m = (ar + (t + dx) * g.K) & 3;
+                        if (4 * j < g.ws + m)                  // else the piece starts past the run
+                            cp_async16(slot + ((q & ~3) + 4 * j) * 4, row0 + (int64_t)(t + dx) * g.K - m + 4 * j);
+                    }
+                    continue;
+                }
+                if (4 * j >= g.ws + mis) continue;
+                if (wraps) {
+                    const int64_t turn = (int64_t)X * g.K;
+                    int x = xs + wr0 + (fold ? g.H * wc : 0);
+                    for (int t = wr0; t < nrows; t += 4) {
+                        cp_async16(dst, src + (x < 0 ? turn : (x >= X ? -turn : 0)));
+                        src += step;
+                        dst += dstep;
+                        x += 4;
+                    }
+                } else {
+#pragma unroll 4
+                    for (int t = wr0; t < nrows; t += 4) {
+                        cp_async16(dst, src);
+                        src += step;
+                        dst += dstep;
+                    }
+                }
+            }
+        }
+        cp_async_commit();
+        return mis4;
+    };
+
+    uint64_t acc[4][8];
+    float asum[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        asum[r] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[r][i] = 0;
+    }
+    int mis4 = 0, mis4_next = 0;
+    if (a.nbuf == 2 && s_begin < s_end) mis4_next = fetch_runs(s_begin, 0);
+
+    CA_PIPE_LOOP(4, {
+        const int mask = stage_mask<4>(s, pw);
+        const uint32_t rowbase = smem_u32(pipe.vec(buf)) + (lr + a.roff) * RB + slab * 16;
+        const int tb = a.nbuf == 2 ? it & 1 : 0;
+        if (a.nbuf == 2) {
+            mis4 = mis4_next;
+            if (s + 1 < s_end) { mis4_next = fetch_runs(s + 1, tb ^ 1); cp_async_wait<1>(); }
+            else cp_async_wait<0>();
+        } else {
+            mis4 = fetch_runs(s, 0);
+            cp_async_wait<0>();
+        }
+        __syncwarp();
+        // shared-space address of this lane's row 0 (transposed: row lrow), per centre column
+        uint32_t pr[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            pr[r] = wbase + (uint32_t)(tb * buf_words + (fold ? 0 : r) * slot_words + lrow * SR + (loose ? 0 : (mis4 >> (2 * r)) & 3)) * 4;
+        // coordinate of this lane's pixel on the window axis (folded: column w0 + s is the one that is on); pixels past
+        // the image take one whose entries all exist
+        const bool here = active && (!kAnyC || !fold || has_pixel(g, h, w0 + s));
+        const int n = !here ? 2 * g.p : (fold ? h + g.H * (w0 + s) : h);
+        const int rot = TRANS || !here ? 0 : run_rot(n, X, g.p, g.ws);
+        auto sweep = [&](auto full_tag, auto loose_tag) {
+            constexpr bool FULL = decltype(full_tag)::value, LOOSE = decltype(loose_tag)::value;
+#pragma unroll 3
+            for (int e = 0; e < g.ws; ++e) {
+                uint64_t v[8];
+                const uint32_t vb = rowbase + e * RB;
+                lds128p(vb, v[0], v[1]);
+                lds128p(vb + 16 * NS, v[2], v[3]);
+                lds128p(vb + 32 * NS, v[4], v[5]);
+                lds128p(vb + 48 * NS, v[6], v[7]);
+                // word of the entry after row lrow's start: the same for the four centre columns, except for the
+                // misalignment of wrapped rows (LOOSE)
+                int off = 0, sh = 0;
+                if (!TRANS) {
+                    off = e + rot;
+                    off -= off >= g.ws ? g.ws : 0;
+                } else {
+                    off = e * SR + transposed_pos(n, e, X, g.p, g.ws);
+                    if (LOOSE) {
+                        const int x = xs + lrow + e + (fold ? g.H * (w0 + s) : 0);
+                        sh = (wrap_axis(x, X) - x) * g.K;
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    if (!FULL && !((mask >> r) & 1)) continue;
+                    const float av = lds32(pr[r] + (uint32_t)(off + (LOOSE ? ((mis4 >> (2 * r)) + sh) & 3 : 0)) * 4);
+                    asum[r] += av;
+                    const uint64_t a2 = dup2(av);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) fma_outer(acc[r][i], a2, v[i]);
+                }
+            }
+        };
+        if (TRANS && loose) {
+            if (mask == 15) sweep(std::true_type{}, std::true_type{});
+            else sweep(std::false_type{}, std::true_type{});
+        } else {
+            if (mask == 15) sweep(std::true_type{}, std::false_type{});
+            else sweep(std::false_type{}, std::false_type{});
+        }
+        __syncwarp();
+    })
+
+    // parts 1.. publish their partial sums, part 0 adds them up
+    if (a.nsplit > 1) {
+        float* xch = reinterpret_cast<float*>(smem_al);
+        if (part > 0) {
+            float* x = xch + (size_t)(part - 1) * 68 * PT + lt;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                x[(64 + r) * PT] = asum[r];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const u64 t = split2(acc[r][i]);
+                    x[(r * 16 + 2 * i) * PT] = t.x;
+                    x[(r * 16 + 2 * i + 1) * PT] = t.y;
+                }
+            }
+        }
+        __syncthreads();
+        if (part > 0) return;
+    }
+    u64 res[4][8];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) res[r][i] = split2(acc[r][i]);
+    for (int q = 1; q < a.nsplit; ++q) {
+        const float* x = reinterpret_cast<float*>(smem_al) + (size_t)(q - 1) * 68 * PT + lt;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            asum[r] += x[(64 + r) * PT];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) res[r][i] = add2(res[r][i], pack2(x[(r * 16 + 2 * i) * PT], x[(r * 16 + 2 * i + 1) * PT]));
+        }
+    }
+    if (a.c0) {
+        u64 ctr[4][8];
+        load_centre<CPE, 4, NCRT>(a.c0, g, u, h, w0, active, 1.f, ctr, 16 * slab);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const u64 ns = pack2(-asum[r], -asum[r]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) res[r][i] = fma2(ns, ctr[r][i], res[r][i]);
+        }
+    }
+    CA_OUT_DISPATCH(
+        _Pragma("unroll")
+        for (int r = 0; r < 4; ++r)
+            _Pragma("unroll")
+            for (int i = 0; i < 8; ++i)
+                store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, a.scale * res[r][i].x + ca_poison,
+                                            a.scale * res[r][i].y + ca_poison, 16 * slab);)
+}
+
+}  // namespace
+
+// Measured, before and after (one thread per pixel row, 4-byte copies with offset tables -> this kernel), per launch:
+// 128 x 96 x 64 x 2, ws 15, 4 heads: plain 124 -> 65 us, transposed 142 -> 97 us (88 MB of values: 14 us at the HBM peak);
+// 320 x 320 x 32 complex, 8 units, ws 7: plain 566 -> 428 us.
+template <>
+int run_apply<kAnyC>(const Geo& g, const Padded& P, const float* nz, const float* packed, const float* centre, float* out,
+                     float alpha, int transposed, cudaStream_t st) {
+    Launch L{};
+    const int ns = slabs_of(g);
+    int rc = CA_OK;
+    const bool loose = transposed && ((g.wsw == 1 ? g.Np : g.H) & 3);
+    const int rows = 32 / ns + (transposed ? g.ws - 1 : 0);
+    auto setup = [&](int nbuf, int max_split, int max_warps) {
+        L = Launch{};
+        rc = prepare(g, P, 4, 68, "CIRCATT_APPLY_WARPS", packed, nullptr, &L, max_split, max_warps, ns, true, 2);
+        L.a.nbuf = nbuf;
+        const size_t words = (size_t)nbuf * run_area(g, rows, g.wsw == 1 ? 1 : 4, loose);
+        const size_t need = (size_t)L.a.nsplit * 2 * L.a.stage_bytes + (size_t)L.threads / 32 * words * sizeof(float) + 1024;
+        if (!rc && need > L.smem) L.smem = need;
+        return rc;
+    };
+    // run buffers of a warp: two when three CTAs still fit on an SM (the registers allow three), else one; wide
+    // windows, whose runs fill the shared memory, run fewer warps per CTA
+    if (setup(2, 4, 4)) return rc;
+    if (3 * (L.smem + 1024) > 227 * 1024 && setup(1, 4, 4)) return rc;
+    for (int split = 2; L.smem > 200 * 1024 && split >= 1; --split)
+        if (setup(1, split, 1)) return rc;
+    if (L.smem > 200 * 1024) {
+        set_error("tiled apply: window %d with %d channels per unit needs %zu bytes of shared memory", g.ws, g.cr, L.smem);
+        return CA_ERR_UNSUPPORTED;
+    }
+    L.a.scale = alpha; L.a.c0 = centre; L.a.cs0 = nz; L.a.o0 = out;
+#define CA_APPLY(NSV)                                                                     \
+    do {                                                                                  \
+        if (g.cpe == 1) {                                                                 \
+            if (transposed) CA_LAUNCH_TILED((apply_tiled_kernel<1, true, NSV>), L, st);   \
+            else CA_LAUNCH_TILED((apply_tiled_kernel<1, false, NSV>), L, st);             \
+        } else {                                                                          \
+            if (transposed) CA_LAUNCH_TILED((apply_tiled_kernel<2, true, NSV>), L, st);   \
+            else CA_LAUNCH_TILED((apply_tiled_kernel<2, false, NSV>), L, st);             \
+        }                                                                                 \
+    } while (0)
+    if (ns == 1) CA_APPLY(16);
+    else if (ns == 2) CA_APPLY(32);
+    else CA_APPLY(64);
+#undef CA_APPLY
+    CA_CHECK_LAUNCH("tiled apply kernel");
+    return CA_OK;
+}
+
+}  // namespace ca

@@ -1,0 +1,3 @@
+// Units of any other channel count up to 64.
+#define CA_ANY_CHANNELS 1
+#include "bwd_sweep.cuh"

@@ -1,0 +1,459 @@
+// Backward sweeps of the tiled kernels and the sweeps of the entmax forward (compiled by bwd_exact.cu and bwd_any.cu; the
+// scheme is described in tiled.cu).
+#include "tile_common.cuh"
+
+namespace ca {
+namespace {
+
+#define CA_MASK_SWITCH(FULL, mask, CALL)                            \
+    if ((mask) == (FULL)) { constexpr int MK = (FULL); CALL; }      \
+    else { constexpr int MK = 0; CALL; }
+
+// =====================================================================
+// Backward, query-owned: dq.  The s chain starts at -L (log2 domain) and the
+// dP chain at -D, so P = 2^chain and dS = P * chain'.
+// =====================================================================
+// MODE 0: softmax, P = 2^chain.  MODE 1: 1.5-entmax, g = max(chain, 0) with the chain = s/2 - tau, dS = g*(dP - D).
+// MODE 2: the entmax pre-pass: only num += g*dP and den += g (in aux and sumds), D = num/den.
+// The same query-owned sweep serves the entmax forward, which has no dy: MODE 3 the row maximum of s/2 (in aux);
+// MODE 4 one step of the threshold search: with t = chain = s/2 - tau, the sum of max(t, 0) (sumds), of its
+// square (aux), the size of the support {t > 0}, its smallest member and the largest t outside (ex[0..2]);
+// MODE 5 the apply: dq (here y) += max(chain, 0)^2 * v.
+template <bool DIST, int MASK, int NQ, int MODE, int NS = 1>
+__device__ __forceinline__ void dq_stage(uint32_t rowbase, int ws, int rm, float sl2, const u64 (&q)[NQ][8],
+                                         const u64 (&dy)[NQ][8], u64 (&dq)[NQ][8], const u64 (&nL2)[NQ],
+                                         const u64 (&nD2)[NQ], const float (&bq)[NQ], float (&sumds)[NQ],
+                                         float (&aux)[NQ], float (&ex)[NQ][3], int slab = 0) {
+#pragma unroll 2      // two keys in flight: the second key's loads overlap the first key's FMAs
+    for (int di = 0; di < ws; ++di) {
+        const uint32_t a0 = rowbase + di * (kRowBytes * NS);
+        float dp[NQ];
+        if (MODE <= 2) {
+            u64 v2[8];
+            lds_slab16<NS>(a0, 1, slab, v2);
+#pragma unroll
+            for (int r = 0; r < NQ; ++r)
+                if (CA_ON(r)) {
+                    u64 t = nD2[r];                               // (-D, 0)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) t = fma2(dy[r][i], v2[i], t);
+                    dp[r] = lane_sum<NS>(hsum2(t));              // -D sits on slab 0 only; rm is warp-uniform
+                }
+        }
+        u64 k2[8];
+        lds_slab16<NS>(a0, 0, slab, k2);
+        float bk = 0.f;
+        if (DIST) {
+            u64 n = zero2();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) n = fma2(k2[i], k2[i], n);
+            bk = -0.5f * sl2 * hsum2(n);
+        }
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+            if (CA_ON(r)) {
+                u64 t = nL2[r];                                   // (-L, 0), log2 domain
+                if (DIST) t = add2(t, pack2(bq[r] + bk, 0.f));
+#pragma unroll
+                for (int i = 0; i < 8; ++i) t = fma2(q[r][i], k2[i], t);
+                const float chain = lane_sum<NS>(hsum2(t));
+                if (MODE == 3) {
+                    aux[r] = fmaxf(aux[r], chain);
+                } else if (MODE == 4) {
+                    const bool in = chain > 0.f;
+                    const float tp = fmaxf(chain, 0.f);
+                    sumds[r] += tp;
+                    aux[r] = fmaf(tp, tp, aux[r]);
+                    ex[r][0] += in ? 1.f : 0.f;
+                    ex[r][1] = fminf(ex[r][1], in ? chain : INFINITY);
+                    ex[r][2] = fmaxf(ex[r][2], in ? -INFINITY : chain);
+                } else if (MODE == 5) {
+                    u64 v2[8];
+                    lds_slab16<NS>(a0, 1, slab, v2);
+                    const float tp = fmaxf(chain, 0.f);
+                    const float w = tp * tp;
+                    const u64 w2 = pack2(w, w);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) dq[r][i] = fma2(w2, v2[i], dq[r][i]);
+                } else if (MODE == 2) {
+                    const float gg = fmaxf(chain, 0.f);
+                    aux[r] = fmaf(gg, dp[r], aux[r]);
+                    sumds[r] += gg;
+                } else {
+                    const float ds = (MODE == 0 ? fast_exp2(chain) : fmaxf(chain, 0.f)) * dp[r];
+                    if (DIST) sumds[r] += ds;
+                    const u64 d2 = pack2(ds, ds);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) dq[r][i] = fma2(d2, k2[i], dq[r][i]);
+                }
+            }
+    }
+}
+
+template <bool DIST, int CPE, int NQ, int MODE, int NCRT = 16>
+__global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dq_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+                                                          const __grid_constant__ CUtensorMap msc) {
+    constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
+    const Geo& g = a.g;
+    const int ROWS = a.TH + 2 * (g.p + a.roff);
+    const int NSTAGES = g.wsw + NQ - 1;
+    const int w0 = blockIdx.x * NQ, h0 = blockIdx.y * a.TH, u = blockIdx.z;
+    const float sl2 = MODE ? 0.5f * a.scale : a.scale * kLog2e;     // entmax: the chain is s/2 - tau
+    bool settled[NQ];                                               // MODE 4: rows whose threshold is final
+    if (MODE == 4) {
+        // a block whose rows all have their final threshold leaves before any barrier or copy exists
+        // (launched without a stage split and for one-slab units: thread = row)
+        const int hh = h0 + (int)threadIdx.x;
+        bool mine = true;
+#pragma unroll
+        for (int r = 0; r < NQ; ++r) {
+            settled[r] = true;
+            if (hh < g.H && has_pixel(g, hh, w0 + r)) settled[r] = __ldg(a.cs1 + (int64_t)u * g.Np + hh + g.H * (w0 + r)) != 0.f;
+            mine = mine && settled[r];
+        }
+        if (__syncthreads_and(mine)) return;
+    }
+    CA_PIPE_PROLOGUE(false, 2)
+    const int slab = NS == 1 ? 0 : (lt % NS);
+    const int lr = NS == 1 ? lt : (lt >> 5) * (32 / NS) + (lt & 31) / NS, h = h0 + lr;
+    const bool active = h < g.H;
+
+    u64 q[NQ][8], dy[NQ][8], dq[NQ][8];
+    load_centre<CPE, NQ, NCRT>(a.c0, g, u, h, w0, active, sl2, q, 16 * slab);
+    if (MODE <= 2) {
+        load_centre<CPE, NQ, NCRT>(a.c1, g, u, h, w0, active, 1.f, dy, 16 * slab);
+    } else {
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) dy[r][i] = zero2();
+    }
+    u64 nL2[NQ], nD2[NQ];
+    float bq[NQ], sumds[NQ], aux[NQ], ex[NQ][3];
+#pragma unroll
+    for (int r = 0; r < NQ; ++r) {
+        const bool ok = active && (has_pixel(g, h, w0 + r)) && slab == 0;       // row scalars enter the lane sums once
+        const int64_t o = (int64_t)u * g.Np + h + g.H * (w0 + r);
+        nL2[r] = pack2((ok && MODE != 3) ? -__ldg(a.cs0 + o) * (MODE ? 1.f : kLog2e) : 0.f, 0.f);
+        nD2[r] = pack2((ok && MODE <= 1) ? -__ldg(a.cs1 + o) : 0.f, 0.f);
+        sumds[r] = 0.f;
+        aux[r] = MODE == 3 ? -INFINITY : 0.f;
+        ex[r][0] = 0.f;
+        ex[r][1] = INFINITY;
+        ex[r][2] = -INFINITY;
+        bq[r] = 0.f;
+        if (DIST) {
+            u64 n = zero2();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) n = fma2(q[r][i], q[r][i], n);
+            bq[r] = -0.5f * hsum2(n) / sl2;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dq[r][i] = zero2();
+    }
+
+    CA_PIPE_LOOP(2, {
+        const int mask = stage_mask<NQ>(s, radius_w(g));
+        CA_MASK_SWITCH(((1 << NQ) - 1), mask, (dq_stage<DIST, MK, NQ, MODE, NS>(smem_u32(pipe.vec(buf)) + (lr + a.roff) * (kRowBytes * NS), g.ws, mask,
+                                                     sl2, q, dy, dq, nL2, nD2, bq, sumds, aux, ex, slab)));
+    })
+
+    if (MODE == 3) {
+        // first threshold of the search: tau >= max - 1 always
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+            if (active && slab == 0 && has_pixel(g, h, w0 + r))
+                a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = aux[r] - 1.f + ca_poison;
+        return;
+    }
+    if (MODE == 4) {
+        // the quadratic sum_S (t - d)^2 = 1 solved on the support S of the current tau; final when tau + d has
+        // the same support and the step was short against the distances it was computed from
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+            if (active && slab == 0 && has_pixel(g, h, w0 + r) && !settled[r]) {
+                const int64_t o = (int64_t)u * g.Np + h + g.H * (w0 + r);
+                const float n = ex[r][0], sa = sumds[r], sb = aux[r];
+                float d = 0.f;
+                bool same = true;
+                if (n > 0.f) {
+                    const float disc = fmaxf(fmaf(sa, sa, -n * (sb - 1.f)), 0.f);
+                    d = (sa - sqrtf(disc)) / n;
+                    same = (d >= 0.f ? d < ex[r][1] : d >= ex[r][2]) && d * n <= 0.5f * sa;
+                    if (!same && a.iter >= 10) d = 0.5f * (sb - 1.f) / sa;     // late steps: Newton on the convex sum
+                }
+                float ntau, zero;
+                unpack2(nL2[r], ntau, zero);
+                a.ostats[o] = d - ntau + ca_poison;
+                a.o1[o] = same ? 1.f : 0.f;
+            }
+        return;
+    }
+    if (MODE == 2) {
+        // pre-pass of the entmax pullback: D = sum g*dP / sum g per query row (launched without a stage split)
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+            if (active && slab == 0 && has_pixel(g, h, w0 + r))
+                a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = (sumds[r] > 0.f ? aux[r] / sumds[r] : 0.f) + ca_poison;
+        return;
+    }
+    if (a.nsplit == 2) {
+        float* xch = reinterpret_cast<float*>(smem_al);
+        if (part == 1) {
+#pragma unroll
+            for (int r = 0; r < NQ; ++r) {
+                xch[(r * 17 + 16) * PT + lt] = sumds[r];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    float x, y;
+                    unpack2(dq[r][i], x, y);
+                    xch[(r * 17 + 2 * i) * PT + lt] = x;
+                    xch[(r * 17 + 2 * i + 1) * PT + lt] = y;
+                }
+            }
+        }
+        __syncthreads();
+        if (part == 1) return;
+#pragma unroll
+        for (int r = 0; r < NQ; ++r) {
+            sumds[r] += xch[(r * 17 + 16) * PT + lt];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                dq[r][i] = add2(dq[r][i], pack2(xch[(r * 17 + 2 * i) * PT + lt], xch[(r * 17 + 2 * i + 1) * PT + lt]));
+        }
+    }
+    // dq = scale * (sum ds*k - [distance] sum(ds) * q);  q registers hold q*scale*log2(e) (entmax: q*scale/2)
+    const float qfac = MODE ? 2.f : kLn2;
+    CA_OUT_DISPATCH(
+        _Pragma("unroll")
+        for (int r = 0; r < NQ; ++r) {
+            _Pragma("unroll")
+            for (int i = 0; i < 8; ++i) {
+                float x, y, qx, qy;
+                unpack2(dq[r][i], x, y);
+                unpack2(q[r][i], qx, qy);
+                if (MODE == 5) {
+                    x += ca_poison;
+                    y += ca_poison;
+                } else {
+                    x = a.scale * x - (DIST ? sumds[r] * qx * qfac : 0.f) + ca_poison;
+                    y = a.scale * y - (DIST ? sumds[r] * qy * qfac : 0.f) + ca_poison;
+                }
+                store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, x, y, 16 * slab);
+            }
+        })
+}
+
+// =====================================================================
+// Backward, key-owned: dk and dv of three key pixels per thread.  The stage
+// rows carry (q | dy) of the query pixels plus their L and D.
+// =====================================================================
+template <bool DIST, int MASK, int NQ, bool ENT, int NS = 1>
+__device__ __forceinline__ void dkdv_stage(uint32_t base, const float* Lb, const float* Db, int row0, int ws, int rm,
+                                           float sl2, const u64 (&k)[NQ][8], const u64 (&v)[NQ][8], u64 (&dk)[NQ][8],
+                                           u64 (&dv)[NQ][8], const float (&bk)[NQ], float (&sumds)[NQ], int slab = 0) {
+#pragma unroll 1
+    for (int di = 0; di < ws; ++di) {
+        const int row = row0 + di;
+        const uint32_t a0 = base + row * (kRowBytes * NS);
+        // the row scalars enter the lane sums once: on slab 0
+        const float nLj = (NS == 1 || slab == 0) ? -Lb[row] : 0.f, nDj = (NS == 1 || slab == 0) ? -Db[row] : 0.f;
+        u64 y2[8];
+        lds_slab16<NS>(a0, 1, slab, y2);
+        float dp[NQ];
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+            if (CA_ON(r)) {
+                u64 t = pack2(nDj, 0.f);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) t = fma2(v[r][i], y2[i], t);
+                dp[r] = lane_sum<NS>(hsum2(t));
+            }
+        u64 q2[8];
+        lds_slab16<NS>(a0, 0, slab, q2);
+        float bqj = 0.f;
+        if (DIST) {
+            u64 n = zero2();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) n = fma2(q2[i], q2[i], n);
+            bqj = -0.5f * sl2 * hsum2(n);
+        }
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+            if (CA_ON(r)) {
+                u64 t = pack2(DIST ? nLj + bk[r] + bqj : nLj, 0.f);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) t = fma2(k[r][i], q2[i], t);
+                const float chain = lane_sum<NS>(hsum2(t));
+                float P, ds;
+                if (!ENT) {
+                    P = fast_exp2(chain);
+                    ds = P * dp[r];
+                } else {                                     // g = max(s/2 - tau, 0): P = g^2, dS = g*(dP - D)
+                    const float gg = fmaxf(chain, 0.f);
+                    P = gg * gg;
+                    ds = gg * dp[r];
+                }
+                if (DIST) sumds[r] += ds;
+                const u64 d2 = pack2(ds, ds), p2 = pack2(P, P);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    dk[r][i] = fma2(d2, q2[i], dk[r][i]);
+                    dv[r][i] = fma2(p2, y2[i], dv[r][i]);
+                }
+            }
+    }
+}
+
+template <bool DIST, int CPE, int NQ, bool ENT, int NCRT = 16>
+__global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dkdv_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+                                                            const __grid_constant__ CUtensorMap msc) {
+    constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
+    const Geo& g = a.g;
+    const int ROWS = a.TH + 2 * (g.p + a.roff);
+    const int NSTAGES = g.wsw + NQ - 1;
+    const int w0 = blockIdx.x * NQ, h0 = blockIdx.y * a.TH, u = blockIdx.z;
+    const float sl2 = ENT ? 0.5f * a.scale : a.scale * kLog2e;      // entmax: the chain is s/2 - tau
+    CA_PIPE_PROLOGUE(true, 2)
+    const int slab = NS == 1 ? 0 : (lt % NS);
+    const int lr = NS == 1 ? lt : (lt >> 5) * (32 / NS) + (lt & 31) / NS, h = h0 + lr;
+    const bool active = h < g.H;
+
+    u64 k[NQ][8], v[NQ][8], dk[NQ][8], dv[NQ][8];
+    load_centre<CPE, NQ, NCRT>(a.c0, g, u, h, w0, active, sl2, k, 16 * slab);
+    load_centre<CPE, NQ, NCRT>(a.c1, g, u, h, w0, active, 1.f, v, 16 * slab);
+    float bk[NQ], sumds[NQ];
+#pragma unroll
+    for (int r = 0; r < NQ; ++r) {
+        sumds[r] = 0.f;
+        bk[r] = 0.f;
+        if (DIST) {
+            u64 n = zero2();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) n = fma2(k[r][i], k[r][i], n);
+            bk[r] = -0.5f * hsum2(n) / sl2;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            dk[r][i] = zero2();
+            dv[r][i] = zero2();
+        }
+    }
+
+    CA_PIPE_LOOP(2, {
+        const int mask = stage_mask<NQ>(s, radius_w(g));
+        CA_MASK_SWITCH(((1 << NQ) - 1), mask, (dkdv_stage<DIST, MK, NQ, ENT, NS>(smem_u32(pipe.vec(buf)), pipe.sc0(buf), pipe.sc1(buf),
+                                                      lr + a.roff, g.ws, mask, sl2, k, v, dk, dv, bk, sumds, slab)));
+    })
+
+    if (a.nsplit == 2) {
+        float* xch = reinterpret_cast<float*>(smem_al);
+        if (part == 1) {
+#pragma unroll
+            for (int r = 0; r < NQ; ++r) {
+                xch[(r * 33 + 32) * PT + lt] = sumds[r];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    float x, y;
+                    unpack2(dk[r][i], x, y);
+                    xch[(r * 33 + 2 * i) * PT + lt] = x;
+                    xch[(r * 33 + 2 * i + 1) * PT + lt] = y;
+                    unpack2(dv[r][i], x, y);
+                    xch[(r * 33 + 16 + 2 * i) * PT + lt] = x;
+                    xch[(r * 33 + 17 + 2 * i) * PT + lt] = y;
+                }
+            }
+        }
+        __syncthreads();
+        if (part == 1) return;
+#pragma unroll
+        for (int r = 0; r < NQ; ++r) {
+            sumds[r] += xch[(r * 33 + 32) * PT + lt];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                dk[r][i] = add2(dk[r][i], pack2(xch[(r * 33 + 2 * i) * PT + lt], xch[(r * 33 + 2 * i + 1) * PT + lt]));
+                dv[r][i] = add2(dv[r][i], pack2(xch[(r * 33 + 16 + 2 * i) * PT + lt], xch[(r * 33 + 17 + 2 * i) * PT + lt]));
+            }
+        }
+    }
+    // dk = scale * (sum ds*q - [distance] sum(ds) * k);  k registers hold k*scale*log2(e)
+    CA_OUT_DISPATCH(
+        _Pragma("unroll")
+        for (int r = 0; r < NQ; ++r) {
+            _Pragma("unroll")
+            for (int i = 0; i < 8; ++i) {
+                float x, y, kx, ky, vx, vy;
+                unpack2(dk[r][i], x, y);
+                unpack2(k[r][i], kx, ky);
+                unpack2(dv[r][i], vx, vy);
+                x = a.scale * x - (DIST ? sumds[r] * kx * (ENT ? 2.f : kLn2) : 0.f) + ca_poison;
+                y = a.scale * y - (DIST ? sumds[r] * ky * (ENT ? 2.f : kLn2) : 0.f) + ca_poison;
+                store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, x, y, 16 * slab);
+                store_centre<CPE, NCRV, BF>(a.o1, g, u, h, w0, active, r, i, vx + ca_poison, vy + ca_poison, 16 * slab);
+            }
+        })
+}
+
+}  // namespace
+
+// The entmax variants exist for four centre pixels per thread and run without a stage split.
+template <>
+int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* dy, const float* stats,
+           const float* D, const float* kv, float* dq, cudaStream_t st, int mode, float* Dout) {
+    Launch L{};
+    const int ns = slabs_of(g);
+    if (ns > 1 && mode) return CA_ERR_UNSUPPORTED;             // the entmax variants exist for one-slab units
+    if (mode >= 3) return CA_ERR_UNSUPPORTED;                  // the forward's sweeps go through run_entmax_fwd_sweep
+    // two query columns per thread measured faster than four at every size for the softmax dq sweep of one-slab
+    // units (160 registers, three blocks per SM, against 255 and two)
+    const int nq = mode ? 4 : (ns > 1 ? (g.ws <= 9 ? 2 : 4) : tune_int("CIRCATT_DQ_NQ", 2));
+    int rc = prepare(g, P, nq, 17 * nq, "CIRCATT_DQ_WARPS", kv, nullptr, &L, mode == 0 && ns == 1 ? 2 : 1, 4, ns);
+    if (rc) return rc;
+    L.a.scale = scale; L.a.c0 = q; L.a.c1 = dy; L.a.cs0 = stats; L.a.cs1 = D; L.a.o0 = dq; L.a.ostats = Dout;
+    if (ns == 2 && nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 32, L, st);
+    else if (ns == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 32, L, st);
+    else if (ns == 4 && nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 64, L, st);
+    else if (ns == 4) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 64, L, st);
+    else if (mode == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 2, 16, L, st);
+    else if (mode == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 1, 16, L, st);
+    else if (nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 16, L, st);
+    else CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 16, L, st);
+    CA_CHECK_LAUNCH("tiled dq kernel");
+    return CA_OK;
+}
+
+template <>
+int run_entmax_fwd_sweep<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* kv,
+                         float* tau, float* settled, float* y, int mode, int iter, cudaStream_t st) {
+    Launch L{};
+    if (slabs_of(g) > 1) return CA_ERR_UNSUPPORTED;
+    int rc = prepare(g, P, 4, 17 * 4, "CIRCATT_DQ_WARPS", kv, nullptr, &L, 1, 4, 1);
+    if (rc) return rc;
+    L.a.scale = scale; L.a.c0 = q; L.a.cs0 = tau; L.a.cs1 = settled; L.a.o0 = y; L.a.o1 = settled; L.a.ostats = tau;
+    L.a.iter = iter;
+    if (mode == 3) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 3, 16, L, st);
+    else if (mode == 4) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 4, 16, L, st);
+    else CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 5, 16, L, st);
+    CA_CHECK_LAUNCH("tiled entmax forward sweep");
+    return CA_OK;
+}
+
+template <>
+int run_dkdv<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* k, const float* v, const float* qdy,
+             const float* planes, float* dk, float* dv, cudaStream_t st, bool entmax) {
+    Launch L{};
+    const int ns = slabs_of(g);
+    if (ns > 1 && entmax) return CA_ERR_UNSUPPORTED;
+    const int nq = 3;
+    int rc = prepare(g, P, nq, 33 * nq, "CIRCATT_DKDV_WARPS", qdy, planes, &L, ns == 1 ? 2 : 1, 4, ns);
+    if (rc) return rc;
+    L.a.scale = scale; L.a.c0 = k; L.a.c1 = v; L.a.o0 = dk; L.a.o1 = dv;
+    if (ns == 2) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 32, L, st);
+    else if (ns == 4) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 64, L, st);
+    else if (entmax) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, true, 16, L, st);
+    else CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 16, L, st);
+    CA_CHECK_LAUNCH("tiled dk/dv kernel");
+    return CA_OK;
+}
+
+}  // namespace ca

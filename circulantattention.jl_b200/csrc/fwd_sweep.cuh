@@ -1,0 +1,340 @@
+// Forward sweep of the tiled kernels (compiled by fwd_exact.cu and fwd_any.cu; the scheme is described in tiled.cu).
+#include "tile_common.cuh"
+
+namespace ca {
+namespace {
+
+// =====================================================================
+// Forward
+// =====================================================================
+// Scores are kept relative to a running reference ref = (largest score seen when
+// the reference was last set) + kHeadroom: the dot-product chain starts at -ref,
+// so sc = s - ref and p = 2^sc needs no subtraction.  The reference moves only
+// when some relative score of the chunk is non-negative (a score jumped more than
+// kHeadroom log2 units above every earlier one), which the AND of the sign bits
+// of the chunk reveals; with O(1) scores that happens almost never after the
+// first key.  2^-kHeadroom only rescales p, l and acc together; it cancels in y.
+constexpr float kHeadroom = 12.f;
+// NS lanes share a pixel (units of 16*NS real channels): every lane holds one 16-channel slab of q and
+// of the accumulator, scores are the lane sums of the per-slab partial dot products, and the terms that
+// enter a score once (the running reference, in nm2) sit on slab 0 only.
+template <int DC, bool DIST, int MASK, int NQ, int NS = 1>
+__device__ __forceinline__ void fwd_stage(uint32_t rowbase, int ws, int rm, float sl2, const u64 (&q)[NQ][8],
+                                          u64 (&acc)[NQ][8], u64 (&nm2)[NQ], float (&l)[NQ], const float (&bq)[NQ],
+                                          int slab = 0) {
+    constexpr int RB = kRowBytes * NS;
+    for (int c0 = 0; c0 < ws; c0 += DC) {
+        const uint32_t cb = rowbase + c0 * RB;
+        float sc[NQ][DC];
+        // one vector ahead: the next key (or the first v) is requested before this key's FMAs
+        u64 nxt[8];
+        lds_slab16<NS>(cb, 0, slab, nxt);
+#pragma unroll
+        for (int t = 0; t < DC; ++t) {
+            {
+                u64 k2[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) k2[i] = nxt[i];
+                if (t + 1 < DC) lds_slab16<NS>(cb + (t + 1) * RB, 0, slab, nxt);
+                else lds_slab16<NS>(cb, 1, slab, nxt);
+                float bk = 0.f;
+                if (DIST) {
+                    u64 n = zero2();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) n = fma2(k2[i], k2[i], n);
+                    bk = -0.5f * sl2 * hsum2(n);
+                }
+                if (MASK != 0) {
+                    // all four chains advance together (4 independent FMAs in flight)
+                    u64 sa[NQ];
+#pragma unroll
+                    for (int r = 0; r < NQ; ++r) {
+                        sa[r] = nm2[r];                           // (-ref, 0)
+                        if (DIST) sa[r] = add2(sa[r], pack2(bq[r] + bk, 0.f));
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int r = 0; r < NQ; ++r) sa[r] = fma2(q[r][i], k2[i], sa[r]);
+#pragma unroll
+                    for (int r = 0; r < NQ; ++r) sc[r][t] = lane_sum<NS>(hsum2(sa[r]));
+                } else {
+#pragma unroll
+                    for (int r = 0; r < NQ; ++r)
+                        if (CA_ON(r)) {
+                            u64 sa = nm2[r];
+                            if (DIST) sa = add2(sa, pack2(bq[r] + bk, 0.f));
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) sa = fma2(q[r][i], k2[i], sa);
+                            sc[r][t] = lane_sum<NS>(hsum2(sa));       // rm is warp-uniform: all lanes shuffle
+                        } else {
+                            sc[r][t] = -INFINITY;
+                        }
+                }
+            }
+        }
+        // any relative score >= 0 ?  (sign bit clear)
+        uint32_t allneg = 0x80000000u;
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+#pragma unroll
+            for (int t = 0; t < DC; ++t) allneg &= __float_as_uint(sc[r][t]);
+        if (__any_sync(0xffffffffu, allneg == 0u)) {
+#pragma unroll
+            for (int r = 0; r < NQ; ++r) {
+                float cm = sc[r][0];
+#pragma unroll
+                for (int t = 1; t < DC; ++t) cm = fmaxf(cm, sc[r][t]);
+                if (cm >= 0.f) {                // move the reference of this row up by cm + headroom
+                    cm += kHeadroom;
+                    const float corr = fast_exp2(-cm);
+                    float nm, zero;
+                    unpack2(nm2[r], nm, zero);
+                    nm2[r] = pack2(nm - (NS == 1 || slab == 0 ? cm : 0.f), 0.f);
+                    l[r] *= corr;
+                    const u64 c2 = pack2(corr, corr);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[r][i] = mul2(acc[r][i], c2);
+#pragma unroll
+                    for (int t = 0; t < DC; ++t) sc[r][t] -= cm;
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < DC; ++t) {
+            {
+                u64 v2[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v2[i] = nxt[i];
+                if (t + 1 < DC) lds_slab16<NS>(cb + (t + 1) * RB, 1, slab, nxt);
+#pragma unroll
+                for (int r = 0; r < NQ; ++r)
+                    if (CA_ON(r)) {
+                        const float pt = fast_exp2(sc[r][t]);
+                        l[r] += pt;
+                        const u64 p2 = pack2(pt, pt);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[r][i] = fma2(p2, v2[i], acc[r][i]);
+                    }
+            }
+        }
+    }
+}
+
+// The ws keys of one window column.  EXACT: ws is a multiple of DC.  Otherwise (DC == 4): chunks of four keys, then
+// the remaining one to three keys as one chunk of exactly that length, so that no chunk carries bounds checks
+// (a checked chunk keeps its prefetched vector alive across branches, which costs a register copy per loaded
+// word and made windows such as 13 slower than 15).
+template <int DC, bool DIST, bool EXACT, int NQ, int NS>
+__device__ __forceinline__ void fwd_window(uint32_t rowbase, int ws, int rm, float sl2, const u64 (&q)[NQ][8],
+                                           u64 (&acc)[NQ][8], u64 (&nm2)[NQ], float (&l)[NQ], const float (&bq)[NQ],
+                                           int slab) {
+    constexpr int FULLM = (1 << NQ) - 1;
+    if (EXACT) {
+        fwd_stage<DC, DIST, FULLM, NQ, NS>(rowbase, ws, rm, sl2, q, acc, nm2, l, bq, slab);
+        return;
+    }
+    static_assert(EXACT || DC == 4, "windows without a dividing chunk length run chunks of four plus a tail");
+    const int main = ws & ~3;
+    fwd_stage<4, DIST, FULLM, NQ, NS>(rowbase, main, rm, sl2, q, acc, nm2, l, bq, slab);
+    const uint32_t tail = rowbase + main * (kRowBytes * NS);
+    switch (ws - main) {                                     // warp-uniform
+        case 1: fwd_stage<1, DIST, FULLM, NQ, NS>(tail, 1, rm, sl2, q, acc, nm2, l, bq, slab); break;
+        case 2: fwd_stage<2, DIST, FULLM, NQ, NS>(tail, 2, rm, sl2, q, acc, nm2, l, bq, slab); break;
+        case 3: fwd_stage<3, DIST, FULLM, NQ, NS>(tail, 3, rm, sl2, q, acc, nm2, l, bq, slab); break;
+        default: break;
+    }
+}
+
+// First score of each centre pixel that starts in this stage: the reference
+// point of its running maximum.
+template <bool DIST, int NQ, int NS = 1>
+__device__ __forceinline__ void fwd_init_max(uint32_t rowbase, int init, float sl2, const u64 (&q)[NQ][8],
+                                             u64 (&nm2)[NQ], const float (&bq)[NQ], int slab = 0) {
+    u64 k2[8];
+    lds_slab16<NS>(rowbase, 0, slab, k2);
+    float bk = 0.f;
+    if (DIST) {
+        u64 n = zero2();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) n = fma2(k2[i], k2[i], n);
+        bk = -0.5f * sl2 * hsum2(n);
+    }
+#pragma unroll
+    for (int r = 0; r < NQ; ++r)
+        if ((init >> r) & 1) {
+            u64 sa = zero2();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sa = fma2(q[r][i], k2[i], sa);
+            const float s0 = lane_sum<NS>(hsum2(sa) + (DIST ? bq[r] + bk : 0.f));     // init is warp-uniform
+            nm2[r] = pack2((NS == 1 || slab == 0) ? -s0 - kHeadroom : 0.f, 0.f);
+        }
+}
+
+// NCRT = real channels per unit the kernel is compiled for: 16 (narrower units are zero-extended),
+// 32 or 64 (NS = 2 or 4 lanes per pixel, one 16-channel slab each; launched without a stage split).
+template <int DC, bool DIST, int CPE, bool EXACT, int NQ, int NCRT = 16>
+__global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) fwd_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+                                                           const __grid_constant__ CUtensorMap msc) {
+    constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
+    constexpr int RB = kRowBytes * NS;
+    const Geo& g = a.g;
+    const int ROWS = a.TH + 2 * (g.p + a.roff);
+    const int NSTAGES = g.wsw + NQ - 1;
+    const int w0 = blockIdx.x * NQ, h0 = blockIdx.y * a.TH, u = blockIdx.z;
+    const float sl2 = a.scale * kLog2e;
+    CA_PIPE_PROLOGUE(false, 2)
+    const int slab = NS == 1 ? 0 : (lt % NS);
+    const int lr = NS == 1 ? lt : (lt >> 5) * (32 / NS) + (lt & 31) / NS, h = h0 + lr;
+    const bool active = h < g.H;
+
+    u64 q[NQ][8], acc[NQ][8];
+    load_centre<CPE, NQ, NCRT>(a.c0, g, u, h, w0, active, sl2, q, 16 * slab);
+    u64 nm2[NQ];
+    float l[NQ], bq[NQ];
+#pragma unroll
+    for (int r = 0; r < NQ; ++r) {
+        nm2[r] = pack2(INFINITY, 0.f);           // (-m, 0); running maximum -inf: no key seen yet
+        l[r] = 0.f;
+        bq[r] = 0.f;
+        if (DIST) {
+            u64 n = zero2();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) n = fma2(q[r][i], q[r][i], n);
+            bq[r] = -0.5f * hsum2(n) / sl2;      // q is pre-scaled by sl2
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[r][i] = zero2();
+    }
+
+    CA_PIPE_LOOP(2, {
+        const int mask = stage_mask<NQ>(s, radius_w(g));
+        const uint32_t rowbase = smem_u32(pipe.vec(buf)) + (lr + a.roff) * RB;
+        // pixels whose first stage (of this part) is s
+        const int init = (s == s_begin) ? mask : (mask & ~stage_mask<NQ>(s - 1, radius_w(g)));
+        if (init) fwd_init_max<DIST, NQ, NS>(rowbase, init, sl2, q, nm2, bq, slab);
+        if (mask != (1 << NQ) - 1) {
+            // a stage that pairs with only some of the columns: the all-slots code (interleaved chains) with the
+            // unpaired slots' scores forced to -inf, so that they contribute exact zeros; measured 6-7 % faster
+            // over a forward than computing the paired slots one after the other
+            u64 nmE[NQ];
+#pragma unroll
+            for (int r = 0; r < NQ; ++r) nmE[r] = ((mask >> r) & 1) ? nm2[r] : pack2(-INFINITY, 0.f);
+            fwd_window<DC, DIST, EXACT, NQ, NS>(rowbase, g.ws, mask, sl2, q, acc, nmE, l, bq, slab);
+#pragma unroll
+            for (int r = 0; r < NQ; ++r)
+                if ((mask >> r) & 1) nm2[r] = nmE[r];
+        } else {
+            fwd_window<DC, DIST, EXACT, NQ, NS>(rowbase, g.ws, mask, sl2, q, acc, nm2, l, bq, slab);
+        }
+    })
+
+    float nm[NQ];
+#pragma unroll
+    for (int r = 0; r < NQ; ++r) {
+        float zero;
+        unpack2(nm2[r], nm[r], zero);
+    }
+    if (a.nsplit == 2) {
+        // merge the two partial softmaxes: part 1 publishes (m, l, acc), part 0 combines
+        float* xch = reinterpret_cast<float*>(smem_al);
+        if (part == 1) {
+#pragma unroll
+            for (int r = 0; r < NQ; ++r) {
+                xch[(r * 18 + 0) * PT + lt] = nm[r];
+                xch[(r * 18 + 1) * PT + lt] = l[r];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    float x, y;
+                    unpack2(acc[r][i], x, y);
+                    xch[(r * 18 + 2 + 2 * i) * PT + lt] = x;
+                    xch[(r * 18 + 3 + 2 * i) * PT + lt] = y;
+                }
+            }
+        }
+        __syncthreads();
+        if (part == 1) return;
+#pragma unroll
+        for (int r = 0; r < NQ; ++r) {
+            const float nm1 = xch[(r * 18 + 0) * PT + lt], l1 = xch[(r * 18 + 1) * PT + lt];
+            const float nmn = fminf(nm[r], nm1);           // -max(m0, m1)
+            const float c0 = (nm[r] == INFINITY) ? 0.f : fast_exp2(nmn - nm[r]);
+            const float c1 = (nm1 == INFINITY) ? 0.f : fast_exp2(nmn - nm1);
+            l[r] = l[r] * c0 + l1 * c1;
+            nm[r] = nmn;
+            const u64 c02 = pack2(c0, c0), c12 = pack2(c1, c1);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const u64 o = pack2(xch[(r * 18 + 2 + 2 * i) * PT + lt], xch[(r * 18 + 3 + 2 * i) * PT + lt]);
+                acc[r][i] = fma2(o, c12, mul2(acc[r][i], c02));
+            }
+        }
+    }
+    CA_OUT_DISPATCH(
+        _Pragma("unroll")
+        for (int r = 0; r < NQ; ++r) {
+            const float inv = 1.f / l[r] + ca_poison;
+            _Pragma("unroll")
+            for (int i = 0; i < 8; ++i) {
+                float x, y;
+                unpack2(acc[r][i], x, y);
+                store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, x * inv, y * inv, 16 * slab);
+            }
+        })
+#pragma unroll
+    for (int r = 0; r < NQ; ++r)
+        if (a.ostats && active && slab == 0 && has_pixel(g, h, w0 + r))
+            a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = (log2f(l[r]) - nm[r]) * kLn2 + ca_poison;
+}
+
+}  // namespace
+
+template <>
+int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* kv, float* y, float* stats,
+                   cudaStream_t st) {
+    Launch L{};
+    const int ns = slabs_of(g);
+    // four columns per thread, or two when the grid is small or the window is short (with ws <= 9 most
+    // stages of a four-column tile pair with only some of its columns: measured 18 % faster at ws 7)
+    const int nq = g.ws <= 9 ? tune_int("CIRCATT_FWD_NQ", 2) : (ns > 1 ? 4 : pick_nq(g, 4, 2, "CIRCATT_FWD_NQ"));
+    int rc = prepare(g, P, nq, 18 * nq, "CIRCATT_FWD_WARPS", kv, nullptr, &L, ns == 1 ? 2 : 1, 4, ns);
+    if (rc) return rc;
+    L.a.scale = scale; L.a.c0 = q; L.a.o0 = y; L.a.ostats = stats;
+#define CA_FWD2(DCV, EX, NQV, NCRV_)                                                            \
+    do {                                                                                 \
+        if (g.cpe == 1) {                                                                \
+            if (dist) CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, true, 1, EX, NQV, NCRV_>), L, st); \
+            else CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, false, 1, EX, NQV, NCRV_>), L, st);     \
+        } else {                                                                         \
+            if (dist) CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, true, 2, EX, NQV, NCRV_>), L, st); \
+            else CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, false, 2, EX, NQV, NCRV_>), L, st);     \
+        }                                                                                \
+    } while (0)
+#define CA_FWD(DCV)                                                                      \
+    do {                                                                                 \
+        if (nq == 2) CA_FWD2(DCV, true, 2, 16);                                          \
+        else CA_FWD2(DCV, true, 4, 16);                                                  \
+    } while (0)
+    // wide units: chunks of 7 or 5 keys where they divide the window, else chunks of four plus a tail
+    if (ns == 2 && nq == 2 && g.ws % 7 == 0) CA_FWD2(7, true, 2, 32);
+    else if (ns == 4 && nq == 2 && g.ws % 7 == 0) CA_FWD2(7, true, 2, 64);
+    else if (ns == 2 && nq == 4 && g.ws % 7 == 0) CA_FWD2(7, true, 4, 32);       // windows 21, 35, 49, 63
+    else if (ns == 4 && nq == 4 && g.ws % 7 == 0) CA_FWD2(7, true, 4, 64);
+    else if (ns == 2 && nq == 4 && g.ws % 5 == 0) CA_FWD2(5, true, 4, 32);       // windows 15, 25, 45, 55
+    else if (ns == 4 && nq == 4 && g.ws % 5 == 0) CA_FWD2(5, true, 4, 64);
+    else if (ns == 2 && nq == 2) CA_FWD2(4, false, 2, 32);
+    else if (ns == 2) CA_FWD2(4, false, 4, 32);
+    else if (ns == 4 && nq == 2) CA_FWD2(4, false, 2, 64);
+    else if (ns == 4) CA_FWD2(4, false, 4, 64);
+    else if (g.ws % 7 == 0) CA_FWD(7);
+    else if (g.ws % 5 == 0) CA_FWD(5);
+    else if (g.ws % 3 == 0) CA_FWD(3);
+    else if (nq == 2) CA_FWD2(4, false, 2, 16);
+    else CA_FWD2(4, false, 4, 16);
+#undef CA_FWD2
+#undef CA_FWD
+    CA_CHECK_LAUNCH("tiled forward kernel");
+    return CA_OK;
+}
+
+}  // namespace ca
