@@ -24,7 +24,7 @@ __device__ __forceinline__ void dq_stage(uint32_t rowbase, int ws, int rm, float
                                          const u64 (&dy)[NQ][8], u64 (&dq)[NQ][8], const u64 (&nL2)[NQ],
                                          const u64 (&nD2)[NQ], const float (&bq)[NQ], float (&sumds)[NQ],
                                          float (&aux)[NQ], float (&ex)[NQ][3], int slab = 0) {
-#pragma unroll 2      // two keys in flight: the second key's loads overlap the first key's FMAs
+#pragma unroll (NQ == 1 ? 4 : 2)      // keys in flight: the next key's loads overlap this key's FMAs
     for (int di = 0; di < ws; ++di) {
         const uint32_t a0 = rowbase + di * (kRowBytes * NS);
         float dp[NQ];
@@ -91,7 +91,7 @@ __device__ __forceinline__ void dq_stage(uint32_t rowbase, int ws, int rm, float
 }
 
 template <bool DIST, int CPE, int NQ, int MODE, int NCRT = 16>
-__global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dq_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+__global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) dq_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
                                                           const __grid_constant__ CUtensorMap msc) {
     constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
     const Geo& g = a.g;
@@ -252,7 +252,7 @@ template <bool DIST, int MASK, int NQ, bool ENT, int NS = 1>
 __device__ __forceinline__ void dkdv_stage(uint32_t base, const float* Lb, const float* Db, int row0, int ws, int rm,
                                            float sl2, const u64 (&k)[NQ][8], const u64 (&v)[NQ][8], u64 (&dk)[NQ][8],
                                            u64 (&dv)[NQ][8], const float (&bk)[NQ], float (&sumds)[NQ], int slab = 0) {
-#pragma unroll 1
+#pragma unroll (NQ == 1 ? 2 : 1)
     for (int di = 0; di < ws; ++di) {
         const int row = row0 + di;
         const uint32_t a0 = base + row * (kRowBytes * NS);
@@ -306,7 +306,7 @@ __device__ __forceinline__ void dkdv_stage(uint32_t base, const float* Lb, const
 }
 
 template <bool DIST, int CPE, int NQ, bool ENT, int NCRT = 16>
-__global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) dkdv_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+__global__ void __launch_bounds__(128, (NQ == 1 ? 4 : NQ == 2 ? 3 : 2)) dkdv_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
                                                             const __grid_constant__ CUtensorMap msc) {
     constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
     const Geo& g = a.g;
@@ -406,11 +406,16 @@ int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const fl
     if (mode >= 3) return CA_ERR_UNSUPPORTED;                  // the forward's sweeps go through run_entmax_fwd_sweep
     // two query columns per thread measured faster than four at every size for the softmax dq sweep of one-slab
     // units (160 registers, three blocks per SM, against 255 and two)
-    const int nq = mode ? 4 : (ns > 1 ? (g.ws <= 9 ? 2 : 4) : tune_int("CIRCATT_DQ_NQ", 2));
-    int rc = prepare(g, P, nq, 17 * nq, "CIRCATT_DQ_WARPS", kv, nullptr, &L, mode == 0 && ns == 1 ? 2 : 1, 4, ns);
+    // (folded signals: one, see run_fwd)
+    const bool fold = g.wsw == 1 && mode == 0;
+    const int nq = fold ? 1 : (mode ? 4 : (ns > 1 ? (g.ws <= 9 ? 2 : 4) : tune_int("CIRCATT_DQ_NQ", 2)));
+    int rc = prepare(g, P, nq, 17 * nq, "CIRCATT_DQ_WARPS", kv, nullptr, &L, mode == 0 && ns == 1 && !fold ? 2 : 1, 4, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.c1 = dy; L.a.cs0 = stats; L.a.cs1 = D; L.a.o0 = dq; L.a.ostats = Dout;
-    if (ns == 2 && nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 32, L, st);
+    if (fold && ns == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 1, 0, 16, L, st);
+    else if (fold && ns == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 1, 0, 32, L, st);
+    else if (fold) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 1, 0, 64, L, st);
+    else if (ns == 2 && nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 32, L, st);
     else if (ns == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 32, L, st);
     else if (ns == 4 && nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 64, L, st);
     else if (ns == 4) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 64, L, st);
@@ -444,11 +449,15 @@ int run_dkdv<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const 
     Launch L{};
     const int ns = slabs_of(g);
     if (ns > 1 && entmax) return CA_ERR_UNSUPPORTED;
-    const int nq = 3;
-    int rc = prepare(g, P, nq, 33 * nq, "CIRCATT_DKDV_WARPS", qdy, planes, &L, ns == 1 ? 2 : 1, 4, ns);
+    const bool fold = g.wsw == 1 && !entmax;
+    const int nq = fold ? 1 : 3;
+    int rc = prepare(g, P, nq, 33 * nq, "CIRCATT_DKDV_WARPS", qdy, planes, &L, ns == 1 && !fold ? 2 : 1, 4, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = k; L.a.c1 = v; L.a.o0 = dk; L.a.o1 = dv;
-    if (ns == 2) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 32, L, st);
+    if (fold && ns == 1) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 1, false, 16, L, st);
+    else if (fold && ns == 2) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 1, false, 32, L, st);
+    else if (fold) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 1, false, 64, L, st);
+    else if (ns == 2) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 32, L, st);
     else if (ns == 4) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 64, L, st);
     else if (entmax) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, true, 16, L, st);
     else CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 16, L, st);

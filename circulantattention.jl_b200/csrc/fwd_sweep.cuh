@@ -174,7 +174,7 @@ __device__ __forceinline__ void fwd_init_max(uint32_t rowbase, int init, float s
 // NCRT = real channels per unit the kernel is compiled for: 16 (narrower units are zero-extended),
 // 32 or 64 (NS = 2 or 4 lanes per pixel, one 16-channel slab each; launched without a stage split).
 template <int DC, bool DIST, int CPE, bool EXACT, int NQ, int NCRT = 16>
-__global__ void __launch_bounds__(128, (NQ <= 2 ? 3 : 2)) fwd_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+__global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) fwd_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
                                                            const __grid_constant__ CUtensorMap msc) {
     constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
     constexpr int RB = kRowBytes * NS;
@@ -296,8 +296,11 @@ int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const f
     const int ns = slabs_of(g);
     // four columns per thread, or two when the grid is small or the window is short (with ws <= 9 most
     // stages of a four-column tile pair with only some of its columns: measured 18 % faster at ws 7)
-    const int nq = g.ws <= 9 ? tune_int("CIRCATT_FWD_NQ", 2) : (ns > 1 ? 4 : pick_nq(g, 4, 2, "CIRCATT_FWD_NQ"));
-    int rc = prepare(g, P, nq, 18 * nq, "CIRCATT_FWD_WARPS", kv, nullptr, &L, ns == 1 ? 2 : 1, 4, ns);
+    // a folded signal has one column per thread: a streamed column pairs with one centre column only, and a wider tile
+    // computes the others for nothing (8192 x 64 x 4, ws 63, 64 channels: 92 us, see below)
+    const bool fold = g.wsw == 1;
+    const int nq = fold ? 1 : (g.ws <= 9 ? tune_int("CIRCATT_FWD_NQ", 2) : (ns > 1 ? 4 : pick_nq(g, 4, 2, "CIRCATT_FWD_NQ")));
+    int rc = prepare(g, P, nq, 18 * nq, "CIRCATT_FWD_WARPS", kv, nullptr, &L, ns == 1 && !fold ? 2 : 1, 4, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.o0 = y; L.a.ostats = stats;
 #define CA_FWD2(DCV, EX, NQV, NCRV_)                                                            \
@@ -315,8 +318,17 @@ int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const f
         if (nq == 2) CA_FWD2(DCV, true, 2, 16);                                          \
         else CA_FWD2(DCV, true, 4, 16);                                                  \
     } while (0)
-    // wide units: chunks of 7 or 5 keys where they divide the window, else chunks of four plus a tail
-    if (ns == 2 && nq == 2 && g.ws % 7 == 0) CA_FWD2(7, true, 2, 32);
+    // chunks of 7 or 5 keys where they divide the window, else chunks of four plus a tail
+#define CA_FWD_FOLD(NCRV_)                                                               \
+    do {                                                                                 \
+        if (g.ws % 7 == 0) CA_FWD2(7, true, 1, NCRV_);                                   \
+        else if (g.ws % 5 == 0) CA_FWD2(5, true, 1, NCRV_);                              \
+        else CA_FWD2(4, false, 1, NCRV_);                                                \
+    } while (0)
+    if (fold && ns == 1) CA_FWD_FOLD(16);
+    else if (fold && ns == 2) CA_FWD_FOLD(32);
+    else if (fold) CA_FWD_FOLD(64);
+    else if (ns == 2 && nq == 2 && g.ws % 7 == 0) CA_FWD2(7, true, 2, 32);
     else if (ns == 4 && nq == 2 && g.ws % 7 == 0) CA_FWD2(7, true, 2, 64);
     else if (ns == 2 && nq == 4 && g.ws % 7 == 0) CA_FWD2(7, true, 4, 32);       // windows 21, 35, 49, 63
     else if (ns == 4 && nq == 4 && g.ws % 7 == 0) CA_FWD2(7, true, 4, 64);
@@ -331,6 +343,7 @@ int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const f
     else if (g.ws % 3 == 0) CA_FWD(3);
     else if (nq == 2) CA_FWD2(4, false, 2, 16);
     else CA_FWD2(4, false, 4, 16);
+#undef CA_FWD_FOLD
 #undef CA_FWD2
 #undef CA_FWD
     CA_CHECK_LAUNCH("tiled forward kernel");
