@@ -630,7 +630,7 @@ int ca_scale_batch(int64_t inner, int32_t o1, int32_t o2, const float* a, int32_
     if (!a || !c || !out) { set_error("a/c/out is NULL"); return CA_ERR_NULL; }
     int rc;
     if ((rc = check_bcast("values", a1, a2, o1, o2)) || (rc = check_bcast("scale", c1, c2, o1, o2))) return rc;
-    dim3 grid(elementwise_grid(inner), o1, o2);
+    dim3 grid(elementwise_grid((inner + kScaleRun - 1) / kScaleRun), o1, o2);
     scale_batch_kernel<<<grid, 256, 0, as_stream(stream)>>>(inner, o1, o2, a, a1, a2, c, c1, c2, out);
     CA_CHECK_LAUNCH("scale kernel");
     return CA_OK;

@@ -70,8 +70,9 @@ __host__ __device__ inline int run_area(const Geo& g, int rows, int nslots, bool
 // column n is the n-th entry, and end at its back, where it is the (X - n)-th from the end.
 __device__ __forceinline__ int transposed_pos(int n, int e, int X, int p, int ws) { return max(min(2 * p - e, n), n - X + ws); }
 
-template <int CPE, bool TRANS, int NCRT>
-__global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+// NQ = centre columns per thread (1: folded signals).
+template <int CPE, bool TRANS, int NQ, int NCRT>
+__global__ void __launch_bounds__(128, (NQ == 1 ? 6 : 4)) apply_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
                                                              const __grid_constant__ CUtensorMap msc) {
     constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;             // 16-channel slabs = lanes per pixel
     constexpr int RW = 32 / NS;                                // pixel rows per warp
@@ -79,9 +80,9 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
     const Geo& g = a.g;
     const int ROWS = a.TH + 2 * (g.p + a.roff);
     const int pw = radius_w(g), p2 = TRANS ? g.p : 0;
-    const bool fold = g.wsw == 1;                              // folded 1-D signal: rows continue into neighbour columns
-    const int w0 = blockIdx.x * 4, h0 = blockIdx.y * a.TH, u = blockIdx.z;
-    const int NSTAGES = g.wsw + min(3, g.W - 1 - w0);          // no stages for centre columns past the image
+    const bool fold = NQ == 1;                                 // folded 1-D signal: rows continue into neighbour columns
+    const int w0 = blockIdx.x * NQ, h0 = blockIdx.y * a.TH, u = blockIdx.z;
+    const int NSTAGES = g.wsw + min(NQ - 1, g.W - 1 - w0);          // no stages for centre columns past the image
     CA_PIPE_PROLOGUE(false, 4)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int slab = lane % NS, lrow = lane / NS;              // this lane's channel slab and row inside the warp
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
     const bool loose = TRANS && (X & 3);
     const int SR = run_pitch(g, loose), C = run_pieces(g.ws);
     const int NR = RW + (TRANS ? g.ws - 1 : 0);                // staged rows per centre column
-    const int slot_words = run_area(g, NR, 1, loose), buf_words = (fold ? 1 : 4) * slot_words;
+    const int slot_words = run_area(g, NR, 1, loose), buf_words = NQ * slot_words;
     const uint32_t wbase = smem_u32(smem_al) + (uint32_t)a.nsplit * a.nstages * a.stage_bytes + (uint32_t)warp * a.nbuf * buf_words * 4;
     const int hw0 = h0 + (lt >> 5) * RW;                       // first image row of this warp
     const int xs = hw0 - p2;                                   // first staged row (plain: the warp's own)
@@ -105,21 +106,21 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
     const int wr0 = lane >> 3, j0 = lane & 7;
     const int64_t step = 4 * (int64_t)g.K;
     auto fetch_runs = [&](int s, int tb) {
-        const int mask = stage_mask<4>(s, pw), wc = stage_column(g, w0, s);
+        const int mask = stage_mask<NQ>(s, pw), wc = stage_column(g, w0, s);
         // staged rows that some pixel of the image needs: the rest of a ragged tile is not copied
         const int hc = kAnyC && fold ? min(g.H, g.Np - g.H * (w0 + s)) : g.H;
         const int nrows = hw0 >= hc ? 0 : min(NR, hc - hw0 + 2 * p2);
         const float* col = TRANS ? nzw + colstep * wc : own;
         int mis4 = 0;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int r = 0; r < NQ; ++r) {
             const int posw = TRANS ? axis_pos(r + pw - s, wc, g.W, pw, g.wsw) : axis_pos(s - pw - r, w0 + r, g.W, pw, g.wsw);
             const float* row0 = col + posw * g.ws;             // run of staged row 0
             if (!TRANS) col += colstep;
             if (!((mask >> r) & 1) || w0 + r >= g.W) continue;
             const int ar = (int)((uintptr_t)row0 >> 2) & 3;
             mis4 |= ar << (2 * r);
-            const uint32_t slot = wbase + (uint32_t)(tb * buf_words + (fold ? 0 : r) * slot_words) * 4;
+            const uint32_t slot = wbase + (uint32_t)(tb * buf_words + r * slot_words) * 4;
             for (int j = j0; j < C; j += 8) {
                 const int mis = (ar + wr0 * g.K) & 3;          // the same for every fourth row
                 const float* src = row0 + (wr0 * g.K - mis + 4 * j);
@@ -159,10 +160,10 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
         return mis4;
     };
 
-    uint64_t acc[4][8];
-    float asum[4];
+    uint64_t acc[NQ][8];
+    float asum[NQ];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < NQ; ++r) {
         asum[r] = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[r][i] = 0;
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
     if (a.nbuf == 2 && s_begin < s_end) mis4_next = fetch_runs(s_begin, 0);
 
     CA_PIPE_LOOP(4, {
-        const int mask = stage_mask<4>(s, pw);
+        const int mask = stage_mask<NQ>(s, pw);
         const uint32_t rowbase = smem_u32(pipe.vec(buf)) + (lr + a.roff) * RB + slab * 16;
         const int tb = a.nbuf == 2 ? it & 1 : 0;
         if (a.nbuf == 2) {
@@ -184,10 +185,10 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
         }
         __syncwarp();
         // shared-space address of this lane's row 0 (transposed: row lrow), per centre column
-        uint32_t pr[4];
+        uint32_t pr[NQ];
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-            pr[r] = wbase + (uint32_t)(tb * buf_words + (fold ? 0 : r) * slot_words + lrow * SR + (loose ? 0 : (mis4 >> (2 * r)) & 3)) * 4;
+        for (int r = 0; r < NQ; ++r)
+            pr[r] = wbase + (uint32_t)(tb * buf_words + r * slot_words + lrow * SR + (loose ? 0 : (mis4 >> (2 * r)) & 3)) * 4;
         // coordinate of this lane's pixel on the window axis (folded: column w0 + s is the one that is on); pixels past
         // the image take one whose entries all exist
         const bool here = active && (!kAnyC || !fold || has_pixel(g, h, w0 + s));
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
         const int rot = TRANS || !here ? 0 : run_rot(n, X, g.p, g.ws);
         auto sweep = [&](auto full_tag, auto loose_tag) {
             constexpr bool FULL = decltype(full_tag)::value, LOOSE = decltype(loose_tag)::value;
-#pragma unroll 3
+#pragma unroll (NQ == 1 ? 4 : 3)
             for (int e = 0; e < g.ws; ++e) {
                 uint64_t v[8];
                 const uint32_t vb = rowbase + e * RB;
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
                 lds128p(vb + 16 * NS, v[2], v[3]);
                 lds128p(vb + 32 * NS, v[4], v[5]);
                 lds128p(vb + 48 * NS, v[6], v[7]);
-                // word of the entry after row lrow's start: the same for the four centre columns, except for the
+                // word of the entry after row lrow's start: the same for all centre columns, except for the
                 // misalignment of wrapped rows (LOOSE)
                 int off = 0, sh = 0;
                 if (!TRANS) {
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
                     }
                 }
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
+                for (int r = 0; r < NQ; ++r) {
                     if (!FULL && !((mask >> r) & 1)) continue;
                     const float av = lds32(pr[r] + (uint32_t)(off + (LOOSE ? ((mis4 >> (2 * r)) + sh) & 3 : 0)) * 4);
                     asum[r] += av;
@@ -228,10 +229,10 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
             }
         };
         if (TRANS && loose) {
-            if (mask == 15) sweep(std::true_type{}, std::true_type{});
+            if (mask == (1 << NQ) - 1) sweep(std::true_type{}, std::true_type{});
             else sweep(std::false_type{}, std::true_type{});
         } else {
-            if (mask == 15) sweep(std::true_type{}, std::false_type{});
+            if (mask == (1 << NQ) - 1) sweep(std::true_type{}, std::false_type{});
             else sweep(std::false_type{}, std::false_type{});
         }
         __syncwarp();
@@ -241,10 +242,10 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
     if (a.nsplit > 1) {
         float* xch = reinterpret_cast<float*>(smem_al);
         if (part > 0) {
-            float* x = xch + (size_t)(part - 1) * 68 * PT + lt;
+            float* x = xch + (size_t)(part - 1) * (17 * NQ) * PT + lt;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                x[(64 + r) * PT] = asum[r];
+            for (int r = 0; r < NQ; ++r) {
+                x[(16 * NQ + r) * PT] = asum[r];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const u64 t = split2(acc[r][i]);
@@ -256,25 +257,25 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
         __syncthreads();
         if (part > 0) return;
     }
-    u64 res[4][8];
+    u64 res[NQ][8];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < NQ; ++r)
 #pragma unroll
         for (int i = 0; i < 8; ++i) res[r][i] = split2(acc[r][i]);
     for (int q = 1; q < a.nsplit; ++q) {
-        const float* x = reinterpret_cast<float*>(smem_al) + (size_t)(q - 1) * 68 * PT + lt;
+        const float* x = reinterpret_cast<float*>(smem_al) + (size_t)(q - 1) * (17 * NQ) * PT + lt;
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            asum[r] += x[(64 + r) * PT];
+        for (int r = 0; r < NQ; ++r) {
+            asum[r] += x[(16 * NQ + r) * PT];
 #pragma unroll
             for (int i = 0; i < 8; ++i) res[r][i] = add2(res[r][i], pack2(x[(r * 16 + 2 * i) * PT], x[(r * 16 + 2 * i + 1) * PT]));
         }
     }
     if (a.c0) {
-        u64 ctr[4][8];
-        load_centre<CPE, 4, NCRT>(a.c0, g, u, h, w0, active, 1.f, ctr, 16 * slab);
+        u64 ctr[NQ][8];
+        load_centre<CPE, NQ, NCRT>(a.c0, g, u, h, w0, active, 1.f, ctr, 16 * slab);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
+        for (int r = 0; r < NQ; ++r) {
             const u64 ns = pack2(-asum[r], -asum[r]);
 #pragma unroll
             for (int i = 0; i < 8; ++i) res[r][i] = fma2(ns, ctr[r][i], res[r][i]);
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
     }
     CA_OUT_DISPATCH(
         _Pragma("unroll")
-        for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < NQ; ++r)
             _Pragma("unroll")
             for (int i = 0; i < 8; ++i)
                 store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, a.scale * res[r][i].x + ca_poison,
@@ -292,8 +293,9 @@ __global__ void __launch_bounds__(128, 3) apply_tiled_kernel(TileArgs a, const _
 }  // namespace
 
 // Measured, before and after (one thread per pixel row, 4-byte copies with offset tables -> this kernel), per launch:
-// 128 x 96 x 64 x 2, ws 15, 4 heads: plain 124 -> 65 us, transposed 142 -> 97 us (88 MB of values: 14 us at the HBM peak);
-// 320 x 320 x 32 complex, 8 units, ws 7: plain 566 -> 428 us.
+// 128 x 96 x 64 x 2, ws 15, 4 heads: plain 124 -> 58 us, transposed 142 -> 72 us (88 MB of values: 14 us at the HBM peak);
+// 320 x 320 x 32 complex, 8 units, ws 7: plain 566 -> 382 us.  Four columns per thread (162 registers, three CTAs per SM)
+// against two: 62 / 94 us and 412 us.
 template <>
 int run_apply<kAnyC>(const Geo& g, const Padded& P, const float* nz, const float* packed, const float* centre, float* out,
                      float alpha, int transposed, cudaStream_t st) {
@@ -302,19 +304,21 @@ int run_apply<kAnyC>(const Geo& g, const Padded& P, const float* nz, const float
     int rc = CA_OK;
     const bool loose = transposed && ((g.wsw == 1 ? g.Np : g.H) & 3);
     const int rows = 32 / ns + (transposed ? g.ws - 1 : 0);
+    const int nq = g.wsw == 1 ? 1 : 2;
+    const size_t most = nq == 1 ? 6 : 4;                     // CTAs per SM that the registers allow
     auto setup = [&](int nbuf, int max_split, int max_warps) {
         L = Launch{};
-        rc = prepare(g, P, 4, 68, "CIRCATT_APPLY_WARPS", packed, nullptr, &L, max_split, max_warps, ns, true, 2);
+        rc = prepare(g, P, nq, 17 * nq, "CIRCATT_APPLY_WARPS", packed, nullptr, &L, nq == 1 ? 1 : max_split, max_warps, ns, true, 2);
         L.a.nbuf = nbuf;
-        const size_t words = (size_t)nbuf * run_area(g, rows, g.wsw == 1 ? 1 : 4, loose);
+        const size_t words = (size_t)nbuf * run_area(g, rows, nq, loose);
         const size_t need = (size_t)L.a.nsplit * 2 * L.a.stage_bytes + (size_t)L.threads / 32 * words * sizeof(float) + 1024;
         if (!rc && need > L.smem) L.smem = need;
         return rc;
     };
-    // run buffers of a warp: two when three CTAs still fit on an SM (the registers allow three), else one; wide
+    // run buffers of a warp: two when as many CTAs still fit on an SM as the registers allow, else one; wide
     // windows, whose runs fill the shared memory, run fewer warps per CTA
     if (setup(2, 4, 4)) return rc;
-    if (3 * (L.smem + 1024) > 227 * 1024 && setup(1, 4, 4)) return rc;
+    if (most * (L.smem + 1024) > 227 * 1024 && setup(1, 4, 4)) return rc;
     for (int split = 2; L.smem > 200 * 1024 && split >= 1; --split)
         if (setup(1, split, 1)) return rc;
     if (L.smem > 200 * 1024) {
@@ -322,19 +326,25 @@ int run_apply<kAnyC>(const Geo& g, const Padded& P, const float* nz, const float
         return CA_ERR_UNSUPPORTED;
     }
     L.a.scale = alpha; L.a.c0 = centre; L.a.cs0 = nz; L.a.o0 = out;
-#define CA_APPLY(NSV)                                                                     \
+#define CA_APPLY(NQV, NSV)                                                                     \
     do {                                                                                  \
         if (g.cpe == 1) {                                                                 \
-            if (transposed) CA_LAUNCH_TILED((apply_tiled_kernel<1, true, NSV>), L, st);   \
-            else CA_LAUNCH_TILED((apply_tiled_kernel<1, false, NSV>), L, st);             \
+            if (transposed) CA_LAUNCH_TILED((apply_tiled_kernel<1, true, NQV, NSV>), L, st);   \
+            else CA_LAUNCH_TILED((apply_tiled_kernel<1, false, NQV, NSV>), L, st);             \
         } else {                                                                          \
-            if (transposed) CA_LAUNCH_TILED((apply_tiled_kernel<2, true, NSV>), L, st);   \
-            else CA_LAUNCH_TILED((apply_tiled_kernel<2, false, NSV>), L, st);             \
+            if (transposed) CA_LAUNCH_TILED((apply_tiled_kernel<2, true, NQV, NSV>), L, st);   \
+            else CA_LAUNCH_TILED((apply_tiled_kernel<2, false, NQV, NSV>), L, st);             \
         }                                                                                 \
     } while (0)
-    if (ns == 1) CA_APPLY(16);
-    else if (ns == 2) CA_APPLY(32);
-    else CA_APPLY(64);
+#define CA_APPLY_NQ(NSV)                                                                  \
+    do {                                                                                  \
+        if (nq == 1) CA_APPLY(1, NSV);                                                    \
+        else CA_APPLY(2, NSV);                                                            \
+    } while (0)
+    if (ns == 1) CA_APPLY_NQ(16);
+    else if (ns == 2) CA_APPLY_NQ(32);
+    else CA_APPLY_NQ(64);
+#undef CA_APPLY_NQ
 #undef CA_APPLY
     CA_CHECK_LAUNCH("tiled apply kernel");
     return CA_OK;

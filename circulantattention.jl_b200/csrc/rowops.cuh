@@ -401,17 +401,26 @@ __global__ void __launch_bounds__(256) axpby_kernel(int64_t n, float alpha, cons
     }
 }
 
+// A block scales runs of 2048 entries of one slice, eight loads in flight per thread (one entry per thread: 43 us for 16
+// slices of 2 MB; slices start at any word, so the accesses stay four bytes wide).
+constexpr int kScaleRun = 8;
 __global__ void __launch_bounds__(256) scale_batch_kernel(int64_t inner, int o1, int o2,
                                                           const float* __restrict__ a, int a1, int a2,
                                                           const float* __restrict__ c, int c1, int c2,
                                                           float* __restrict__ out) {
     const int i1 = blockIdx.y, i2 = blockIdx.z;
-    const int64_t ao = ((int64_t)(a1 > 1 ? i1 : 0) + (int64_t)a1 * (a2 > 1 ? i2 : 0)) * inner;
+    const float* src = a + ((int64_t)(a1 > 1 ? i1 : 0) + (int64_t)a1 * (a2 > 1 ? i2 : 0)) * inner;
     const float cv = c[(c1 > 1 ? i1 : 0) + c1 * (c2 > 1 ? i2 : 0)];
-    const int64_t oo = ((int64_t)i1 + (int64_t)o1 * i2) * inner;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < inner; t += stride)
-        out[oo + t] = cv * a[ao + t];
+    float* dst = out + ((int64_t)i1 + (int64_t)o1 * i2) * inner;
+    for (int64_t t0 = (int64_t)blockIdx.x * (256 * kScaleRun) + threadIdx.x; t0 < inner; t0 += (int64_t)gridDim.x * (256 * kScaleRun)) {
+        float v[kScaleRun];
+#pragma unroll
+        for (int i = 0; i < kScaleRun; ++i)
+            if (t0 + 256 * i < inner) v[i] = src[t0 + 256 * i];
+#pragma unroll
+        for (int i = 0; i < kScaleRun; ++i)
+            if (t0 + 256 * i < inner) dst[t0 + 256 * i] = cv * v[i];
+    }
 }
 
 // One block per batch slice, fixed summation order: deterministic, no scratch.

@@ -589,7 +589,7 @@ inline int prepare(const Geo& g, const Padded& P, int nq, int xch_floats, const 
 
 template <typename K>
 int set_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) {
+    if (bytes > 47 * 1024) {                // the default limit of 48 KB counts the kernel's static shared memory too
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(shared memory)");
     }
