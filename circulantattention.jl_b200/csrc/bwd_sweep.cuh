@@ -72,9 +72,8 @@ __device__ __forceinline__ void dq_stage(uint32_t rowbase, int ws, int rm, float
                     lds_slab16<NS>(a0, 1, slab, v2);
                     const float tp = fmaxf(chain, 0.f);
                     const float w = tp * tp;
-                    const u64 w2 = pack2(w, w);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) dq[r][i] = fma2(w2, v2[i], dq[r][i]);
+                    for (int i = 0; i < 8; ++i) dq[r][i] = outer2(w, v2[i], dq[r][i]);
                 } else if (MODE == 2) {
                     const float gg = fmaxf(chain, 0.f);
                     aux[r] = fmaf(gg, dp[r], aux[r]);
@@ -82,9 +81,8 @@ __device__ __forceinline__ void dq_stage(uint32_t rowbase, int ws, int rm, float
                 } else {
                     const float ds = (MODE == 0 ? fast_exp2(chain) : fmaxf(chain, 0.f)) * dp[r];
                     if (DIST) sumds[r] += ds;
-                    const u64 d2 = pack2(ds, ds);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) dq[r][i] = fma2(d2, k2[i], dq[r][i]);
+                    for (int i = 0; i < 8; ++i) dq[r][i] = outer2(ds, k2[i], dq[r][i]);
                 }
             }
     }
@@ -295,12 +293,10 @@ __device__ __forceinline__ void dkdv_stage(uint32_t base, const float* Lb, const
                     ds = gg * dp[r];
                 }
                 if (DIST) sumds[r] += ds;
-                const u64 d2 = pack2(ds, ds), p2 = pack2(P, P);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    dk[r][i] = fma2(d2, q2[i], dk[r][i]);
-                    dv[r][i] = fma2(p2, y2[i], dv[r][i]);
-                }
+                for (int i = 0; i < 8; ++i) dk[r][i] = outer2(ds, q2[i], dk[r][i]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) dv[r][i] = outer2(P, y2[i], dv[r][i]);
             }
     }
 }

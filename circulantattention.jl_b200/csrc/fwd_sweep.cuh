@@ -112,9 +112,8 @@ __device__ __forceinline__ void fwd_stage(uint32_t rowbase, int ws, int rm, floa
                     if (CA_ON(r)) {
                         const float pt = fast_exp2(sc[r][t]);
                         l[r] += pt;
-                        const u64 p2 = pack2(pt, pt);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) acc[r][i] = fma2(p2, v2[i], acc[r][i]);
+                        for (int i = 0; i < 8; ++i) acc[r][i] = outer2(pt, v2[i], acc[r][i]);
                     }
             }
         }
@@ -174,7 +173,7 @@ __device__ __forceinline__ void fwd_init_max(uint32_t rowbase, int init, float s
 // NCRT = real channels per unit the kernel is compiled for: 16 (narrower units are zero-extended),
 // 32 or 64 (NS = 2 or 4 lanes per pixel, one 16-channel slab each; launched without a stage split).
 template <int DC, bool DIST, int CPE, bool EXACT, int NQ, int NCRT = 16>
-__global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) fwd_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+__global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
                                                            const __grid_constant__ CUtensorMap msc) {
     constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
     constexpr int RB = kRowBytes * NS;
@@ -294,12 +293,17 @@ int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const f
                    cudaStream_t st) {
     Launch L{};
     const int ns = slabs_of(g);
-    // four columns per thread, or two when the grid is small or the window is short (with ws <= 9 most
-    // stages of a four-column tile pair with only some of its columns: measured 18 % faster at ws 7)
+    // three columns per thread (168 registers, three CTAs per SM), or two where the window is short (with ws <= 9 most
+    // stages of a wide tile pair with only some of its columns) or the grid smaller than the chip.  Measured, with packed
+    // outer products: three against four columns (255 registers, two CTAs) 5.68 and 6.07 ms at 1024 x 1024, 8 units, ws 21;
+    // three against two 54 and 61 us at 128 x 96, 8 units, ws 15, 22 and 17 us at 64 x 64, one unit.  Wide units: four once
+    // there are eight warps of such tiles per SM (200 x 150, two units of 64 channels, ws 21: 263 against 270 us; 128 x 96:
+    // 77 against 63 us).
     // a folded signal has one column per thread: a streamed column pairs with one centre column only, and a wider tile
     // computes the others for nothing (8192 x 64 x 4, ws 63, 64 channels: 92 us, see below)
     const bool fold = g.wsw == 1;
-    const int nq = fold ? 1 : (g.ws <= 9 ? tune_int("CIRCATT_FWD_NQ", 2) : (ns > 1 ? 4 : pick_nq(g, 4, 2, "CIRCATT_FWD_NQ")));
+    auto warps_at = [&](int n) { return (long)((g.W + n - 1) / n) * ((g.H * ns + 31) / 32) * g.units; };
+    const int nq = fold ? 1 : (g.ws <= 9 ? 2 : (ns > 1 ? (warps_at(4) >= 8L * sm_count() ? 4 : 3) : (warps_at(3) < sm_count() ? 2 : 3)));
     int rc = prepare(g, P, nq, 18 * nq, "CIRCATT_FWD_WARPS", kv, nullptr, &L, ns == 1 && !fold ? 2 : 1, 4, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.o0 = y; L.a.ostats = stats;
@@ -316,7 +320,7 @@ int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const f
 #define CA_FWD(DCV)                                                                      \
     do {                                                                                 \
         if (nq == 2) CA_FWD2(DCV, true, 2, 16);                                          \
-        else CA_FWD2(DCV, true, 4, 16);                                                  \
+        else CA_FWD2(DCV, true, 3, 16);                                                  \
     } while (0)
     // chunks of 7 or 5 keys where they divide the window, else chunks of four plus a tail
 #define CA_FWD_FOLD(NCRV_)                                                               \
@@ -328,21 +332,25 @@ int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const f
     if (fold && ns == 1) CA_FWD_FOLD(16);
     else if (fold && ns == 2) CA_FWD_FOLD(32);
     else if (fold) CA_FWD_FOLD(64);
-    else if (ns == 2 && nq == 2 && g.ws % 7 == 0) CA_FWD2(7, true, 2, 32);
-    else if (ns == 4 && nq == 2 && g.ws % 7 == 0) CA_FWD2(7, true, 2, 64);
-    else if (ns == 2 && nq == 4 && g.ws % 7 == 0) CA_FWD2(7, true, 4, 32);       // windows 21, 35, 49, 63
-    else if (ns == 4 && nq == 4 && g.ws % 7 == 0) CA_FWD2(7, true, 4, 64);
-    else if (ns == 2 && nq == 4 && g.ws % 5 == 0) CA_FWD2(5, true, 4, 32);       // windows 15, 25, 45, 55
-    else if (ns == 4 && nq == 4 && g.ws % 5 == 0) CA_FWD2(5, true, 4, 64);
-    else if (ns == 2 && nq == 2) CA_FWD2(4, false, 2, 32);
-    else if (ns == 2) CA_FWD2(4, false, 4, 32);
-    else if (ns == 4 && nq == 2) CA_FWD2(4, false, 2, 64);
-    else if (ns == 4) CA_FWD2(4, false, 4, 64);
+#define CA_FWD_WIDE(NCRV_)                                                               \
+    do {                                                                                 \
+        if (nq == 2 && g.ws % 7 == 0) CA_FWD2(7, true, 2, NCRV_);                        \
+        else if (nq == 2) CA_FWD2(4, false, 2, NCRV_);                                   \
+        else if (nq == 4 && g.ws % 7 == 0) CA_FWD2(7, true, 4, NCRV_);                   \
+        else if (nq == 4 && g.ws % 5 == 0) CA_FWD2(5, true, 4, NCRV_);                   \
+        else if (nq == 4) CA_FWD2(4, false, 4, NCRV_);                                   \
+        else if (g.ws % 7 == 0) CA_FWD2(7, true, 3, NCRV_);                              \
+        else if (g.ws % 5 == 0) CA_FWD2(5, true, 3, NCRV_);                              \
+        else CA_FWD2(4, false, 3, NCRV_);                                                \
+    } while (0)
+    else if (ns == 2) CA_FWD_WIDE(32);
+    else if (ns == 4) CA_FWD_WIDE(64);
     else if (g.ws % 7 == 0) CA_FWD(7);
     else if (g.ws % 5 == 0) CA_FWD(5);
     else if (g.ws % 3 == 0) CA_FWD(3);
     else if (nq == 2) CA_FWD2(4, false, 2, 16);
-    else CA_FWD2(4, false, 4, 16);
+    else CA_FWD2(4, false, 3, 16);
+#undef CA_FWD_WIDE
 #undef CA_FWD_FOLD
 #undef CA_FWD2
 #undef CA_FWD

@@ -115,10 +115,14 @@ __device__ __forceinline__ float fast_rcp(float x) {
     return y;
 }
 
+// y += w * x, channel pairs as packed FMAs (an outer product reuses its coefficient: it runs at the packed rate).
 template <int CR>
 __device__ __forceinline__ void axpy(float w, const float (&x)[CR], float (&y)[CR]) {
 #pragma unroll
-    for (int i = 0; i < CR; ++i) y[i] = fmaf(w, x[i], y[i]);
+    for (int i = 0; i < CR; i += 2)
+        asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %2};\n\tmov.b64 b, {%3, %4};\n\tmov.b64 c, {%0, %1};\n\t"
+            "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+            : "+f"(y[i]), "+f"(y[i + 1]) : "f"(w), "f"(x[i]), "f"(x[i + 1]));
 }
 
 // factor * |x|^2 per staged pixel, from the staged groups.
@@ -626,7 +630,7 @@ int prepare(LineArgs& a, int nq, int groups, int scalar_planes, size_t* smem) {
 
 template <typename Kern>
 int launch(Kern kern, const LineArgs& a, int nq, size_t smem, cudaStream_t st, const char* what) {
-    if (smem > 48 * 1024) {
+    if (smem > 47 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
     }

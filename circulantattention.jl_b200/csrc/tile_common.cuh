@@ -74,6 +74,15 @@ struct u64 { float x, y; };
 __device__ __forceinline__ u64 pack2(float a, float b) { return u64{a, b}; }
 __device__ __forceinline__ void unpack2(u64 v, float& a, float& b) { a = v.x; b = v.y; }
 __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) { return u64{fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)}; }
+// acc + w * v with one coefficient for the pair, packed: consecutive outer-product instructions reuse the coefficient, so
+// they run at the packed rate (61 against 50 TFLOP/s in registers, which dot products do not).
+__device__ __forceinline__ u64 outer2(float w, u64 v, u64 acc) {
+    u64 r;
+    asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %2};\n\tmov.b64 b, {%3, %4};\n\tmov.b64 c, {%5, %6};\n\t"
+        "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(w), "f"(v.x), "f"(v.y), "f"(acc.x), "f"(acc.y));
+    return r;
+}
 __device__ __forceinline__ u64 mul2(u64 a, u64 b) { return u64{a.x * b.x, a.y * b.y}; }
 __device__ __forceinline__ u64 add2(u64 a, u64 b) { return u64{a.x + b.x, a.y + b.y}; }
 __device__ __forceinline__ u64 zero2() { return u64{0.f, 0.f}; }
@@ -625,15 +634,6 @@ int set_smem(K kernel, size_t bytes) {
             else CA_LAUNCH_TILED((KERNEL_T<false, 2, NQV, XV, NCRV_>), L, st);        \
         }                                                                             \
     } while (0)
-
-// Centre pixels per thread.  Large problems use the widest tile the registers allow (least
-// shared-memory traffic per FMA); problems too small to fill the GPU use narrower tiles, which
-// means more, shorter-lived warps.
-inline int pick_nq(const Geo& g, int wide, int narrow, const char* env) {
-    const long tasks = ((long)(g.W + wide - 1) / wide) * ((g.H + 31) / 32) * g.units;     // warps at the wide tile
-    const int nq = tasks < 12L * sm_count() ? narrow : wide;
-    return tune_int(env, nq);
-}
 
 }  // namespace
 }  // namespace ca
