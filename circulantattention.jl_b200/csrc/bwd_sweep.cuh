@@ -15,7 +15,7 @@ namespace {
 // =====================================================================
 // MODE 0: softmax, P = 2^chain.  MODE 1: 1.5-entmax, g = max(chain, 0) with the chain = s/2 - tau, dS = g*(dP - D).
 // MODE 2: the entmax pre-pass: only num += g*dP and den += g (in aux and sumds), D = num/den.
-// The same query-owned sweep serves the entmax forward, which has no dy: MODE 3 the row maximum of s/2 (in aux);
+// The same query-owned sweep serves the entmax forward, which has no dy: MODE 3 the largest s/2 of a stage (in aux);
 // MODE 4 one step of the threshold search: with t = chain = s/2 - tau, the sum of max(t, 0) (sumds), of its
 // square (aux), the size of the support {t > 0}, its smallest member and the largest t outside (ex[0..2]);
 // MODE 5 the apply: dq (here y) += max(chain, 0)^2 * v.
@@ -150,18 +150,38 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) dq_tiled
         for (int i = 0; i < 8; ++i) dq[r][i] = zero2();
     }
 
+    // MODE 3: the largest scores of eight classes of keys, window columns dealt out in turn (the stage's maxima always
+    // enter the same register: the others move up)
+    constexpr int kClasses = 8;
+    float top[NQ][kClasses];
+    if (MODE == 3) {
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+#pragma unroll
+            for (int i = 0; i < kClasses; ++i) top[r][i] = -INFINITY;
+    }
     CA_PIPE_LOOP(2, {
         const int mask = stage_mask<NQ>(s, radius_w(g));
         CA_MASK_SWITCH(((1 << NQ) - 1), mask, (dq_stage<DIST, MK, NQ, MODE, NS>(smem_u32(pipe.vec(buf)) + (lr + a.roff) * (kRowBytes * NS), g.ws, mask,
                                                      sl2, q, dy, dq, nL2, nD2, bq, sumds, aux, ex, slab)));
+        if (MODE == 3) {
+            _Pragma("unroll")
+            for (int r = 0; r < NQ; ++r) {
+                const float first = fmaxf(top[r][0], aux[r]);
+                _Pragma("unroll")
+                for (int i = 0; i + 1 < kClasses; ++i) top[r][i] = top[r][i + 1];
+                top[r][kClasses - 1] = first;
+                aux[r] = -INFINITY;
+            }
+        }
     })
 
     if (MODE == 3) {
-        // first threshold of the search: tau >= max - 1 always
+        // first threshold of the search
 #pragma unroll
         for (int r = 0; r < NQ; ++r)
             if (active && slab == 0 && has_pixel(g, h, w0 + r))
-                a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = aux[r] - 1.f + ca_poison;
+                a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = entmax_start(top[r]) + ca_poison;
         return;
     }
     if (MODE == 4) {
@@ -404,7 +424,7 @@ int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const fl
     // units (160 registers, three blocks per SM, against 255 and two)
     // (folded signals: one, see run_fwd)
     const bool fold = g.wsw == 1 && mode == 0;
-    const int nq = fold ? 1 : (mode ? 4 : (ns > 1 ? (g.ws <= 9 ? 2 : 4) : tune_int("CIRCATT_DQ_NQ", 2)));
+    const int nq = fold ? 1 : (mode ? 4 : (ns > 1 ? (g.ws <= 9 ? 2 : 4) : 2));
     int rc = prepare(g, P, nq, 17 * nq, "CIRCATT_DQ_WARPS", kv, nullptr, &L, mode == 0 && ns == 1 && !fold ? 2 : 1, 4, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.c1 = dy; L.a.cs0 = stats; L.a.cs1 = D; L.a.o0 = dq; L.a.ostats = Dout;
@@ -417,8 +437,7 @@ int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const fl
     else if (ns == 4) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 64, L, st);
     else if (mode == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 2, 16, L, st);
     else if (mode == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 1, 16, L, st);
-    else if (nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 16, L, st);
-    else CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 16, L, st);
+    else CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 16, L, st);
     CA_CHECK_LAUNCH("tiled dq kernel");
     return CA_OK;
 }

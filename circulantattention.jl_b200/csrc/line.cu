@@ -9,8 +9,8 @@
 // padding per NQ pixels, which makes the 128-bit loads of a warp (lanes NQ pixels apart) conflict-free.
 //
 // The softmax forward is one sweep with an online sum.  Without the scores of a row in memory, a row quantity
-// that needs all of them is found by sweeping the window again: the entmax forward sweeps once for the row
-// maximum and once to accumulate; the 1.5-entmax
+// that needs all of them is found by sweeping the window again: the entmax forward sweeps once for a
+// first threshold and once to accumulate; the 1.5-entmax
 // threshold tau (sum_k max(z_k - tau, 0)^2 = 1, z = s/2) takes a few sweeps in between, each of which
 // solves the quadratic exactly on the current support {z > tau} and stops when that support reproduces
 // itself; the backward recomputes the weights from the saved row statistic (log-sum-exp or tau).
@@ -173,6 +173,49 @@ __device__ __forceinline__ void sweep(int tb, int ws, F&& f) {
     sweep_tail<NQ, 0>(f, tb, ws);
 }
 
+// The same sweep for the largest score of each of 2*NQ classes of keys: `f(mask, class, slot)` gets the class as a
+// compile-time value.  Steps 0 .. 2*NQ-1 are classes 0 .. 2*NQ-1 and so on; the last few of a window that is no
+// multiple of 2*NQ go to the first classes again (any partition of the keys will do).
+template <int NQ, int T, class F>
+__device__ __forceinline__ void class_head(F& f, int slot0) {
+    if constexpr (T < NQ - 1) {
+        f(ic<(1 << (T + 1)) - 1>{}, ic<T>{}, slot0 + T);
+        class_head<NQ, T + 1>(f, slot0);
+    }
+}
+template <int NQ, int FIRST, int I, class F>
+__device__ __forceinline__ void class_group(F& f, int slot0) {
+    if constexpr (I < NQ) {
+        f(ic<(1 << NQ) - 1>{}, ic<FIRST + I>{}, slot0 + I);
+        class_group<NQ, FIRST, I + 1>(f, slot0);
+    }
+}
+template <int NQ, int E, class F>
+__device__ __forceinline__ void class_tail(F& f, int tb, int ws) {
+    if constexpr (E < NQ - 1) {
+        f(ic<((1 << NQ) - 1) & ~((1 << (E + 1)) - 1)>{}, ic<E + 1>{}, pad<NQ>(tb + ws + E));
+        class_tail<NQ, E + 1>(f, tb, ws);
+    }
+}
+template <int NQ, class F>
+__device__ __forceinline__ void sweep_classes(int tb, int ws, F&& f) {
+    int slot0 = pad<NQ>(tb);
+    class_head<NQ, 0>(f, slot0);
+    f(ic<(1 << NQ) - 1>{}, ic<NQ - 1>{}, slot0 + NQ - 1);
+    int t = NQ;
+    slot0 += NQ + 1;
+    for (; t + 2 * NQ <= ws; t += 2 * NQ, slot0 += 2 * (NQ + 1)) {
+        class_group<NQ, NQ, 0>(f, slot0);
+        class_group<NQ, 0, 0>(f, slot0 + NQ + 1);
+    }
+    if (t + NQ <= ws) {
+        class_group<NQ, NQ, 0>(f, slot0);
+        t += NQ;
+    }
+    for (; t < ws; ++t) f(ic<(1 << NQ) - 1>{}, ic<0>{}, pad<NQ>(tb + t));
+    class_tail<NQ, 0>(f, tb, ws);
+}
+
 // One step of the entmax threshold search from the statistics of a sweep at the current tau, with t = z - tau:
 // n = |{t > 0}| (the support S), sa = sum_S t, sb = sum_S t^2, rmax = max 1/t = 1 / (smallest t > 0),
 // rmin = min 1/t = 1 / (largest t < 0).  Returns the step d that solves sum_S (t - d)^2 = 1 and sets `same` when
@@ -231,7 +274,7 @@ __global__ void __launch_bounds__(kLT, CR <= 8 ? 3 : 2) line_fwd_kernel(LineArgs
         bq[r] = DIST ? -0.5f * invf * dot<CR>(q[r], q[r], 0.f) : 0.f;
     }
 
-    // entmax: the row maximum.  softmax: an online sum against a reference that starts kLineHeadroom above the
+    // softmax: an online sum against a reference that starts kLineHeadroom above the
     // score of the centre key and moves only when a score climbs past it (then the sums are rescaled)
     float m[NQ];
 #pragma unroll
@@ -244,29 +287,41 @@ __global__ void __launch_bounds__(kLT, CR <= 8 ? 3 : 2) line_fwd_kernel(LineArgs
             m[r] = dot<CR>(q[r], kk, DIST ? bq[r] + bk[pad<NQ>(tb + r + g.p)] : 0.f) + kLineHeadroom;
         }
     }
-    if (ENT) sweep<NQ>(tb, ws, [&](auto mk, int slot) {
-        constexpr int M = decltype(mk)::value;
-        float kk[CR];
-        ld_vec<CR>(Kg, a.PP, slot, kk);
-        const float bkk = DIST ? bk[slot] : 0.f;
+    // entmax: the first threshold comes from the largest scores of 2*NQ classes of keys, which cost the sweep no more
+    // than the row maximum does.  Against a start at max - 1 the threshold sweeps fall from four to two
+    // (127 keys of 8 channels, standard normal: 128, 123, 63, 0.5 of a warp's 128 rows open after each, now 92 and 3);
+    // 16384 x 64 x 16, 8 units, ws 127, Distance: 1046 -> 786 us.
+    if (ENT) {
+        constexpr int kClasses = 2 * NQ;
+        float top[NQ][kClasses];
 #pragma unroll
         for (int r = 0; r < NQ; ++r)
-            if ((M >> r) & 1) m[r] = fmaxf(m[r], dot<CR>(q[r], kk, DIST ? bq[r] + bkk : 0.f));
-    });
+#pragma unroll
+            for (int i = 0; i < kClasses; ++i) top[r][i] = -INFINITY;
+        sweep_classes<NQ>(tb, ws, [&](auto mk, auto cls, int slot) {
+            constexpr int M = decltype(mk)::value;
+            constexpr int I = decltype(cls)::value;
+            float kk[CR];
+            ld_vec<CR>(Kg, a.PP, slot, kk);
+            const float bkk = DIST ? bk[slot] : 0.f;
+#pragma unroll
+            for (int r = 0; r < NQ; ++r)
+                if ((M >> r) & 1) top[r][I] = fmaxf(top[r][I], dot<CR>(q[r], kk, DIST ? bq[r] + bkk : 0.f));
+        });
+#pragma unroll
+        for (int r = 0; r < NQ; ++r) m[r] = entmax_start(top[r]);
+    }
 
-    // offset of the weights: p = 2^(z - m) (softmax) or max(z - tau, 0)^2 (entmax)
+    // offset of the weights: p = 2^(z - m) (softmax) or max(z - tau, 0)^2 (entmax, m = the first tau)
     float off[NQ];
 #pragma unroll
     for (int r = 0; r < NQ; ++r) off[r] = m[r];
     if (ENT) {
-        // tau >= max - 1; every sweep solves sum_{S} (z - tau)^2 = 1 on the support S = {z > tau} of the
-        // current tau and is final when the new tau has the same support
+        // every sweep solves sum_{S} (z - tau)^2 = 1 on the support S = {z > tau} of the current tau < max and is
+        // final when the new tau has the same support
         bool done[NQ];
 #pragma unroll
-        for (int r = 0; r < NQ; ++r) {
-            off[r] = m[r] - 1.f;
-            done[r] = false;
-        }
+        for (int r = 0; r < NQ; ++r) done[r] = false;
         for (int it = 0; it < kMaxTauSweeps; ++it) {
             // the support's nearest members on both sides of tau through reciprocals: max 1/t is 1/(smallest t > 0),
             // min 1/t is 1/(largest t < 0) -- one reciprocal and two min/max per pair, no selects

@@ -47,7 +47,7 @@ int run_fwd(const Geo& g, const Padded& P, float scale, int dist, const float* q
 template <bool ANYC>
 int run_dq(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* dy, const float* stats,
            const float* D, const float* kv, float* dq, cudaStream_t st, int mode, float* Dout);
-// One sweep of the entmax forward over the packed (k|v): mode 3 row maximum -> first threshold (tau),
+// One sweep of the entmax forward over the packed (k|v): mode 3 class maxima -> first threshold (tau),
 // 4 one step of the threshold search (tau and `settled` updated in place), 5 y = sum max(s/2 - tau, 0)^2 v.
 template <bool ANYC>
 int run_entmax_fwd_sweep(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* kv,
@@ -611,17 +611,6 @@ int set_smem(K kernel, size_t bytes) {
         if (rc__) return rc__;                                                        \
         KERNEL<<<(L).grid, (L).threads, (L).smem, st>>>((L).a, (L).mv, (L).msc);      \
         count_tiled_launch();                                                         \
-    } while (0)
-
-#define CA_DIST_CPE(KERNEL_T, dist, cpe, L, st)                                       \
-    do {                                                                              \
-        if ((cpe) == 1) {                                                             \
-            if (dist) CA_LAUNCH_TILED((KERNEL_T<true, 1>), L, st);                    \
-            else CA_LAUNCH_TILED((KERNEL_T<false, 1>), L, st);                        \
-        } else {                                                                      \
-            if (dist) CA_LAUNCH_TILED((KERNEL_T<true, 2>), L, st);                    \
-            else CA_LAUNCH_TILED((KERNEL_T<false, 2>), L, st);                        \
-        }                                                                             \
     } while (0)
 
 #define CA_DIST_CPE_NQ(KERNEL_T, dist, cpe, NQV, XV, NCRV_, L, st)                    \

@@ -222,8 +222,8 @@ int tiled_attention_bwd_entmax(const Geo& gin, float scale, int dist, const floa
     return CA_CHANNELS(g, run_dkdv, g, P, scale, dist, k, v, qdy, planes, dk, dv, st, true);
 }
 
-// The 1.5-entmax forward in flash mode without A-sized memory: the packed (k|v) is swept once for the row
-// maxima, a fixed number of times for the thresholds (blocks whose rows are all final leave at once) and once
+// The 1.5-entmax forward in flash mode without A-sized memory: the packed (k|v) is swept once for the first
+// thresholds, a fixed number of times for the thresholds (blocks whose rows are all final leave at once) and once
 // for y.  `stats` (nullable) receives tau and doubles as the search's state; the `settled` plane and a tau plane
 // for callers without `stats` live behind the pair in the workspace (tiled_fwd_entmax_workspace bytes).
 size_t tiled_fwd_entmax_workspace(const Geo& gin) {

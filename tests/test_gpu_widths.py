@@ -1,6 +1,6 @@
-"""Shapes at the edges of the tiled kernels' dispatch: channel counts that are zero-extended to 16, 32 or 64, 1-D
-signals whose folded last column is short, stored values applied at every alignment, and rows at the limits of the
-row kernels' register shapes."""
+"""Shapes at the edges of the tiled and 1-D kernels' dispatch: channel counts that are zero-extended to 16, 32 or 64, 1-D
+signals whose folded last column is short, stored values applied at every alignment, rows at the limits of the row
+kernels' register shapes, columns per thread of the forward, and the classes of the first entmax threshold."""
 import numpy as np
 import pytest
 
@@ -85,3 +85,40 @@ def test_rows_at_the_limits_of_the_row_kernels(ca, spatial, ws):
     back = ca.ops.row_normalize_bwd(got, d, spatial, ws, 0)
     assert rel_err(ca.jl.to_numpy(back), ds.reshape((rows * K, 3), order="F")) < TOL
     assert rel_err(ca.jl.to_numpy(ca.ops.sum_rows(s, spatial, ws)), z.sum(axis=0)[:, None, :]) < TOL
+
+
+@pytest.mark.parametrize("shape,ws", [
+    ((30, 25, 16, 17), 11),     # 153 warps of three-column tiles: one column in the last tile
+    ((30, 26, 16, 17), 13),     # two
+    ((30, 27, 8, 17), 21),      # full tiles, chunks of seven
+    ((30, 26, 16, 10), 15),     # fewer warps than SMs: two columns per thread
+    ((32, 33, 32, 66), 11),     # two slabs, 1188 warps of four-column tiles, one column in the last
+    ((17, 19, 64, 2), 11),      # four slabs, three columns per thread
+])
+def test_forward_column_tiles(ca, shape, ws):
+    rng = np.random.default_rng(44)
+    qn, kn, vn = (randn(rng, shape) for _ in range(3))
+    y, _ = ca.circulant_attention(ca.DotSimilarity(), *(ca.jl.from_numpy(t) for t in (qn, kn, vn)), ws, return_A=False)
+    units = range(0, shape[-1], max(1, shape[-1] // 4))
+    for u in units:
+        one = slice(u, u + 1)
+        yo, _ = orc.attention(orc.DOT, up(qn[..., one]), up(kn[..., one]), up(vn[..., one]), ws)
+        assert_close(ca.jl.to_numpy(y)[..., one], yo, f"y of unit {u}")
+
+
+@pytest.mark.parametrize("c", [8, 16])
+@pytest.mark.parametrize("ws", [5, 7, 9, 11, 13, 15, 17, 19, 33])
+def test_entmax_first_threshold(ca, ws, c):
+    """1-D windows of every remainder modulo the classes the first threshold is taken from; units of ordinary rows, of
+    equal scores (everything in the support) and of one score far above the others (nothing else in it)."""
+    rng = np.random.default_rng(45)
+    qn, kn, vn = (randn(rng, (141, c, 3)) for _ in range(3))
+    kn[..., 1] = kn[:1, :, 1]
+    qn[..., 2] = 1.0
+    kn[::ws + 1, :, 2] += 6.0
+    y, _ = ca.circulant_attention(ca.DotSimilarity(), *(ca.jl.from_numpy(t) for t in (qn, kn, vn)), ws,
+                                  normalizer=ca.ENTMAX15, return_A=False)
+    for u in range(3):
+        one = slice(u, u + 1)
+        yo, _ = orc.attention(orc.DOT, up(qn[..., one]), up(kn[..., one]), up(vn[..., one]), ws, orc.ENTMAX15)
+        assert_close(ca.jl.to_numpy(y)[..., one], yo, f"y of unit {u}", tol=3e-5, elem_tol=6e-5)
