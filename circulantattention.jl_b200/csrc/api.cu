@@ -155,11 +155,8 @@ static int launch_row_normalize(int64_t rows, int K, int entmax, const float* s,
     const int64_t blocks = (rows * 32 + 255) / 256;
     if (blocks > INT32_MAX) { set_error("too many rows"); return CA_ERR_TOO_LARGE; }
     if (entmax) {
-        if (K <= 64) row_entmax15_reg_kernel<2><<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
-        else if (K <= 128) row_entmax15_reg_kernel<4><<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
-        else if (K <= 256) row_entmax15_reg_kernel<8><<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
-        else if (K <= 512) row_entmax15_reg_kernel<16><<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
-        else row_entmax15_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats);
+        CA_ENTMAX_SHAPE(K, (row_entmax15_reg_kernel<G, R><<<(unsigned)((rows * G + 255) / 256), 256, 0, st>>>(rows, K, s, p, stats)),
+                        (row_entmax15_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats)));
     }
     else CA_ROW_SHAPE(K, (row_softmax_reg_kernel<G, R><<<(unsigned)((rows * G + 255) / 256), 256, 0, st>>>(rows, K, s, p, stats)),
                       (row_softmax_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, K, s, p, stats)));

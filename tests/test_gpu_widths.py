@@ -80,6 +80,9 @@ def test_rows_at_the_limits_of_the_row_kernels(ca, spatial, ws):
     got, stats = ca.ops.row_normalize(s, spatial, ws, 0, want_stats=True)
     assert rel_err(ca.jl.to_numpy(got), p.reshape((rows * K, 3), order="F")) < TOL
     assert rel_err(ca.jl.to_numpy(stats), z.max(axis=0) + np.log(e.sum(axis=0))) < TOL
+    pe = orc.row_entmax15(z.copy())
+    got_e = ca.ops.row_normalize(s, spatial, ws, 1)
+    assert rel_err(ca.jl.to_numpy(got_e), pe.reshape((rows * K, 3), order="F")) < TOL
     dp = up(dn).reshape((K, rows, 3), order="F")
     ds = p * (dp - (p * dp).sum(axis=0))
     back = ca.ops.row_normalize_bwd(got, d, spatial, ws, 0)
