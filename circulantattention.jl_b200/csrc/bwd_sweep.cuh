@@ -412,7 +412,6 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 4 : NQ == 2 ? 3 : 2)) dkdv_til
 
 }  // namespace
 
-// The entmax variants exist for four centre pixels per thread and run without a stage split.
 template <>
 int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* dy, const float* stats,
            const float* D, const float* kv, float* dq, cudaStream_t st, int mode, float* Dout) {
@@ -420,12 +419,13 @@ int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const fl
     const int ns = slabs_of(g);
     if (ns > 1 && mode) return CA_ERR_UNSUPPORTED;             // the entmax variants exist for one-slab units
     if (mode >= 3) return CA_ERR_UNSUPPORTED;                  // the forward's sweeps go through run_entmax_fwd_sweep
-    // two query columns per thread measured faster than four at every size for the softmax dq sweep of one-slab
-    // units (160 registers, three blocks per SM, against 255 and two)
+    // two query columns per thread measured faster than four at every size for the dq sweeps of one-slab units (160
+    // registers, three blocks per SM, against 255 and two), the entmax ones included: 128 x 96, 8 units, ws 15, dq
+    // 105 -> 67 us, its pre-pass 84 -> 63 us.  The pre-pass runs without a stage split.
     // (folded signals: one, see run_fwd)
     const bool fold = g.wsw == 1 && mode == 0;
-    const int nq = fold ? 1 : (mode ? 4 : (ns > 1 ? (g.ws <= 9 ? 2 : 4) : 2));
-    int rc = prepare(g, P, nq, 17 * nq, "CIRCATT_DQ_WARPS", kv, nullptr, &L, mode == 0 && ns == 1 && !fold ? 2 : 1, 4, ns);
+    const int nq = fold ? 1 : (ns > 1 ? (g.ws <= 9 ? 2 : 4) : 2);
+    int rc = prepare(g, P, nq, 17 * nq, "CIRCATT_DQ_WARPS", kv, nullptr, &L, mode < 2 && ns == 1 && !fold ? 2 : 1, 4, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.c1 = dy; L.a.cs0 = stats; L.a.cs1 = D; L.a.o0 = dq; L.a.ostats = Dout;
     if (fold && ns == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 1, 0, 16, L, st);
@@ -435,13 +435,15 @@ int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const fl
     else if (ns == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 32, L, st);
     else if (ns == 4 && nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 64, L, st);
     else if (ns == 4) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 64, L, st);
-    else if (mode == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 2, 16, L, st);
-    else if (mode == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 1, 16, L, st);
+    else if (mode == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 2, 16, L, st);
+    else if (mode == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 1, 16, L, st);
     else CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 16, L, st);
     CA_CHECK_LAUNCH("tiled dq kernel");
     return CA_OK;
 }
 
+// Four columns per thread and no stage split: these sweeps serve large problems (smaller ones normalise stored scores),
+// where two measured slower (300 x 280, 8 units, ws 11: first threshold 149 and 173 us, apply 252 and 266 us).
 template <>
 int run_entmax_fwd_sweep<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* kv,
                          float* tau, float* settled, float* y, int mode, int iter, cudaStream_t st) {
