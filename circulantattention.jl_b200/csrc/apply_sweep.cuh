@@ -52,11 +52,6 @@ __device__ __forceinline__ u64 split2(uint64_t v) {
 __device__ __forceinline__ void lds128p(uint32_t addr, uint64_t& lo, uint64_t& hi) {
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(addr));
 }
-__device__ __forceinline__ float lds32(uint32_t addr) {
-    float x;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(addr));
-    return x;
-}
 
 // 16-byte pieces that cover a run of ws words at any misalignment, and the row pitch in words.  Rows that wrap around
 // an axis whose length is no multiple of four change their misalignment, which takes one more piece of room.
@@ -83,7 +78,7 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 6 : 4)) apply_tiled_kernel(Til
     const bool fold = NQ == 1;                                 // folded 1-D signal: rows continue into neighbour columns
     const int w0 = blockIdx.x * NQ, h0 = blockIdx.y * a.TH, u = blockIdx.z;
     const int NSTAGES = g.wsw + min(NQ - 1, g.W - 1 - w0);          // no stages for centre columns past the image
-    CA_PIPE_PROLOGUE(false, 4)
+    CA_PIPE_PROLOGUE(false, kParts)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int slab = lane % NS, lrow = lane / NS;              // this lane's channel slab and row inside the warp
     const int lr = (lt >> 5) * RW + lrow, h = h0 + lr;         // row inside the tile, image row
@@ -171,10 +166,10 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 6 : 4)) apply_tiled_kernel(Til
     int mis4 = 0, mis4_next = 0;
     if (a.nbuf == 2 && s_begin < s_end) mis4_next = fetch_runs(s_begin, 0);
 
-    CA_PIPE_LOOP(4, {
+    CA_PIPE_LOOP({
         const int mask = stage_mask<NQ>(s, pw);
-        const uint32_t rowbase = smem_u32(pipe.vec(buf)) + (lr + a.roff) * RB + slab * 16;
-        const int tb = a.nbuf == 2 ? it & 1 : 0;
+        const uint32_t rowbase = pipe.vec(buf, a) + (lr + a.roff) * RB + slab * 16;
+        const int tb = a.nbuf == 2 ? (s - s_begin) & 1 : 0;
         if (a.nbuf == 2) {
             mis4 = mis4_next;
             if (s + 1 < s_end) { mis4_next = fetch_runs(s + 1, tb ^ 1); cp_async_wait<1>(); }

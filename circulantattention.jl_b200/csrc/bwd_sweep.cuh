@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) dq_tiled
         }
         if (__syncthreads_and(mine)) return;
     }
-    CA_PIPE_PROLOGUE(false, 2)
+    CA_PIPE_PROLOGUE(false, (NS == 1 ? kParts : 1))
     const int slab = NS == 1 ? 0 : (lt % NS);
     const int lr = NS == 1 ? lt : (lt >> 5) * (32 / NS) + (lt & 31) / NS, h = h0 + lr;
     const bool active = h < g.H;
@@ -160,9 +160,9 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) dq_tiled
 #pragma unroll
             for (int i = 0; i < kClasses; ++i) top[r][i] = -INFINITY;
     }
-    CA_PIPE_LOOP(2, {
+    CA_PIPE_LOOP({
         const int mask = stage_mask<NQ>(s, radius_w(g));
-        CA_MASK_SWITCH(((1 << NQ) - 1), mask, (dq_stage<DIST, MK, NQ, MODE, NS>(smem_u32(pipe.vec(buf)) + (lr + a.roff) * (kRowBytes * NS), g.ws, mask,
+        CA_MASK_SWITCH(((1 << NQ) - 1), mask, (dq_stage<DIST, MK, NQ, MODE, NS>(pipe.vec(buf, a) + (lr + a.roff) * (kRowBytes * NS), g.ws, mask,
                                                      sl2, q, dy, dq, nL2, nD2, bq, sumds, aux, ex, slab)));
         if (MODE == 3) {
             _Pragma("unroll")
@@ -215,9 +215,9 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) dq_tiled
                 a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = (sumds[r] > 0.f ? aux[r] / sumds[r] : 0.f) + ca_poison;
         return;
     }
-    if (a.nsplit == 2) {
-        float* xch = reinterpret_cast<float*>(smem_al);
-        if (part == 1) {
+    if (NS == 1 && a.nsplit > 1) {                                    // parts 1.. publish their partial sums, part 0 adds them up
+        float* xch = reinterpret_cast<float*>(smem_al) + (size_t)max(part - 1, 0) * (17 * NQ) * PT;
+        if (part > 0) {
 #pragma unroll
             for (int r = 0; r < NQ; ++r) {
                 xch[(r * 17 + 16) * PT + lt] = sumds[r];
@@ -231,7 +231,9 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) dq_tiled
             }
         }
         __syncthreads();
-        if (part == 1) return;
+        if (part > 0) return;
+#pragma unroll 1
+        for (int o = 1; o < a.nsplit; ++o, xch += (17 * NQ) * PT)
 #pragma unroll
         for (int r = 0; r < NQ; ++r) {
             sumds[r] += xch[(r * 17 + 16) * PT + lt];
@@ -267,15 +269,16 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) dq_tiled
 // rows carry (q | dy) of the query pixels plus their L and D.
 // =====================================================================
 template <bool DIST, int MASK, int NQ, bool ENT, int NS = 1>
-__device__ __forceinline__ void dkdv_stage(uint32_t base, const float* Lb, const float* Db, int row0, int ws, int rm,
+__device__ __forceinline__ void dkdv_stage(uint32_t a0, uint32_t sa, uint32_t plane, int ws, int rm,
                                            float sl2, const u64 (&k)[NQ][8], const u64 (&v)[NQ][8], u64 (&dk)[NQ][8],
                                            u64 (&dv)[NQ][8], const float (&bk)[NQ], float (&sumds)[NQ], int slab = 0) {
+    // row statistics as C++ loads: the compiler places them, the vector loads are pinned (2 % at ws 21)
+    const float* Lr = reinterpret_cast<const float*>(__cvta_shared_to_generic(sa));
+    const float* Dr = reinterpret_cast<const float*>(__cvta_shared_to_generic(sa + plane));
 #pragma unroll (NQ == 1 ? 2 : 1)
     for (int di = 0; di < ws; ++di) {
-        const int row = row0 + di;
-        const uint32_t a0 = base + row * (kRowBytes * NS);
         // the row scalars enter the lane sums once: on slab 0
-        const float nLj = (NS == 1 || slab == 0) ? -Lb[row] : 0.f, nDj = (NS == 1 || slab == 0) ? -Db[row] : 0.f;
+        const float nLj = (NS == 1 || slab == 0) ? -*Lr : 0.f, nDj = (NS == 1 || slab == 0) ? -*Dr : 0.f;
         u64 y2[8];
         lds_slab16<NS>(a0, 1, slab, y2);
         float dp[NQ];
@@ -318,6 +321,9 @@ __device__ __forceinline__ void dkdv_stage(uint32_t base, const float* Lb, const
 #pragma unroll
                 for (int i = 0; i < 8; ++i) dv[r][i] = outer2(P, y2[i], dv[r][i]);
             }
+        a0 += kRowBytes * NS;
+        ++Lr;
+        ++Dr;
     }
 }
 
@@ -330,7 +336,7 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 4 : NQ == 2 ? 3 : 2)) dkdv_til
     const int NSTAGES = g.wsw + NQ - 1;
     const int w0 = blockIdx.x * NQ, h0 = blockIdx.y * a.TH, u = blockIdx.z;
     const float sl2 = ENT ? 0.5f * a.scale : a.scale * kLog2e;      // entmax: the chain is s/2 - tau
-    CA_PIPE_PROLOGUE(true, 2)
+    CA_PIPE_PROLOGUE(true, (NS == 1 ? kParts : 1))
     const int slab = NS == 1 ? 0 : (lt % NS);
     const int lr = NS == 1 ? lt : (lt >> 5) * (32 / NS) + (lt & 31) / NS, h = h0 + lr;
     const bool active = h < g.H;
@@ -356,15 +362,15 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 4 : NQ == 2 ? 3 : 2)) dkdv_til
         }
     }
 
-    CA_PIPE_LOOP(2, {
+    CA_PIPE_LOOP({
         const int mask = stage_mask<NQ>(s, radius_w(g));
-        CA_MASK_SWITCH(((1 << NQ) - 1), mask, (dkdv_stage<DIST, MK, NQ, ENT, NS>(smem_u32(pipe.vec(buf)), pipe.sc0(buf), pipe.sc1(buf),
-                                                      lr + a.roff, g.ws, mask, sl2, k, v, dk, dv, bk, sumds, slab)));
+        CA_MASK_SWITCH(((1 << NQ) - 1), mask, (dkdv_stage<DIST, MK, NQ, ENT, NS>(pipe.vec(buf, a) + (lr + a.roff) * (kRowBytes * NS),
+                                                      pipe.sc0(buf, a, ROWS) + (lr + a.roff) * 4, pipe.plane_bytes(ROWS), g.ws, mask, sl2, k, v, dk, dv, bk, sumds, slab)));
     })
 
-    if (a.nsplit == 2) {
-        float* xch = reinterpret_cast<float*>(smem_al);
-        if (part == 1) {
+    if (NS == 1 && a.nsplit > 1) {
+        float* xch = reinterpret_cast<float*>(smem_al) + (size_t)max(part - 1, 0) * (33 * NQ) * PT;
+        if (part > 0) {
 #pragma unroll
             for (int r = 0; r < NQ; ++r) {
                 xch[(r * 33 + 32) * PT + lt] = sumds[r];
@@ -381,7 +387,9 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 4 : NQ == 2 ? 3 : 2)) dkdv_til
             }
         }
         __syncthreads();
-        if (part == 1) return;
+        if (part > 0) return;
+#pragma unroll 1
+        for (int o = 1; o < a.nsplit; ++o, xch += (33 * NQ) * PT)
 #pragma unroll
         for (int r = 0; r < NQ; ++r) {
             sumds[r] += xch[(r * 33 + 32) * PT + lt];

@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 6 : 4)) emit_a_tiled_kernel(Ti
     const int w0 = blockIdx.x * NQ, h0 = blockIdx.y * a.TH, u = blockIdx.z;
     const int NSTAGES = g.wsw + min(NQ - 1, g.W - 1 - w0);          // no stages for centre columns past the image
     const float sl2 = a.scale * kLog2e;
-    CA_PIPE_PROLOGUE(false, 2)
+    CA_PIPE_PROLOGUE(false, kParts)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int slab = lane % NS, lrow = lane / NS;              // this lane's channel slab and row inside the warp
     const int lr = (lt >> 5) * RW + lrow, h = h0 + lr;         // row inside the tile, image row
@@ -75,9 +75,9 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 6 : 4)) emit_a_tiled_kernel(Ti
     }
     const int64_t warp_row0 = (int64_t)u * g.Np + hw0;
 
-    CA_PIPE_LOOP(2, {
+    CA_PIPE_LOOP({
         const int mask = stage_mask<NQ>(s, pw);
-        const uint32_t rowbase = smem_u32(pipe.vec(buf)) + (lr + a.roff) * RB;
+        const uint32_t rowbase = pipe.vec(buf, a) + (lr + a.roff) * RB;
         for (int d0 = 0; d0 < g.ws; d0 += CH) {
             const int len = min(CH, g.ws - d0);                // window rows d0 .. d0 + len - 1
             // the dot products of all centre columns run interleaved (the columns that do not pair with this stage are

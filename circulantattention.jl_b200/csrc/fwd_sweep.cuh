@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tile
     const int NSTAGES = g.wsw + NQ - 1;
     const int w0 = blockIdx.x * NQ, h0 = blockIdx.y * a.TH, u = blockIdx.z;
     const float sl2 = a.scale * kLog2e;
-    CA_PIPE_PROLOGUE(false, 2)
+    CA_PIPE_PROLOGUE(false, (NS == 1 ? kParts : 1))
     const int slab = NS == 1 ? 0 : (lt % NS);
     const int lr = NS == 1 ? lt : (lt >> 5) * (32 / NS) + (lt & 31) / NS, h = h0 + lr;
     const bool active = h < g.H;
@@ -206,9 +206,9 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tile
         for (int i = 0; i < 8; ++i) acc[r][i] = zero2();
     }
 
-    CA_PIPE_LOOP(2, {
+    CA_PIPE_LOOP({
         const int mask = stage_mask<NQ>(s, radius_w(g));
-        const uint32_t rowbase = smem_u32(pipe.vec(buf)) + (lr + a.roff) * RB;
+        const uint32_t rowbase = pipe.vec(buf, a) + (lr + a.roff) * RB;
         // pixels whose first stage (of this part) is s
         const int init = (s == s_begin) ? mask : (mask & ~stage_mask<NQ>(s - 1, radius_w(g)));
         if (init) fwd_init_max<DIST, NQ, NS>(rowbase, init, sl2, q, nm2, bq, slab);
@@ -234,10 +234,10 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tile
         float zero;
         unpack2(nm2[r], nm[r], zero);
     }
-    if (a.nsplit == 2) {
-        // merge the two partial softmaxes: part 1 publishes (m, l, acc), part 0 combines
-        float* xch = reinterpret_cast<float*>(smem_al);
-        if (part == 1) {
+    if (NS == 1 && a.nsplit > 1) {
+        // merge the partial softmaxes: parts 1.. publish (m, l, acc), part 0 combines
+        float* xch = reinterpret_cast<float*>(smem_al) + (size_t)max(part - 1, 0) * (18 * NQ) * PT;
+        if (part > 0) {
 #pragma unroll
             for (int r = 0; r < NQ; ++r) {
                 xch[(r * 18 + 0) * PT + lt] = nm[r];
@@ -252,7 +252,9 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tile
             }
         }
         __syncthreads();
-        if (part == 1) return;
+        if (part > 0) return;
+#pragma unroll 1
+        for (int o = 1; o < a.nsplit; ++o, xch += (18 * NQ) * PT)
 #pragma unroll
         for (int r = 0; r < NQ; ++r) {
             const float nm1 = xch[(r * 18 + 0) * PT + lt], l1 = xch[(r * 18 + 1) * PT + lt];

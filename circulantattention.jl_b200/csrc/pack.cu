@@ -231,10 +231,10 @@ __global__ void __launch_bounds__(32) stage_timeout_probe_kernel(uint32_t tries,
     __syncthreads();
     bool ok = true;
     if (threadIdx.x == 0) {
-        mbar_arrive_expect_tx(&bar, 64);                      // 64 bytes expected ...
+        mbar_arrive_expect_tx(smem_u32(&bar), 64);                      // 64 bytes expected ...
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 32, [%2];"
                      ::"r"(smem_u32(dst)), "l"(g_probe_src), "r"(smem_u32(&bar)) : "memory");   // ... 32 delivered
-        ok = mbar_wait(&bar, 0, tries);
+        ok = mbar_wait(smem_u32(&bar), 0, tries);
         // the copy in flight gets a bounded chance to land before the CTA (and its shared memory) goes away
         for (uint32_t i = 0; i < (1u << 16) && *reinterpret_cast<volatile float*>(&dst[7]) != 8.f; ++i) {}
         if (!ok) {

@@ -89,6 +89,11 @@ __device__ __forceinline__ u64 zero2() { return u64{0.f, 0.f}; }
 __device__ __forceinline__ void lds128(uint32_t addr, u64& lo, u64& hi) {
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(lo.x), "=f"(lo.y), "=f"(hi.x), "=f"(hi.y) : "r"(addr));
 }
+__device__ __forceinline__ float lds32(uint32_t addr) {
+    float x;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(addr));
+    return x;
+}
 __device__ __forceinline__ float hsum2(u64 v) {
     float a, b;
     unpack2(v, a, b);
@@ -109,7 +114,7 @@ struct TileArgs {
     int TH;                 // rows per CTA
     int roff;               // p' - p: first window row inside a stage buffer
     int stage_bytes;        // bytes of one stage buffer (multiple of 128)
-    int nsplit;             // 1, 2 or (operators) 4 groups of warps sharing the stages of a tile
+    int nsplit;             // 1 to kParts groups of warps sharing the stages of a tile
     int iter;               // entmax threshold search: number of the step (late steps fall back to Newton)
     int row_bytes;          // bytes of one packed pixel row: 144 per 16-channel slab
     int nstages;            // copy stages in flight per part: 2 or 3 (kStages)
@@ -127,6 +132,7 @@ struct TileArgs {
 };
 
 constexpr int kStages = 3;
+constexpr int kParts = 4;                      // groups of warps that can share the stages of a tile
 constexpr uint32_t kWaitTries = 1u << 20;
 constexpr int kEntmaxFwdSteps = 16;            // launches of the entmax threshold step (settled blocks leave at once)
 
@@ -189,14 +195,18 @@ __device__ __forceinline__ int stage_mask(int s, int p) {
     return mask;
 }
 
-// Barrier of one group of warps (ids 1..PARTS; id 0 stays the CTA-wide barrier).  Immediate ids: one in a register
-// reserves all sixteen, and every branch counts where stages are short (windows of 7: 5 % of the sweeps).
-template <int PARTS>
-__device__ __forceinline__ void part_sync(int part, int nthreads) {
-    if (part == 0) asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
-    else if (PARTS == 2 || part == 1) asm volatile("bar.sync 2, %0;" ::"r"(nthreads) : "memory");
-    else if (part == 2) asm volatile("bar.sync 3, %0;" ::"r"(nthreads) : "memory");
-    else asm volatile("bar.sync 4, %0;" ::"r"(nthreads) : "memory");
+// Barrier of one group of warps (ids 1..PARTS; id 0 stays the CTA-wide barrier) that also tells whether any thread of it
+// passes a true `flag`.  A group of one warp needs no barrier.  Immediate ids: one in a register reserves all sixteen.
+__device__ __forceinline__ bool part_any(int part, int nthreads, bool flag) {
+    int any;
+#define CA_BAR_OR(ID)                                                                                                 \
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %2, 0;\n\tbar.red.or.pred q, " #ID ", %1, p;\n\t"          \
+                 "selp.s32 %0, 1, 0, q;\n\t}" : "=r"(any) : "r"(nthreads), "r"((int)flag) : "memory")
+    if (nthreads == 32) return __any_sync(0xffffffffu, flag);
+    if (part == 0) CA_BAR_OR(1);
+    else CA_BAR_OR(2);                                   // groups of more than one warp come in pairs at most
+#undef CA_BAR_OR
+    return any != 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -206,75 +216,76 @@ __device__ __forceinline__ void part_sync(int part, int nthreads) {
 // ---------------------------------------------------------------------------
 template <bool NSC>
 struct StagePipe {
-    uint64_t* full;          // kStages barriers of this part
-    unsigned char* base;     // kStages stage buffers of this part
-    const CUtensorMap* mv;
-    const CUtensorMap* msc;
-    int ROWS, stage_bytes, row_bytes, u, h0, w0;
+    uint32_t full;           // kStages barriers of this part (shared-space address)
+    uint32_t base;           // stage buffers of this part
+    int kc;                  // next column to copy
 
-    __device__ __forceinline__ unsigned char* vec(int buf) const { return base + (size_t)buf * stage_bytes; }
-    __device__ __forceinline__ int sstride() const { return (ROWS * 4 + 127) & ~127; }
-    __device__ __forceinline__ int vbytes() const { return (ROWS * row_bytes + 127) & ~127; }
-    __device__ __forceinline__ float* sc0(int buf) const { return reinterpret_cast<float*>(vec(buf) + vbytes()); }
-    __device__ __forceinline__ float* sc1(int buf) const { return reinterpret_cast<float*>(vec(buf) + vbytes() + sstride()); }
+    __device__ __forceinline__ uint32_t bar(int buf) const { return full + 8 * buf; }
+    __device__ __forceinline__ uint32_t vec(int buf, const TileArgs& a) const { return base + buf * a.stage_bytes; }
+    // the two scalar planes of a stage, behind its rows
+    static __device__ __forceinline__ uint32_t plane_bytes(int rows) { return (rows * 4 + 127) & ~127; }
+    __device__ __forceinline__ uint32_t sc0(int buf, const TileArgs& a, int rows) const { return vec(buf, a) + ((rows * a.row_bytes + 127) & ~127); }
 
-    __device__ __forceinline__ void issue(const Geo& g, int s, int buf) const {
-        const int kc = stage_column(g, w0, s);
-        mbar_arrive_expect_tx(&full[buf], (uint32_t)(ROWS * row_bytes + (NSC ? ROWS * 8 : 0)));
-        tma_load_4d(vec(buf), mv, 0, h0, kc, u, &full[buf]);
+    __device__ __forceinline__ void issue(int buf, const TileArgs& a, const CUtensorMap* mv, const CUtensorMap* msc, int rows, int u, int h0) {
+        mbar_arrive_expect_tx(bar(buf), (uint32_t)(rows * a.row_bytes + (NSC ? rows * 8 : 0)));
+        tma_load_4d(vec(buf, a), mv, 0, h0, kc, u, bar(buf));
         if (NSC) {
-            tma_load_3d(sc0(buf), msc, h0, kc, 2 * u, &full[buf]);
-            tma_load_3d(sc1(buf), msc, h0, kc, 2 * u + 1, &full[buf]);
+            const uint32_t s0 = sc0(buf, a, rows);
+            tma_load_3d(s0, msc, h0, kc, 2 * u, bar(buf));
+            tma_load_3d(s0 + plane_bytes(rows), msc, h0, kc, 2 * u + 1, bar(buf));
         }
+        kc = kc + 1 == a.g.Wk ? 0 : kc + 1;
     }
 };
 
 // Declares the pipeline of this thread's part and starts the first copies.
 // Needs in scope: a (TileArgs), g, ROWS, u, h0, w0, NSTAGES (stages of the tile), mv, msc.
-#define CA_PIPE_PROLOGUE(NSCV, PARTS)                                                                       \
+// PARTS: most groups of warps that the kernel is launched with.
+#define CA_PIPE_PROLOGUE(NSCV, PARTS)                                                                \
     extern __shared__ unsigned char smem_raw[];                                                      \
-    __shared__ __align__(8) uint64_t full_bar[PARTS * kStages];                                          \
-    __shared__ int s_err;                                                                            \
-    const int PT = blockDim.x / a.nsplit;          /* threads per part */                            \
-    const int part = threadIdx.x / PT;                                                               \
+    __shared__ __align__(8) uint64_t full_bar[PARTS * kStages];                                         \
+    const int PT = PARTS == 1 ? blockDim.x : blockDim.x / a.nsplit;          /* threads per part */  \
+    const int part = PARTS == 1 ? 0 : threadIdx.x / PT;                                              \
     const int lt = threadIdx.x - part * PT;                                                          \
-    const int s_begin = PARTS == 2 ? part * (NSTAGES / a.nsplit) : part * NSTAGES / a.nsplit;        \
-    const int s_end = (part + 1 == a.nsplit) ? NSTAGES : (PARTS == 2 ? (part + 1) * (NSTAGES / a.nsplit) : (part + 1) * NSTAGES / a.nsplit); \
+    const int s_begin = PARTS == 1 ? 0 : part * NSTAGES / a.nsplit;                                  \
+    const int s_end = PARTS == 1 ? NSTAGES : (part + 1) * NSTAGES / a.nsplit;                        \
     unsigned char* smem_al = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);            \
     StagePipe<NSCV> pipe;                                                                            \
-    pipe.full = full_bar + part * kStages;                                                           \
-    pipe.base = smem_al + (size_t)part * a.nstages * a.stage_bytes;                                  \
-    pipe.mv = &mv; pipe.msc = &msc;                                                                  \
-    pipe.ROWS = ROWS; pipe.stage_bytes = a.stage_bytes; pipe.row_bytes = a.row_bytes;                \
-    pipe.u = u; pipe.h0 = h0; pipe.w0 = w0;                                                          \
+    pipe.full = smem_u32(full_bar) + part * kStages * 8;                                             \
+    pipe.base = smem_u32(smem_al) + part * a.nstages * a.stage_bytes;                                \
+    pipe.kc = stage_column(g, w0, s_begin);                                                          \
     if (threadIdx.x == 0) {                                                                          \
-        for (int i = 0; i < PARTS * kStages; ++i) mbar_init(&full_bar[i], 1);                            \
-        s_err = 0;                                                                                   \
+        for (int i = 0; i < PARTS * kStages; ++i) mbar_init(&full_bar[i], 1);                        \
         mbar_fence_init();                                                                           \
     }                                                                                                \
     __syncthreads();                                                                                 \
     if (lt == 0)                                                                                     \
-        for (int i = 0; i < a.nstages && s_begin + i < s_end; ++i) pipe.issue(g, s_begin + i, i);
+        for (int i = 0; i < a.nstages && s_begin + i < s_end; ++i) pipe.issue(i, a, &mv, &msc, ROWS, u, h0);
 
-// Consumer loop over the stages of this part: bounded wait, BODY, recycle the buffer.
-#define CA_PIPE_LOOP(PARTS, ...)                                                                            \
+// Consumer loop over the stages of this part: bounded wait, BODY (sees s and buf), recycle the buffer.  What a stage costs
+// besides its window rows counts where windows are short: running counters instead of divisions, one barrier that
+// also collects the error flag, 32-bit shared addresses (320 x 320, 4 units of 64 channels, ws 7: dq 464 -> 313 us, dk/dv
+// 588 -> 435, forward 281 -> 249, apply 196 -> 178; a fifth to a third of each).
+#define CA_PIPE_LOOP(...)                                                                            \
+    bool s_err = false;                                                                              \
+    int buf = 0;                                                                                     \
+    uint32_t full_phase = 0;                                                                         \
     for (int s = s_begin; s < s_end; ++s) {                                                          \
-        const int it = s - s_begin;                                                                  \
-        const int buf = it % a.nstages;                                                              \
-        if (!mbar_wait(&pipe.full[buf], (uint32_t)((it / a.nstages) & 1), a.wait_tries)) s_err = 1;  \
+        const bool lost = !mbar_wait(pipe.bar(buf), full_phase, a.wait_tries);                       \
         __VA_ARGS__                                                                                  \
-        part_sync<PARTS>(part, PT);                                                                         \
+        s_err = part_any(part, PT, lost);                                                            \
         if (s_err) break;                                                                            \
-        if (lt == 0 && s + a.nstages < s_end) pipe.issue(g, s + a.nstages, buf);                     \
+        if (lt == 0 && s + a.nstages < s_end) pipe.issue(buf, a, &mv, &msc, ROWS, u, h0);                \
+        if (++buf == a.nstages) { buf = 0; full_phase ^= 1; }                                        \
     }                                                                                                \
-    __syncthreads();                                                                                 \
+    s_err = __syncthreads_or(s_err);                                                                 \
     /* A wait that ran out: the CTA stops computing, reports (device counter, caller's status word)  \
        and poisons what it still stores with NaN, so that the failure cannot pass for a result. */   \
     float ca_poison = 0.f;                                                                           \
     if (s_err) {                                                                                     \
         /* give copies still in flight a bounded chance to land before the CTA exits */              \
         if (lt == 0)                                                                                 \
-            for (int i = 0; i < a.nstages; ++i) mbar_wait(&pipe.full[i], 0, 1u << 12);               \
+            for (int i = 0; i < a.nstages; ++i) mbar_wait(pipe.bar(i), 0, 1u << 12);               \
         if (threadIdx.x == 0) {                                                                      \
             atomicAdd(a.timeouts, 1);                                                         \
             if (a.status) atomicOr(a.status, 1);                                                     \
