@@ -303,7 +303,7 @@ int run_apply<kAnyC>(const Geo& g, const Padded& P, const float* nz, const float
     const size_t most = nq == 1 ? 6 : 4;                     // CTAs per SM that the registers allow
     auto setup = [&](int nbuf, int max_split, int max_warps) {
         L = Launch{};
-        rc = prepare(g, P, nq, 17 * nq, "CIRCATT_APPLY_WARPS", packed, nullptr, &L, nq == 1 ? 1 : max_split, max_warps, ns, true, 2);
+        rc = prepare(g, P, operator_tile(g, ns, nq, nq == 1 ? 1 : max_split, max_warps), 17 * nq, packed, nullptr, &L, ns, true, 2);
         L.a.nbuf = nbuf;
         const size_t words = (size_t)nbuf * run_area(g, rows, nq, loose);
         const size_t need = (size_t)L.a.nsplit * 2 * L.a.stage_bytes + (size_t)L.threads / 32 * words * sizeof(float) + 1024;

@@ -420,6 +420,12 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 4 : NQ == 2 ? 3 : 2)) dkdv_til
 
 }  // namespace
 
+// Columns per thread: 1 (for short windows and small grids, and folded signals, whose streamed column pairs with one centre
+// column only), 2 (160 registers, three blocks per SM) or 3 (255, two blocks).
+static const SweepCost kDqCost[3][3] = {{{1, 20, 0, 123, 501, 4921}, {2, 12, 9, 135, 936, 7404}, {3, 8, 22, 183, 1437, 10612}},
+                                        {{1, 20, 59, 112, 0, 6247}, {2, 12, 15, 158, 146, 9951}, {3, 8, 53, 207, 0, 15865}},
+                                        {{1, 20, 79, 124, 645, 0}, {2, 12, 55, 167, 964, 0}, {3, 8, 122, 192, 1635, 0}}};
+
 template <>
 int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* dy, const float* stats,
            const float* D, const float* kv, float* dq, cudaStream_t st, int mode, float* Dout) {
@@ -427,25 +433,26 @@ int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const fl
     const int ns = slabs_of(g);
     if (ns > 1 && mode) return CA_ERR_UNSUPPORTED;             // the entmax variants exist for one-slab units
     if (mode >= 3) return CA_ERR_UNSUPPORTED;                  // the forward's sweeps go through run_entmax_fwd_sweep
-    // two query columns per thread measured faster than four at every size for the dq sweeps of one-slab units (160
-    // registers, three blocks per SM, against 255 and two), the entmax ones included: 128 x 96, 8 units, ws 15, dq
-    // 105 -> 67 us, its pre-pass 84 -> 63 us.  The pre-pass runs without a stage split.
-    // (folded signals: one, see run_fwd)
+    // the entmax variants have two columns per thread (128 x 96, 8 units, ws 15, against four: dq 105 -> 67 us, its
+    // pre-pass 84 -> 63 us); the pre-pass does not share stages
     const bool fold = g.wsw == 1 && mode == 0;
-    const int nq = fold ? 1 : (ns > 1 ? (g.ws <= 9 ? 2 : 4) : 2);
-    int rc = prepare(g, P, nq, 17 * nq, "CIRCATT_DQ_WARPS", kv, nullptr, &L, mode < 2 && ns == 1 && !fold ? 2 : 1, 4, ns);
+    const SweepCost* cost = kDqCost[ns == 1 ? 0 : ns / 2] + (mode ? 1 : 0);
+    const TileShape t = choose_tile(g, P, ns, cost, fold || mode ? 1 : 3, mode < 2 && ns == 1 ? kParts : 1, false);
+    int rc = prepare(g, P, t, 17 * t.nq, kv, nullptr, &L, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.c1 = dy; L.a.cs0 = stats; L.a.cs1 = D; L.a.o0 = dq; L.a.ostats = Dout;
-    if (fold && ns == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 1, 0, 16, L, st);
-    else if (fold && ns == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 1, 0, 32, L, st);
-    else if (fold) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 1, 0, 64, L, st);
-    else if (ns == 2 && nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 32, L, st);
-    else if (ns == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 32, L, st);
-    else if (ns == 4 && nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 64, L, st);
-    else if (ns == 4) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 4, 0, 64, L, st);
-    else if (mode == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 2, 16, L, st);
+#define CA_DQ(NCRV_)                                                                          \
+    do {                                                                                      \
+        if (t.nq == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 1, 0, NCRV_, L, st);      \
+        else if (t.nq == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, NCRV_, L, st); \
+        else CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 3, 0, NCRV_, L, st);                \
+    } while (0)
+    if (mode == 2) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 2, 16, L, st);
     else if (mode == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 1, 16, L, st);
-    else CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 2, 0, 16, L, st);
+    else if (ns == 1) CA_DQ(16);
+    else if (ns == 2) CA_DQ(32);
+    else CA_DQ(64);
+#undef CA_DQ
     CA_CHECK_LAUNCH("tiled dq kernel");
     return CA_OK;
 }
@@ -457,7 +464,7 @@ int run_entmax_fwd_sweep<kAnyC>(const Geo& g, const Padded& P, float scale, int 
                          float* tau, float* settled, float* y, int mode, int iter, cudaStream_t st) {
     Launch L{};
     if (slabs_of(g) > 1) return CA_ERR_UNSUPPORTED;
-    int rc = prepare(g, P, 4, 17 * 4, "CIRCATT_DQ_WARPS", kv, nullptr, &L, 1, 4, 1);
+    int rc = prepare(g, P, TileShape{4, std::min(4, (g.H + 31) / 32), 1}, 17 * 4, kv, nullptr, &L, 1);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.cs0 = tau; L.a.cs1 = settled; L.a.o0 = y; L.a.o1 = settled; L.a.ostats = tau;
     L.a.iter = iter;
@@ -468,6 +475,12 @@ int run_entmax_fwd_sweep<kAnyC>(const Geo& g, const Padded& P, float scale, int 
     return CA_OK;
 }
 
+// Columns per thread: 1 (three or four blocks per SM) or 3 (255 registers, two).  Two measured slower than one of them at
+// every shape.
+static const SweepCost kDkdvCost[3][2] = {{{1, 16, 13, 135, 190, 7335}, {3, 8, 201, 188, 1070, 14075}},
+                                          {{1, 16, 82, 118, 0, 6933}, {3, 8, 138, 239, 0, 15999}},
+                                          {{1, 16, 70, 146, 804, 0}, {3, 8, 234, 225, 1472, 0}}};
+
 template <>
 int run_dkdv<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* k, const float* v, const float* qdy,
              const float* planes, float* dk, float* dv, cudaStream_t st, bool entmax) {
@@ -475,17 +488,21 @@ int run_dkdv<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const 
     const int ns = slabs_of(g);
     if (ns > 1 && entmax) return CA_ERR_UNSUPPORTED;
     const bool fold = g.wsw == 1 && !entmax;
-    const int nq = fold ? 1 : 3;
-    int rc = prepare(g, P, nq, 33 * nq, "CIRCATT_DKDV_WARPS", qdy, planes, &L, ns == 1 && !fold ? 2 : 1, 4, ns);
+    const SweepCost* cost = kDkdvCost[ns == 1 ? 0 : ns / 2] + (entmax ? 1 : 0);
+    const TileShape t = choose_tile(g, P, ns, cost, fold || entmax ? 1 : 2, ns == 1 ? kParts : 1, true);
+    int rc = prepare(g, P, t, 33 * t.nq, qdy, planes, &L, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = k; L.a.c1 = v; L.a.o0 = dk; L.a.o1 = dv;
-    if (fold && ns == 1) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 1, false, 16, L, st);
-    else if (fold && ns == 2) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 1, false, 32, L, st);
-    else if (fold) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 1, false, 64, L, st);
-    else if (ns == 2) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 32, L, st);
-    else if (ns == 4) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 64, L, st);
-    else if (entmax) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, true, 16, L, st);
-    else CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, 16, L, st);
+#define CA_DKDV(NCRV_)                                                                                \
+    do {                                                                                              \
+        if (t.nq == 1) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 1, false, NCRV_, L, st);        \
+        else CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, false, NCRV_, L, st);                  \
+    } while (0)
+    if (entmax) CA_DIST_CPE_NQ(dkdv_tiled_kernel, dist, g.cpe, 3, true, 16, L, st);
+    else if (ns == 1) CA_DKDV(16);
+    else if (ns == 2) CA_DKDV(32);
+    else CA_DKDV(64);
+#undef CA_DKDV
     CA_CHECK_LAUNCH("tiled dk/dv kernel");
     return CA_OK;
 }

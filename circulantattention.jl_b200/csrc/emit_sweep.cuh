@@ -166,8 +166,7 @@ int run_emit<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const 
     int rc = CA_OK;
     auto setup = [&](int stages) {
         L = Launch{};
-        rc = prepare(g, P, nq, 0, "CIRCATT_EMIT_WARPS", packed, nullptr, &L, nq == 1 ? 1 : 2, 4, ns,
-                     single, stages);
+        rc = prepare(g, P, operator_tile(g, ns, nq, nq == 1 ? 1 : 2, 4), 0, packed, nullptr, &L, ns, single, stages);
         // per warp: staging tile, run rotations, offset table
         if (!rc) L.smem += (size_t)L.threads / 32 * (32 / ns) * (nq * (ch + 1) + nq + ch) * sizeof(float);
         return rc;
@@ -176,9 +175,8 @@ int run_emit<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const 
     {
         const size_t per_sm = 227 * 1024, with3 = L.smem + 1024;          // + the driver's per-CTA reservation
         const size_t with2 = with3 - (size_t)L.a.nsplit * L.a.stage_bytes;
-        const int want = tune_int("CIRCATT_EMIT_STAGES", 0);
         const size_t most = nq == 1 ? 6 : 4;                 // CTAs per SM that the registers allow
-        if (want == 2 || (want == 0 && std::min(most, per_sm / with2) > std::min(most, per_sm / with3)))
+        if (std::min(most, per_sm / with2) > std::min(most, per_sm / with3))
             if (setup(2)) return rc;
     }
     if (L.smem > 200 * 1024) return CA_ERR_UNSUPPORTED;

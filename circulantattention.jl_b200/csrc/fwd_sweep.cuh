@@ -290,23 +290,20 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tile
 
 }  // namespace
 
+// Columns per thread: 1 (five blocks per SM; short windows, small grids, folded signals), 2 or 3 (168 registers, three
+// blocks per SM; with packed outer products three beat four, 255 registers and two blocks, 5.68 against 6.07 ms at
+// 1024 x 1024, 8 units, ws 21).
+static const SweepCost kFwdCost[3][3] = {{{1, 20, 0, 129, 216, 3265}, {2, 12, 0, 121, 532, 5634}, {3, 12, 16, 138, 684, 8536}},
+                                         {{1, 20, 36, 105, 145, 4276}, {2, 12, 0, 131, 130, 8597}, {3, 12, 53, 125, 0, 14976}},
+                                         {{1, 20, 3, 141, 421, 0}, {2, 12, 0, 154, 726, 0}, {3, 12, 6, 166, 1454, 0}}};
+
 template <>
 int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* kv, float* y, float* stats,
                    cudaStream_t st) {
     Launch L{};
     const int ns = slabs_of(g);
-    // three columns per thread (168 registers, three CTAs per SM), or two where the window is short (with ws <= 9 most
-    // stages of a wide tile pair with only some of its columns) or the grid smaller than the chip.  Measured, with packed
-    // outer products: three against four columns (255 registers, two CTAs) 5.68 and 6.07 ms at 1024 x 1024, 8 units, ws 21;
-    // three against two 54 and 61 us at 128 x 96, 8 units, ws 15, 22 and 17 us at 64 x 64, one unit.  Wide units: four once
-    // there are eight warps of such tiles per SM (200 x 150, two units of 64 channels, ws 21: 263 against 270 us; 128 x 96:
-    // 77 against 63 us).
-    // a folded signal has one column per thread: a streamed column pairs with one centre column only, and a wider tile
-    // computes the others for nothing (8192 x 64 x 4, ws 63, 64 channels: 92 us, see below)
-    const bool fold = g.wsw == 1;
-    auto warps_at = [&](int n) { return (long)((g.W + n - 1) / n) * ((g.H * ns + 31) / 32) * g.units; };
-    const int nq = fold ? 1 : (g.ws <= 9 ? 2 : (ns > 1 ? (warps_at(4) >= 8L * sm_count() ? 4 : 3) : (warps_at(3) < sm_count() ? 2 : 3)));
-    int rc = prepare(g, P, nq, 18 * nq, "CIRCATT_FWD_WARPS", kv, nullptr, &L, ns == 1 && !fold ? 2 : 1, 4, ns);
+    const TileShape t = choose_tile(g, P, ns, kFwdCost[ns == 1 ? 0 : ns / 2], g.wsw == 1 ? 1 : 3, ns == 1 ? kParts : 1, false);
+    int rc = prepare(g, P, t, 18 * t.nq, kv, nullptr, &L, ns);
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.o0 = y; L.a.ostats = stats;
 #define CA_FWD2(DCV, EX, NQV, NCRV_)                                                            \
@@ -319,43 +316,26 @@ int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const f
             else CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, false, 2, EX, NQV, NCRV_>), L, st);     \
         }                                                                                \
     } while (0)
-#define CA_FWD(DCV)                                                                      \
+    // chunks of 7, 5 or 3 keys where they divide the window, else chunks of four plus a tail
+#define CA_FWD(NQV, NCRV_)                                                               \
     do {                                                                                 \
-        if (nq == 2) CA_FWD2(DCV, true, 2, 16);                                          \
-        else CA_FWD2(DCV, true, 3, 16);                                                  \
+        if (g.ws % 7 == 0) CA_FWD2(7, true, NQV, NCRV_);                                 \
+        else if (g.ws % 5 == 0) CA_FWD2(5, true, NQV, NCRV_);                            \
+        else if (NQV > 1 && NCRV_ == 16 && g.ws % 3 == 0) CA_FWD2((NQV > 1 && NCRV_ == 16 ? 3 : 5), true, NQV, NCRV_); \
+        else CA_FWD2(4, false, NQV, NCRV_);                                              \
     } while (0)
-    // chunks of 7 or 5 keys where they divide the window, else chunks of four plus a tail
-#define CA_FWD_FOLD(NCRV_)                                                               \
+#define CA_FWD_NQ(NCRV_)                                                                 \
     do {                                                                                 \
-        if (g.ws % 7 == 0) CA_FWD2(7, true, 1, NCRV_);                                   \
-        else if (g.ws % 5 == 0) CA_FWD2(5, true, 1, NCRV_);                              \
-        else CA_FWD2(4, false, 1, NCRV_);                                                \
+        if (t.nq == 1) CA_FWD(1, NCRV_);                                                 \
+        else if (t.nq == 2) CA_FWD(2, NCRV_);                                            \
+        else CA_FWD(3, NCRV_);                                                           \
     } while (0)
-    if (fold && ns == 1) CA_FWD_FOLD(16);
-    else if (fold && ns == 2) CA_FWD_FOLD(32);
-    else if (fold) CA_FWD_FOLD(64);
-#define CA_FWD_WIDE(NCRV_)                                                               \
-    do {                                                                                 \
-        if (nq == 2 && g.ws % 7 == 0) CA_FWD2(7, true, 2, NCRV_);                        \
-        else if (nq == 2) CA_FWD2(4, false, 2, NCRV_);                                   \
-        else if (nq == 4 && g.ws % 7 == 0) CA_FWD2(7, true, 4, NCRV_);                   \
-        else if (nq == 4 && g.ws % 5 == 0) CA_FWD2(5, true, 4, NCRV_);                   \
-        else if (nq == 4) CA_FWD2(4, false, 4, NCRV_);                                   \
-        else if (g.ws % 7 == 0) CA_FWD2(7, true, 3, NCRV_);                              \
-        else if (g.ws % 5 == 0) CA_FWD2(5, true, 3, NCRV_);                              \
-        else CA_FWD2(4, false, 3, NCRV_);                                                \
-    } while (0)
-    else if (ns == 2) CA_FWD_WIDE(32);
-    else if (ns == 4) CA_FWD_WIDE(64);
-    else if (g.ws % 7 == 0) CA_FWD(7);
-    else if (g.ws % 5 == 0) CA_FWD(5);
-    else if (g.ws % 3 == 0) CA_FWD(3);
-    else if (nq == 2) CA_FWD2(4, false, 2, 16);
-    else CA_FWD2(4, false, 3, 16);
-#undef CA_FWD_WIDE
-#undef CA_FWD_FOLD
-#undef CA_FWD2
+    if (ns == 1) CA_FWD_NQ(16);
+    else if (ns == 2) CA_FWD_NQ(32);
+    else CA_FWD_NQ(64);
+#undef CA_FWD_NQ
 #undef CA_FWD
+#undef CA_FWD2
     CA_CHECK_LAUNCH("tiled forward kernel");
     return CA_OK;
 }

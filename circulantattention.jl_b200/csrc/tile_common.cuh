@@ -4,9 +4,9 @@
 #include "tiled.cuh"
 #include "tma.cuh"
 #include <cuda_bf16.h>
-#include <stdlib.h>
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <type_traits>
 
 namespace ca {
@@ -513,17 +513,6 @@ inline bool fold_geo(const Geo& in, Geo* out) {
     return true;
 }
 
-// Launch-shape overrides for tuning sessions.  Compiled out of the shipped library (the build
-// never defines CA_TUNING): no launch reads the environment.
-#ifdef CA_TUNING
-inline int tune_int(const char* name, int dflt) {
-    const char* v = getenv(name);
-    return v && *v ? atoi(v) : dflt;
-}
-#else
-inline int tune_int(const char*, int dflt) { return dflt; }
-#endif
-
 struct Launch {
     TileArgs a;
     CUtensorMap mv, msc;
@@ -545,28 +534,80 @@ inline int sm_count() {
     return n;
 }
 
-// Fills the launch geometry and the tensor maps of the packed pair (and of the
-// scalar planes when given).  `nq` centre pixels per thread, `xch_floats` per
-// thread for the merge of a split tile.  CTAs have at most 128 threads: four
-// warps of rows, or two warps of rows times two stage groups on small grids.
-inline int prepare(const Geo& g, const Padded& P, int nq, int xch_floats, const char* env_warps, const float* pair,
-            const float* planes, Launch* L, int max_split = 2, int max_warps = 4, int ns = 1,
-            bool single = false, int stages = kStages) {
+// How a sweep is cut into blocks: `nq` centre columns per thread, `warps` warps of pixel rows per block and `nsplit` groups
+// of such warps that share the stages of a tile (warps * nsplit <= 4).
+struct TileShape {
+    int nq, warps, nsplit;
+};
+
+// What a sweep with `nq` columns per thread costs, in cycles: a window row takes a warp `lat` + `issue` for each warp on its
+// scheduler, a stage `stage` more, a block `block`; an SM holds `sm_warps` warps of it.  Fitted to the measured times of
+// 25 shapes (32 x 32 to 512 x 512, 1 to 16 units of 16, 32 and 64 channels, windows 5 to 21) in every cut; rms error of a
+// predicted time 5 to 11 %.
+struct SweepCost {
+    int nq, sm_warps;
+    float lat, issue, stage, block;
+};
+
+inline int tile_stage_bytes(int rows, int row_bytes, bool planes, bool single) {
+    const int vbytes = (rows * row_bytes + 127) & ~127;
+    return single ? vbytes : (vbytes + (planes ? 2 * ((rows * 4 + 127) & ~127) : 0) + 1023) & ~1023;
+}
+
+// The cut with the least predicted time.  What decides: rows of a tile past the image (75 rows are three warps, not two
+// tiles of 64), whole waves of blocks, window rows left to a warp when the stages are shared, and few wide tiles
+// against many narrow ones where a window is short or a grid small (a tile of nq columns streams ws + nq - 1).  Over the
+// 25 shapes the choice is within 10 % of the best cut but for two.  Against four warps of rows and fixed columns:
+// 75 x 53, 9 units, ws 11: forward 27 -> 21 us, dq 40 -> 24, dk/dv 66 -> 35; 128 x 96, 4 units of 64 channels, ws 15: dq
+// 211 -> 160, dk/dv 262 -> 202; 32 x 32, 1 unit, ws 7: forward 8.0 -> 5.1, dq 10 -> 6, dk/dv 20 -> 6.8.
+inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepCost* cost, int n, int max_split, bool planes) {
+    TileShape best{cost[0].nq, 1, 1};
+    float least = INFINITY;
     const int rw = 32 / ns;                             // pixel rows per warp (ns lanes share a pixel)
+    const float sms = (float)sm_count();
+    for (const SweepCost* c = cost; c < cost + n; ++c) {
+        const int nst = g.wsw + c->nq - 1;
+        const float cols = (float)((g.W + c->nq - 1) / c->nq) * g.units;
+        for (int w = 4; w >= 1; --w) {
+            if (w > 1 && rw * (w - 1) >= g.H) continue;
+            const int stage = tile_stage_bytes(rw * w + 2 * P.pp, kRowBytes * ns, planes, false);
+            const float blocks = cols * ((g.H + rw * w - 1) / (rw * w));
+            for (int s = 1; w * s <= 4 && s <= max_split && s <= nst; ++s) {
+                if (s * 2 * stage > 216 * 1024) break;              // not even two copies in flight
+                const int resident = std::max(1, std::min(c->sm_warps / (w * s), 227 * 1024 / (s * kStages * stage + 2048)));
+                const float waves = blocks / (resident * sms);
+                // warps per scheduler, and how many times a block's time passes: whole waves while there are few (the
+                // blocks of a wave end together), later half a wave is lost at the end
+                const float k = waves <= 1.f ? std::ceil(std::ceil(blocks / sms) * (w * s) / 4) : std::max(1.f, resident * (w * s) / 4.f);
+                const float turns = waves <= 2.f ? std::ceil(waves) : std::min(std::ceil(waves), waves + 0.5f);
+                float t = turns * (((nst + s - 1) / s) * (g.ws * (c->lat + c->issue * k) + c->stage) + c->block);
+                // tiles of one or two warps copy more halo rows; it shows once blocks follow one another (the forward
+                // at 500 x 400, 3 units, ws 11: 209 us with one warp, 172 with two, 167 with four)
+                if (waves > 1.f) t *= w == 1 ? 1.08f : (w == 2 ? 1.02f : 1.f);
+                if (t < least) { least = t; best = TileShape{c->nq, w, s}; }
+            }
+        }
+    }
+    return best;
+}
+
+// Operators: four warps of rows; fewer than 6 warps per SM share the stages of a tile (in four where the kernel can,
+// in two up to 12 warps per SM).
+inline TileShape operator_tile(const Geo& g, int ns, int nq, int max_split, int max_warps) {
+    const int rw = 32 / ns;
+    const int warps = std::min(max_warps, (g.H + rw - 1) / rw);
+    const long tasks = (long)((g.W + nq - 1) / nq) * ((g.H + rw * warps - 1) / (rw * warps)) * g.units * warps;
+    int nsplit = max_split == 4 ? (tasks < 6L * sm_count() ? 4 : (tasks < 12L * sm_count() ? 2 : 1)) : (tasks < 6L * sm_count() ? 2 : 1);
+    nsplit = std::min(nsplit, max_split);
+    return TileShape{nq, warps * nsplit > 4 ? 4 / nsplit : warps, nsplit};
+}
+
+// Fills the launch geometry and the tensor maps of the packed pair (and of the scalar planes when given).
+// `xch_floats` per thread for the merge of a split tile.
+inline int prepare(const Geo& g, const Padded& P, TileShape t, int xch_floats, const float* pair, const float* planes, Launch* L,
+                   int ns, bool single = false, int stages = kStages) {
+    const int rw = 32 / ns, warps = t.warps, nsplit = t.nsplit;
     const int rf = (single ? kSingleFloats : kRowFloats) * ns, rb = rf * 4;
-    int warps = (g.H + rw - 1) / rw;
-    if (warps > max_warps) warps = max_warps;
-    const long cols = (g.W + nq - 1) / nq;
-    const long ctas4 = cols * ((g.H + rw * warps - 1) / (rw * warps)) * g.units;
-    // fewer than 6 warps per SM without a split: split the stages of a tile (in four where the kernel can and 12
-    // warps per SM fit, in two otherwise)
-    const long tasks = ctas4 * warps;
-    int nsplit = max_split == 4 ? (tasks < 6L * sm_count() ? 4 : (tasks < 12L * sm_count() ? 2 : 1))
-                                : (tasks < 6L * sm_count() ? 2 : 1);
-    nsplit = tune_int("CIRCATT_SPLIT", nsplit);
-    if (nsplit > max_split) nsplit = max_split;
-    warps = tune_int(env_warps, warps);
-    if (warps * nsplit > 4) warps = 4 / nsplit;
     TileArgs& a = L->a;
     a.g = g;
     a.status = status_word();
@@ -578,10 +619,8 @@ inline int prepare(const Geo& g, const Padded& P, int nq, int xch_floats, const 
     a.row_bytes = rb;
     const int ROWS = a.TH + 2 * P.pp;
     if (ROWS > 256) { set_error("tile of %d rows exceeds the TMA box limit", ROWS); return CA_ERR_UNSUPPORTED; }
-    const int sstride = (ROWS * 4 + 127) & ~127;
-    const int vbytes = (ROWS * rb + 127) & ~127;
-    a.stage_bytes = single ? vbytes : (vbytes + (planes ? 2 * sstride : 0) + 1023) & ~1023;
-    L->grid = dim3((unsigned)cols, (g.H + a.TH - 1) / a.TH, g.units);
+    a.stage_bytes = tile_stage_bytes(ROWS, rb, planes != nullptr, single);
+    L->grid = dim3((unsigned)((g.W + t.nq - 1) / t.nq), (g.H + a.TH - 1) / a.TH, g.units);
     L->threads = 32 * warps * nsplit;
     // long windows of wide units: two copies in flight where three do not fit
     if (stages > 2 && (size_t)nsplit * stages * a.stage_bytes > 216 * 1024) stages = 2;
@@ -595,12 +634,12 @@ inline int prepare(const Geo& g, const Padded& P, int nq, int xch_floats, const 
     const uint64_t strides[3] = {(uint64_t)rb, (uint64_t)P.Hp * rb, (uint64_t)P.Hp * rb * g.Wk};
     const uint32_t box[4] = {(uint32_t)rf, (uint32_t)ROWS, 1, 1};
     int rc;
-    if ((rc = encode_tensor_map(&L->mv, pair, 4, dims, strides, box, false))) return rc;
+    if ((rc = encode_tensor_map(&L->mv, pair, 4, dims, strides, box))) return rc;
     if (planes) {
         const uint64_t sdims[3] = {(uint64_t)P.Hp, (uint64_t)g.Wk, (uint64_t)2 * g.units};
         const uint64_t sstr[2] = {(uint64_t)P.Hp * 4, (uint64_t)P.Hp * 4 * g.Wk};
         const uint32_t sbox[3] = {(uint32_t)ROWS, 1, 1};
-        if ((rc = encode_tensor_map(&L->msc, planes, 3, sdims, sstr, sbox, false))) return rc;
+        if ((rc = encode_tensor_map(&L->msc, planes, 3, sdims, sstr, sbox))) return rc;
     } else {
         L->msc = L->mv;
     }

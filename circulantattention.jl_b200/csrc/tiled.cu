@@ -177,7 +177,7 @@ int tiled_attention_bwd(const Geo& gin, float scale, int dist, const float* q, c
     int rc = launch_pack(pa, st);
     if (rc) return rc;
     const bool small = (long)g.Np * g.units < 2048L * sm_count();      // fewer than ~4 CTAs per SM per sweep
-    if (small && tune_int("CIRCATT_CONCURRENT", 1)) {
+    if (small) {
         ForkJoin* f = fork_join_for_current_device();
         if (f && cudaEventRecord(f->fork, st) == cudaSuccess && cudaStreamWaitEvent(f->side, f->fork, 0) == cudaSuccess) {
             rc = CA_CHANNELS(g, run_dkdv, g, P, scale, dist, k, v, qdy, planes, dk, dv, f->side, false);

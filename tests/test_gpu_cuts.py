@@ -1,0 +1,49 @@
+"""How the tiled sweeps are cut into blocks: one to three columns per thread, one to four warps of rows, stages shared by one
+to four groups of warps.  The shapes reach those cuts on a B200 (148 SMs)."""
+import numpy as np
+import pytest
+
+from oracle import circatt_oracle as orc
+from tests.helpers import KIND, assert_close, randn, up
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("simname", ["dot", "distance"])
+@pytest.mark.parametrize("shape,ws,nheads,cplx", [
+    ((32, 32, 16, 1), 7, 1, False),       # one column, one warp, stages in four
+    ((48, 48, 32, 1), 5, 2, False),       # stages in two and three; fewer stages than a thread's share would round to
+    ((16, 17, 8, 1), 3, 1, False),        # three stages among four groups at most
+    ((60, 50, 16, 2), 21, 1, False),      # three columns, stages in four
+    ((75, 53, 36, 3), 11, 3, False),      # one and two columns, three warps of rows, 12 channels
+    ((64, 64, 32, 4), 9, 2, False),       # two columns, two warps, stages in two
+    ((70, 31, 32, 2), 9, 1, False),       # two slabs: rows of 16 per warp, no shared stages
+    ((40, 40, 32, 2), 7, 1, True),        # four slabs, one column
+])
+def test_cuts(ca, shape, ws, nheads, cplx, simname):
+    rng = np.random.default_rng(61)
+    qn, kn, vn, rn = (randn(rng, shape, cplx) for _ in range(4))
+    q, k, v = (ca.jl.from_numpy(t).requires_grad_(True) for t in (qn, kn, vn))
+    sim = ca.DotSimilarity() if simname == "dot" else ca.DistanceSimilarity()
+    n0 = ca.lib.ca_probe_tiled_launch_count()
+    y, _ = ca.circulant_mh_attention(sim, q, k, v, ws, nheads, return_A=False)
+    r = ca.jl.from_numpy(rn)
+    ((y * r.conj()).real.sum() if cplx else (y * r).sum()).backward()
+    assert ca.lib.ca_probe_tiled_launch_count() - n0 == 3
+    yo, _ = orc.mh_attention(KIND[simname], up(qn), up(kn), up(vn), ws, nheads)
+    dqo, dko, dvo = orc.mh_attention_pullback(KIND[simname], up(qn), up(kn), up(vn), ws, nheads, up(rn))
+    for name, got, want in (("y", y, yo), ("dq", q.grad, dqo), ("dk", k.grad, dko), ("dv", v.grad, dvo)):
+        assert_close(ca.jl.to_numpy(got), want, name)
+
+
+@pytest.mark.parametrize("shape,ws,nheads", [((32, 32, 16, 1), 7, 1), ((75, 53, 36, 3), 11, 3)])
+def test_cuts_entmax(ca, shape, ws, nheads):
+    rng = np.random.default_rng(62)
+    qn, kn, vn, rn = (randn(rng, shape) for _ in range(4))
+    q, k, v = (ca.jl.from_numpy(t).requires_grad_(True) for t in (qn, kn, vn))
+    y, _ = ca.circulant_mh_attention(ca.DotSimilarity(), q, k, v, ws, nheads, normalizer=ca.ENTMAX15, return_A=False)
+    (y * ca.jl.from_numpy(rn)).sum().backward()
+    yo, _ = orc.mh_attention(orc.DOT, up(qn), up(kn), up(vn), ws, nheads, orc.ENTMAX15)
+    dqo, dko, dvo = orc.mh_attention_pullback(orc.DOT, up(qn), up(kn), up(vn), ws, nheads, up(rn), norm=orc.ENTMAX15)
+    for name, got, want in (("y", y, yo), ("dq", q.grad, dqo), ("dk", k.grad, dko), ("dv", v.grad, dvo)):
+        assert_close(ca.jl.to_numpy(got), want, name)
