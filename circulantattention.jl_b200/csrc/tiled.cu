@@ -201,7 +201,7 @@ int tiled_attention_bwd_entmax(const Geo& gin, float scale, int dist, const floa
                                void* workspace, cudaStream_t st) {
     Geo g;
     if (!fold_geo(gin, &g)) return CA_ERR_UNSUPPORTED;
-    if (!tiled_shape_ok(g) || g.Wk != g.W || g.bf16) return CA_ERR_UNSUPPORTED;
+    if (!tiled_shape_ok(g) || g.Wk != g.W || g.bf16 || slabs_of(g) > 1) return CA_ERR_UNSUPPORTED;
     if (!workspace) { set_error("workspace is NULL"); return CA_ERR_NULL; }
     const Padded P = padded_of(g);
     float* kv = static_cast<float*>(workspace);

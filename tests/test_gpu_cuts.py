@@ -47,3 +47,14 @@ def test_cuts_entmax(ca, shape, ws, nheads):
     dqo, dko, dvo = orc.mh_attention_pullback(orc.DOT, up(qn), up(kn), up(vn), ws, nheads, up(rn), norm=orc.ENTMAX15)
     for name, got, want in (("y", y, yo), ("dq", q.grad, dqo), ("dk", k.grad, dko), ("dv", v.grad, dvo)):
         assert_close(ca.jl.to_numpy(got), want, name)
+
+
+@pytest.mark.parametrize("c", [24, 48])
+def test_wide_entmax_backward_launches(ca, c):
+    """Units past one slab take the operator chain at once: no pack is made for the fused sweeps they do not have."""
+    rng = np.random.default_rng(64)
+    q, k, v = (ca.jl.from_numpy(randn(rng, (20, 18, c, 1))).requires_grad_(True) for _ in range(3))
+    y, _ = ca.circulant_attention(ca.DotSimilarity(), q, k, v, 5, normalizer=ca.ENTMAX15, return_A=False)
+    n0 = ca.lib.ca_probe_launch_count()
+    y.sum().backward()
+    assert ca.lib.ca_probe_launch_count() - n0 == 12      # scores, weights, dv, dP, dS, dq, dk, and five packs
