@@ -43,6 +43,10 @@ struct Padded {
 template <bool ANYC>
 int run_fwd(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* kv, float* y, float* stats,
             cudaStream_t st);
+// The same and A's values in CSR order; CA_ERR_UNSUPPORTED where the rows of A do not fit the shared memory (values_fit).
+template <bool ANYC>
+int run_fwd_values(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* kv, float* y, float* stats,
+                   float* nz, cudaStream_t st);
 // mode 0: softmax; 1: entmax; 2: entmax pre-pass (writes D, needs no D and no dq).
 template <bool ANYC>
 int run_dq(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* dy, const float* stats,
@@ -94,6 +98,7 @@ __device__ __forceinline__ float lds32(uint32_t addr) {
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(addr));
     return x;
 }
+__device__ __forceinline__ void sts32(uint32_t addr, float x) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(x) : "memory"); }
 __device__ __forceinline__ float hsum2(u64 v) {
     float a, b;
     unpack2(v, a, b);
@@ -118,6 +123,7 @@ struct TileArgs {
     int iter;               // entmax threshold search: number of the step (late steps fall back to Newton)
     int row_bytes;          // bytes of one packed pixel row: 144 per 16-channel slab
     int nstages;            // copy stages in flight per part: 2 or 3 (kStages)
+    int extra_off;          // shared memory of the kernel's own behind the stages and the merge buffers, bytes
     int nbuf;               // apply: buffers for the staged values of A per warp (1 or 2)
     const float* c0;        // centre tensors (reference layout)
     const float* c1;
@@ -462,6 +468,13 @@ __device__ __forceinline__ void store_centre(float* dst, const Geo& g, int u, in
 // 16-channel slabs of a packed pixel row: 1, 2 or 4 (the channels past the unit's are zero).
 inline int slabs_of(const Geo& g) { return g.cr <= 16 ? 1 : (g.cr <= 32 ? 2 : 4); }
 
+// Whether the forward keeps the rows of A in shared memory and writes them itself: up to 11.6 KB per warp and column, past which
+// too few warps are left on an SM.  Forward and values in one kernel against two: 320 x 320, 8 units of 64 channels,
+// ws 7 (1.6 KB): 565 and 867 us; 150 x 140, 4 of 32, ws 11 (7.7 KB): 104 and 130; 100 x 100, 2 of 64, ws 19 (11.6 KB): 156
+// and 197; 128 x 96, 8 of 16, ws 9 (10.4 KB): 55 and 67; 128 x 96, 4 of 32, ws 15 (14.4 KB): 115 and 109; 128 x 96, 8 of
+// 16, ws 11 (15.5 KB): 85 and 72; folded signals 8192 x 64 x 4, ws 63 (2 KB): 60 and 95.
+inline bool values_fit(const Geo& g, int ns) { return 32 / ns * g.K * 4 <= 11600; }
+
 inline bool exact_shape(const Geo& g) {
     return (g.cr == 8 || g.cr == 16 || g.cr == 32 || g.cr == 64) && (int64_t)g.H * g.W == g.Np;
 }
@@ -560,7 +573,10 @@ inline int tile_stage_bytes(int rows, int row_bytes, bool planes, bool single) {
 // 25 shapes the choice is within 10 % of the best cut but for two.  Against four warps of rows and fixed columns:
 // 75 x 53, 9 units, ws 11: forward 27 -> 21 us, dq 40 -> 24, dk/dv 66 -> 35; 128 x 96, 4 units of 64 channels, ws 15: dq
 // 211 -> 160, dk/dv 262 -> 202; 32 x 32, 1 unit, ws 7: forward 8.0 -> 5.1, dq 10 -> 6, dk/dv 20 -> 6.8.
-inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepCost* cost, int n, int max_split, bool planes) {
+// `planes`: the stages carry the scalar planes; `single`: packed rows of one tensor; `col_bytes`: shared memory of a warp of
+// rows for each centre column besides the stages, `warp_bytes` of every warp; `stages` copies in flight.
+inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepCost* cost, int n, int max_split, bool planes = false,
+                             bool single = false, int col_bytes = 0, int stages = kStages, int warp_bytes = 0) {
     TileShape best{cost[0].nq, 1, 1};
     float least = INFINITY;
     const int rw = 32 / ns;                             // pixel rows per warp (ns lanes share a pixel)
@@ -570,11 +586,13 @@ inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepC
         const float cols = (float)((g.W + c->nq - 1) / c->nq) * g.units;
         for (int w = 4; w >= 1; --w) {
             if (w > 1 && rw * (w - 1) >= g.H) continue;
-            const int stage = tile_stage_bytes(rw * w + 2 * P.pp, kRowBytes * ns, planes, false);
+            const int stage = tile_stage_bytes(rw * w + 2 * P.pp, (single ? kSingleFloats : kRowFloats) * 4 * ns, planes, single);
+            const int rows_bytes = w * c->nq * col_bytes;
             const float blocks = cols * ((g.H + rw * w - 1) / (rw * w));
             for (int s = 1; w * s <= 4 && s <= max_split && s <= nst; ++s) {
-                if (s * 2 * stage > 216 * 1024) break;              // not even two copies in flight
-                const int resident = std::max(1, std::min(c->sm_warps / (w * s), 227 * 1024 / (s * kStages * stage + 2048)));
+                const int own = rows_bytes + w * s * warp_bytes;
+                if (s * 2 * stage + own > 216 * 1024) break;        // not even two copies in flight
+                const int resident = std::max(1, std::min(c->sm_warps / (w * s), 227 * 1024 / (s * stages * stage + own + 2048)));
                 const float waves = blocks / (resident * sms);
                 // warps per scheduler, and how many times a block's time passes: whole waves while there are few (the
                 // blocks of a wave end together), later half a wave is lost at the end
@@ -603,9 +621,9 @@ inline TileShape operator_tile(const Geo& g, int ns, int nq, int max_split, int 
 }
 
 // Fills the launch geometry and the tensor maps of the packed pair (and of the scalar planes when given).
-// `xch_floats` per thread for the merge of a split tile.
+// `xch_floats` per thread for the merge of a split tile; `extra` bytes of the kernel's own.
 inline int prepare(const Geo& g, const Padded& P, TileShape t, int xch_floats, const float* pair, const float* planes, Launch* L,
-                   int ns, bool single = false, int stages = kStages) {
+                   int ns, bool single = false, int stages = kStages, size_t extra = 0) {
     const int rw = 32 / ns, warps = t.warps, nsplit = t.nsplit;
     const int rf = (single ? kSingleFloats : kRowFloats) * ns, rb = rf * 4;
     TileArgs& a = L->a;
@@ -628,6 +646,8 @@ inline int prepare(const Geo& g, const Padded& P, TileShape t, int xch_floats, c
     size_t smem = (size_t)nsplit * stages * a.stage_bytes;
     const size_t xch = (size_t)(nsplit - 1) * xch_floats * 32 * warps * sizeof(float);
     if (xch > smem) smem = xch;
+    a.extra_off = (int)smem;
+    smem += extra;
     L->smem = smem + 1024;
     if (L->smem > 220 * 1024) return CA_ERR_UNSUPPORTED;     // window too large for the stage ring: generic kernels
     const uint64_t dims[4] = {(uint64_t)rf, (uint64_t)P.Hp, (uint64_t)g.Wk, (uint64_t)g.units};
