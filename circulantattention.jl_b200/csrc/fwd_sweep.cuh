@@ -1,8 +1,18 @@
 // Forward sweep of the tiled kernels (compiled by fwd_exact.cu and fwd_any.cu; the scheme is described in tiled.cu).
+// fwd_values_exact.cu and fwd_values_any.cu compile the form that also writes A's values.
 #include "tile_common.cuh"
+#ifndef CA_FWD_VALUES
+#define CA_FWD_VALUES 0
+#endif
+#if CA_FWD_VALUES
+#define CA_VALUES_PARAM float* nz,
+#else
+#define CA_VALUES_PARAM
+#endif
 
 namespace ca {
 namespace {
+constexpr bool kValues = CA_FWD_VALUES != 0;
 
 // =====================================================================
 // Forward
@@ -18,10 +28,18 @@ constexpr float kHeadroom = 12.f;
 // NS lanes share a pixel (units of 16*NS real channels): every lane holds one 16-channel slab of q and
 // of the accumulator, scores are the lane sums of the per-slab partial dot products, and the terms that
 // enter a score once (the running reference, in nm2) sit on slab 0 only.
-template <int DC, bool DIST, int MASK, int NQ, int NS = 1>
+//
+// VALUES: the scores of the window also go to shared memory (struct Values), from where A's values leave at the end.
+template <int NQ>
+struct Values {
+    uint32_t run[NQ];        // where the runs of this lane's row start: window column fixed, window rows varying
+    int pos, wrap;           // byte position of the next window row inside a run, which turns to 0 at `wrap`
+    bool on;                 // this lane stores
+};
+template <int DC, bool DIST, int MASK, int NQ, int NS, bool VALUES>
 __device__ __forceinline__ void fwd_stage(uint32_t rowbase, int ws, int rm, float sl2, const u64 (&q)[NQ][8],
                                           u64 (&acc)[NQ][8], u64 (&nm2)[NQ], float (&l)[NQ], const float (&bq)[NQ],
-                                          int slab = 0) {
+                                          int slab, Values<NQ>& vals) {
     constexpr int RB = kRowBytes * NS;
     for (int c0 = 0; c0 < ws; c0 += DC) {
         const uint32_t cb = rowbase + c0 * RB;
@@ -71,6 +89,15 @@ __device__ __forceinline__ void fwd_stage(uint32_t rowbase, int ws, int rm, floa
                             sc[r][t] = -INFINITY;
                         }
                 }
+            }
+        }
+        if constexpr (VALUES) {
+#pragma unroll
+            for (int t = 0; t < DC; ++t) {
+#pragma unroll
+                for (int r = 0; r < NQ; ++r)
+                    if (vals.on && ((rm >> r) & 1)) sts32(vals.run[r] + vals.pos, sc[r][t] - nm2[r].x);
+                vals.pos = vals.pos + 4 == vals.wrap ? 0 : vals.pos + 4;
             }
         }
         // any relative score >= 0 ?  (sign bit clear)
@@ -124,23 +151,23 @@ __device__ __forceinline__ void fwd_stage(uint32_t rowbase, int ws, int rm, floa
 // the remaining one to three keys as one chunk of exactly that length, so that no chunk carries bounds checks
 // (a checked chunk keeps its prefetched vector alive across branches, which costs a register copy per loaded
 // word and made windows such as 13 slower than 15).
-template <int DC, bool DIST, bool EXACT, int NQ, int NS>
+template <int DC, bool DIST, bool EXACT, int NQ, int NS, bool VALUES>
 __device__ __forceinline__ void fwd_window(uint32_t rowbase, int ws, int rm, float sl2, const u64 (&q)[NQ][8],
                                            u64 (&acc)[NQ][8], u64 (&nm2)[NQ], float (&l)[NQ], const float (&bq)[NQ],
-                                           int slab) {
+                                           int slab, Values<NQ>& vals) {
     constexpr int FULLM = (1 << NQ) - 1;
     if (EXACT) {
-        fwd_stage<DC, DIST, FULLM, NQ, NS>(rowbase, ws, rm, sl2, q, acc, nm2, l, bq, slab);
+        fwd_stage<DC, DIST, FULLM, NQ, NS, VALUES>(rowbase, ws, rm, sl2, q, acc, nm2, l, bq, slab, vals);
         return;
     }
     static_assert(EXACT || DC == 4, "windows without a dividing chunk length run chunks of four plus a tail");
     const int main = ws & ~3;
-    fwd_stage<4, DIST, FULLM, NQ, NS>(rowbase, main, rm, sl2, q, acc, nm2, l, bq, slab);
+    fwd_stage<4, DIST, FULLM, NQ, NS, VALUES>(rowbase, main, rm, sl2, q, acc, nm2, l, bq, slab, vals);
     const uint32_t tail = rowbase + main * (kRowBytes * NS);
     switch (ws - main) {                                     // warp-uniform
-        case 1: fwd_stage<1, DIST, FULLM, NQ, NS>(tail, 1, rm, sl2, q, acc, nm2, l, bq, slab); break;
-        case 2: fwd_stage<2, DIST, FULLM, NQ, NS>(tail, 2, rm, sl2, q, acc, nm2, l, bq, slab); break;
-        case 3: fwd_stage<3, DIST, FULLM, NQ, NS>(tail, 3, rm, sl2, q, acc, nm2, l, bq, slab); break;
+        case 1: fwd_stage<1, DIST, FULLM, NQ, NS, VALUES>(tail, 1, rm, sl2, q, acc, nm2, l, bq, slab, vals); break;
+        case 2: fwd_stage<2, DIST, FULLM, NQ, NS, VALUES>(tail, 2, rm, sl2, q, acc, nm2, l, bq, slab, vals); break;
+        case 3: fwd_stage<3, DIST, FULLM, NQ, NS, VALUES>(tail, 3, rm, sl2, q, acc, nm2, l, bq, slab, vals); break;
         default: break;
     }
 }
@@ -172,7 +199,11 @@ __device__ __forceinline__ void fwd_init_max(uint32_t rowbase, int init, float s
 
 // NCRT = real channels per unit the kernel is compiled for: 16 (narrower units are zero-extended),
 // 32 or 64 (NS = 2 or 4 lanes per pixel, one 16-channel slab each; launched without a stage split).
-template <int DC, bool DIST, int CPE, bool EXACT, int NQ, int NCRT = 16>
+// VALUES: also writes A's values, for windows whose rows fit the shared memory: the raw scores of the warp's pixels stay
+// there at their final positions, and once a row's log-sum-exp is known 2^(score - it) leaves as one contiguous piece per
+// centre column.  That costs a store per score and two more instructions on the way out, where a second sweep over the keys
+// forms every score again.
+template <int DC, bool DIST, int CPE, bool EXACT, int NQ, int NCRT, bool VALUES>
 __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
                                                            const __grid_constant__ CUtensorMap msc) {
     constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
@@ -206,9 +237,28 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tile
         for (int i = 0; i < 8; ++i) acc[r][i] = zero2();
     }
 
+    constexpr int RW = 32 / NS;
+    float* tile = nullptr;                       // VALUES: [NQ][RW][K] scores of the warp's rows, then [NQ][RW] log-sum-exps
+    const int hw0 = h0 + (lt >> 5) * RW;
+    Values<NQ> vals{};
+    int rot = 0;
+    if constexpr (VALUES) {
+        tile = reinterpret_cast<float*>(smem_al + a.extra_off) + (lt >> 5) * (NQ * RW * (g.K + 1));
+        rot = active && has_pixel(g, h, w0) ? run_rot(axis_coord(g, h, w0), axis_len(g), g.p, g.ws) : 0;    // 2-D: for all columns
+        vals.wrap = 4 * g.ws;
+        vals.on = slab == 0;
+    }
+
     CA_PIPE_LOOP({
         const int mask = stage_mask<NQ>(s, radius_w(g));
         const uint32_t rowbase = pipe.vec(buf, a) + (lr + a.roff) * RB;
+        if constexpr (VALUES) {
+            vals.pos = 4 * rot;
+            for (int r = 0; r < NQ; ++r) {
+                const bool here = ((mask >> r) & 1) && w0 + r < g.W;
+                vals.run[r] = smem_u32(tile + (r * RW + (lr & (RW - 1))) * g.K + (here ? axis_pos(s - radius_w(g) - r, w0 + r, g.W, radius_w(g), g.wsw) * g.ws : 0));
+            }
+        }
         // pixels whose first stage (of this part) is s
         const int init = (s == s_begin) ? mask : (mask & ~stage_mask<NQ>(s - 1, radius_w(g)));
         if (init) fwd_init_max<DIST, NQ, NS>(rowbase, init, sl2, q, nm2, bq, slab);
@@ -219,12 +269,12 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tile
             u64 nmE[NQ];
 #pragma unroll
             for (int r = 0; r < NQ; ++r) nmE[r] = ((mask >> r) & 1) ? nm2[r] : pack2(-INFINITY, 0.f);
-            fwd_window<DC, DIST, EXACT, NQ, NS>(rowbase, g.ws, mask, sl2, q, acc, nmE, l, bq, slab);
+            fwd_window<DC, DIST, EXACT, NQ, NS, VALUES>(rowbase, g.ws, mask, sl2, q, acc, nmE, l, bq, slab, vals);
 #pragma unroll
             for (int r = 0; r < NQ; ++r)
                 if ((mask >> r) & 1) nm2[r] = nmE[r];
         } else {
-            fwd_window<DC, DIST, EXACT, NQ, NS>(rowbase, g.ws, mask, sl2, q, acc, nm2, l, bq, slab);
+            fwd_window<DC, DIST, EXACT, NQ, NS, VALUES>(rowbase, g.ws, mask, sl2, q, acc, nm2, l, bq, slab, vals);
         }
     })
 
@@ -286,6 +336,29 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ <= 3 ? 3 : 2)) fwd_tile
     for (int r = 0; r < NQ; ++r)
         if (a.ostats && active && slab == 0 && has_pixel(g, h, w0 + r))
             a.ostats[(int64_t)u * g.Np + h + g.H * (w0 + r)] = (log2f(l[r]) - nm[r]) * kLn2 + ca_poison;
+    if constexpr (VALUES) {
+        float* lse = tile + NQ * RW * g.K;
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+            if (slab == 0) lse[r * RW + (lr & (RW - 1))] = log2f(l[r]) - nm[r];
+        __syncwarp();
+        const int lane = threadIdx.x & 31;
+#pragma unroll 1
+        for (int r = 0; r < NQ && w0 + r < g.W; ++r) {
+            // rows of this column (the last column of a folded signal may be shorter)
+            const int n = min(RW, (kAnyC ? min(g.H, g.Np - g.H * (w0 + r)) : g.H) - hw0) * g.K;
+            float* dst = a.o1 + ((int64_t)u * g.Np + hw0 + (int64_t)g.H * (w0 + r)) * g.K;
+            const float* src = tile + r * RW * g.K;
+            int row = 0, e = lane;
+            for (; e >= g.K; e -= g.K) ++row;
+#pragma unroll 4
+            for (int i = lane; i < n; i += 32) {
+                dst[i] = fast_exp2(src[i] - lse[r * RW + row]) + ca_poison;
+                e += 32;
+                while (e >= g.K) { e -= g.K; ++row; }
+            }
+        }
+    }
 }
 
 }  // namespace
@@ -297,23 +370,36 @@ static const SweepCost kFwdCost[3][3] = {{{1, 20, 0, 129, 216, 3265}, {2, 12, 0,
                                          {{1, 20, 36, 105, 145, 4276}, {2, 12, 0, 131, 130, 8597}, {3, 12, 53, 125, 0, 14976}},
                                          {{1, 20, 3, 141, 421, 0}, {2, 12, 0, 154, 726, 0}, {3, 12, 6, 166, 1454, 0}}};
 
+#if CA_FWD_VALUES
+#define RUN_FWD run_fwd_values
+#else
+#define RUN_FWD run_fwd
+#endif
 template <>
-int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* kv, float* y, float* stats,
-                   cudaStream_t st) {
+int RUN_FWD<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* kv, float* y, float* stats,
+                   CA_VALUES_PARAM cudaStream_t st) {
     Launch L{};
     const int ns = slabs_of(g);
-    const TileShape t = choose_tile(g, P, ns, kFwdCost[ns == 1 ? 0 : ns / 2], g.wsw == 1 ? 1 : 3, ns == 1 ? kParts : 1, false);
+#if CA_FWD_VALUES
+    const int col_bytes = 32 / ns * (g.K + 1) * (int)sizeof(float);
+    if (!values_fit(g, ns)) return CA_ERR_UNSUPPORTED;
+    const TileShape t = choose_tile(g, P, ns, kFwdCost[ns == 1 ? 0 : ns / 2], g.wsw == 1 ? 1 : 2, ns == 1 ? kParts : 1, false, false, col_bytes, 2);
+    int rc = prepare(g, P, t, 18 * t.nq, kv, nullptr, &L, ns, false, 2, t.warps * t.nq * col_bytes);
+    L.a.o1 = nz;
+#else
+    const TileShape t = choose_tile(g, P, ns, kFwdCost[ns == 1 ? 0 : ns / 2], g.wsw == 1 ? 1 : 3, ns == 1 ? kParts : 1);
     int rc = prepare(g, P, t, 18 * t.nq, kv, nullptr, &L, ns);
+#endif
     if (rc) return rc;
     L.a.scale = scale; L.a.c0 = q; L.a.o0 = y; L.a.ostats = stats;
 #define CA_FWD2(DCV, EX, NQV, NCRV_)                                                            \
     do {                                                                                 \
         if (g.cpe == 1) {                                                                \
-            if (dist) CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, true, 1, EX, NQV, NCRV_>), L, st); \
-            else CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, false, 1, EX, NQV, NCRV_>), L, st);     \
+            if (dist) CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, true, 1, EX, NQV, NCRV_, kValues>), L, st); \
+            else CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, false, 1, EX, NQV, NCRV_, kValues>), L, st);     \
         } else {                                                                         \
-            if (dist) CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, true, 2, EX, NQV, NCRV_>), L, st); \
-            else CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, false, 2, EX, NQV, NCRV_>), L, st);     \
+            if (dist) CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, true, 2, EX, NQV, NCRV_, kValues>), L, st); \
+            else CA_LAUNCH_TILED((fwd_tiled_kernel<DCV, false, 2, EX, NQV, NCRV_, kValues>), L, st);     \
         }                                                                                \
     } while (0)
     // chunks of 7, 5 or 3 keys where they divide the window, else chunks of four plus a tail
@@ -327,8 +413,8 @@ int run_fwd<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const f
 #define CA_FWD_NQ(NCRV_)                                                                 \
     do {                                                                                 \
         if (t.nq == 1) CA_FWD(1, NCRV_);                                                 \
-        else if (t.nq == 2) CA_FWD(2, NCRV_);                                            \
-        else CA_FWD(3, NCRV_);                                                           \
+        else if (kValues || t.nq == 2) CA_FWD(2, NCRV_);                                 \
+        else CA_FWD((kValues ? 2 : 3), NCRV_);                                           \
     } while (0)
     if (ns == 1) CA_FWD_NQ(16);
     else if (ns == 2) CA_FWD_NQ(32);

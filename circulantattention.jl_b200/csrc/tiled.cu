@@ -79,6 +79,10 @@ int tiled_attention_fwd(const Geo& gin, float scale, int dist, const float* q, c
     pa.src[0] = k; pa.src[1] = v; pa.dst[0] = kv;
     int rc = launch_pack(pa, st);
     if (rc) return rc;
+    if (nz && values_fit(g, slabs_of(g))) {
+        rc = CA_CHANNELS(g, run_fwd_values, g, P, scale, dist, q, kv, y, stats, nz, st);
+        if (rc != CA_ERR_UNSUPPORTED) return rc;
+    }
     if ((rc = CA_CHANNELS(g, run_fwd, g, P, scale, dist, q, kv, y, stats, st))) return rc;
     if (nz) return CA_CHANNELS(g, run_emit, g, P, scale, dist, q, stats, nz, kv, st, false);
     return CA_OK;

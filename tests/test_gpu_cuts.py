@@ -49,6 +49,33 @@ def test_cuts_entmax(ca, shape, ws, nheads):
         assert_close(ca.jl.to_numpy(got), want, name)
 
 
+@pytest.mark.parametrize("shape,ws,nheads,cplx", [
+    ((32, 32, 16, 1), 7, 1, False),       # rows of A kept by the forward: one column, stages in four
+    ((37, 23, 24, 2), 9, 2, False),       # short channel count, rows past the image, wrapped rows
+    ((41, 30, 32, 1), 9, 1, False),       # two slabs, at the limit of what the forward keeps
+    ((33, 19, 32, 2), 7, 1, True),        # four slabs, an odd last column
+    ((26, 25, 64, 1), 19, 1, False),      # four slabs, the largest window the forward keeps
+    ((35, 26, 32, 1), 15, 1, False),      # past it: runs staged per window column
+    ((36, 37, 16, 2), 35, 1, False),      # runs in two pieces
+    ((131, 40, 1), 9, 1, False),          # folded signal, short last column
+    ((300, 24, 2), 127, 1, False),        # folded signal, rows of 127
+])
+@pytest.mark.parametrize("simname", ["dot", "distance"])
+def test_values(ca, shape, ws, nheads, cplx, simname):
+    """A's values: written by the forward where a warp's rows fit, else by a second sweep; and the raw scores of the similarity."""
+    rng = np.random.default_rng(63)
+    qn, kn, vn = (randn(rng, shape, cplx) for _ in range(3))
+    sim = ca.DotSimilarity() if simname == "dot" else ca.DistanceSimilarity()
+    q, k, v = (ca.jl.from_numpy(t) for t in (qn, kn, vn))
+    y, A = ca.circulant_mh_attention(sim, q, k, v, ws, nheads)
+    yo, nzo = orc.mh_attention(KIND[simname], up(qn), up(kn), up(vn), ws, nheads)
+    assert_close(ca.jl.to_numpy(y), yo, "y")
+    assert_close(ca.jl.to_numpy(A.nzVal), nzo, "A")
+    if nheads == 1:
+        S = ca.circulant_similarity(sim, q, k, ws)
+        assert_close(ca.jl.to_numpy(S.nzVal), orc.similarity(KIND[simname], up(qn), up(kn), ws), "scores")
+
+
 @pytest.mark.parametrize("c", [24, 48])
 def test_wide_entmax_backward_launches(ca, c):
     """Units past one slab take the operator chain at once: no pack is made for the fused sweeps they do not have."""
