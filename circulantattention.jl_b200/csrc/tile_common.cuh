@@ -574,9 +574,10 @@ inline int tile_stage_bytes(int rows, int row_bytes, bool planes, bool single) {
 // 75 x 53, 9 units, ws 11: forward 27 -> 21 us, dq 40 -> 24, dk/dv 66 -> 35; 128 x 96, 4 units of 64 channels, ws 15: dq
 // 211 -> 160, dk/dv 262 -> 202; 32 x 32, 1 unit, ws 7: forward 8.0 -> 5.1, dq 10 -> 6, dk/dv 20 -> 6.8.
 // `planes`: the stages carry the scalar planes; `single`: packed rows of one tensor; `col_bytes`: shared memory of a warp of
-// rows for each centre column besides the stages, `warp_bytes` of every warp; `stages` copies in flight.
+// rows for each centre column besides the stages, `warp_bytes` of every warp; `stages` copies in flight; `lone` weighs blocks of
+// one warp within one wave.
 inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepCost* cost, int n, int max_split, bool planes = false,
-                             bool single = false, int col_bytes = 0, int stages = kStages, int warp_bytes = 0) {
+                             bool single = false, int col_bytes = 0, int stages = kStages, int warp_bytes = 0, float lone = 1.f) {
     TileShape best{cost[0].nq, 1, 1};
     float least = INFINITY;
     const int rw = 32 / ns;                             // pixel rows per warp (ns lanes share a pixel)
@@ -602,6 +603,7 @@ inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepC
                 // tiles of one or two warps copy more halo rows; it shows once blocks follow one another (the forward
                 // at 500 x 400, 3 units, ws 11: 209 us with one warp, 172 with two, 167 with four)
                 if (waves > 1.f) t *= w == 1 ? 1.08f : (w == 2 ? 1.02f : 1.f);
+                else if (w * s == 1) t *= lone;
                 if (t < least) { least = t; best = TileShape{c->nq, w, s}; }
             }
         }

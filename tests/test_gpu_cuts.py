@@ -85,3 +85,32 @@ def test_wide_entmax_backward_launches(ca, c):
     n0 = ca.lib.ca_probe_launch_count()
     y.sum().backward()
     assert ca.lib.ca_probe_launch_count() - n0 == 12      # scores, weights, dv, dP, dS, dq, dk, and five packs
+
+
+@pytest.mark.parametrize("spatial,ws,c,units,cplx", [
+    ((32, 32), 7, 16, 1, False),      # whole rows: one column, stages in four
+    ((75, 53), 9, 12, 3, False),      # whole rows at their limit for one slab, rows past the image
+    ((38, 31), 11, 32, 2, False),     # two slabs, at the limit of the window
+    ((41, 30), 7, 32, 2, True),       # four slabs, an odd last column, every alignment of a row
+    ((131,), 21, 40, 2, False),       # folded signal, short last column
+    ((75, 53), 11, 16, 3, False),     # runs, stages in three
+    ((60, 40), 21, 16, 2, False),     # runs, stages in four
+    ((39, 45), 13, 32, 2, False),     # loose runs of the transposed form (39 rows), two slabs
+])
+def test_apply_cuts(ca, spatial, ws, c, units, cplx):
+    """A (x) v, its transpose and, for Distance, the pullback that subtracts the row sums times the centre."""
+    rng = np.random.default_rng(65)
+    K = ws ** len(spatial)
+    nzn = rng.standard_normal((int(np.prod(spatial)) * K, units)).astype(np.float32)
+    xn, yn = randn(rng, spatial + (c, units), cplx), randn(rng, spatial + (c, units), cplx)
+    nz, x = ca.jl.from_numpy(np.asfortranarray(nzn)), ca.jl.from_numpy(xn)
+    dS = up(nzn).reshape((K, -1, units), order="F")
+    for transpose in (False, True):
+        assert_close(ca.jl.to_numpy(ca.ops.apply(nz, x, ws, transpose)), orc.apply(dS, up(xn), ws, transpose), f"transpose {transpose}")
+    xt, yt = ca.jl.from_numpy(xn).requires_grad_(True), ca.jl.from_numpy(yn).requires_grad_(True)
+    S = ca.circulant_similarity(ca.DistanceSimilarity(), xt, yt, ws)
+    S.nzVal.backward(nz.reshape(S.nzVal.shape) if S.nzVal.shape != nz.shape else nz)
+    dxo, dyo = orc.similarity_pullback(orc.DISTANCE, up(xn), up(yn), ws, dS)
+    # a sum of K differences of O(1) vectors: the centre enters with the sum of K weights
+    assert_close(ca.jl.to_numpy(xt.grad), dxo, "dx")
+    assert_close(ca.jl.to_numpy(yt.grad), dyo, "dy")
