@@ -4,6 +4,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <stdarg.h>
+#include <atomic>
 #include "../../include/circatt_b200.h"
 #include "../../include/circatt_b200_probe.h"
 
@@ -69,6 +70,20 @@ __host__ __device__ inline int axis_pos(int d, int x, int X, int p, int ws) {
 int make_geo(const ca_desc* d, Geo* g, bool allow_band);
 
 static inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
+
+// ---------------------------------------------------------------- host
+// SM count of the current device (cached per device ordinal).
+inline int sm_count() {
+    static std::atomic<int> cache[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    int n = cache[dev].load(std::memory_order_relaxed);
+    if (!n) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        cache[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
 
 // ---------------------------------------------------------------- device math
 __device__ __forceinline__ float fast_exp2(float x) {

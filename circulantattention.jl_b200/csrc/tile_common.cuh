@@ -138,6 +138,7 @@ struct TileArgs {
 };
 
 constexpr int kStages = 3;
+constexpr int kMaxDynamicSmem = 220 * 1024;
 constexpr int kParts = 4;                      // groups of warps that can share the stages of a tile
 constexpr uint32_t kWaitTries = 1u << 20;
 constexpr int kEntmaxFwdSteps = 16;            // launches of the entmax threshold step (settled blocks leave at once)
@@ -534,19 +535,6 @@ struct Launch {
     size_t smem;
 };
 
-// SM count of the current device (cached per device ordinal).
-inline int sm_count() {
-    static std::atomic<int> cache[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    int n = cache[dev].load(std::memory_order_relaxed);
-    if (!n) {
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        cache[dev].store(n, std::memory_order_relaxed);
-    }
-    return n;
-}
-
 // How a sweep is cut into blocks: `nq` centre columns per thread, `warps` warps of pixel rows per block and `nsplit` groups
 // of such warps that share the stages of a tile (warps * nsplit <= 4).
 struct TileShape {
@@ -576,12 +564,12 @@ inline int tile_stage_bytes(int rows, int row_bytes, bool planes, bool single) {
 // `planes`: the stages carry the scalar planes; `single`: packed rows of one tensor; `col_bytes`: shared memory of a warp of
 // rows for each centre column besides the stages, `warp_bytes` of every warp; `stages` copies in flight; `lone` weighs blocks of
 // one warp within one wave.
-inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepCost* cost, int n, int max_split, bool planes = false,
-                             bool single = false, int col_bytes = 0, int stages = kStages, int warp_bytes = 0, float lone = 1.f) {
+inline TileShape search_tile(const Geo& g, const Padded& P, int ns, const SweepCost* cost, int n, int max_split, bool planes, bool single,
+                             int col_bytes, int stages, int warp_bytes, float lone, int sm) {
     TileShape best{cost[0].nq, 1, 1};
     float least = INFINITY;
     const int rw = 32 / ns;                             // pixel rows per warp (ns lanes share a pixel)
-    const float sms = (float)sm_count();
+    const float sms = (float)sm;
     for (const SweepCost* c = cost; c < cost + n; ++c) {
         const int nst = g.wsw + c->nq - 1;
         const float cols = (float)((g.W + c->nq - 1) / c->nq) * g.units;
@@ -609,6 +597,25 @@ inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepC
         }
     }
     return best;
+}
+
+// The search takes about a microsecond of a launch's three: a thread keeps the cuts of its last launches.
+inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepCost* cost, int n, int max_split, bool planes = false,
+                             bool single = false, int col_bytes = 0, int stages = kStages, int warp_bytes = 0, float lone = 1.f) {
+    struct Key {
+        const SweepCost* cost;
+        int v[14];
+        bool operator==(const Key& o) const { return cost == o.cost && std::equal(v, v + 14, o.v); }
+    };
+    struct Entry { Key key; TileShape shape; };
+    static thread_local Entry kept[16] = {};
+    const int sm = sm_count();
+    const Key key{cost, {g.H, g.W, g.units, g.ws, g.wsw, P.pp, ns, n, max_split, planes * 2 + single, col_bytes, stages, warp_bytes * 4 + (lone < 1.f), sm}};
+    unsigned h = (unsigned)(reinterpret_cast<uintptr_t>(cost) >> 4);
+    for (int x : key.v) h = h * 31u + (unsigned)x;
+    Entry& e = kept[h % 16];
+    if (!(e.key == key)) e = Entry{key, search_tile(g, P, ns, cost, n, max_split, planes, single, col_bytes, stages, warp_bytes, lone, sm)};
+    return e.shape;
 }
 
 // Operators: four warps of rows; fewer than 6 warps per SM share the stages of a tile (in four where the kernel can,
@@ -651,7 +658,7 @@ inline int prepare(const Geo& g, const Padded& P, TileShape t, int xch_floats, c
     a.extra_off = (int)smem;
     smem += extra;
     L->smem = smem + 1024;
-    if (L->smem > 220 * 1024) return CA_ERR_UNSUPPORTED;     // window too large for the stage ring: generic kernels
+    if (L->smem > kMaxDynamicSmem) return CA_ERR_UNSUPPORTED;     // window too large for the stage ring: generic kernels
     const uint64_t dims[4] = {(uint64_t)rf, (uint64_t)P.Hp, (uint64_t)g.Wk, (uint64_t)g.units};
     const uint64_t strides[3] = {(uint64_t)rb, (uint64_t)P.Hp * rb, (uint64_t)P.Hp * rb * g.Wk};
     const uint32_t box[4] = {(uint32_t)rf, (uint32_t)ROWS, 1, 1};
@@ -668,18 +675,24 @@ inline int prepare(const Geo& g, const Padded& P, TileShape t, int xch_floats, c
     return CA_OK;
 }
 
+// Raises a kernel's limit of dynamic shared memory to the most that any launch asks for (prepare()), once per kernel and
+// device: `have` remembers the device of the last call.  Always the same value, so threads cannot lower each other's.
 template <typename K>
-int set_smem(K kernel, size_t bytes) {
-    if (bytes > 47 * 1024) {                // the default limit of 48 KB counts the kernel's static shared memory too
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(shared memory)");
-    }
+int set_smem(K kernel, size_t bytes, std::atomic<int>& have) {
+    if (bytes <= 47 * 1024) return CA_OK;   // the default limit of 48 KB counts the kernel's static shared memory too
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess && have.load(std::memory_order_relaxed) == dev + 1) return CA_OK;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(shared memory)");
+    have.store(dev + 1, std::memory_order_relaxed);
     return CA_OK;
 }
 
 #define CA_LAUNCH_TILED(KERNEL, L, st)                                                \
     do {                                                                              \
-        int rc__ = set_smem(KERNEL, (L).smem);                                        \
+        static std::atomic<int> have__{0};                                            \
+        int rc__ = set_smem(KERNEL, (L).smem, have__);                                \
         if (rc__) return rc__;                                                        \
         KERNEL<<<(L).grid, (L).threads, (L).smem, st>>>((L).a, (L).mv, (L).msc);      \
         count_tiled_launch();                                                         \
