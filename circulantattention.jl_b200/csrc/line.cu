@@ -173,9 +173,10 @@ __device__ __forceinline__ void sweep(int tb, int ws, F&& f) {
     sweep_tail<NQ, 0>(f, tb, ws);
 }
 
-// The same sweep for the largest score of each of 2*NQ classes of keys: `f(mask, class, slot)` gets the class as a
-// compile-time value.  Steps 0 .. 2*NQ-1 are classes 0 .. 2*NQ-1 and so on; the last few of a window that is no
-// multiple of 2*NQ go to the first classes again (any partition of the keys will do).
+// The same sweep for the largest score of each of kClasses classes of keys: `f(mask, class, slot)` gets the class as a
+// compile-time value.  Step t is of class t mod kClasses; the last few of a window that is no multiple of NQ go to the first
+// classes again (any partition of the keys will do).
+constexpr int kClasses = 8;
 template <int NQ, int T, class F>
 __device__ __forceinline__ void class_head(F& f, int slot0) {
     if constexpr (T < NQ - 1) {
@@ -197,21 +198,25 @@ __device__ __forceinline__ void class_tail(F& f, int tb, int ws) {
         class_tail<NQ, E + 1>(f, tb, ws);
     }
 }
+// Groups of NQ steps from class C on, as far as the classes go; returns the step behind the last one.
+template <int NQ, int C, class F>
+__device__ __forceinline__ int class_turn(F& f, int t, int slot0, int ws) {
+    if constexpr (C < kClasses) {
+        if (t + NQ > ws) return t;
+        class_group<NQ, C, 0>(f, slot0);
+        return class_turn<NQ, C + NQ>(f, t + NQ, slot0 + NQ + 1, ws);
+    } else {
+        return t;
+    }
+}
 template <int NQ, class F>
 __device__ __forceinline__ void sweep_classes(int tb, int ws, F&& f) {
     int slot0 = pad<NQ>(tb);
     class_head<NQ, 0>(f, slot0);
     f(ic<(1 << NQ) - 1>{}, ic<NQ - 1>{}, slot0 + NQ - 1);
-    int t = NQ;
-    slot0 += NQ + 1;
-    for (; t + 2 * NQ <= ws; t += 2 * NQ, slot0 += 2 * (NQ + 1)) {
-        class_group<NQ, NQ, 0>(f, slot0);
-        class_group<NQ, 0, 0>(f, slot0 + NQ + 1);
-    }
-    if (t + NQ <= ws) {
-        class_group<NQ, NQ, 0>(f, slot0);
-        t += NQ;
-    }
+    constexpr int TURN = kClasses / NQ * (NQ + 1);          // slots of a turn through all classes
+    int t = class_turn<NQ, NQ>(f, NQ, slot0 + NQ + 1, ws);
+    for (slot0 += TURN; t + NQ <= ws; slot0 += TURN) t = class_turn<NQ, 0>(f, t, slot0, ws);
     for (; t < ws; ++t) f(ic<(1 << NQ) - 1>{}, ic<0>{}, pad<NQ>(tb + t));
     class_tail<NQ, 0>(f, tb, ws);
 }
@@ -245,7 +250,7 @@ constexpr float kLineHeadroom = 12.f;          // log2 units between the softmax
 
 // ------------------------------------------------------------------------------------------------ forward
 template <int CR, int NQ, bool DIST, bool ENT>
-__global__ void __launch_bounds__(kLT, CR <= 8 ? 3 : 2) line_fwd_kernel(LineArgs a) {
+__global__ void __launch_bounds__(kLT, NQ == 4 ? (CR <= 8 ? 3 : 2) : (CR <= 8 ? 5 : 4)) line_fwd_kernel(LineArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const Geo& g = a.g;
     const int N = g.Np, ws = g.ws, lt = threadIdx.x, u = blockIdx.y;
@@ -287,12 +292,11 @@ __global__ void __launch_bounds__(kLT, CR <= 8 ? 3 : 2) line_fwd_kernel(LineArgs
             m[r] = dot<CR>(q[r], kk, DIST ? bq[r] + bk[pad<NQ>(tb + r + g.p)] : 0.f) + kLineHeadroom;
         }
     }
-    // entmax: the first threshold comes from the largest scores of 2*NQ classes of keys, which cost the sweep no more
+    // entmax: the first threshold comes from the largest scores of eight classes of keys, which cost the sweep no more
     // than the row maximum does.  Against a start at max - 1 the threshold sweeps fall from four to two
     // (127 keys of 8 channels, standard normal: 128, 123, 63, 0.5 of a warp's 128 rows open after each, now 92 and 3);
     // 16384 x 64 x 16, 8 units, ws 127, Distance: 1046 -> 786 us.
     if (ENT) {
-        constexpr int kClasses = 2 * NQ;
         float top[NQ][kClasses];
 #pragma unroll
         for (int r = 0; r < NQ; ++r)
@@ -332,30 +336,39 @@ __global__ void __launch_bounds__(kLT, CR <= 8 ? 3 : 2) line_fwd_kernel(LineArgs
                 rmax[r] = 0.f;
                 rmin[r] = 0.f;
             }
-            sweep<NQ>(tb, ws, [&](auto mk, int slot) {
-                constexpr int M = decltype(mk)::value;
-                float kk[CR];
-                ld_vec<CR>(Kg, a.PP, slot, kk);
-                const float bkk = DIST ? bk[slot] : 0.f;
+            auto search = [&](auto near) {
+                sweep<NQ>(tb, ws, [&](auto mk, int slot) {
+                    constexpr int M = decltype(mk)::value;
+                    float kk[CR];
+                    ld_vec<CR>(Kg, a.PP, slot, kk);
+                    const float bkk = DIST ? bk[slot] : 0.f;
 #pragma unroll
-                for (int r = 0; r < NQ; ++r)
-                    if ((M >> r) & 1) {
-                        const float tt = dot<CR>(q[r], kk, DIST ? (bq[r] - off[r]) + bkk : -off[r]);
-                        const float tp = fmaxf(tt, 0.f);
-                        sa[r] += tp;
-                        sb[r] = fmaf(tp, tp, sb[r]);
-                        n[r] += tt > 0.f ? 1.f : 0.f;
-                        const float rt = fast_rcp(tt);
-                        rmax[r] = fmaxf(rmax[r], rt);
-                        rmin[r] = fminf(rmin[r], rt);
-                    }
-            });
+                    for (int r = 0; r < NQ; ++r)
+                        if ((M >> r) & 1) {
+                            const float tt = dot<CR>(q[r], kk, DIST ? (bq[r] - off[r]) + bkk : -off[r]);
+                            const float tp = fmaxf(tt, 0.f);
+                            sa[r] += tp;
+                            sb[r] = fmaf(tp, tp, sb[r]);
+                            n[r] += tt > 0.f ? 1.f : 0.f;
+                            if constexpr (decltype(near)::value) {
+                                const float rt = fast_rcp(tt);
+                                rmax[r] = fmaxf(rmax[r], rt);
+                                rmin[r] = fminf(rmin[r], rt);
+                            }
+                        }
+                });
+            };
+            // the first sweep of a long window leaves most rows open (93 of 128 at 127 keys, 50 at 31) and is followed by
+            // another in any case: it goes without the nearest members, its rows all stay open
+            const bool first = it == 0 && ws >= 31;
+            if (first) search(std::false_type{});
+            else search(std::true_type{});
 #pragma unroll
             for (int r = 0; r < NQ; ++r)
                 if (!done[r]) {
                     bool same;
                     off[r] += tau_step(n[r], sa[r], sb[r], rmax[r], rmin[r], it >= kNewtonAfter, same);
-                    done[r] = same;
+                    done[r] = same && !first;
                 }
             // rows of this warp that are still open; when only a few are left (after the fourth sweep about
             // one row in a hundred), the warp finishes them one at a time, the window's keys spread over its
@@ -472,7 +485,7 @@ __global__ void __launch_bounds__(kLT, CR <= 8 ? 3 : 2) line_fwd_kernel(LineArgs
 // Query-owned.  softmax: D = dy . y, dS = P (dP - D); entmax: g = max(z - tau, 0), D = sum g dP / sum g,
 // dS = g (dP - D).  dq = scale * sum dS k  (Distance: - scale * q * sum dS).
 template <int CR, int NQ, bool DIST, bool ENT>
-__global__ void __launch_bounds__(kLT, CR <= 8 ? 3 : 2) line_dq_kernel(LineArgs a) {
+__global__ void __launch_bounds__(kLT, CR <= 8 ? 5 : 2) line_dq_kernel(LineArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const Geo& g = a.g;
     const int N = g.Np, ws = g.ws, lt = threadIdx.x, u = blockIdx.y;
@@ -702,7 +715,27 @@ int launch(Kern kern, const LineArgs& a, int nq, size_t smem, cudaStream_t st, c
             : ((ent) ? launch(KERN<CRV, NQV, false, true>, __VA_ARGS__)                          \
                      : launch(KERN<CRV, NQV, false, false>, __VA_ARGS__)))
 
-constexpr int kFwdNQ8 = 4, kFwdNQ16 = 4, kBwdNQ8 = 4, kBwdNQ16 = 2;
+// Pixels per thread.  Four use every vector they load four times; two leave twice the blocks, with half the registers.  Per
+// launch, four against two pixels (N x units, window; us):
+//   dq, 8 channels: two at every size (16384 x 32, ws 127: softmax 106 -> 100, entmax 128 -> 118; 2000 x 4, ws 63: 17 -> 11); 16
+//   channels: two (the registers of four spill).
+//   dk/dv, 8 channels: 5001 x 12, ws 63: 18.9 -> 14.5; 16384 x 64, ws 15: 83 -> 70, ws 63: 131 = 131, ws 127: 210 against 220;
+//   16384 x 16, ws 127 (512 blocks of four): 68 -> 62; 16 channels: two.
+//   forward, softmax, 8 channels: 5001 x 12, ws 63: 20.7 -> 14.7; 16384 x 96, ws 63: 181 -> 166; 8192 x 16, ws 127 (256 blocks): 38 -> 30;
+//   4096 x 48, ws 127 (384): 44 against 51; entmax: 5001 x 12, ws 127 (120): 41 -> 39; 4096 x 48, ws 63 (384): 49 against 54;
+//   16384 x 32, ws 63 (1024): 125 -> 114, ws 127: 193 against 200.
+//   forward, 16 channels: 16384 x 32, ws 63: softmax 231 -> 167, entmax 312 -> 267; but where four fill each SM's two blocks once and no
+//   more, 8192 x 16 (256), ws 63: softmax 51 against 57, entmax 70 against 89.
+int fwd_pixels(const Geo& g, bool entmax) {
+    const long blocks = (long)((g.Np + 4 * kLT - 1) / (4 * kLT)) * g.units, sms = sm_count();
+    if (g.cr > 8) return g.ws >= 32 && blocks > sms && blocks <= 2 * sms ? 4 : 2;
+    if (entmax) return blocks <= sms || (g.ws < 96 && blocks > 3 * sms) ? 2 : 4;
+    return g.ws < 96 || blocks <= 2 * sms ? 2 : 4;
+}
+int dkdv_pixels(const Geo& g) {
+    const long blocks = (long)((g.Np + 4 * kLT - 1) / (4 * kLT)) * g.units;
+    return g.cr > 8 || g.ws < 96 || blocks <= 4L * sm_count() ? 2 : 4;
+}
 
 }  // namespace
 
@@ -718,14 +751,12 @@ int line_attention_fwd(const Geo& g, float scale, int dist, int entmax, const fl
     LineArgs a{};
     a.g = g; a.scale = scale; a.q = q; a.k = k; a.v = v; a.o = y; a.ostats = stats;
     size_t smem;
-    if (g.cr <= 8) {
-        const int rc = prepare(a, kFwdNQ8, 4, 1, &smem);
-        if (rc) return rc;
-        return CA_LINE_DISPATCH(line_fwd_kernel, 8, kFwdNQ8, dist, entmax, a, kFwdNQ8, smem, st, "1-D forward kernel");
-    }
-    const int rc = prepare(a, kFwdNQ16, 8, 1, &smem);
+    const int nq = fwd_pixels(g, entmax), rc = prepare(a, nq, g.cr <= 8 ? 4 : 8, 1, &smem);
     if (rc) return rc;
-    return CA_LINE_DISPATCH(line_fwd_kernel, 16, kFwdNQ16, dist, entmax, a, kFwdNQ16, smem, st, "1-D forward kernel");
+#define CA_LINE_FWD(CRV, NQV) CA_LINE_DISPATCH(line_fwd_kernel, CRV, NQV, dist, entmax, a, nq, smem, st, "1-D forward kernel")
+    if (g.cr <= 8) return nq == 2 ? CA_LINE_FWD(8, 2) : CA_LINE_FWD(8, 4);
+    return nq == 2 ? CA_LINE_FWD(16, 2) : CA_LINE_FWD(16, 4);
+#undef CA_LINE_FWD
 }
 
 int line_attention_bwd(const Geo& g, float scale, int dist, int entmax, const float* q, const float* k,
@@ -737,16 +768,17 @@ int line_attention_bwd(const Geo& g, float scale, int dist, int entmax, const fl
     a.D = D; a.dq = dq; a.dk = dk; a.dv = dv;
     size_t smem_q, smem_k;
     int rc;
-    if (g.cr <= 8) {
-        if ((rc = prepare(a, kBwdNQ8, 4, 1, &smem_q))) return rc;
-        if ((rc = CA_LINE_DISPATCH(line_dq_kernel, 8, kBwdNQ8, dist, entmax, a, kBwdNQ8, smem_q, st, "1-D dq kernel"))) return rc;
-        if ((rc = prepare(a, kBwdNQ8, 5, 0, &smem_k))) return rc;
-        return CA_LINE_DISPATCH(line_dkdv_kernel, 8, kBwdNQ8, dist, entmax, a, kBwdNQ8, smem_k, st, "1-D dk/dv kernel");
-    }
-    if ((rc = prepare(a, kBwdNQ16, 8, 1, &smem_q))) return rc;
-    if ((rc = CA_LINE_DISPATCH(line_dq_kernel, 16, kBwdNQ16, dist, entmax, a, kBwdNQ16, smem_q, st, "1-D dq kernel"))) return rc;
-    if ((rc = prepare(a, kBwdNQ16, 9, 0, &smem_k))) return rc;
-    return CA_LINE_DISPATCH(line_dkdv_kernel, 16, kBwdNQ16, dist, entmax, a, kBwdNQ16, smem_k, st, "1-D dk/dv kernel");
+    const bool wide = g.cr > 8;
+    if ((rc = prepare(a, 2, wide ? 8 : 4, 1, &smem_q))) return rc;
+    rc = wide ? CA_LINE_DISPATCH(line_dq_kernel, 16, 2, dist, entmax, a, 2, smem_q, st, "1-D dq kernel")
+              : CA_LINE_DISPATCH(line_dq_kernel, 8, 2, dist, entmax, a, 2, smem_q, st, "1-D dq kernel");
+    if (rc) return rc;
+    const int nq = dkdv_pixels(g);
+    if ((rc = prepare(a, nq, wide ? 9 : 5, 0, &smem_k))) return rc;
+#define CA_LINE_DKDV(CRV, NQV) CA_LINE_DISPATCH(line_dkdv_kernel, CRV, NQV, dist, entmax, a, nq, smem_k, st, "1-D dk/dv kernel")
+    if (wide) return CA_LINE_DKDV(16, 2);
+    return nq == 2 ? CA_LINE_DKDV(8, 2) : CA_LINE_DKDV(8, 4);
+#undef CA_LINE_DKDV
 }
 
 }  // namespace ca

@@ -114,3 +114,27 @@ def test_apply_cuts(ca, spatial, ws, c, units, cplx):
     # a sum of K differences of O(1) vectors: the centre enters with the sum of K weights
     assert_close(ca.jl.to_numpy(xt.grad), dxo, "dx")
     assert_close(ca.jl.to_numpy(yt.grad), dyo, "dy")
+
+
+@pytest.mark.parametrize("shape,ws", [
+    ((513, 8, 300), 97),      # 600 blocks of four pixels per thread, a block of one pixel at the end of each signal
+    ((515, 6, 80), 33),       # 160: entmax with four, softmax with two
+    ((513, 16, 100), 33),     # 16 channels, 200 blocks: forward with four
+    ((514, 12, 4), 99),       # two everywhere
+])
+@pytest.mark.parametrize("norm", ["softmax", "entmax"])
+def test_line_pixels(ca, shape, ws, norm):
+    """1-D kernels with two and with four pixels per thread."""
+    rng = np.random.default_rng(66)
+    qn, kn, vn, rn = (randn(rng, shape) for _ in range(4))
+    q, k, v = (ca.jl.from_numpy(t).requires_grad_(True) for t in (qn, kn, vn))
+    y, _ = ca.circulant_attention(ca.DistanceSimilarity(), q, k, v, ws, normalizer=ca.ENTMAX15 if norm == "entmax" else ca.SOFTMAX, return_A=False)
+    (y * ca.jl.from_numpy(rn)).sum().backward()
+    which = orc.ENTMAX15 if norm == "entmax" else orc.SOFTMAX
+    for u in (0, shape[-1] // 2, shape[-1] - 1):
+        one = slice(u, u + 1)
+        qo, ko, vo, ro = (up(t[..., one]) for t in (qn, kn, vn, rn))
+        yo, _ = orc.attention(orc.DISTANCE, qo, ko, vo, ws, which)
+        dqo, dko, dvo = orc.attention_pullback(orc.DISTANCE, qo, ko, vo, ws, ro, None, which)
+        for name, got, want in (("y", y, yo), ("dq", q.grad, dqo), ("dk", k.grad, dko), ("dv", v.grad, dvo)):
+            assert_close(ca.jl.to_numpy(got)[..., one], want, f"{name} of unit {u}")
