@@ -19,11 +19,13 @@ namespace {
 // MODE 4 one step of the threshold search: with t = chain = s/2 - tau, the sum of max(t, 0) (sumds), of its
 // square (aux), the size of the support {t > 0}, its smallest member and the largest t outside (ex[0..2]);
 // MODE 5 the apply: dq (here y) += max(chain, 0)^2 * v.
-template <bool DIST, int MASK, int NQ, int MODE, int NS = 1>
+// STORE: the weights P and dS also go to memory, for dkdv_stored_kernel: `w[r]` is where this lane's entry of the stage's
+// first key goes (lanes of slab 0 write P, of slab 1 dS), `step` the words to the next key's.
+template <bool DIST, int MASK, int NQ, int MODE, int NS, bool STORE>
 __device__ __forceinline__ void dq_stage(uint32_t rowbase, int ws, int rm, float sl2, const u64 (&q)[NQ][8],
                                          const u64 (&dy)[NQ][8], u64 (&dq)[NQ][8], const u64 (&nL2)[NQ],
                                          const u64 (&nD2)[NQ], const float (&bq)[NQ], float (&sumds)[NQ],
-                                         float (&aux)[NQ], float (&ex)[NQ][3], int slab = 0) {
+                                         float (&aux)[NQ], float (&ex)[NQ][3], int slab, float* (&w)[NQ], int step, int keep) {
 #pragma unroll (NQ == 1 ? 4 : 2)      // keys in flight: the next key's loads overlap this key's FMAs
     for (int di = 0; di < ws; ++di) {
         const uint32_t a0 = rowbase + di * (kRowBytes * NS);
@@ -79,7 +81,12 @@ __device__ __forceinline__ void dq_stage(uint32_t rowbase, int ws, int rm, float
                     aux[r] = fmaf(gg, dp[r], aux[r]);
                     sumds[r] += gg;
                 } else {
-                    const float ds = (MODE == 0 ? fast_exp2(chain) : fmaxf(chain, 0.f)) * dp[r];
+                    const float P = MODE == 0 ? fast_exp2(chain) : fmaxf(chain, 0.f);
+                    const float ds = P * dp[r];
+                    if (STORE) {
+                        if ((keep >> r) & 1) *w[r] = slab ? ds : P;
+                        w[r] += step;
+                    }
                     if (DIST) sumds[r] += ds;
 #pragma unroll
                     for (int i = 0; i < 8; ++i) dq[r][i] = outer2(ds, k2[i], dq[r][i]);
@@ -88,7 +95,7 @@ __device__ __forceinline__ void dq_stage(uint32_t rowbase, int ws, int rm, float
     }
 }
 
-template <bool DIST, int CPE, int NQ, int MODE, int NCRT = 16>
+template <bool DIST, int CPE, int NQ, int MODE, int NCRT = 16, bool STORE = false>
 __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) dq_tiled_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
                                                           const __grid_constant__ CUtensorMap msc) {
     constexpr int NS = NCRT <= 16 ? 1 : NCRT / 16;
@@ -160,10 +167,22 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 5 : NQ == 2 ? 3 : 2)) dq_tiled
 #pragma unroll
             for (int i = 0; i < kClasses; ++i) top[r][i] = -INFINITY;
     }
+    int keep = 0;                                // STORE: columns whose weights this lane writes
+    if (STORE) {
+#pragma unroll
+        for (int r = 0; r < NQ; ++r)
+            if (active && slab < 2 && has_pixel(g, h, w0 + r)) keep |= 1 << r;
+    }
     CA_PIPE_LOOP({
         const int mask = stage_mask<NQ>(s, radius_w(g));
-        CA_MASK_SWITCH(((1 << NQ) - 1), mask, (dq_stage<DIST, MK, NQ, MODE, NS>(pipe.vec(buf, a) + (lr + a.roff) * (kRowBytes * NS), g.ws, mask,
-                                                     sl2, q, dy, dq, nL2, nD2, bq, sumds, aux, ex, slab)));
+        float* kept[NQ];
+        if (STORE) {
+            _Pragma("unroll")
+            for (int r = 0; r < NQ; ++r)
+                kept[r] = a.o1 + ((int64_t)(2 * u + (slab & 1)) * g.K + (s - r) * g.ws) * g.Np + h + g.H * (w0 + r);
+        }
+        CA_MASK_SWITCH(((1 << NQ) - 1), mask, (dq_stage<DIST, MK, NQ, MODE, NS, STORE>(pipe.vec(buf, a) + (lr + a.roff) * (kRowBytes * NS), g.ws, mask,
+                                                     sl2, q, dy, dq, nL2, nD2, bq, sumds, aux, ex, slab, kept, g.Np, keep)));
         if (MODE == 3) {
             _Pragma("unroll")
             for (int r = 0; r < NQ; ++r) {
@@ -418,6 +437,129 @@ __global__ void __launch_bounds__(128, (NQ == 1 ? 4 : NQ == 2 ? 3 : 2)) dkdv_til
         })
 }
 
+// =====================================================================
+// dk and dv of wide units from the stored weights of the dq sweep: dv = sum P dy, dk = scale * sum dS q over the queries
+// whose window holds the key.  Recomputing P and dS takes two of the four contractions, two shuffles for each of their
+// scores and an exp2 in each of the NS lanes; stored they are 8 bytes per pair, written and read once, for
+// 64 * NS FMAs saved.  [unit][P | dS][window entry][query pixel]: lanes on consecutive rows write and read consecutive words.
+// The entry that key i needs of query j is the one at offset i - j (window symmetry).  The weights of the next stage are on
+// their way to shared memory while one is used; pairs that do not exist weigh zero.  (Loaded into registers two keys
+// ahead they were waited for in the move to the next key's: 1031 us, 320 x 320, 8 units of 64 channels, ws 7.)
+// Bound: shared-memory reads, 32 cycles of vectors for NQ columns, next to 32 packed FMAs (8 cycles) per column.
+// =====================================================================
+// Copies four bytes to shared memory, or zero.
+__device__ __forceinline__ void cp_async4_or_zero(uint32_t dst, const float* src, bool on) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(on ? 4 : 0) : "memory");
+}
+
+template <bool DIST, int CPE, int NQ, int NCRT>
+__global__ void __launch_bounds__(128, (NQ == 1 ? 5 : 3)) dkdv_stored_kernel(TileArgs a, const __grid_constant__ CUtensorMap mv,
+                                                            const __grid_constant__ CUtensorMap msc) {
+    constexpr int NS = NCRT / 16;
+    constexpr int RW = 32 / NS;
+    const Geo& g = a.g;
+    const int ROWS = a.TH + 2 * (g.p + a.roff);
+    const int NSTAGES = g.wsw + NQ - 1;
+    const int w0 = blockIdx.x * NQ, h0 = blockIdx.y * a.TH, u = blockIdx.z, p = g.p;
+    CA_PIPE_PROLOGUE(false, 1)
+    const int slab = lt % NS, lr = (lt >> 5) * RW + (lt & 31) / NS, h = h0 + lr;
+    const bool active = h < g.H;
+
+    const float* unit = a.cs0 + (int64_t)(2 * u) * g.K * g.Np;
+    const int64_t second = (int64_t)g.K * g.Np;                  // from P to dS
+    const int64_t column = (int64_t)g.ws * g.Np;                 // from one window column's entries to the next's
+    const int half = g.ws * (2 * NQ * RW * 4);                   // bytes of a stage's weights: [key row][P | dS][column][row]
+    const uint32_t mine = smem_u32(smem_al) + a.extra_off + (lt >> 5) * (2 * half) + ((lt & 31) / NS) * 4;
+    // starts the copies of the weights of stage s with the centre columns; the lanes of a pixel share them out
+    auto fetch = [&](int s, int tb) {
+        int wq = w0 - p + s;
+        for (; wq < 0; wq += g.W) {}
+        for (; wq >= g.W; wq -= g.W) {}
+        const float* stage = unit + (int64_t)((2 * p - s) * g.ws + 2 * p) * g.Np + (int64_t)g.H * wq;
+#pragma unroll
+        for (int c0 = 0; c0 < 2 * NQ; c0 += NS) {
+            const int c = c0 + slab, r = c % NQ;
+            if (c >= 2 * NQ) break;
+            const bool on = active && w0 + r < g.W && s >= r && s <= r + 2 * p;
+            const float* at = on ? stage + r * column + (c >= NQ ? second : 0) : unit;
+            uint32_t to = mine + tb * half + c * (RW * 4);
+            int hq = h - p;
+            for (int di = 0; di < g.ws; ++di) {
+                cp_async4_or_zero(to, at + (on ? wrap_axis(hq, g.H) : 0), on);
+                at -= on ? g.Np : 0;
+                to += 2 * NQ * RW * 4;
+                ++hq;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    u64 dk[NQ][8], dv[NQ][8];
+    float sumds[NQ];
+#pragma unroll
+    for (int r = 0; r < NQ; ++r) {
+        sumds[r] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            dk[r][i] = zero2();
+            dv[r][i] = zero2();
+        }
+    }
+    fetch(0, 0);
+
+    CA_PIPE_LOOP({
+        uint32_t a0 = pipe.vec(buf, a) + (lr + a.roff) * (kRowBytes * NS);
+        uint32_t at = mine + (s & 1) * half;
+        if (s + 1 < s_end) {
+            fetch(s + 1, (s + 1) & 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();
+        const int mask = stage_mask<NQ>(s, p);
+        auto sweep = [&](auto full_tag) {
+            constexpr bool FULL = decltype(full_tag)::value;
+            _Pragma("unroll 2")
+            for (int di = 0; di < g.ws; ++di) {
+                u64 q2[8];
+                u64 y2[8];
+                lds_slab16<NS>(a0, 0, slab, q2);
+                lds_slab16<NS>(a0, 1, slab, y2);
+                _Pragma("unroll")
+                for (int r = 0; r < NQ; ++r) {
+                    if (!FULL && !((mask >> r) & 1)) continue;
+                    const float P = lds32(at + r * (RW * 4));
+                    const float S = lds32(at + (NQ + r) * (RW * 4));
+                    if (DIST) sumds[r] += S;
+                    _Pragma("unroll")
+                    for (int i = 0; i < 8; ++i) dk[r][i] = outer2(S, q2[i], dk[r][i]);
+                    _Pragma("unroll")
+                    for (int i = 0; i < 8; ++i) dv[r][i] = outer2(P, y2[i], dv[r][i]);
+                }
+                a0 += kRowBytes * NS;
+                at += 2 * NQ * RW * 4;
+            }
+        };
+        if (mask == (1 << NQ) - 1) sweep(std::true_type{});
+        else sweep(std::false_type{});
+        __syncwarp();                                            // the next stage but one writes what was read here
+    })
+
+    u64 k[NQ][8];
+    if (DIST) load_centre<CPE, NQ, NCRT>(a.c0, g, u, h, w0, active, 1.f, k, 16 * slab);
+    CA_OUT_DISPATCH(
+        _Pragma("unroll")
+        for (int r = 0; r < NQ; ++r) {
+            _Pragma("unroll")
+            for (int i = 0; i < 8; ++i) {
+                const float x = dk[r][i].x - (DIST ? sumds[r] * k[r][i].x : 0.f);
+                const float y = dk[r][i].y - (DIST ? sumds[r] * k[r][i].y : 0.f);
+                store_centre<CPE, NCRV, BF>(a.o0, g, u, h, w0, active, r, i, a.scale * x + ca_poison, a.scale * y + ca_poison, 16 * slab);
+                store_centre<CPE, NCRV, BF>(a.o1, g, u, h, w0, active, r, i, dv[r][i].x + ca_poison, dv[r][i].y + ca_poison, 16 * slab);
+            }
+        })
+}
+
 }  // namespace
 
 // Columns per thread: 1 (for short windows and small grids, and folded signals, whose streamed column pairs with one centre
@@ -428,7 +570,7 @@ static const SweepCost kDqCost[3][3] = {{{1, 20, 0, 123, 501, 4921}, {2, 12, 9, 
 
 template <>
 int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* dy, const float* stats,
-           const float* D, const float* kv, float* dq, cudaStream_t st, int mode, float* Dout) {
+           const float* D, const float* kv, float* dq, cudaStream_t st, int mode, float* Dout, float* weights) {
     Launch L{};
     const int ns = slabs_of(g);
     if (ns > 1 && mode) return CA_ERR_UNSUPPORTED;             // the entmax variants exist for one-slab units
@@ -437,10 +579,28 @@ int run_dq<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const fl
     // pre-pass 84 -> 63 us); the pre-pass does not share stages
     const bool fold = g.wsw == 1 && mode == 0;
     const SweepCost* cost = kDqCost[ns == 1 ? 0 : ns / 2] + (mode ? 1 : 0);
-    const TileShape t = choose_tile(g, P, ns, cost, fold || mode ? 1 : 3, mode < 2 && ns == 1 ? kParts : 1, false);
+    const TileShape t = choose_tile(g, P, ns, cost, fold || mode ? 1 : (weights ? 2 : 3), mode < 2 && ns == 1 ? kParts : 1);
     int rc = prepare(g, P, t, 17 * t.nq, kv, nullptr, &L, ns);
     if (rc) return rc;
-    L.a.scale = scale; L.a.c0 = q; L.a.c1 = dy; L.a.cs0 = stats; L.a.cs1 = D; L.a.o0 = dq; L.a.ostats = Dout;
+    L.a.scale = scale; L.a.c0 = q; L.a.c1 = dy; L.a.cs0 = stats; L.a.cs1 = D; L.a.o0 = dq; L.a.o1 = weights; L.a.ostats = Dout;
+    if (weights) {
+        if (ns != 4 || mode) return CA_ERR_UNSUPPORTED;
+#define CA_DQ_STORE(NQV, NCRV_)                                                                       \
+    do {                                                                                              \
+        if (g.cpe == 1) {                                                                             \
+            if (dist) CA_LAUNCH_TILED((dq_tiled_kernel<true, 1, NQV, 0, NCRV_, true>), L, st);        \
+            else CA_LAUNCH_TILED((dq_tiled_kernel<false, 1, NQV, 0, NCRV_, true>), L, st);            \
+        } else {                                                                                      \
+            if (dist) CA_LAUNCH_TILED((dq_tiled_kernel<true, 2, NQV, 0, NCRV_, true>), L, st);        \
+            else CA_LAUNCH_TILED((dq_tiled_kernel<false, 2, NQV, 0, NCRV_, true>), L, st);            \
+        }                                                                                             \
+    } while (0)
+        if (t.nq == 1) CA_DQ_STORE(1, 64);
+        else CA_DQ_STORE(2, 64);
+#undef CA_DQ_STORE
+        CA_CHECK_LAUNCH("tiled dq kernel");
+        return CA_OK;
+    }
 #define CA_DQ(NCRV_)                                                                          \
     do {                                                                                      \
         if (t.nq == 1) CA_DIST_CPE_NQ(dq_tiled_kernel, dist, g.cpe, 1, 0, NCRV_, L, st);      \
@@ -503,6 +663,37 @@ int run_dkdv<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const 
     else if (ns == 2) CA_DKDV(32);
     else CA_DKDV(64);
 #undef CA_DKDV
+    CA_CHECK_LAUNCH("tiled dk/dv kernel");
+    return CA_OK;
+}
+
+// One column per thread (five blocks per SM) or three (three blocks).
+static const SweepCost kStoredCost[2] = {{1, 20, 60, 90, 0, 5000}, {3, 12, 100, 120, 0, 9000}};
+
+template <>
+int run_dkdv_stored<kAnyC>(const Geo& g, const Padded& P, float scale, int dist, const float* k, const float* qdy, const float* weights,
+                           float* dk, float* dv, cudaStream_t st) {
+    Launch L{};
+    const int ns = slabs_of(g);
+    if (ns != 4) return CA_ERR_UNSUPPORTED;
+    const int col_bytes = 2 * g.ws * 2 * (32 / ns) * (int)sizeof(float);       // weights of two stages
+    const TileShape t = choose_tile(g, P, ns, kStoredCost, 2, 1, false, false, col_bytes, 2);
+    int rc = prepare(g, P, t, 0, qdy, nullptr, &L, ns, false, 2, (size_t)t.warps * t.nq * col_bytes);
+    if (rc) return rc;
+    L.a.scale = scale; L.a.c0 = k; L.a.cs0 = weights; L.a.o0 = dk; L.a.o1 = dv;
+#define CA_STORED(NQV, NCRV_)                                                                      \
+    do {                                                                                           \
+        if (g.cpe == 1) {                                                                          \
+            if (dist) CA_LAUNCH_TILED((dkdv_stored_kernel<true, 1, NQV, NCRV_>), L, st);           \
+            else CA_LAUNCH_TILED((dkdv_stored_kernel<false, 1, NQV, NCRV_>), L, st);               \
+        } else {                                                                                   \
+            if (dist) CA_LAUNCH_TILED((dkdv_stored_kernel<true, 2, NQV, NCRV_>), L, st);           \
+            else CA_LAUNCH_TILED((dkdv_stored_kernel<false, 2, NQV, NCRV_>), L, st);               \
+        }                                                                                          \
+    } while (0)
+    if (t.nq == 1) CA_STORED(1, 64);
+    else CA_STORED(3, 64);
+#undef CA_STORED
     CA_CHECK_LAUNCH("tiled dk/dv kernel");
     return CA_OK;
 }

@@ -50,7 +50,7 @@ int run_fwd_values(const Geo& g, const Padded& P, float scale, int dist, const f
 // mode 0: softmax; 1: entmax; 2: entmax pre-pass (writes D, needs no D and no dq).
 template <bool ANYC>
 int run_dq(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* dy, const float* stats,
-           const float* D, const float* kv, float* dq, cudaStream_t st, int mode, float* Dout);
+           const float* D, const float* kv, float* dq, cudaStream_t st, int mode, float* Dout, float* weights = nullptr);
 // One sweep of the entmax forward over the packed (k|v): mode 3 class maxima -> first threshold (tau),
 // 4 one step of the threshold search (tau and `settled` updated in place), 5 y = sum max(s/2 - tau, 0)^2 v.
 template <bool ANYC>
@@ -59,6 +59,10 @@ int run_entmax_fwd_sweep(const Geo& g, const Padded& P, float scale, int dist, c
 template <bool ANYC>
 int run_dkdv(const Geo& g, const Padded& P, float scale, int dist, const float* k, const float* v, const float* qdy,
              const float* planes, float* dk, float* dv, cudaStream_t st, bool entmax);
+// dk and dv from the weights that run_dq stored (`weights` of weight_floats()).
+template <bool ANYC>
+int run_dkdv_stored(const Geo& g, const Padded& P, float scale, int dist, const float* k, const float* qdy, const float* weights, float* dk,
+                    float* dv, cudaStream_t st);
 // A's values in CSR order: from q, a packed operand and the row statistics, or the raw scores without them.
 template <bool ANYC>
 int run_emit(const Geo& g, const Padded& P, float scale, int dist, const float* q, const float* stats, float* nz,
@@ -475,6 +479,17 @@ inline int slabs_of(const Geo& g) { return g.cr <= 16 ? 1 : (g.cr <= 32 ? 2 : 4)
 // and 197; 128 x 96, 8 of 16, ws 9 (10.4 KB): 55 and 67; 128 x 96, 4 of 32, ws 15 (14.4 KB): 115 and 109; 128 x 96, 8 of
 // 16, ws 11 (15.5 KB): 85 and 72; folded signals 8192 x 64 x 4, ws 63 (2 KB): 60 and 95.
 inline bool values_fit(const Geo& g, int ns) { return 32 / ns * g.K * 4 <= 11600; }
+
+// Words of the weights (P and dS) that the backward of wide units keeps between its dq and dk/dv sweeps; 0: dk/dv recomputes them.
+// 33 to 64 real channels: at 32 the weights cost as much to move as the contractions they save (150 x 140, 4 units, ws 11: 206
+// and 211 us for both sweeps, 320 x 240, 4 units, ws 5: 210 and 195).  Windows whose weights take no more memory than the
+// two packed pairs, and enough pixels to fill the chip: recomputing sweeps run side by side, which a few pixels need
+// (40 x 40, 2 units, ws 7: 21 us side by side, 27 one after the other; 100 x 64, 6 units, ws 11: 246 and 211).
+inline size_t weight_floats(const Geo& g) {
+    if (slabs_of(g) != 4 || g.wsw != g.ws || g.Wk != g.W || g.K > 288 || (int64_t)g.Np * g.units < 20000) return 0;
+    const size_t words = (size_t)2 * g.units * g.K * g.Np;
+    return words <= ((size_t)1 << 28) ? words : 0;          // at most 1 GiB
+}
 
 inline bool exact_shape(const Geo& g) {
     return (g.cr == 8 || g.cr == 16 || g.cr == 32 || g.cr == 64) && (int64_t)g.H * g.W == g.Np;

@@ -62,7 +62,7 @@ size_t tiled_bwd_workspace(const Geo& gin) {
     if (!fold_geo(gin, &g)) return 0;
     if (!tiled_shape_ok(g)) return 0;
     const Padded P = padded_of(g);
-    return (2 * P.pair_floats + P.plane_floats) * sizeof(float);
+    return (2 * P.pair_floats + P.plane_floats + weight_floats(g)) * sizeof(float);
 }
 
 int tiled_attention_fwd(const Geo& gin, float scale, int dist, const float* q, const float* k, const float* v,
@@ -180,6 +180,11 @@ int tiled_attention_bwd(const Geo& gin, float scale, int dist, const float* q, c
     pa.planes = planes; pa.stats = stats; pa.stat_mul = kLog2e; pa.y = y; pa.dy = dy; pa.Dout = D;
     int rc = launch_pack(pa, st);
     if (rc) return rc;
+    if (weight_floats(g)) {
+        float* weights = planes + P.plane_floats;
+        if ((rc = CA_CHANNELS(g, run_dq, g, P, scale, dist, q, dy, stats, D, kv, dq, st, 0, nullptr, weights))) return rc;
+        return CA_CHANNELS(g, run_dkdv_stored, g, P, scale, dist, k, qdy, weights, dk, dv, st);
+    }
     const bool small = (long)g.Np * g.units < 2048L * sm_count();      // fewer than ~4 CTAs per SM per sweep
     if (small) {
         ForkJoin* f = fork_join_for_current_device();

@@ -138,3 +138,26 @@ def test_line_pixels(ca, shape, ws, norm):
         dqo, dko, dvo = orc.attention_pullback(orc.DISTANCE, qo, ko, vo, ws, ro, None, which)
         for name, got, want in (("y", y, yo), ("dq", q.grad, dqo), ("dk", k.grad, dko), ("dv", v.grad, dvo)):
             assert_close(ca.jl.to_numpy(got)[..., one], want, f"{name} of unit {u}")
+
+
+@pytest.mark.parametrize("simname", ["dot", "distance"])
+@pytest.mark.parametrize("shape,ws,cplx", [
+    ((100, 53, 64, 4), 5, False),      # the weights of the dq sweep stored: an odd last column, rows past the image
+    ((75, 70, 40, 4), 7, False),       # 40 channels in four slabs
+    ((71, 71, 32, 4), 9, True),        # complex, three columns do not divide the width
+    ((41, 37, 64, 14), 17, False),     # the largest window whose weights are stored
+    ((41, 37, 64, 14), 19, False),     # past it: recomputed
+])
+def test_wide_backward(ca, shape, ws, cplx, simname):
+    rng = np.random.default_rng(67)
+    qn, kn, vn, rn = (randn(rng, shape, cplx) for _ in range(4))
+    q, k, v = (ca.jl.from_numpy(t).requires_grad_(True) for t in (qn, kn, vn))
+    sim = ca.DotSimilarity() if simname == "dot" else ca.DistanceSimilarity()
+    y, _ = ca.circulant_attention(sim, q, k, v, ws, return_A=False)
+    r = ca.jl.from_numpy(rn)
+    ((y * r.conj()).real.sum() if cplx else (y * r).sum()).backward()
+    for u in (0, shape[-1] - 1):
+        one = slice(u, u + 1)
+        dqo, dko, dvo = orc.attention_pullback(KIND[simname], *(up(t[..., one]) for t in (qn, kn, vn)), ws, up(rn[..., one]))
+        for name, got, want in (("dq", q.grad, dqo), ("dk", k.grad, dko), ("dv", v.grad, dvo)):
+            assert_close(ca.jl.to_numpy(got)[..., one], want, f"{name} of unit {u}")
