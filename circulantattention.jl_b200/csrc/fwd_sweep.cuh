@@ -63,7 +63,7 @@ __device__ __forceinline__ void fwd_stage(uint32_t rowbase, int ws, int rm, floa
                     bk = -0.5f * sl2 * hsum2(n);
                 }
                 if (MASK != 0) {
-                    // all four chains advance together (4 independent FMAs in flight)
+                    // the chains of all columns advance together
                     u64 sa[NQ];
 #pragma unroll
                     for (int r = 0; r < NQ; ++r) {

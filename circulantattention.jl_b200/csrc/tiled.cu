@@ -1,11 +1,11 @@
-// Tiled sm_100a kernels for 2-D windows with 16 real channels per unit
-// (16 Float32 or 8 ComplexF32 channels per head) and softmax.
+// Tiled sm_100a kernels for 2-D windows and folded 1-D signals of up to 64 real channels per unit (Float32 or ComplexF32;
+// bfloat16 storage at 8 and 16), softmax, and for one slab of channels the 1.5-entmax.
 //
-// Work decomposition.  A CTA owns TH consecutive rows (the fast axis h) of NQ
-// consecutive columns w0..w0+NQ-1 of one unit (NQ = 4 in the forward and dq
-// kernels, 3 in the dk/dv kernel).  A thread owns one row and the NQ pixels of
-// that row ("centre" pixels: queries in the forward and dq kernels, keys in
-// the dk/dv kernel) and keeps their 16-channel vectors in registers.  The other
+// Work decomposition.  A CTA owns TH consecutive rows (the fast axis h) of NQ consecutive columns w0..w0+NQ-1 of one unit.
+// A thread owns one row and the NQ pixels of that row ("centre" pixels: queries in the forward and dq kernels, keys in
+// the dk/dv kernels) and keeps their 16-channel vectors in registers; units of more channels give a pixel two or four
+// lanes.  NQ, the rows and how many groups of warps share the stages of a tile follow from a prediction of the time
+// (choose_tile).  The other
 // side of the window is streamed through shared memory one image column at a
 // time: column stage s holds column w0 - p + s (wrapped circularly, or taken
 // from the neighbour halo in band mode) for rows h0-p' .. h0+TH+p'-1.  Centre
@@ -28,15 +28,14 @@
 // conflict free without any address swizzle and every chunk of every row of a
 // window column is the thread's row base plus a compile-time constant.
 //
-// Arithmetic: FP32 on the FMA pipe, channel pairs as two scalar FMAs.  Softmax in
+// Arithmetic: FP32 on the FMA pipe, dot products scalar, outer products as packed FMAs.  Softmax in
 // the log2 domain with ex2.approx.  The running maximum (forward) or the saved row
 // statistic (backward) is folded into the initial value of the dot-product
 // chain, and the forward only touches the maximum when the sign bits of a chunk
 // of relative scores say that one of them is positive.
 //
-// Small grids.  When the grid would not fill the GPU, the column stages of a
-// tile are split between two groups of warps of the same CTA (each with its own
-// copy pipeline) whose partial results are merged through shared memory.
+// Small grids.  Where it pays, the column stages of a tile are split between up to four groups of warps of the same CTA
+// (each with its own copy pipeline) whose partial results are merged through shared memory.
 #include "tile_common.cuh"
 
 namespace ca {
@@ -151,7 +150,8 @@ static ForkJoin* fork_join_for_current_device() {
     return &f;
 }
 
-// Whole backward in three launches: pack (both pairs, D, planes), dq, dk/dv.
+// Whole backward in three launches: pack (both pairs, D, planes), dq, dk/dv.  The two sweeps run side by side on small
+// problems; where dq stores the weights for dk/dv (weight_floats) they run one after the other.
 int tiled_attention_bwd(const Geo& gin, float scale, int dist, const float* q, const float* k, const float* v,
                         const float* y, const float* dy, const float* stats, float* D, float* dq, float* dk,
                         float* dv, void* workspace, const void* fwd_workspace, cudaStream_t st) {
