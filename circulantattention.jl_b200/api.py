@@ -273,7 +273,14 @@ def circulant_adjacency(simfun, x, y, W: int, normalizer=SOFTMAX, lazy=False):
         _check_odd(W)
         _check_xy(x, y)
         return LazyAdjacency([(1, simfun, x, y, normalizer)], W, 1, tuple(x.shape[:-2]), x.shape[-1], False)
-    return softmax(circulant_similarity(simfun, x, y, W), normalizer)
+    _check_odd(W)
+    _check_xy(x, y)
+    return _adjacency(simfun, x, y, W, 1, normalizer)
+
+
+def _adjacency(simfun, x, y, W, nheads, normalizer):
+    nz = host.adjacency(x, y, _kind(simfun), int(W), int(nheads), normalizer)
+    return Circulant._from_nz(nz, int(W), tuple(x.shape[:-2]))
 
 
 def circulant_adjacency_(A: Circulant, simfun, x, y) -> Circulant:
@@ -342,8 +349,7 @@ def circulant_mh_adjacency(simfun, x, y, W: int, nheads: int, normalizer=SOFTMAX
     _check_odd(W)
     _check_xy(x, y)
     assert x.shape[-2] % nheads == 0, f"channels ({x.shape[-2]}) must be divisible by nheads ({nheads})"
-    nz = host.similarity(x, y, _kind(simfun), int(W), int(nheads))
-    return softmax(Circulant._from_nz(nz, int(W), tuple(x.shape[:-2])), normalizer)
+    return _adjacency(simfun, x, y, W, nheads, normalizer)
 
 
 def _apply(A: Circulant, x, transpose, nheads=1):

@@ -306,6 +306,42 @@ Tensor normalize(const Tensor& nz, const std::vector<int64_t>& spatial, int64_t 
     return NormalizeFn::apply(nz, spatial, ws, normalizer);
 }
 
+// ---------------------------------------------------------------- adjacency
+// softmax o circulant_similarity and the composition of their rrules (src/similarity.jl:157-161, src/rrules.jl:1-56) as one
+// node instead of two (a host-bound graph of two adjacencies, 96 x 80 x 32 x 2, ws 9, with every gradient: 276 -> 254 us).
+Tensor adjacency_raw(const Tensor& x, const Tensor& y, int64_t kind, int64_t ws, int64_t heads, int64_t normalizer) {
+    const Tensor s = similarity_raw(kind, x, y, ws, 1.0, heads);          // checks x and y
+    const std::vector<int64_t> spatial(x.sizes().begin(), x.sizes().end() - 2);
+    return std::get<0>(normalize_raw(s, spatial, ws, normalizer, std::nullopt, false));
+}
+
+struct AdjacencyFn : public Function<AdjacencyFn> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& y, int64_t kind, int64_t ws, int64_t heads, int64_t normalizer) {
+        Tensor p = adjacency_raw(x, y, kind, ws, heads, normalizer);
+        ctx->save_for_backward({x, y, p});
+        ctx->saved_data["kind"] = kind;
+        ctx->saved_data["ws"] = ws;
+        ctx->saved_data["heads"] = heads;
+        ctx->saved_data["normalizer"] = normalizer;
+        return p;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const auto s = ctx->get_saved_variables();
+        const Tensor &x = s[0], &y = s[1];
+        const int64_t ws = ctx->saved_data["ws"].toInt();
+        const std::vector<int64_t> spatial(x.sizes().begin(), x.sizes().end() - 2);
+        const Tensor ds = normalize_bwd_raw(s[2], g[0], spatial, ws, ctx->saved_data["normalizer"].toInt());
+        auto [dx, dy] = similarity_bwd_raw(ctx->saved_data["kind"].toInt(), x, y, ws, ds, 1.0, ctx->saved_data["heads"].toInt(),
+                                           ctx->needs_input_grad(0), ctx->needs_input_grad(1));
+        return {dx, dy, Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+Tensor adjacency(const Tensor& x, const Tensor& y, int64_t kind, int64_t ws, int64_t heads, int64_t normalizer) {
+    if (!tracked({&x, &y})) return adjacency_raw(x, y, kind, ws, heads, normalizer);
+    return AdjacencyFn::apply(x, y, kind, ws, heads, normalizer);
+}
+
 // ---------------------------------------------------------------- apply
 // A (x) v or A^T (x) v.  nz: (Np*K, batch...); v: (spatial..., C, B) of `heads` heads.  Where the units of A are
 // broadcast over those of v or the other way round, the result has the larger number of units.
@@ -610,6 +646,7 @@ PYBIND11_MODULE(_circatt_host, m) {
     });
     m.def("attention", &attention, release());
     m.def("similarity", &similarity, release());
+    m.def("adjacency", &adjacency, release());
     m.def("similarity_raw", [](int64_t kind, const Tensor& x, const Tensor& y, int64_t ws, double scale) {
         const Tensor nz = similarity_raw(kind, x, y, ws, scale, 1);
         return view_cm(nz, {nz.size(0), nz.size(2)});
