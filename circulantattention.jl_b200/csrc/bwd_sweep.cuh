@@ -45,12 +45,7 @@ __device__ __forceinline__ void dq_stage(uint32_t rowbase, int ws, int rm, float
         u64 k2[8];
         lds_slab16<NS>(a0, 0, slab, k2);
         float bk = 0.f;
-        if (DIST) {
-            u64 n = zero2();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) n = fma2(k2[i], k2[i], n);
-            bk = -0.5f * sl2 * hsum2(n);
-        }
+        if (DIST) bk = -0.5f * sl2 * lds_norm(a0, 128 * NS, slab);
 #pragma unroll
         for (int r = 0; r < NQ; ++r)
             if (CA_ON(r)) {
@@ -312,12 +307,7 @@ __device__ __forceinline__ void dkdv_stage(uint32_t a0, uint32_t sa, uint32_t pl
         u64 q2[8];
         lds_slab16<NS>(a0, 0, slab, q2);
         float bqj = 0.f;
-        if (DIST) {
-            u64 n = zero2();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) n = fma2(q2[i], q2[i], n);
-            bqj = -0.5f * sl2 * hsum2(n);
-        }
+        if (DIST) bqj = -0.5f * sl2 * lds_norm(a0, 128 * NS, slab);
 #pragma unroll
         for (int r = 0; r < NQ; ++r)
             if (CA_ON(r)) {

@@ -41,17 +41,12 @@ struct Scatter {
 
 // Partial scores (this lane's slab) of the key at a0 with all centre columns, chains interleaved.
 template <bool DIST, int NQ, int NS>
-__device__ __forceinline__ void emit_scores(uint32_t a0, int slab, float sl2, const u64 (&q)[NQ][8], const u64 (&nL2)[NQ],
+__device__ __forceinline__ void emit_scores(uint32_t a0, int RB, int slab, float sl2, const u64 (&q)[NQ][8], const u64 (&nL2)[NQ],
                                             const float (&bq)[NQ], float (&sc)[NQ]) {
     u64 k2[8], t[NQ];
     lds_slab16<NS>(a0, 0, slab, k2);
     float bk = 0.f;
-    if (DIST) {
-        u64 n = zero2();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) n = fma2(k2[i], k2[i], n);
-        bk = -0.5f * sl2 * hsum2(n);
-    }
+    if (DIST) bk = -0.5f * sl2 * lds_norm(a0, RB - 16 * NS, slab);
 #pragma unroll
     for (int r = 0; r < NQ; ++r) {
         t[r] = nL2[r];
@@ -78,8 +73,8 @@ __device__ __forceinline__ void emit_keys(uint32_t a0, int RB, int len, int slab
 #pragma unroll 2
     for (; len >= 2; len -= 2, a0 += 2 * RB) {
         float s0[NQ], s1[NQ];
-        emit_scores<DIST, NQ, NS>(a0, slab, sl2, q, nL2, bq, s0);
-        emit_scores<DIST, NQ, NS>(a0 + RB, slab, sl2, q, nL2, bq, s1);
+        emit_scores<DIST, NQ, NS>(a0, RB, slab, sl2, q, nL2, bq, s0);
+        emit_scores<DIST, NQ, NS>(a0 + RB, RB, slab, sl2, q, nL2, bq, s1);
         const int pos1 = pos + 4 == wrap ? 0 : pos + 4;
         if constexpr (NS == 1) {
 #pragma unroll
@@ -101,7 +96,7 @@ __device__ __forceinline__ void emit_keys(uint32_t a0, int RB, int len, int slab
     }
     if (len) {
         float s0[NQ];
-        emit_scores<DIST, NQ, NS>(a0, slab, sl2, q, nL2, bq, s0);
+        emit_scores<DIST, NQ, NS>(a0, RB, slab, sl2, q, nL2, bq, s0);
         if constexpr (NS == 1) {
 #pragma unroll
             for (int r = 0; r < NQ; ++r)

@@ -81,7 +81,13 @@ __device__ __forceinline__ void pack_rows_body(const PackArgs& a, float* tile) {
         for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int c = 0; c < 4; ++c) trow[t * (4 * NS) + c * NS + slab] = make_float4(vals[t][4 * c], vals[t][4 * c + 1], vals[t][4 * c + 2], vals[t][4 * c + 3]);
-        trow[4 * NT * NS + slab] = make_float4(0.f, 0.f, 0.f, 0.f);            // padding words
+        float2 norm = make_float2(0.f, 0.f);               // squared, of the first tensor, for the Distance sweeps
+#pragma unroll
+        for (int e = 0; e < 16; e += 2) {
+            norm.x = fmaf(vals[0][e], vals[0][e], norm.x);
+            norm.y = fmaf(vals[0][e + 1], vals[0][e + 1], norm.y);
+        }
+        trow[4 * NT * NS + slab] = make_float4(norm.x + norm.y, 0.f, 0.f, 0.f);         // padding words
         __syncthreads();
         const int nrows = min(RB, a.Hp - rr0);
         float4* out = reinterpret_cast<float4*>(a.dst[slot] + (((int64_t)u * g.Wk + w) * a.Hp + rr0) * RF);

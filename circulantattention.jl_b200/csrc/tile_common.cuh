@@ -167,6 +167,12 @@ __device__ __forceinline__ void lds_slab16(uint32_t a0, int which, int slab, u64
     lds128(b + 48 * NS, v[6], v[7]);
 }
 
+// The squared norm of slab `slab` of the first tensor of the pixel row at `a0`: the pack leaves it in the slab's padding words
+// (`pad` bytes into the row), so that the Distance sweeps do not form it for every key they meet, 16 FMAs each in every
+// thread (600 x 500, 8 units, ws 21: forward 2123 -> 1918 us, dq 3029 -> 2668, dk/dv 4070 -> 3768; 128 x 96, 8 units, ws 15: 61 -> 55,
+// 81 -> 72, 120 -> 111).
+__device__ __forceinline__ float lds_norm(uint32_t a0, int pad, int slab) { return lds32(a0 + pad + 16 * slab); }
+
 // Global offset of real channel cc of unit u at pixel pix (npix pixels per plane, cr real channels per unit).
 template <int CPE>
 __device__ __forceinline__ int64_t goff(int u, int cr, int cc, int npix, int pix) {
