@@ -325,10 +325,11 @@ __device__ __forceinline__ void dkdv_stage(uint32_t a0, uint32_t sa, uint32_t pl
                     ds = gg * dp[r];
                 }
                 if (DIST) sumds[r] += ds;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) dk[r][i] = outer2(ds, q2[i], dk[r][i]);
+                // dv first: its vector was loaded first and is free again sooner (1024 x 1024, 2 units, ws 21: 3009 -> 2966 us)
 #pragma unroll
                 for (int i = 0; i < 8; ++i) dv[r][i] = outer2(P, y2[i], dv[r][i]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) dk[r][i] = outer2(ds, q2[i], dk[r][i]);
             }
         a0 += kRowBytes * NS;
         ++Lr;
