@@ -638,8 +638,8 @@ inline TileShape choose_tile(const Geo& g, const Padded& P, int ns, const SweepC
     return e.shape;
 }
 
-// Operators: four warps of rows; fewer than 6 warps per SM share the stages of a tile (in four where the kernel can,
-// in two up to 12 warps per SM).
+// The apply runs of folded signals, and of windows whose runs fill the shared memory: `max_warps` warps of rows; fewer than 6
+// warps per SM share the stages of a tile (in four where the kernel can, in two up to 12 warps per SM).
 inline TileShape operator_tile(const Geo& g, int ns, int nq, int max_split, int max_warps) {
     const int rw = 32 / ns;
     const int warps = std::min(max_warps, (g.H + rw - 1) / rw);
