@@ -1,0 +1,596 @@
+// Shared parts of the tensor-core sweeps (split_*.cu): softmax attention on 2-D windows with every Float32 operand as a pair
+// of half-precision numbers.
+//
+// Arithmetic.  A Float32 number x is the sum of hi = half(x / s) and lo = half(x / s - hi), times a power of two s: 22 to 24
+// of its bits.  A product of two such numbers is hi*hi + hi*lo + lo*hi on the tensor cores (mma.sync m16n8k16, Float32
+// accumulators); lo*lo is below the last bit.  That is three tensor products where three-way bfloat16 splits take six and
+// tf32 pairs three of twice the time: the warp-level unit runs 1024 half-precision FMAs per SM and cycle, 512 of tf32.
+// tcgen05 is not used: its scores would leave and enter through tensor memory for the mask, the exponential and the
+// split, which costs more than its rate gains at 16 to 64 channels (forward 70.6 us against 62.5 on the FMA pipe).
+//
+// Tiles.  Rows of a product are 16 centre pixels: 8 rows (h) of two neighbouring columns (w), whose windows share all but two
+// columns.  Columns are 8 pixels of the streamed column, so a window column takes NT = ceil((8 + 2p) / 8) tiles and 62 %
+// (window 21) to 44 % (window 7) of the scores are inside the window; 16 rows of one column would leave 52 and 29 %.
+// Scores outside start at -inf in the accumulator, which costs nothing.
+//
+// Streamed rows.  [unit][column][row'][128 NS + 16 bytes] = hi then lo of the first tensor, hi then lo of the second, 16 bytes of
+// scalars; row' = h + p with the circular halo unrolled.  The pitch is an odd number of 16-byte words, so ldmatrix
+// reads eight rows without bank conflicts.  The power of two is common to a group of eight rows starting at a multiple of eight
+// (a warp's window starts at one), so it is uniform over a tile.  It puts the group's largest magnitude into [2^11, 2^15): an
+// element 2^13 below it keeps all bits, the least step is 2^-36 of the largest.
+//
+// Rows with a NaN or an infinity mark their group; a block that meets one recomputes its pixels from the tensors one
+// by one (exact_*), since a product of a tile would carry them to pixels outside their window.
+#pragma once
+#include "tile_common.cuh"
+#include <cuda_fp16.h>
+
+namespace ca {
+
+struct SplitArgs {
+    Geo g;
+    float scale;
+    int dist;
+    const float* c0;        // centre tensors
+    const float* c1;
+    const float* stats;     // statistics of the centre pixels (dq)
+    const float* D;
+    float* o0;              // outputs
+    float* o1;
+    float* ostats;
+    const float* x0;        // streamed tensors and their pixels' statistics in the reference layout, for the pixels that are recomputed
+    const float* x1;
+    const float* xstats;
+    const float* xD;
+    int* status;            // nullable device word of the caller: bit 0 is set when a stage wait ran out
+    int* timeouts;          // device counter of the blocks that gave up waiting for a copy
+    uint32_t wait_tries;    // polls before a wait gives up
+};
+
+struct SplitPackArgs {
+    Geo g;
+    int Hp;                 // padded rows per column: roundup4(H + 2p)
+    const float* x0;
+    const float* x1;
+    float norm_mul;         // Distance: the scalar of a row is norm_mul |x0|^2 ...
+    const float* stats;     // ... - stats log2(e), and -D goes with it (nullable: neither)
+    const float* y;         // D = y . x1 ...
+    const float* Din;       // ... or given
+    float* Dout;            // nullable
+    float* dst;
+};
+
+// 2-D softmax windows the sweeps take.
+bool split_shape_ok(const Geo& g, float scale);
+// Packs (x0|x1); with `stats` also the scalars of the backward, D = y . x1 (written to Dout) or given.
+int launch_split_pack(const Geo& g, float scale, int dist, const float* x0, const float* x1, const float* stats, const float* y, const float* Din,
+                      float* Dout, float* dst, cudaStream_t st);
+int run_split_fwd(const Geo& g, float scale, int dist, const float* q, const float* k, const float* v, const float* kv, float* y, float* stats,
+                  cudaStream_t st);
+// A's values in CSR order from the row statistics.
+int run_split_emit(const Geo& g, float scale, int dist, const float* q, const float* k, const float* stats, const float* kv, float* nz,
+                   cudaStream_t st);
+int run_split_dq(const Geo& g, float scale, int dist, const float* q, const float* k, const float* v, const float* dy, const float* stats,
+                 const float* D, const float* kv, float* dq, cudaStream_t st);
+int run_split_dkdv(const Geo& g, float scale, int dist, const float* q, const float* k, const float* v, const float* dy, const float* stats,
+                   const float* D, const float* qdy, float* dk, float* dv, cudaStream_t st);
+
+namespace {
+
+__host__ __device__ constexpr int split_row_bytes(int ns) { return 128 * ns + 16; }
+constexpr int kSplitSteps = 3, kSplitWarps = 4;
+__host__ __device__ constexpr int split_rows(int nt) { return 8 * (kSplitWarps - 1) + 8 * nt; }
+__host__ __device__ constexpr int split_stage_bytes(int ns, int nt) { return (split_rows(nt) * split_row_bytes(ns) + 127) & ~127; }
+__host__ __device__ inline int split_hp(const Geo& g) { return (g.H + 2 * g.p + 3) & ~3; }
+inline int split_tiles(const Geo& g) { return (8 + 2 * g.p + 7) / 8; }
+
+// ---------------------------------------------------------------- device
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+// d = a b + c, 16 x 16 by 16 x 8.
+__device__ __forceinline__ void mma16(float (&d)[4], const uint32_t* a, uint32_t b0, uint32_t b1, const float (&c)[4]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %12, %13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+__device__ __forceinline__ void mma16(float (&d)[4], const uint32_t* a, uint32_t b0, uint32_t b1) {                // d = a b
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// hi and lo of two numbers below 2^15.  The remainder as a mixed-precision FMA: 1.34 SM cycles a warp and pair; with a conversion
+// back to Float32 and a subtraction 1.59, with the low bits masked off 1.82.
+__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    float rx, ry;
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(rx) : "h"(__half_as_ushort(__low2half(h))), "h"((unsigned short)0xbc00), "f"(x));
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(ry) : "h"(__half_as_ushort(__high2half(h))), "h"((unsigned short)0xbc00), "f"(y));
+    const __half2 l = __floats2half2_rn(rx, ry);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// Pairs of Float32 numbers for the two-lane instructions, kept as one register pair: a coefficient that stands twice in a pair is
+// then formed once and not for every use.
+typedef unsigned long long pair_t;
+__device__ __forceinline__ pair_t pair(float x, float y) {
+    pair_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpair(pair_t p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ pair_t fma_pair(pair_t a, pair_t b, pair_t c) {
+    pair_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ pair_t add_pair(pair_t a, pair_t b) {
+    pair_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair_t mul_pair(pair_t a, pair_t b) {
+    pair_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// Biased exponent of the power of two that brings magnitudes up to `bits` below 2^15: a multiple of `step`, 0 for zero,
+// 255 for a NaN or an infinity.
+// `least` is the smallest that is given (also to zeros, where it is not 0).
+__device__ __forceinline__ int scale_exp(uint32_t bits, int step, int least) {
+    const int e = (int)(bits >> 23);
+    if (bits == 0) return least;
+    if (e == 255) return 255;
+    return max((e - 14 + step - 1) / step * step, max(least, 4));
+}
+// Least exponent of a score's operands, 2^-55: the product of two scales is no denormal, so a start of -inf stays -inf.
+constexpr int kLeastExp = 72;
+__device__ __forceinline__ float exp_scale(int e) { return __uint_as_float((uint32_t)e << 23); }
+__device__ __forceinline__ float exp_inverse(int e) { return e ? __uint_as_float((uint32_t)(254 - e) << 23) : 0.f; }
+
+// One real channel of a dense tensor, whatever its storage.
+__device__ __forceinline__ float ld_channel(const float* src, const Geo& g, int u, int cc, int npix, int pix) {
+    if (g.cpe == 2) return __ldg(src + goff<2>(u, g.cr, cc, npix, pix));
+    return g.bf16 ? ld_real<true>(src, goff<1>(u, g.cr, cc, npix, pix)) : ld_real<false>(src, goff<1>(u, g.cr, cc, npix, pix));
+}
+__device__ __forceinline__ void st_channel(float* dst, const Geo& g, int u, int cc, int npix, int pix, float x) {
+    if (g.cpe == 2) dst[goff<2>(u, g.cr, cc, npix, pix)] = x;
+    else if (g.bf16) st_real<true>(dst, goff<1>(u, g.cr, cc, npix, pix), x);
+    else st_real<false>(dst, goff<1>(u, g.cr, cc, npix, pix), x);
+}
+
+// The channels 2t, 2t+1, 2t+8, 2t+9 of every slab (t = lane % 4) of the two pixels of a lane's row: what a lane holds of a row of an A
+// operand and of a result.  Pixels outside the image and channels past the unit's read some other element of the tensor and
+// are zeroed in Centre::form: without conditions all loads of a warp are in flight together.
+template <int NS>
+struct Raw {
+    float x[2][NS][4];
+    __device__ __forceinline__ void load(const float* src, const Geo& g, int u, int h, int w, int tq) {
+        const int hc = min(h, g.H - 1);
+        const int pix[2] = {hc + g.H * w, hc + g.H * min(w + 1, g.W - 1)};
+        if (g.cpe == 2) {
+            const float2* s2 = reinterpret_cast<const float2*>(src) + (int64_t)u * g.c * g.Np;
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const float2 z = __ldg(s2 + (int64_t)min(8 * s + tq + 4 * i, g.c - 1) * g.Np + pix[r]);
+                        x[r][s][2 * i] = z.x;
+                        x[r][s][2 * i + 1] = z.y;
+                    }
+            return;
+        }
+        const int64_t o = (int64_t)u * g.cr * g.Np;
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int64_t c = o + (int64_t)min(16 * s + 2 * tq + (i & 1) + 8 * (i >> 1), g.cr - 1) * g.Np;
+#pragma unroll
+                for (int r = 0; r < 2; ++r) x[r][s][i] = g.bf16 ? ld_real<true>(src, c + pix[r]) : ld_real<false>(src, c + pix[r]);
+            }
+    }
+};
+// The channel of element i of slab s.
+__device__ __forceinline__ int lane_channel(const Geo& g, int s, int i, int tq) { return 16 * s + 2 * tq + (i & 1) + 8 * (i >> 1); }
+
+// The four channels of one slab of a pixel: x[0..1] in the result's first eight channels, x[2..3] in its second.
+__device__ __forceinline__ void store_pixel(float* dst, const Geo& g, int u, int slab, int pix, int tq, float x0, float x1, float x2, float x3) {
+    if (g.cpe == 2) {
+        float2* d2 = reinterpret_cast<float2*>(dst);
+        const int c = 8 * slab + tq;
+        if (c < g.c) d2[((int64_t)u * g.c + c) * g.Np + pix] = make_float2(x0, x1);
+        if (c + 4 < g.c) d2[((int64_t)u * g.c + c + 4) * g.Np + pix] = make_float2(x2, x3);
+        return;
+    }
+    const float x[4] = {x0, x1, x2, x3};
+    const int64_t o = (int64_t)u * g.cr * g.Np + pix;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int c = 16 * slab + 2 * tq + (i & 1) + 8 * (i >> 1);
+        if (c >= g.cr) continue;
+        if (g.bf16) st_real<true>(dst, o + (int64_t)c * g.Np, x[i]);
+        else st_real<false>(dst, o + (int64_t)c * g.Np, x[i]);
+    }
+}
+__device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t quad_max(uint32_t x) {
+    x = max(x, __shfl_xor_sync(0xffffffffu, x, 1));
+    return max(x, __shfl_xor_sync(0xffffffffu, x, 2));
+}
+__device__ __forceinline__ float quad_max(float x) {
+    x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+    return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+}
+__device__ __forceinline__ float quad_sum(float x) {
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    return x + __shfl_xor_sync(0xffffffffu, x, 2);
+}
+
+// An A operand: the split vectors of the two pixels of each row of a tile, with each pixel's scale and squared norm.
+template <int NS>
+struct Centre {
+    uint32_t hi[NS][4], lo[NS][4];
+    float scale[2], norm2[2];
+    bool bad;
+    __device__ __forceinline__ void form(const Raw<NS>& raw, const Geo& g, int h, int w, int tq, int least) {
+        bad = false;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const bool ok = h < g.H && w + r < g.W;
+            float x[NS][4];
+            uint32_t m = 0;
+            float n = 0.f;
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    x[s][i] = ok && lane_channel(g, s, i, tq) < g.cr ? raw.x[r][s][i] : 0.f;
+                    m = max(m, abs_bits(x[s][i]));
+                    n = fmaf(x[s][i], x[s][i], n);
+                }
+            const int e = scale_exp(quad_max(m), 1, least);
+            norm2[r] = quad_sum(n);
+            bad |= e == 255;
+            scale[r] = exp_scale(e);
+            const float inv = exp_inverse(e == 255 ? 0 : e);
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                split2(x[s][0] * inv, x[s][1] * inv, hi[s][r], lo[s][r]);
+                split2(x[s][2] * inv, x[s][3] * inv, hi[s][2 + r], lo[s][2 + r]);
+            }
+        }
+    }
+};
+
+// Tiles of a step: NT of its first column, then NT of its second; offset of tile f from the step's first row.
+template <int NS, int NT>
+__device__ __forceinline__ constexpr int tile_offset(int f) {
+    return (f / NT) * split_stage_bytes(NS, NT) + 8 * (f % NT) * split_row_bytes(NS);
+}
+
+// x[f] = centre . streamed over the channels for the tiles of a step: `b` is this lane's ldmatrix address inside the first tensor or
+// the second.  The chains of the tiles advance together (a warp issues in order and a dependent product waits 20 cycles);
+// small products first, since the unit cuts its sums.
+template <int NS, int NT>
+__device__ __forceinline__ void dot_tiles(const Centre<NS>& a, uint32_t b, float (&x)[2 * NT][4]) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        uint32_t f[2 * NT][4];
+#pragma unroll
+        for (int t = 0; t < 2 * NT; ++t) ldsm4(b + tile_offset<NS, NT>(t) + 32 * s, f[t]);      // hi of 8 + 8 channels, lo of 8 + 8
+#pragma unroll
+        for (int t = 0; t < 2 * NT; ++t) {
+            if (s == 0) mma16(x[t], a.lo[s], f[t][0], f[t][1]);
+            else mma16(x[t], a.lo[s], f[t][0], f[t][1], x[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < 2 * NT; ++t) mma16(x[t], a.hi[s], f[t][2], f[t][3], x[t]);
+#pragma unroll
+        for (int t = 0; t < 2 * NT; ++t) mma16(x[t], a.hi[s], f[t][0], f[t][1], x[t]);
+    }
+}
+
+// acc += S * (weights . streamed) over the pixels of a step.  The weights of its tiles are split pairs as A operands: two tiles of a
+// column make one of 16 pixels, the odd last ones of the two columns another.  `b`: this lane's transposing ldmatrix address
+// for 16 rows of a column, `bt` the one for 8 rows of each column.  The unit cuts its sums instead of rounding them, 0.7
+// units of the last place of a partial sum on average; the sums of a step therefore start at zero, the products of the
+// upper halves apart from the small ones, and are added to the running ones in Float32.
+template <int NS, int NT>
+__device__ __forceinline__ void outer_tiles(const uint32_t (&hi)[2 * NT][2], const uint32_t (&lo)[2 * NT][2], uint32_t b, uint32_t bt, const pair_t (&S)[2],
+                                            pair_t (&acc)[NS][2][2]) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        float c[2][4], d[2][4];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+            const bool tail = (NT & 1) && k == NT - 1;
+            const int t = tail ? NT - 1 : (k < NT / 2 ? 2 * k : NT + 2 * (k - NT / 2)), t1 = tail ? 2 * NT - 1 : t + 1;
+            const uint32_t at = (tail ? bt : b) + tile_offset<NS, NT>(t) + 32 * s;
+            uint32_t x[4], y[4];
+            ldsm4t(at, x);                                 // hi: channels 0-7 of 8 + 8 rows, channels 8-15
+            ldsm4t(at + 32 * NS, y);                       // lo
+            const uint32_t ah[4] = {hi[t][0], hi[t][1], hi[t1][0], hi[t1][1]};
+            const uint32_t al[4] = {lo[t][0], lo[t][1], lo[t1][0], lo[t1][1]};
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                if (k == 0) mma16(c[n], ah, x[2 * n], x[2 * n + 1]);
+                else mma16(c[n], ah, x[2 * n], x[2 * n + 1], c[n]);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                if (k == 0) mma16(d[n], al, x[2 * n], x[2 * n + 1]);
+                else mma16(d[n], al, x[2 * n], x[2 * n + 1], d[n]);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) mma16(d[n], ah, y[2 * n], y[2 * n + 1], d[n]);
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; i += 2)
+                acc[s][n][i / 2] = fma_pair(add_pair(pair(c[n][i], c[n][i + 1]), pair(d[n][i], d[n][i + 1])), S[i / 2], acc[s][n][i / 2]);
+    }
+}
+
+// The same two products a column at a time, for the backward, whose four products need no other independent work.  Scores of one
+// column against two centre operands: x from the first tensor (`b`), y from the second.
+template <int NS, int NT>
+__device__ __forceinline__ void dot_column(const Centre<NS>& a0, const Centre<NS>& a1, uint32_t b, float (&x)[NT][4], float (&y)[NT][4]) {
+    constexpr int RB = split_row_bytes(NS);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        uint32_t f[NT][4], e[NT][4];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            ldsm4(b + 8 * t * RB + 32 * s, f[t]);
+            ldsm4(b + 8 * t * RB + 32 * s + 64 * NS, e[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            if (s == 0) mma16(x[t], a0.lo[s], f[t][0], f[t][1]);
+            else mma16(x[t], a0.lo[s], f[t][0], f[t][1], x[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            if (s == 0) mma16(y[t], a1.lo[s], e[t][0], e[t][1]);
+            else mma16(y[t], a1.lo[s], e[t][0], e[t][1], y[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) mma16(x[t], a0.hi[s], f[t][2], f[t][3], x[t]);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) mma16(y[t], a1.hi[s], e[t][2], e[t][3], y[t]);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) mma16(x[t], a0.hi[s], f[t][0], f[t][1], x[t]);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) mma16(y[t], a1.hi[s], e[t][0], e[t][1], y[t]);
+    }
+}
+// acc += S * (weights . streamed) over one column.  An odd last tile of the first column (TAIL 0) waits in `tail` for that of the
+// second (TAIL 1), with which it makes one operand.
+struct Tail {
+    uint32_t hi[2], lo[2];
+};
+template <int NS, int NT, int TAIL>
+__device__ __forceinline__ void outer_column(const uint32_t (&hi)[NT][2], const uint32_t (&lo)[NT][2], Tail& tail, uint32_t b, uint32_t bt,
+                                             const pair_t (&S)[2], pair_t (&acc)[NS][2][2]) {
+    constexpr int RB = split_row_bytes(NS), K = NT / 2 + ((NT & 1) && TAIL ? 1 : 0);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        float c[2][4], d[2][4];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const bool last = k == NT / 2;                 // the tails of both columns
+            const uint32_t at = (last ? bt : b) + (last ? 8 * (NT - 1) : 16 * k) * RB + 32 * s;
+            const int t = last ? NT - 1 : 2 * k, t1 = last ? NT - 1 : 2 * k + 1;
+            uint32_t x[4], y[4];
+            ldsm4t(at, x);
+            ldsm4t(at + 32 * NS, y);
+            const uint32_t ah[4] = {last ? tail.hi[0] : hi[t][0], last ? tail.hi[1] : hi[t][1], hi[t1][0], hi[t1][1]};
+            const uint32_t al[4] = {last ? tail.lo[0] : lo[t][0], last ? tail.lo[1] : lo[t][1], lo[t1][0], lo[t1][1]};
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                if (k == 0) mma16(c[n], ah, x[2 * n], x[2 * n + 1]);
+                else mma16(c[n], ah, x[2 * n], x[2 * n + 1], c[n]);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                if (k == 0) mma16(d[n], al, x[2 * n], x[2 * n + 1]);
+                else mma16(d[n], al, x[2 * n], x[2 * n + 1], d[n]);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) mma16(d[n], ah, y[2 * n], y[2 * n + 1], d[n]);
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; i += 2)
+                acc[s][n][i / 2] = fma_pair(add_pair(pair(c[n][i], c[n][i + 1]), pair(d[n][i], d[n][i + 1])), S[i / 2], acc[s][n][i / 2]);
+    }
+    if ((NT & 1) && !TAIL) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            tail.hi[r] = hi[NT - 1][r];
+            tail.lo[r] = lo[NT - 1][r];
+        }
+    }
+}
+
+// 0 for a score inside the window of the lane's row, -inf outside (tile t, element i of the lane's four).
+__device__ __forceinline__ float window_mask(int lane, int p, int t, int i) {
+    const int d = 8 * t + 2 * (lane & 3) + (i & 1) - (lane >> 2);
+    return d >= 0 && d <= 2 * p ? 0.f : -INFINITY;
+}
+
+__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+    return done;
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Runs a sweep: a block of four warps owns 32 rows of two columns, each warp eight of them.  The columns meet the ws + 1 columns of
+// their windows two at a time ("steps"); thread 0 copies them, and every warp with rows in the image reads at its own
+// pace.  A step's buffer is refilled one step after it was read, when the other warps have mostly left it as well.  Every
+// wait is bounded.
+// Sweep: begin(w0, own) with the shared address behind the buffers, step(rb, first, last) with the shared address of the warp's first row in the first of the step's columns (the
+// second follows one stage on), end(w0, poison).  A wait that ran out ends the warp's sweep: the block reports it (device
+// counter, caller's status word), and what it stores is poisoned with NaN.
+// Measured against this cut at 512 x 512, 8 units, ws 21 (forward 1090 us): two pairs of columns per block on the same buffers with
+// half the copies 1100, several pairs of columns one after the other 1100, two buffers instead of three 1170.
+template <int NS, int NT, class Sweep>
+__device__ __forceinline__ void split_run(const SplitArgs& a, const CUtensorMap* map, Sweep& sweep) {
+    constexpr int SB = split_stage_bytes(NS, NT);
+    constexpr uint32_t kBytes = 2 * split_rows(NT) * split_row_bytes(NS);
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bars[2 * kSplitSteps];
+    const Geo& g = a.g;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int steps = (g.ws + 1) / 2, w0 = 2 * blockIdx.x, h0 = blockIdx.y * 8 * kSplitWarps, u = blockIdx.z;
+    const uint32_t full = smem_u32(bars), stages = (smem_u32(smem_raw) + 127u) & ~127u;
+    const bool live = h0 + 8 * warp < g.H;                    // the warp's rows reach into the image
+    int kc = stage_column(g, w0, 0);
+    auto copy = [&](uint32_t bar, uint32_t dst) {
+        mbar_arrive_expect_tx(bar, kBytes);
+        tma_load_4d(dst, map, 0, h0, kc, u, bar);
+        kc = kc + 1 == g.Wk ? 0 : kc + 1;
+        tma_load_4d(dst + SB, map, 0, h0, kc, u, bar);
+        kc = kc + 1 == g.Wk ? 0 : kc + 1;
+    };
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kSplitSteps; ++i) {
+            mbar_init(&bars[i], 1);
+            mbar_init(&bars[kSplitSteps + i], min(kSplitWarps, (g.H - h0 + 7) >> 3));
+        }
+        mbar_fence_init();
+        for (int i = 0; i < kSplitSteps && i < steps; ++i) copy(full + 8 * i, stages + 2 * SB * i);
+    }
+    __syncthreads();
+    bool lost = false;
+    if (live) {
+        sweep.begin(w0, stages + 2 * SB * kSplitSteps);
+        uint32_t bar = full, ring = stages + 8 * warp * split_row_bytes(NS), phase = 0;
+#pragma unroll 1
+        for (int step = 0; step < steps; ++step) {
+            if (!__all_sync(0xffffffffu, mbar_try(bar, phase))) {
+                lost = !__all_sync(0xffffffffu, mbar_wait(bar, phase, a.wait_tries));
+                if (lost) break;
+            }
+            sweep.step(ring, step == 0, step == steps - 1);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar + 8 * kSplitSteps);
+            if (warp == 0 && step > 0 && step - 1 + kSplitSteps < steps) {
+                const bool first = bar == full;
+                const uint32_t b = first ? bar + 8 * (kSplitSteps - 1) : bar - 8;
+                const uint32_t d = (first ? ring + 2 * SB * (kSplitSteps - 1) : ring - 2 * SB);
+                lost = !__all_sync(0xffffffffu, mbar_wait(b + 8 * kSplitSteps, first ? phase ^ 1 : phase, a.wait_tries));
+                if (lost) break;
+                if (lane == 0) copy(b, d);
+            }
+            bar += 8;
+            ring += 2 * SB;
+            if (bar == full + 8 * kSplitSteps) { bar = full; ring -= 2 * SB * kSplitSteps; phase ^= 1; }
+        }
+    }
+    float poison = 0.f;
+    if (__syncthreads_or(lost)) {
+        if (threadIdx.x == 0) {
+            // copies still in flight get a bounded chance to land before the block exits
+            for (int i = 0; i < kSplitSteps; ++i) mbar_wait(full + 8 * i, 0, 1u << 12);
+            atomicAdd(a.timeouts, 1);
+            if (a.status) atomicOr(a.status, 1);
+        }
+        poison = __int_as_float(0x7fc00000);
+    }
+    if (live) sweep.end(w0, poison);
+}
+
+// This lane's ldmatrix offsets inside a stage, relative to the warp's first row.
+__device__ __forceinline__ uint32_t dot_offset(int lane, int ns) {               // [hi 0-7, hi 8-15, lo 0-7, lo 8-15] of 8 rows
+    return (lane & 7) * split_row_bytes(ns) + ((lane >> 3) & 1) * 16 + (lane >> 4) * 32 * ns;
+}
+__device__ __forceinline__ uint32_t outer_offset(int lane, int ns, int next) {   // [rows 0-7, those `next` bytes on] x [channels 0-7, 8-15]
+    return (lane & 7) * split_row_bytes(ns) + ((lane >> 3) & 1) * next + (lane >> 4) * 16;
+}
+// Where the word of scales lies that this lane watches: lanes 0-3 the groups of the step's first column, lanes 4-7 those of its
+// second, and so on; groups past the padded rows do not exist.
+template <int NS, int NT>
+__device__ __forceinline__ uint32_t word_offset(const Geo& g, int lane, int row0) {
+    const int t = min(min(lane & 3, NT - 1), (split_hp(g) - row0 - 1) >> 3);
+    return ((lane >> 2) & 1) * split_stage_bytes(NS, NT) + 8 * t * split_row_bytes(NS) + 128 * NS;
+}
+// Tiles whose group has another scale than the step's largest (byte `shift` of the words), times the ratio; `least`: the smallest
+// exponent of the ratio (0: it may vanish; groups without a scale hold zeros only).
+// `column`: the first of the tiles.
+template <int NT, int N>
+__device__ __forceinline__ void scale_tiles(float (&x)[N][4], uint32_t word, uint32_t cur, int shift, int least, int column = 0) {
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+        const int e = __shfl_sync(0xffffffffu, word, t < NT ? 4 * column + t : 4 + t - NT) >> shift & 255u;
+        const float f = e ? exp_scale(max(127 + e - (int)(cur >> shift & 255u), least)) : 1.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[t][i] *= f;
+    }
+}
+// Two neighbouring rows' scalars (see the layout above) at the shared address of the even or of the odd row's.
+__device__ __forceinline__ pair_t lds_pair(uint32_t addr) {
+    pair_t x;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(x) : "r"(addr));
+    return x;
+}
+__device__ __forceinline__ uint32_t ldsu32(uint32_t addr) {
+    uint32_t x;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x) : "r"(addr));
+    return x;
+}
+
+// ---------------------------------------------------------------- host
+// Launch geometry, shared memory (`extra` bytes of the sweep's own) and the tensor map of a sweep.
+inline int split_prepare(const Geo& g, float scale, int dist, const float* packed, Launch* L, SplitArgs* a, size_t extra = 0) {
+    const int ns = slabs_of(g), nt = split_tiles(g), rb = split_row_bytes(ns), rf = rb / 4, hp = split_hp(g);
+    a->g = g;
+    a->scale = scale;
+    a->dist = dist;
+    a->status = status_word();
+    if (!(a->timeouts = stage_timeout_counter())) return cuda_fail(cudaGetLastError(), "cudaGetSymbolAddress(stage timeouts)");
+    a->wait_tries = kWaitTries;
+    L->grid = dim3((unsigned)((g.W + 1) / 2), (unsigned)((g.H + 8 * kSplitWarps - 1) / (8 * kSplitWarps)), (unsigned)g.units);
+    L->threads = 32 * kSplitWarps;
+    L->smem = (size_t)2 * kSplitSteps * split_stage_bytes(ns, nt) + 128 + extra;
+    if (L->smem > kMaxDynamicSmem || L->grid.y > 65535u) return CA_ERR_UNSUPPORTED;
+    const uint64_t dims[4] = {(uint64_t)rf, (uint64_t)hp, (uint64_t)g.Wk, (uint64_t)g.units};
+    const uint64_t strides[3] = {(uint64_t)rb, (uint64_t)hp * rb, (uint64_t)hp * rb * g.Wk};
+    const uint32_t box[4] = {(uint32_t)rf, (uint32_t)split_rows(nt), 1, 1};
+    return encode_tensor_map(&L->mv, packed, 4, dims, strides, box);
+}
+
+#define CA_LAUNCH_SPLIT(KERNEL, a, L, st)                                             \
+    do {                                                                              \
+        static std::atomic<int> have__{0};                                            \
+        int rc__ = set_smem(KERNEL, (L).smem, have__);                                \
+        if (rc__) return rc__;                                                        \
+        KERNEL<<<(L).grid, (L).threads, (L).smem, st>>>(a, (L).mv);                   \
+        count_tiled_launch();                                                         \
+    } while (0)
+
+}  // namespace
+}  // namespace ca

@@ -1,0 +1,293 @@
+// Backward of the tensor-core sweeps (split.cuh): dq from the streamed (k|v), dk and dv from the streamed (q|dy).
+//   P = 2^(s - L),  dS = P (dP - D),  dq = scale sum dS k,  dk = scale sum dS q,  dv = sum P dy
+// (Distance: sum dS (k - q), sum dS (q - k)).  Weights enter the products as halves, so they are scaled by powers of two: P by
+// 2^14, and dP - D by the reciprocal of a bound that follows from the operands' norms, per row and step (dq) or per warp and
+// step (dk); a step's sums are scaled back when they are added to the running ones.
+#include "split.cuh"
+
+namespace ca {
+namespace {
+
+constexpr float kWeightExp = 14.f;
+
+// Biased exponent of a power of two above |x| (255 for what is no number).
+__device__ __forceinline__ int above(float x) {
+    const uint32_t b = abs_bits(x);
+    return b ? min((int)(b >> 23) + 1, 255) : 0;
+}
+// Biased exponent of the reciprocal of a bound of |dP| + |D|: `norm` above the centre vector's norm, `e` the exponent of the streamed
+// group's scale, whose vectors have norms up to sqrt(16 NS) 2^15, `d` above |D|.
+template <int NS>
+__device__ __forceinline__ int bound_inverse(int norm, int e, int d) {
+    const int x = max(norm + e - 127 + 17 + (NS > 1) , d) + 1;
+    return min(max(254 - x, 1), 250);
+}
+
+// One pixel from the tensors themselves (a warp that met a NaN or an infinity).
+__device__ __noinline__ void exact_dkdv(const SplitArgs& a, int u, int h, int w) {
+    const Geo& g = a.g;
+    const int i = h + g.H * w;
+    float k[64], v[64], dk[64], dv[64];
+    for (int c = 0; c < g.cr; ++c) {
+        k[c] = ld_channel(a.c0, g, u, c, g.Np, i);
+        v[c] = ld_channel(a.c1, g, u, c, g.Np, i);
+        dk[c] = dv[c] = 0.f;
+    }
+    const float sl2 = a.scale * kLog2e;
+    for (int dw = -g.p; dw <= g.p; ++dw) {
+        const int jw = wrap_axis(w + dw + g.wk_off, g.Wk);
+        for (int dh = -g.p; dh <= g.p; ++dh) {
+            const int pix = wrap_axis(h + dh, g.H) + g.H * jw;
+            const int64_t row = (int64_t)u * g.Npk + pix;
+            float s = 0.f, dp = 0.f;
+            for (int c = 0; c < g.cr; ++c) {
+                const float qc = ld_channel(a.x0, g, u, c, g.Npk, pix);
+                s = a.dist ? fmaf(-0.5f * (qc - k[c]), qc - k[c], s) : fmaf(qc, k[c], s);
+                dp = fmaf(ld_channel(a.x1, g, u, c, g.Npk, pix), v[c], dp);
+            }
+            const float p = fast_exp2(s * sl2 - a.xstats[row] * kLog2e), ds = p * (dp - a.xD[row]);
+            for (int c = 0; c < g.cr; ++c) {
+                dk[c] = fmaf(ds, ld_channel(a.x0, g, u, c, g.Npk, pix) - (a.dist ? k[c] : 0.f), dk[c]);
+                dv[c] = fmaf(p, ld_channel(a.x1, g, u, c, g.Npk, pix), dv[c]);
+            }
+        }
+    }
+    for (int c = 0; c < g.cr; ++c) {
+        st_channel(a.o0, g, u, c, g.Np, i, a.scale * dk[c]);
+        st_channel(a.o1, g, u, c, g.Np, i, dv[c]);
+    }
+}
+
+// What the two sweeps share: the tiles of a column against two centre operands.
+template <int NS, int NT>
+struct BwdSweep {
+    static constexpr int RB = split_row_bytes(NS), SB = split_stage_bytes(NS, NT);
+    const SplitArgs& a;
+    int lane, tq, h, u;
+    uint32_t dot_off, outer_off, tail_off, word_off;
+    float sl2;
+    Centre<NS> c0, c1;
+    uint32_t cur, word;                                      // the scales of the step's groups when they are all alike; this lane's
+    bool bad, mixed;
+
+    __device__ __forceinline__ BwdSweep(const SplitArgs& a_) : a(a_) {
+        const int row0 = blockIdx.y * 8 * kSplitWarps + 8 * (threadIdx.x >> 5);
+        lane = threadIdx.x & 31;
+        tq = lane & 3;
+        h = row0 + (lane >> 2);
+        u = blockIdx.z;
+        sl2 = a.scale * kLog2e;
+        dot_off = dot_offset(lane, NS);
+        outer_off = outer_offset(lane, NS, 8 * RB);
+        tail_off = outer_offset(lane, NS, SB);
+        word_off = word_offset<NS, NT>(a.g, lane, row0);
+    }
+    __device__ __forceinline__ void load(int w0) {
+        Raw<NS> r0, r1;
+        r0.load(a.c0, a.g, u, h, w0, tq);
+        r1.load(a.c1, a.g, u, h, w0, tq);
+        c0.form(r0, a.g, h, w0, tq, kLeastExp);
+        c1.form(r1, a.g, h, w0, tq, 0);
+        bad = c0.bad || c1.bad;
+        cur = 0;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) c0.scale[r] = fmaxf(c0.scale[r] * sl2, 0x1p-70f);
+    }
+    // Centre column 0 does not meet the last column of the windows, centre column 1 not the first.
+    template <int HALF>
+    __device__ __forceinline__ void drop(bool first, bool last, float (&x)[NT][4]) {
+        if (HALF == 0 && first) {
+#pragma unroll
+            for (int t = 0; t < NT; ++t) x[t][2] = x[t][3] = -INFINITY;
+        }
+        if (HALF == 1 && last) {
+#pragma unroll
+            for (int t = 0; t < NT; ++t) x[t][0] = x[t][1] = -INFINITY;
+        }
+    }
+};
+
+template <int NS, int NT, bool DIST>
+struct DkdvSweep : BwdSweep<NS, NT> {
+    using B = BwdSweep<NS, NT>;
+    using B::a; using B::lane; using B::tq; using B::h; using B::u; using B::c0; using B::c1; using B::cur; using B::word; using B::bad; using B::mixed;
+    using B::RB; using B::SB;
+    pair_t dk[NS][2][2], dv[NS][2][2], sum[2], mk[NT], bk[2], c[2], e[2], nrm, Sk[2], Sv[2], Sd;      // Sd: Distance, the sums of dS
+    int norm;
+    uint32_t most;                                           // exponent above the |D| met so far
+    Tail tp, td;
+
+    __device__ __forceinline__ DkdvSweep(const SplitArgs& a_) : B(a_) {}
+
+    __device__ __forceinline__ void begin(int w0, uint32_t) {
+        const Geo& g = a.g;
+        B::load(w0);
+        most = 0;
+        nrm = Sd = 0;
+        norm = above(sqrtf(fmaxf(c1.norm2[0], c1.norm2[1])));
+        norm = __reduce_max_sync(0xffffffffu, norm);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) mk[t] = pair(kWeightExp + window_mask(lane, g.p, t, 0), kWeightExp + window_mask(lane, g.p, t, 1));
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const float b = -0.5f * B::sl2 * c0.norm2[r];
+            bk[r] = pair(b, b);
+            sum[r] = c[r] = e[r] = Sk[r] = Sv[r] = 0;
+        }
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) dk[s][n][0] = dk[s][n][1] = dv[s][n][0] = dv[s][n][1] = 0;
+    }
+
+    template <int HALF>
+    __device__ __forceinline__ void column(uint32_t rb, bool first, bool last) {
+        float x[NT][4], y[NT][4];
+        dot_column<NS, NT>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
+        if (mixed) {
+            scale_tiles<NT>(x, word, cur, 0, 1, HALF);
+            scale_tiles<NT>(y, word, cur, 8, 0, HALF);
+        }
+        const uint32_t sc = rb + HALF * SB + 2 * tq * RB + 128 * NS + 8;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const pair_t A = add_pair(mk[t], lds_pair(sc + 8 * t * RB)), Dn = mul_pair(lds_pair(sc + (8 * t + 1) * RB), nrm);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float2 z = unpair(fma_pair(pair(x[t][2 * r], x[t][2 * r + 1]), c[r], DIST ? add_pair(A, bk[r]) : A));
+                const float2 w = unpair(fma_pair(pair(y[t][2 * r], y[t][2 * r + 1]), e[r], Dn));
+                x[t][2 * r] = z.x;
+                x[t][2 * r + 1] = z.y;
+                y[t][2 * r] = w.x;
+                y[t][2 * r + 1] = w.y;
+            }
+        }
+        B::template drop<HALF>(first, last, x);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[t][i] = fast_exp2(x[t][i]);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const pair_t ds = mul_pair(pair(x[t][2 * r], x[t][2 * r + 1]), pair(y[t][2 * r], y[t][2 * r + 1]));
+                if (DIST) sum[r] = fma_pair(ds, Sd, sum[r]);
+                const float2 z = unpair(ds);
+                y[t][2 * r] = z.x;
+                y[t][2 * r + 1] = z.y;
+            }
+        }
+        if (mixed) {
+            scale_tiles<NT>(y, word, cur, 0, 0, HALF);
+            scale_tiles<NT>(x, word, cur, 8, 0, HALF);
+        }
+        uint32_t hi[NT][2], lo[NT][2];
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) split2(x[t][2 * r], x[t][2 * r + 1], hi[t][r], lo[t][r]);
+        outer_column<NS, NT, HALF>(hi, lo, tp, rb + HALF * SB + B::outer_off + 64 * NS, rb + B::tail_off + 64 * NS, Sv, dv);
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) split2(y[t][2 * r], y[t][2 * r + 1], hi[t][r], lo[t][r]);
+        outer_column<NS, NT, HALF>(hi, lo, td, rb + HALF * SB + B::outer_off, rb + B::tail_off, Sk, dk);
+    }
+
+    __device__ __forceinline__ void step(uint32_t rb, bool first, bool last) {
+        word = ldsu32(rb + B::word_off);
+        const uint32_t top = word >> 16;
+        word &= 0xffffu;
+        mixed = false;
+        if (__any_sync(0xffffffffu, word != cur || top > most)) {
+            bad |= (word & 255u) == 255u || (word >> 8) == 255u || top == 255u;
+            const uint32_t eq = __reduce_max_sync(0xffffffffu, word & 255u), ed = __reduce_max_sync(0xffffffffu, word >> 8);
+            most = max(most, __reduce_max_sync(0xffffffffu, top));
+            cur = eq | ed << 8;
+            mixed = __any_sync(0xffffffffu, word != cur);
+            const int nb = bound_inverse<NS>(norm, ed, most);
+            const float n = exp_scale(nb), bv = exp_scale(ed) * 0x1p-14f, bd = exp_scale(254 - nb) * 0x1p-14f, back = exp_scale(eq) * bd;
+            nrm = pair(n, n);
+            Sd = pair(bd, bd);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                c[r] = pair(c0.scale[r] * exp_scale(eq), c0.scale[r] * exp_scale(eq));
+                e[r] = pair(c1.scale[r] * n * exp_scale(ed), c1.scale[r] * n * exp_scale(ed));
+                Sv[r] = pair(bv, bv);
+                Sk[r] = pair(back, back);
+            }
+        }
+        column<0>(rb, first, last);
+        column<1>(rb, first, last);
+    }
+
+    __device__ __forceinline__ void end(int w0, float poison) {
+        const Geo& g = a.g;
+        if (__any_sync(0xffffffffu, bad)) {
+            if (tq < 2 && h < g.H && w0 + tq < g.W) exact_dkdv(a, u, h, w0 + tq);
+            return;
+        }
+        Raw<NS> raw = {};
+        if (DIST) raw.load(a.c0, g, u, h, w0, tq);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const bool ok = h < g.H && w0 + r < g.W;
+            const int pix = ok ? h + g.H * (w0 + r) : 0;
+            float ds = 0.f;
+            if (DIST) {
+                const float2 z = unpair(sum[r]);
+                ds = quad_sum(z.x + z.y);
+            }
+            if (!ok) continue;
+            const float (&kv)[NS][4] = raw.x[r];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                const float2 k0 = unpair(dk[s][0][r]), k1 = unpair(dk[s][1][r]), v0 = unpair(dv[s][0][r]), v1 = unpair(dv[s][1][r]);
+                store_pixel(a.o0, g, u, s, pix, tq, a.scale * (k0.x - ds * kv[s][0]) + poison, a.scale * (k0.y - ds * kv[s][1]) + poison,
+                            a.scale * (k1.x - ds * kv[s][2]) + poison, a.scale * (k1.y - ds * kv[s][3]) + poison);
+                store_pixel(a.o1, g, u, s, pix, tq, v0.x + poison, v0.y + poison, v1.x + poison, v1.y + poison);
+            }
+        }
+    }
+};
+
+template <int NS, int NT, bool DIST>
+__global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 ? 4 : 3) split_dkdv_kernel(const __grid_constant__ SplitArgs a,
+                                                                                             const __grid_constant__ CUtensorMap map) {
+    DkdvSweep<NS, NT, DIST> sweep(a);
+    split_run<NS, NT>(a, &map, sweep);
+}
+
+}  // namespace
+
+#define CA_SPLIT_BWD(KERNEL, NSV, NTV)                                                               \
+    do {                                                                                             \
+        if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true>), a, L, st);                               \
+        else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false>), a, L, st);                                   \
+    } while (0)
+#define CA_SPLIT_BWD_NT(KERNEL, NSV)                                                                 \
+    do {                                                                                             \
+        if (nt == 2) CA_SPLIT_BWD(KERNEL, NSV, 2);                                                   \
+        else if (nt == 3) CA_SPLIT_BWD(KERNEL, NSV, 3);                                              \
+        else if (nt == 4) CA_SPLIT_BWD(KERNEL, NSV, 4);                                              \
+        else return CA_ERR_UNSUPPORTED;                                                              \
+    } while (0)
+#define CA_SPLIT_BWD_NS(KERNEL)                                                                      \
+    do {                                                                                             \
+        if (ns != 1) return CA_ERR_UNSUPPORTED;                                                      \
+        CA_SPLIT_BWD_NT(KERNEL, 1);                                                                  \
+    } while (0)
+
+int run_split_dkdv(const Geo& g, float scale, int dist, const float* q, const float* k, const float* v, const float* dy, const float* stats,
+                   const float* D, const float* qdy, float* dk, float* dv, cudaStream_t st) {
+    Launch L{};
+    SplitArgs a{};
+    const int ns = slabs_of(g), nt = split_tiles(g);
+    const int rc = split_prepare(g, scale, dist, qdy, &L, &a);
+    if (rc) return rc;
+    a.c0 = k; a.c1 = v; a.o0 = dk; a.o1 = dv; a.x0 = q; a.x1 = dy; a.xstats = stats; a.xD = D;
+    CA_SPLIT_BWD_NS(split_dkdv_kernel);
+    CA_CHECK_LAUNCH("split dk/dv kernel");
+    return CA_OK;
+}
+
+}  // namespace ca

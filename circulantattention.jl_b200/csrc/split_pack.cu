@@ -1,0 +1,173 @@
+// Pack kernel of the tensor-core sweeps (split.cuh has the layout): two tensors in the reference layout -> rows of split halves
+// with the circular halo unrolled, the scales of each group of eight rows and the rows' scalars.
+#include "split.cuh"
+
+namespace ca {
+namespace {
+
+// A block gathers RB = 128 / NS packed rows of one column of one unit: thread (row, slab) reads 16 channels of both tensors
+// (consecutive lanes on consecutive rows: coalesced planar loads, all in flight together), the largest magnitude of each
+// group of eight rows comes from shuffles and, over the slabs, shared memory, and the block writes its rows as one
+// contiguous run of 16-byte stores.  Bound: HBM.
+template <int CPE, int NS, bool BF>
+__global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
+    constexpr int RB = 128 / NS, RF = split_row_bytes(NS) / 4;
+    __shared__ __align__(16) uint32_t tile[RB * RF];
+    __shared__ uint32_t gmax[2][NS][RB / 8];
+    __shared__ float sums[2][NS][RB];
+    const Geo& g = a.g;
+    const int rl = threadIdx.x % RB, slab = threadIdx.x / RB;
+    const int rr0 = blockIdx.x * RB, rr = rr0 + rl, w = blockIdx.y, u = blockIdx.z;
+    const bool real_row = rr < g.H + 2 * g.p;
+    const int pix = real_row ? (rr - g.p + g.H) % g.H + g.H * w : 0;
+    float x[2][16];
+    float dot = 0.f;
+    {
+        // all loads first, from clamped addresses
+        const float* src[2] = {a.x0, a.x1};
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int e = 0; e < 16; e += CPE) {
+                const int64_t o = goff<CPE>(u, g.cr, min(16 * slab + e, g.cr - CPE), g.Npk, pix);
+                if (CPE == 2) {
+                    const float2 z = __ldg(reinterpret_cast<const float2*>(src[t] + o));
+                    x[t][e] = z.x;
+                    x[t][e + CPE - 1] = z.y;
+                } else {
+                    x[t][e] = ld_real<BF>(src[t], o);
+                }
+            }
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+                if (!real_row || 16 * slab + e >= g.cr) x[t][e] = 0.f;
+        if (a.y) {
+            float yv[16];
+#pragma unroll
+            for (int e = 0; e < 16; e += CPE) {
+                const int64_t o = goff<CPE>(u, g.cr, min(16 * slab + e, g.cr - CPE), g.Npk, pix);
+                if (CPE == 2) {
+                    const float2 z = __ldg(reinterpret_cast<const float2*>(a.y + o));
+                    yv[e] = z.x;
+                    yv[e + CPE - 1] = z.y;
+                } else {
+                    yv[e] = ld_real<BF>(a.y, o);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+                if (16 * slab + e < g.cr) dot = fmaf(x[1][e], yv[e], dot);
+            if (!real_row) dot = 0.f;
+        }
+    }
+    float2 n2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int e = 0; e < 16; e += 2) {
+        n2.x = fmaf(x[0][e], x[0][e], n2.x);
+        n2.y = fmaf(x[0][e + 1], x[0][e + 1], n2.y);
+    }
+    float norm = n2.x + n2.y;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) m = max(m, abs_bits(x[t][e]));
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+        if ((rl & 7) == 0) gmax[t][slab][rl >> 3] = m;
+    }
+    sums[0][slab][rl] = norm;
+    sums[1][slab][rl] = dot;
+    __syncthreads();
+    uint32_t exps = 0;
+    uint32_t* row = tile + rl * RF;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        uint32_t m = gmax[t][0][rl >> 3];
+#pragma unroll
+        for (int s = 1; s < NS; ++s) m = max(m, gmax[t][s][rl >> 3]);
+        const int e = scale_exp(m, 4, t == 0 ? kLeastExp : 0);
+        exps |= (uint32_t)e << (8 * t);
+        const float inv = exp_inverse(e == 255 ? 0 : e);
+        uint32_t hi[8], lo[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) split2(x[t][2 * i] * inv, x[t][2 * i + 1] * inv, hi[i], lo[i]);
+        uint4* d = reinterpret_cast<uint4*>(row + t * 16 * NS + slab * 8);
+        d[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        d[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+        d += 2 * NS;
+        d[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        d[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+    }
+    if (slab == 0) {
+#pragma unroll
+        for (int s = 1; s < NS; ++s) {
+            norm += sums[0][s][rl];
+            dot += sums[1][s][rl];
+        }
+        float A = a.norm_mul * norm;
+        if (a.stats) {
+            const int64_t so = (int64_t)u * g.Npk + pix;
+            if (real_row) {
+                A = fmaf(__ldg(a.stats + so), -kLog2e, A);
+                if (a.Din) dot = __ldg(a.Din + so);
+                else if (a.Dout && rr >= g.p && rr < g.p + g.H) a.Dout[so] = dot;
+            }
+            uint32_t m = abs_bits(dot);
+#pragma unroll
+            for (int d = 1; d < 8; d <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+            // a power of two above every |D| of the group; a statistic that is no number marks it, too
+            uint32_t bad = abs_bits(A) >= 0x7f800000u;
+            bad = __ballot_sync(0xffffffffu, bad) >> (rl & 24) & 255u;
+            const uint32_t e = bad || m >= 0x7e800000u ? 255u : (m >> 23) + (m ? 1u : 0u);
+            exps |= e << 16;
+        }
+        const float A1 = __shfl_xor_sync(0xffffffffu, A, 1), dot1 = __shfl_xor_sync(0xffffffffu, dot, 1);
+        const uint4 odd = make_uint4(exps, 0u, __float_as_uint(-dot1), __float_as_uint(-dot));
+        *reinterpret_cast<uint4*>(row + 32 * NS) = rl & 1 ? odd : make_uint4(exps, 0u, __float_as_uint(A), __float_as_uint(A1));
+    }
+    __syncthreads();
+    const int nrows = min(RB, a.Hp - rr0);
+    uint4* out = reinterpret_cast<uint4*>(a.dst + (((int64_t)u * g.Wk + w) * a.Hp + rr0) * RF);
+    const uint4* tin = reinterpret_cast<const uint4*>(tile);
+    for (int i = threadIdx.x; i < nrows * (RF / 4); i += 128) out[i] = tin[i];
+}
+
+}  // namespace
+
+// Units of one slab (more channels would need their results in registers for 32 or 64 channels), windows up to 25 (four tiles a
+// column).  From window 9 on, and at 7 on grids of up to 2^18 pixels: what a warp spends outside its steps, and the scores outside
+// the window, weigh more the shorter it is.  dk/dv on the FMA pipe and on the tensor cores: 500 x 400, 8 units: ws 5 289 and 358 us,
+// 7: 431 and 418, 9: 588 and 480, 13: 1022 and 817; 512 x 512, 8 units, ws 21 2966 and 1720; 200 x 180, 4 units: ws 5 40 and 43,
+// 7: 59 and 50, 9: 90 and 56.  A few pixels leave the chip idle either way, and their warps have less to do in the smaller
+// tiles of the FMA kernels (32 x 32, 1 unit, ws 11: 9.2 and 10.4 us).
+bool split_shape_ok(const Geo& g, float scale) {
+    const int64_t pixels = (int64_t)g.Np * g.units;
+    return tiled_shape_ok(g) && g.wsw == g.ws && slabs_of(g) == 1 && split_tiles(g) <= 4 && scale > 0.f && g.Wk <= 65535 && pixels > 8192 &&
+           (g.ws >= 9 || (g.ws == 7 && pixels <= (1 << 18)));
+}
+
+int launch_split_pack(const Geo& g, float scale, int dist, const float* x0, const float* x1, const float* stats, const float* y, const float* Din,
+                      float* Dout, float* dst, cudaStream_t st) {
+    SplitPackArgs a{};
+    a.g = g; a.Hp = split_hp(g); a.x0 = x0; a.x1 = x1; a.stats = stats; a.y = y; a.Din = Din; a.Dout = Dout; a.dst = dst;
+    a.norm_mul = dist ? -0.5f * scale * kLog2e : 0.f;
+    const int ns = slabs_of(a.g), rb = 128 / ns;
+    const dim3 grid((a.Hp + rb - 1) / rb, a.g.Wk, a.g.units);
+    if (a.g.bf16) split_pack_kernel<1, 1, true><<<grid, 128, 0, st>>>(a);
+    else if (a.g.cpe == 1) {
+        if (ns == 1) split_pack_kernel<1, 1, false><<<grid, 128, 0, st>>>(a);
+        else if (ns == 2) split_pack_kernel<1, 2, false><<<grid, 128, 0, st>>>(a);
+        else split_pack_kernel<1, 4, false><<<grid, 128, 0, st>>>(a);
+    } else {
+        if (ns == 1) split_pack_kernel<2, 1, false><<<grid, 128, 0, st>>>(a);
+        else if (ns == 2) split_pack_kernel<2, 2, false><<<grid, 128, 0, st>>>(a);
+        else split_pack_kernel<2, 4, false><<<grid, 128, 0, st>>>(a);
+    }
+    CA_CHECK_LAUNCH("split pack kernel");
+    return CA_OK;
+}
+
+}  // namespace ca

@@ -36,7 +36,7 @@
 //
 // Small grids.  Where it pays, the column stages of a tile are split between up to four groups of warps of the same CTA
 // (each with its own copy pipeline) whose partial results are merged through shared memory.
-#include "tile_common.cuh"
+#include "split.cuh"
 
 namespace ca {
 
@@ -113,6 +113,11 @@ int tiled_attention_bwd_dkdv(const Geo& gin, float scale, int dist, const float*
     if (!workspace) { set_error("workspace of ca_attention_bwd_stage_workspace() bytes is NULL"); return CA_ERR_NULL; }
     const Padded P = padded_of(g);
     float* qdy = static_cast<float*>(workspace);
+    if (split_shape_ok(g, scale)) {
+        int rc = launch_split_pack(g, scale, dist, q, dy, stats, nullptr, D, nullptr, qdy, st);
+        if (rc) return rc;
+        return run_split_dkdv(g, scale, dist, q, k, v, dy, stats, D, qdy, dk, dv, st);
+    }
     float* planes = qdy + P.pair_floats;
     PackArgs pa{};
     pa.g = g; pa.pp = P.pp; pa.Hp = P.Hp; pa.npairs = 1;
@@ -163,11 +168,40 @@ int tiled_attention_bwd(const Geo& gin, float scale, int dist, const float* q, c
     float* kv = static_cast<float*>(workspace);
     float* qdy = kv + P.pair_floats;
     float* planes = qdy + P.pair_floats;
+    // both sweeps: side by side where neither fills the GPU (fewer than ~4 CTAs per SM per sweep)
+    auto run_both = [&](auto sweep_q, auto sweep_k) -> int {
+        if ((long)g.Np * g.units < 2048L * sm_count()) {
+            ForkJoin* f = fork_join_for_current_device();
+            if (f && cudaEventRecord(f->fork, st) == cudaSuccess && cudaStreamWaitEvent(f->side, f->fork, 0) == cudaSuccess) {
+                const int rc = sweep_k(f->side), rc2 = sweep_q(st);
+                cudaError_t e = cudaEventRecord(f->join, f->side);
+                if (e == cudaSuccess) e = cudaStreamWaitEvent(st, f->join, 0);
+                if (e != cudaSuccess) return cuda_fail(e, "joining the helper stream");
+                return rc ? rc : rc2;
+            }
+            cudaGetLastError();
+        }
+        const int rc = sweep_q(st);
+        return rc ? rc : sweep_k(st);
+    };
+    if (split_shape_ok(g, scale)) {
+        int rc;
+        if (fwd_workspace) {
+            kv = const_cast<float*>(static_cast<const float*>(fwd_workspace));
+        } else {
+            PackArgs pa{};
+            pa.g = g; pa.pp = P.pp; pa.Hp = P.Hp; pa.npairs = 1;
+            pa.src[0] = k; pa.src[1] = v; pa.dst[0] = kv;
+            if ((rc = launch_pack(pa, st))) return rc;
+        }
+        if ((rc = launch_split_pack(g, scale, dist, q, dy, stats, y, nullptr, D, qdy, st))) return rc;
+        return run_both([&](cudaStream_t s) { return CA_CHANNELS(g, run_dq, g, P, scale, dist, q, dy, stats, D, kv, dq, s, 0, nullptr); },
+                        [&](cudaStream_t s) { return run_split_dkdv(g, scale, dist, q, k, v, dy, stats, D, qdy, dk, dv, s); });
+    }
     PackArgs pa{};
     pa.g = g; pa.pp = P.pp; pa.Hp = P.Hp;
     if (fwd_workspace) {
-        // the forward of the same problem left its packed (k|v) at the start of its workspace: only
-        // (q|dy) and the planes are packed here
+        // only (q|dy) and the planes are packed here
         kv = const_cast<float*>(static_cast<const float*>(fwd_workspace));
         pa.npairs = 1;
         pa.src[0] = q; pa.src[1] = dy;
@@ -185,21 +219,8 @@ int tiled_attention_bwd(const Geo& gin, float scale, int dist, const float* q, c
         if ((rc = CA_CHANNELS(g, run_dq, g, P, scale, dist, q, dy, stats, D, kv, dq, st, 0, nullptr, weights))) return rc;
         return CA_CHANNELS(g, run_dkdv_stored, g, P, scale, dist, k, qdy, weights, dk, dv, st);
     }
-    const bool small = (long)g.Np * g.units < 2048L * sm_count();      // fewer than ~4 CTAs per SM per sweep
-    if (small) {
-        ForkJoin* f = fork_join_for_current_device();
-        if (f && cudaEventRecord(f->fork, st) == cudaSuccess && cudaStreamWaitEvent(f->side, f->fork, 0) == cudaSuccess) {
-            rc = CA_CHANNELS(g, run_dkdv, g, P, scale, dist, k, v, qdy, planes, dk, dv, f->side, false);
-            int rc2 = CA_CHANNELS(g, run_dq, g, P, scale, dist, q, dy, stats, D, kv, dq, st, 0, nullptr);
-            cudaError_t e = cudaEventRecord(f->join, f->side);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(st, f->join, 0);
-            if (e != cudaSuccess) return cuda_fail(e, "joining the helper stream");
-            return rc ? rc : rc2;
-        }
-        cudaGetLastError();
-    }
-    if ((rc = CA_CHANNELS(g, run_dq, g, P, scale, dist, q, dy, stats, D, kv, dq, st, 0, nullptr))) return rc;
-    return CA_CHANNELS(g, run_dkdv, g, P, scale, dist, k, v, qdy, planes, dk, dv, st, false);
+    return run_both([&](cudaStream_t s) { return CA_CHANNELS(g, run_dq, g, P, scale, dist, q, dy, stats, D, kv, dq, s, 0, nullptr); },
+                    [&](cudaStream_t s) { return CA_CHANNELS(g, run_dkdv, g, P, scale, dist, k, v, qdy, planes, dk, dv, s, false); });
 }
 
 // Entmax-1.5 backward on the fused kernels.  Unlike the softmax, D = sum g*dP / sum g is not dy.y, so

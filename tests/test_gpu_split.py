@@ -1,0 +1,97 @@
+"""The tensor-core sweeps (split halves): tile edges of rows, columns and windows, storage kinds, groups of eight rows whose
+magnitudes differ, and scores of a thousand.
+
+Bars: the usual ones.  A split operand keeps 22 to 24 bits of an element down to 2^-13 of the largest of its group of eight rows and 16
+channels, and steps of 2^-36 of that largest below; the products and sums are Float32's.  The magnitudes below vary by less
+than 2^13 within a group, except for zeros."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import circatt_oracle as orc
+from tests.helpers import KIND, assert_close, randn, up
+
+pytestmark = pytest.mark.gpu
+
+
+def sim_of(ca, name):
+    return ca.DotSimilarity() if name == "dot" else ca.DistanceSimilarity()
+
+
+def run(ca, simname, qn, kn, vn, rn, ws, heads, want_a=False):
+    q, k, v = (ca.jl.from_numpy(t).requires_grad_(True) for t in (qn, kn, vn))
+    y, A = ca.circulant_mh_attention(sim_of(ca, simname), q, k, v, ws, heads, return_A=want_a)
+    grads = torch.autograd.grad(y, (q, k, v), ca.jl.from_numpy(rn))
+    out = dict(zip(("y", "dq", "dk", "dv"), (y,) + grads))
+    if want_a:
+        out["A"] = A.nzVal
+    return {name: ca.jl.to_numpy(t.detach()) for name, t in out.items()}
+
+
+def oracle(simname, qn, kn, vn, rn, ws, heads):
+    y, nz = orc.mh_attention(KIND[simname], up(qn), up(kn), up(vn), ws, heads)
+    dq, dk, dv = orc.mh_attention_pullback(KIND[simname], up(qn), up(kn), up(vn), ws, heads, up(rn))
+    return {"y": y, "A": nz, "dq": dq, "dk": dk, "dv": dv}
+
+
+@pytest.mark.parametrize("simname", ["dot", "distance"])
+@pytest.mark.parametrize("shape,ws,heads,cplx", [
+    ((41, 40, 96, 1), 7, 6, False),      # two tiles a column; one row past a warp's eight, rows past a block's 32
+    ((64, 33, 64, 1), 9, 4, False),      # 16 keys exactly, an odd number of columns
+    ((39, 31, 84, 1), 11, 7, False),     # three tiles, 12 channels
+    ((17, 61, 72, 1), 17, 9, False),     # rows equal to the window: every row wraps; the longest of three tiles; 8 channels
+    ((33, 37, 56, 1), 19, 8, False),     # four tiles, 7 channels
+    ((65, 26, 32, 3), 25, 2, False),     # the longest window; batch of three
+    ((40, 52, 32, 1), 13, 4, True),      # 8 complex channels
+    ((47, 45, 20, 1), 9, 4, True),       # 5 complex channels
+])
+def test_edges(ca, shape, ws, heads, cplx, simname):
+    rng = np.random.default_rng(61)
+    t = [randn(rng, shape, cplx) for _ in range(4)]
+    got = run(ca, simname, *t, ws, heads, want_a=True)
+    want = oracle(simname, *t, ws, heads)
+    for name in got:
+        assert_close(got[name], want[name], name)
+
+
+@pytest.mark.parametrize("what", ["pixels", "zeros", "small", "large", "scores"])
+def test_magnitudes(ca, what):
+    rng = np.random.default_rng(62)
+    shape, ws, heads = (48, 44, 64, 1), 11, 4
+    q, k, v, r = (randn(rng, shape) for _ in range(4))
+    if what == "pixels":                     # every pixel another power of two: the groups of a step rarely share their scale
+        for t, span in ((q, 1), (k, 1), (v, 5), (r, 5)):
+            t *= (2.0 ** rng.integers(-span, span + 1, shape[:2] + (1, 1))).astype(np.float32)
+    elif what == "zeros":                    # padding
+        for t in (q, k, v, r):
+            t[:, :9] = 0
+            t[20:37] = 0
+    elif what == "small":
+        v *= 1e-12
+        r *= 1e-9
+    elif what == "large":
+        v *= 1e9
+        r *= 1e7
+    else:                                    # scores of a thousand: the rows are one-hot
+        q *= 30
+        k[:, ::3] *= 8
+    got = run(ca, "dot", q, k, v, r, ws, heads, want_a=True)
+    want = oracle("dot", q, k, v, r, ws, heads)
+    # an ulp of a score of a thousand is already 1e-4 in the exponential
+    bars = dict(tol=2e-3, elem_tol=2e-2) if what == "scores" else {}
+    for name in got:
+        assert_close(got[name], want[name], name, **bars)
+
+
+def test_bfloat16_storage(ca):
+    rng = np.random.default_rng(64)
+    shape, ws, heads = (50, 46, 64, 1), 15, 4
+    t = [torch.from_numpy(randn(rng, shape)).to(torch.bfloat16).float().numpy() for _ in range(4)]
+    q, k, v, r = (ca.jl.from_numpy(np.asfortranarray(x)).to(torch.bfloat16) for x in t)
+    q, k, v = (x.requires_grad_(True) for x in (q, k, v))
+    y, _ = ca.circulant_mh_attention(ca.DotSimilarity(), q, k, v, ws, heads, return_A=False)
+    grads = torch.autograd.grad(y, (q, k, v), r)
+    want = oracle("dot", *t, ws, heads)
+    for name, got in zip(("y", "dq", "dk", "dv"), (y,) + grads):
+        # results are rounded to 8 bits, dy . y is formed from the rounded y
+        assert_close(ca.jl.to_numpy(got.detach().float()), want[name], name, tol=1e-2, elem_tol=2e-2)
