@@ -10,7 +10,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 OUT = os.path.join(PKG_DIR, "libcircatt_b200.so")
 SOURCES = ["fwd_exact.cu", "fwd_any.cu", "fwd_values_exact.cu", "fwd_values_any.cu", "bwd_exact.cu", "bwd_any.cu", "emit_exact.cu", "emit_any.cu",
-           "apply_exact.cu", "apply_any.cu", "operators.cu", "tiled.cu", "pack.cu", "split_pack.cu", "split_bwd.cu", "line.cu", "api.cu", "static_scratch.cu", "comm.cu"]
+           "apply_exact.cu", "apply_any.cu", "operators.cu", "tiled.cu", "pack.cu", "split_pack.cu", "split_fwd.cu", "split_bwd.cu", "line.cu", "api.cu", "static_scratch.cu", "comm.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "--use_fast_math", "-Xcompiler", "-fPIC"]
 

@@ -24,6 +24,33 @@ __device__ __forceinline__ int bound_inverse(int norm, int e, int d) {
 }
 
 // One pixel from the tensors themselves (a warp that met a NaN or an infinity).
+__device__ __noinline__ void exact_dq(const SplitArgs& a, int u, int h, int w) {
+    const Geo& g = a.g;
+    const int j = h + g.H * w;
+    float q[64], dy[64], acc[64];
+    for (int c = 0; c < g.cr; ++c) {
+        q[c] = ld_channel(a.c0, g, u, c, g.Np, j);
+        dy[c] = ld_channel(a.c1, g, u, c, g.Np, j);
+        acc[c] = 0.f;
+    }
+    const float L = a.stats[(int64_t)u * g.Np + j] * kLog2e, D = a.D[(int64_t)u * g.Np + j], sl2 = a.scale * kLog2e;
+    for (int dw = -g.p; dw <= g.p; ++dw) {
+        const int kw = wrap_axis(w + dw + g.wk_off, g.Wk);
+        for (int dh = -g.p; dh <= g.p; ++dh) {
+            const int pix = wrap_axis(h + dh, g.H) + g.H * kw;
+            float s = 0.f, dp = 0.f;
+            for (int c = 0; c < g.cr; ++c) {
+                const float kc = ld_channel(a.x0, g, u, c, g.Npk, pix);
+                s = a.dist ? fmaf(-0.5f * (q[c] - kc), q[c] - kc, s) : fmaf(q[c], kc, s);
+                dp = fmaf(dy[c], ld_channel(a.x1, g, u, c, g.Npk, pix), dp);
+            }
+            const float ds = fast_exp2(s * sl2 - L) * (dp - D);
+            for (int c = 0; c < g.cr; ++c) acc[c] = fmaf(ds, ld_channel(a.x0, g, u, c, g.Npk, pix) - (a.dist ? q[c] : 0.f), acc[c]);
+        }
+    }
+    for (int c = 0; c < g.cr; ++c) st_channel(a.o0, g, u, c, g.Np, j, a.scale * acc[c]);
+}
+
 __device__ __noinline__ void exact_dkdv(const SplitArgs& a, int u, int h, int w) {
     const Geo& g = a.g;
     const int i = h + g.H * w;
@@ -103,6 +130,139 @@ struct BwdSweep {
         if (HALF == 1 && last) {
 #pragma unroll
             for (int t = 0; t < NT; ++t) x[t][0] = x[t][1] = -INFINITY;
+        }
+    }
+};
+
+template <int NS, int NT, bool DIST>
+struct DqSweep : BwdSweep<NS, NT> {
+    using B = BwdSweep<NS, NT>;
+    using B::a; using B::lane; using B::tq; using B::h; using B::u; using B::c0; using B::c1; using B::cur; using B::word; using B::bad; using B::mixed;
+    using B::RB; using B::SB;
+    pair_t acc[NS][2][2], sum[2], nref[NT][2], c[2], e[2], nd[2], S[2], Sd[2];     // Sd: Distance, the sums of dS
+    float D[2];
+    int norm[2];
+    Tail tail;
+
+    __device__ __forceinline__ DqSweep(const SplitArgs& a_) : B(a_) {}
+
+    __device__ __forceinline__ void begin(int w0, uint32_t) {
+        const Geo& g = a.g;
+        float Ls[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int64_t o = (int64_t)u * g.Np + min(h, g.H - 1) + g.H * min(w0 + r, g.W - 1);
+            Ls[r] = __ldg(a.stats + o);
+            D[r] = __ldg(a.D + o);
+        }
+        B::load(w0);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const bool ok = h < g.H && w0 + r < g.W;
+            const float L = ok ? Ls[r] * kLog2e : 0.f;
+            D[r] = ok ? D[r] : 0.f;
+            bad |= !(fabsf(L) < INFINITY) || !(fabsf(D[r]) < INFINITY);
+            const float b = kWeightExp - L - (DIST ? 0.5f * B::sl2 * c0.norm2[r] : 0.f);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) nref[t][r] = pair(b + window_mask(lane, g.p, t, 0), b + window_mask(lane, g.p, t, 1));
+            norm[r] = above(sqrtf(c1.norm2[r]));
+            sum[r] = c[r] = e[r] = nd[r] = S[r] = Sd[r] = 0;
+        }
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) acc[s][n][0] = acc[s][n][1] = 0;
+    }
+
+    template <int HALF>
+    __device__ __forceinline__ void column(uint32_t rb, bool first, bool last) {
+        float x[NT][4], y[NT][4];
+        dot_column<NS, NT>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
+        if (mixed) {
+            scale_tiles<NT>(x, word, cur, 0, 1, HALF);
+            scale_tiles<NT>(y, word, cur, 8, 0, HALF);
+        }
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const pair_t b = DIST ? lds_pair(rb + HALF * SB + (8 * t + 2 * tq) * RB + 128 * NS + 8) : 0;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float2 z = unpair(fma_pair(pair(x[t][2 * r], x[t][2 * r + 1]), c[r], DIST ? add_pair(nref[t][r], b) : nref[t][r]));
+                x[t][2 * r] = z.x;
+                x[t][2 * r + 1] = z.y;
+            }
+        }
+        B::template drop<HALF>(first, last, x);
+        uint32_t hi[NT][2], lo[NT][2];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[t][i] = fast_exp2(x[t][i]);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const pair_t ds = mul_pair(pair(x[t][2 * r], x[t][2 * r + 1]), fma_pair(pair(y[t][2 * r], y[t][2 * r + 1]), e[r], nd[r]));
+                if (DIST) sum[r] = fma_pair(ds, Sd[r], sum[r]);
+                const float2 z = unpair(ds);
+                x[t][2 * r] = z.x;
+                x[t][2 * r + 1] = z.y;
+            }
+        }
+        if (mixed) scale_tiles<NT>(x, word, cur, 0, 0, HALF);
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) split2(x[t][2 * r], x[t][2 * r + 1], hi[t][r], lo[t][r]);
+        outer_column<NS, NT, HALF>(hi, lo, tail, rb + HALF * SB + B::outer_off, rb + B::tail_off, S, acc);
+    }
+
+    __device__ __forceinline__ void step(uint32_t rb, bool first, bool last) {
+        word = ldsu32(rb + B::word_off) & 0xffffu;
+        mixed = false;
+        if (__any_sync(0xffffffffu, word != cur)) {
+            bad |= (word & 255u) == 255u || (word >> 8) == 255u;
+            const uint32_t ek = __reduce_max_sync(0xffffffffu, word & 255u), ev = __reduce_max_sync(0xffffffffu, word >> 8);
+            cur = ek | ev << 8;
+            mixed = __any_sync(0xffffffffu, word != cur);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int nb = bound_inverse<NS>(norm[r], ev, above(D[r]));
+                const float nrm = exp_scale(nb), bd = exp_scale(254 - nb) * 0x1p-14f, back = exp_scale(ek) * bd;
+                c[r] = pair(c0.scale[r] * exp_scale(ek), c0.scale[r] * exp_scale(ek));
+                e[r] = pair(c1.scale[r] * nrm * exp_scale(ev), c1.scale[r] * nrm * exp_scale(ev));
+                nd[r] = pair(-D[r] * nrm, -D[r] * nrm);
+                S[r] = pair(back, back);
+                Sd[r] = pair(bd, bd);
+            }
+        }
+        column<0>(rb, first, last);
+        column<1>(rb, first, last);
+    }
+
+    __device__ __forceinline__ void end(int w0, float poison) {
+        const Geo& g = a.g;
+        if (__any_sync(0xffffffffu, bad)) {
+            if (tq < 2 && h < g.H && w0 + tq < g.W) exact_dq(a, u, h, w0 + tq);
+            return;
+        }
+        Raw<NS> raw = {};
+        if (DIST) raw.load(a.c0, g, u, h, w0, tq);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const bool ok = h < g.H && w0 + r < g.W;
+            const int pix = ok ? h + g.H * (w0 + r) : 0;
+            float ds = 0.f;
+            if (DIST) {
+                const float2 z = unpair(sum[r]);
+                ds = quad_sum(z.x + z.y);
+            }
+            if (!ok) continue;
+            const float (&qv)[NS][4] = raw.x[r];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                const float2 y0 = unpair(acc[s][0][r]), y1 = unpair(acc[s][1][r]);
+                store_pixel(a.o0, g, u, s, pix, tq, a.scale * (y0.x - ds * qv[s][0]) + poison, a.scale * (y0.y - ds * qv[s][1]) + poison,
+                            a.scale * (y1.x - ds * qv[s][2]) + poison, a.scale * (y1.y - ds * qv[s][3]) + poison);
+            }
         }
     }
 };
@@ -251,6 +411,12 @@ struct DkdvSweep : BwdSweep<NS, NT> {
 };
 
 template <int NS, int NT, bool DIST>
+__global__ void __launch_bounds__(32 * kSplitWarps, 4) split_dq_kernel(const __grid_constant__ SplitArgs a,
+                                                                                           const __grid_constant__ CUtensorMap map) {
+    DqSweep<NS, NT, DIST> sweep(a);
+    split_run<NS, NT>(a, &map, sweep);
+}
+template <int NS, int NT, bool DIST>
 __global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 ? 4 : 3) split_dkdv_kernel(const __grid_constant__ SplitArgs a,
                                                                                              const __grid_constant__ CUtensorMap map) {
     DkdvSweep<NS, NT, DIST> sweep(a);
@@ -276,6 +442,19 @@ __global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 ? 4 : 3) split_dkdv_
         if (ns != 1) return CA_ERR_UNSUPPORTED;                                                      \
         CA_SPLIT_BWD_NT(KERNEL, 1);                                                                  \
     } while (0)
+
+int run_split_dq(const Geo& g, float scale, int dist, const float* q, const float* k, const float* v, const float* dy, const float* stats,
+                 const float* D, const float* kv, float* dq, cudaStream_t st) {
+    Launch L{};
+    SplitArgs a{};
+    const int ns = slabs_of(g), nt = split_tiles(g);
+    const int rc = split_prepare(g, scale, dist, kv, &L, &a);
+    if (rc) return rc;
+    a.c0 = q; a.c1 = dy; a.stats = stats; a.D = D; a.o0 = dq; a.x0 = k; a.x1 = v;
+    CA_SPLIT_BWD_NS(split_dq_kernel);
+    CA_CHECK_LAUNCH("split dq kernel");
+    return CA_OK;
+}
 
 int run_split_dkdv(const Geo& g, float scale, int dist, const float* q, const float* k, const float* v, const float* dy, const float* stats,
                    const float* D, const float* qdy, float* dk, float* dv, cudaStream_t st) {

@@ -140,6 +140,7 @@ struct FwdSweep {
         if (last) {
 #pragma unroll
             for (int t = NT; t < T; ++t) x[t][0] = x[t][1] = -INFINITY;
+            top[2] = -INFINITY;
         }
         // the first step sets the references; later they move when a score lies far above the earlier ones
         if (__any_sync(0xffffffffu, first || max3(fmaxf(top[0], top[1]), top[2], top[3]) > kTop)) {
@@ -267,7 +268,7 @@ struct EmitSweep {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int d = 8 * t + 2 * tq + i - (lane >> 2);
-                at[t][i] = d < 0 || d >= g.ws ? -1 : (int)buf + 4 * ((lane >> 2) * 2 * g.ws + (d + rot >= g.ws ? d + rot - g.ws : d + rot));
+                at[t][i] = h >= g.H || d < 0 || d >= g.ws ? -1 : (int)buf + 4 * ((lane >> 2) * 2 * g.ws + (d + rot >= g.ws ? d + rot - g.ws : d + rot));
             }
     }
 

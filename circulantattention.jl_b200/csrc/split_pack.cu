@@ -139,10 +139,10 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
 
 // Units of one slab (more channels would need their results in registers for 32 or 64 channels), windows up to 25 (four tiles a
 // column).  From window 9 on, and at 7 on grids of up to 2^18 pixels: what a warp spends outside its steps, and the scores outside
-// the window, weigh more the shorter it is.  dk/dv on the FMA pipe and on the tensor cores: 500 x 400, 8 units: ws 5 289 and 358 us,
-// 7: 431 and 418, 9: 588 and 480, 13: 1022 and 817; 512 x 512, 8 units, ws 21 2966 and 1720; 200 x 180, 4 units: ws 5 40 and 43,
-// 7: 59 and 50, 9: 90 and 56.  A few pixels leave the chip idle either way, and their warps have less to do in the smaller
-// tiles of the FMA kernels (32 x 32, 1 unit, ws 11: 9.2 and 10.4 us).
+// the window, weigh more the shorter it is.  Forward + dq + dk/dv, FMA pipe and tensor cores: 500 x 400, 8 units: ws 5 651 and
+// 875 us, 7: 937 and 1013, 9: 1277 and 1158, 13: 2229 and 1905, 1024 x 1024, ws 21: 25900 and 17300; 200 x 180, 4 units: ws 5 95
+// and 103, 7: 143 and 119, 9: 197 and 135.  A few pixels leave the chip idle either way, and their warps have less to do in
+// the smaller tiles of the FMA kernels (32 x 32, 1 unit, ws 11: 24 and 28 us).
 bool split_shape_ok(const Geo& g, float scale) {
     const int64_t pixels = (int64_t)g.Np * g.units;
     return tiled_shape_ok(g) && g.wsw == g.ws && slabs_of(g) == 1 && split_tiles(g) <= 4 && scale > 0.f && g.Wk <= 65535 && pixels > 8192 &&

@@ -72,6 +72,13 @@ int tiled_attention_fwd(const Geo& gin, float scale, int dist, const float* q, c
     if (!workspace) { set_error("workspace of ca_attention_fwd_workspace() bytes is NULL"); return CA_ERR_NULL; }
     const Padded P = padded_of(g);
     float* kv = static_cast<float*>(workspace);
+    if (split_shape_ok(g, scale)) {
+        if (nz && !stats) stats = kv + P.pair_floats;
+        int rc = launch_split_pack(g, scale, dist, k, v, nullptr, nullptr, nullptr, nullptr, kv, st);
+        if (rc) return rc;
+        if ((rc = run_split_fwd(g, scale, dist, q, k, v, kv, y, stats, st)) || !nz) return rc;
+        return run_split_emit(g, scale, dist, q, k, stats, kv, nz, st);
+    }
     if (nz && !stats) stats = kv + P.pair_floats;         // scratch statistics behind the packed pair
     PackArgs pa{};
     pa.g = g; pa.pp = P.pp; pa.Hp = P.Hp; pa.npairs = 1;
@@ -96,6 +103,11 @@ int tiled_attention_bwd_dq(const Geo& gin, float scale, int dist, const float* q
     if (!workspace) { set_error("workspace of ca_attention_bwd_stage_workspace() bytes is NULL"); return CA_ERR_NULL; }
     const Padded P = padded_of(g);
     float* kv = static_cast<float*>(workspace);
+    if (split_shape_ok(g, scale)) {
+        int rc = launch_split_pack(g, scale, dist, k, v, nullptr, nullptr, nullptr, nullptr, kv, st);
+        if (rc) return rc;
+        return run_split_dq(g, scale, dist, q, k, v, dy, stats, D, kv, dq, st);
+    }
     PackArgs pa{};
     pa.g = g; pa.pp = P.pp; pa.Hp = P.Hp; pa.npairs = 1;
     pa.src[0] = k; pa.src[1] = v; pa.dst[0] = kv;
@@ -185,17 +197,12 @@ int tiled_attention_bwd(const Geo& gin, float scale, int dist, const float* q, c
         return rc ? rc : sweep_k(st);
     };
     if (split_shape_ok(g, scale)) {
+        // the forward of the same problem left its packed (k|v) at the start of its workspace
         int rc;
-        if (fwd_workspace) {
-            kv = const_cast<float*>(static_cast<const float*>(fwd_workspace));
-        } else {
-            PackArgs pa{};
-            pa.g = g; pa.pp = P.pp; pa.Hp = P.Hp; pa.npairs = 1;
-            pa.src[0] = k; pa.src[1] = v; pa.dst[0] = kv;
-            if ((rc = launch_pack(pa, st))) return rc;
-        }
+        if (fwd_workspace) kv = const_cast<float*>(static_cast<const float*>(fwd_workspace));
+        else if ((rc = launch_split_pack(g, scale, dist, k, v, nullptr, nullptr, nullptr, nullptr, kv, st))) return rc;
         if ((rc = launch_split_pack(g, scale, dist, q, dy, stats, y, nullptr, D, qdy, st))) return rc;
-        return run_both([&](cudaStream_t s) { return CA_CHANNELS(g, run_dq, g, P, scale, dist, q, dy, stats, D, kv, dq, s, 0, nullptr); },
+        return run_both([&](cudaStream_t s) { return run_split_dq(g, scale, dist, q, k, v, dy, stats, D, kv, dq, s); },
                         [&](cudaStream_t s) { return run_split_dkdv(g, scale, dist, q, k, v, dy, stats, D, qdy, dk, dv, s); });
     }
     PackArgs pa{};

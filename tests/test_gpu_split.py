@@ -1,5 +1,5 @@
 """The tensor-core sweeps (split halves): tile edges of rows, columns and windows, storage kinds, groups of eight rows whose
-magnitudes differ, and scores of a thousand.
+magnitudes differ, references that move, and values that are no numbers.
 
 Bars: the usual ones.  A split operand keeps 22 to 24 bits of an element down to 2^-13 of the largest of its group of eight rows and 16
 channels, and steps of 2^-36 of that largest below; the products and sums are Float32's.  The magnitudes below vary by less
@@ -72,7 +72,7 @@ def test_magnitudes(ca, what):
     elif what == "large":
         v *= 1e9
         r *= 1e7
-    else:                                    # scores of a thousand: the rows are one-hot
+    else:                                    # scores of a thousand: the references move, rows are one-hot
         q *= 30
         k[:, ::3] *= 8
     got = run(ca, "dot", q, k, v, r, ws, heads, want_a=True)
@@ -81,6 +81,27 @@ def test_magnitudes(ca, what):
     bars = dict(tol=2e-3, elem_tol=2e-2) if what == "scores" else {}
     for name in got:
         assert_close(got[name], want[name], name, **bars)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_what_is_no_number_stays_in_its_windows(ca, bad):
+    rng = np.random.default_rng(63)
+    shape, ws, heads = (56, 50, 48, 1), 9, 3
+    q, k, v, r = (randn(rng, shape) for _ in range(4))
+    clean = run(ca, "dot", q, k, v, r, ws, heads, want_a=True)
+    v[30, 20, 5, 0] = bad                    # head 0
+    got = run(ca, "dot", q, k, v, r, ws, heads, want_a=True)
+    near = np.zeros(shape[:2], bool)         # pixels whose window holds the element
+    near[26:35, 16:25] = True
+    assert not np.isfinite(got["y"][26:35, 16:25, 5, 0]).any()
+    assert_close(got["A"], clean["A"], "A")
+    assert_close(got["y"][~near], clean["y"][~near], "y")
+    far = np.ones(shape[:2], bool)           # gradients reach two windows
+    far[22:39, 12:29] = False
+    for name in ("dq", "dk", "dv"):
+        assert_close(got[name][far], clean[name][far], name)
+    for name in ("y", "dq", "dk", "dv"):     # and no other head
+        assert_close(got[name][:, :, 16:], clean[name][:, :, 16:], name)
 
 
 def test_bfloat16_storage(ca):
