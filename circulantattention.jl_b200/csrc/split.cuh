@@ -60,8 +60,9 @@ struct SplitPackArgs {
     float* dst;
 };
 
-// 2-D softmax windows the sweeps take.
+// Whether the forward, A's values and dq run here, and whether dk/dv does (wherever they do, and at more shapes).
 bool split_shape_ok(const Geo& g, float scale);
+bool split_dkdv_ok(const Geo& g, float scale);
 // Packs (x0|x1); with `stats` also the scalars of the backward, D = y . x1 (written to Dout) or given.
 int launch_split_pack(const Geo& g, float scale, int dist, const float* x0, const float* x1, const float* stats, const float* y, const float* Din,
                       float* Dout, float* dst, cudaStream_t st);

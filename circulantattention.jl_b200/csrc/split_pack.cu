@@ -138,15 +138,25 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
 }  // namespace
 
 // Units of one slab (more channels would need their results in registers for 32 or 64 channels), windows up to 25 (four tiles a
-// column).  From window 9 on, and at 7 on grids of up to 2^18 pixels: what a warp spends outside its steps, and the scores outside
-// the window, weigh more the shorter it is.  Forward + dq + dk/dv, FMA pipe and tensor cores: 500 x 400, 8 units: ws 5 651 and
-// 875 us, 7: 937 and 1013, 9: 1277 and 1158, 13: 2229 and 1905, 1024 x 1024, ws 21: 25900 and 17300; 200 x 180, 4 units: ws 5 95
-// and 103, 7: 143 and 119, 9: 197 and 135.  A few pixels leave the chip idle either way, and their warps have less to do in
-// the smaller tiles of the FMA kernels (32 x 32, 1 unit, ws 11: 24 and 28 us).
-bool split_shape_ok(const Geo& g, float scale) {
+// column), and enough pixels to fill the chip: a few are done sooner in the smaller tiles of the FMA kernels (train, 100 x 90,
+// 1 unit, ws 11: under 89 and 109 us; 64 x 64, 3 units: 89 and 87).
+// dk/dv from window 9 on, and at 7 on grids of up to 2^18 pixels: what a warp spends outside its steps, and the scores outside the
+// window, weigh more the shorter it is.  FMA pipe and tensor cores: 500 x 400, 8 units: ws 5 289 and 358 us, 7: 431 and 418,
+// 9: 588 and 480, 13: 1022 and 817; 512 x 512, 8 units: ws 7 555 and 540, ws 21 2966 and 1720; 200 x 180, 4 units: ws 5 40 and
+// 43, 7: 59 and 50, 9: 90 and 56.
+bool split_dkdv_ok(const Geo& g, float scale) {
     const int64_t pixels = (int64_t)g.Np * g.units;
-    return tiled_shape_ok(g) && g.wsw == g.ws && slabs_of(g) == 1 && split_tiles(g) <= 4 && scale > 0.f && g.Wk <= 65535 && pixels > 8192 &&
+    return tiled_shape_ok(g) && g.wsw == g.ws && slabs_of(g) == 1 && split_tiles(g) <= 4 && scale > 0.f && g.Wk <= 65535 && pixels > 12000 &&
            (g.ws >= 9 || (g.ws == 7 && pixels <= (1 << 18)));
+}
+
+// Forward, A's values and dq, which share the packed (k|v): window 9, whose 16 keys are two tiles exactly, and from 13 on; at 11 (18
+// keys of three tiles) where the FMA kernels' warps of 32 rows do not divide the image either.  Evaluation without and
+// with A, start and here: 200 x 180, 4 units: ws 7 43, 61 and 41, 73 us, 9: 55, 92 and 45, 92, 11: 70, 144 and 60, 121, 13:
+// 86, 172 and 66, 134; 256 x 256, 4 units: ws 7 57, 104 and 66, 116, 9: 73, 168 and 72, 145, 11: 91, 201 and 95, 189, 13:
+// 112, 252 and 104, 211.
+bool split_shape_ok(const Geo& g, float scale) {
+    return split_dkdv_ok(g, scale) && g.ws >= 9 && (g.ws != 11 || g.H % 32 != 0);
 }
 
 int launch_split_pack(const Geo& g, float scale, int dist, const float* x0, const float* x1, const float* stats, const float* y, const float* Din,

@@ -125,7 +125,7 @@ int tiled_attention_bwd_dkdv(const Geo& gin, float scale, int dist, const float*
     if (!workspace) { set_error("workspace of ca_attention_bwd_stage_workspace() bytes is NULL"); return CA_ERR_NULL; }
     const Padded P = padded_of(g);
     float* qdy = static_cast<float*>(workspace);
-    if (split_shape_ok(g, scale)) {
+    if (split_dkdv_ok(g, scale)) {
         int rc = launch_split_pack(g, scale, dist, q, dy, stats, nullptr, D, nullptr, qdy, st);
         if (rc) return rc;
         return run_split_dkdv(g, scale, dist, q, k, v, dy, stats, D, qdy, dk, dv, st);
@@ -196,20 +196,31 @@ int tiled_attention_bwd(const Geo& gin, float scale, int dist, const float* q, c
         const int rc = sweep_q(st);
         return rc ? rc : sweep_k(st);
     };
-    if (split_shape_ok(g, scale)) {
-        // the forward of the same problem left its packed (k|v) at the start of its workspace
-        int rc;
-        if (fwd_workspace) kv = const_cast<float*>(static_cast<const float*>(fwd_workspace));
-        else if ((rc = launch_split_pack(g, scale, dist, k, v, nullptr, nullptr, nullptr, nullptr, kv, st))) return rc;
-        if ((rc = launch_split_pack(g, scale, dist, q, dy, stats, y, nullptr, D, qdy, st))) return rc;
-        return run_both([&](cudaStream_t s) { return run_split_dq(g, scale, dist, q, k, v, dy, stats, D, kv, dq, s); },
-                        [&](cudaStream_t s) { return run_split_dkdv(g, scale, dist, q, k, v, dy, stats, D, qdy, dk, dv, s); });
+    // the forward of the same problem left its packed (k|v), split or not by the same rule, at the start of its workspace
+    if (fwd_workspace) kv = const_cast<float*>(static_cast<const float*>(fwd_workspace));
+    if (split_dkdv_ok(g, scale)) {
+        const bool split = split_shape_ok(g, scale);
+        int rc = CA_OK;
+        if (!fwd_workspace && split) {
+            rc = launch_split_pack(g, scale, dist, k, v, nullptr, nullptr, nullptr, nullptr, kv, st);
+        } else if (!fwd_workspace) {
+            PackArgs pa{};
+            pa.g = g; pa.pp = P.pp; pa.Hp = P.Hp; pa.npairs = 1;
+            pa.src[0] = k; pa.src[1] = v; pa.dst[0] = kv;
+            rc = launch_pack(pa, st);
+        }
+        if (rc || (rc = launch_split_pack(g, scale, dist, q, dy, stats, y, nullptr, D, qdy, st))) return rc;
+        return run_both(
+            [&](cudaStream_t s) {
+                return split ? run_split_dq(g, scale, dist, q, k, v, dy, stats, D, kv, dq, s)
+                             : CA_CHANNELS(g, run_dq, g, P, scale, dist, q, dy, stats, D, kv, dq, s, 0, nullptr);
+            },
+            [&](cudaStream_t s) { return run_split_dkdv(g, scale, dist, q, k, v, dy, stats, D, qdy, dk, dv, s); });
     }
     PackArgs pa{};
     pa.g = g; pa.pp = P.pp; pa.Hp = P.Hp;
     if (fwd_workspace) {
         // only (q|dy) and the planes are packed here
-        kv = const_cast<float*>(static_cast<const float*>(fwd_workspace));
         pa.npairs = 1;
         pa.src[0] = q; pa.src[1] = dy;
         pa.dst[0] = qdy;

@@ -36,14 +36,14 @@ def oracle(simname, qn, kn, vn, rn, ws, heads):
 
 @pytest.mark.parametrize("simname", ["dot", "distance"])
 @pytest.mark.parametrize("shape,ws,heads,cplx", [
-    ((41, 40, 96, 1), 7, 6, False),      # two tiles a column; one row past a warp's eight, rows past a block's 32
-    ((64, 33, 64, 1), 9, 4, False),      # 16 keys exactly, an odd number of columns
-    ((39, 31, 84, 1), 11, 7, False),     # three tiles, 12 channels
-    ((17, 61, 72, 1), 17, 9, False),     # rows equal to the window: every row wraps; the longest of three tiles; 8 channels
-    ((33, 37, 56, 1), 19, 8, False),     # four tiles, 7 channels
-    ((65, 26, 32, 3), 25, 2, False),     # the longest window; batch of three
-    ((40, 52, 32, 1), 13, 4, True),      # 8 complex channels
-    ((47, 45, 20, 1), 9, 4, True),       # 5 complex channels
+    ((41, 40, 128, 1), 7, 8, False),     # dk/dv only; two tiles a column; one row past a warp's eight, rows past a block's 32
+    ((64, 33, 96, 1), 9, 6, False),      # 16 keys exactly, an odd number of columns
+    ((39, 47, 84, 1), 11, 7, False),     # three tiles, 12 channels
+    ((17, 91, 72, 1), 17, 9, False),     # rows equal to the window: every row wraps; the longest of three tiles; 8 channels
+    ((33, 47, 56, 1), 19, 8, False),     # four tiles, 7 channels
+    ((65, 32, 32, 3), 25, 2, False),     # the longest window; batch of three
+    ((40, 76, 32, 1), 13, 4, True),      # 8 complex channels
+    ((47, 65, 20, 1), 9, 4, True),       # 5 complex channels
 ])
 def test_edges(ca, shape, ws, heads, cplx, simname):
     rng = np.random.default_rng(61)
@@ -57,7 +57,7 @@ def test_edges(ca, shape, ws, heads, cplx, simname):
 @pytest.mark.parametrize("what", ["pixels", "zeros", "small", "large", "scores"])
 def test_magnitudes(ca, what):
     rng = np.random.default_rng(62)
-    shape, ws, heads = (48, 44, 64, 1), 11, 4
+    shape, ws, heads = (57, 54, 64, 1), 11, 4
     q, k, v, r = (randn(rng, shape) for _ in range(4))
     if what == "pixels":                     # every pixel another power of two: the groups of a step rarely share their scale
         for t, span in ((q, 1), (k, 1), (v, 5), (r, 5)):
@@ -86,7 +86,7 @@ def test_magnitudes(ca, what):
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 def test_what_is_no_number_stays_in_its_windows(ca, bad):
     rng = np.random.default_rng(63)
-    shape, ws, heads = (56, 50, 48, 1), 9, 3
+    shape, ws, heads = (56, 74, 48, 1), 9, 3
     q, k, v, r = (randn(rng, shape) for _ in range(4))
     clean = run(ca, "dot", q, k, v, r, ws, heads, want_a=True)
     v[30, 20, 5, 0] = bad                    # head 0
@@ -106,7 +106,7 @@ def test_what_is_no_number_stays_in_its_windows(ca, bad):
 
 def test_bfloat16_storage(ca):
     rng = np.random.default_rng(64)
-    shape, ws, heads = (50, 46, 64, 1), 15, 4
+    shape, ws, heads = (50, 62, 64, 1), 15, 4
     t = [torch.from_numpy(randn(rng, shape)).to(torch.bfloat16).float().numpy() for _ in range(4)]
     q, k, v, r = (ca.jl.from_numpy(np.asfortranarray(x)).to(torch.bfloat16) for x in t)
     q, k, v = (x.requires_grad_(True) for x in (q, k, v))
