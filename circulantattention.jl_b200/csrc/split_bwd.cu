@@ -86,14 +86,14 @@ __device__ __noinline__ void exact_dkdv(const SplitArgs& a, int u, int h, int w)
 }
 
 // What the two sweeps share: the tiles of a column against two centre operands.
-template <int NS, int NT>
+template <int NS, int NT, bool LO>
 struct BwdSweep {
     static constexpr int RB = split_row_bytes(NS), SB = split_stage_bytes(NS, NT);
     const SplitArgs& a;
     int lane, tq, h, u;
     uint32_t dot_off, outer_off, tail_off, word_off;
     float sl2;
-    Centre<NS> c0, c1;
+    Centre<NS, LO> c0, c1;
     uint32_t cur, word;                                      // the scales of the step's groups when they are all alike; this lane's
     bool bad, mixed;
 
@@ -134,9 +134,9 @@ struct BwdSweep {
     }
 };
 
-template <int NS, int NT, bool DIST>
-struct DqSweep : BwdSweep<NS, NT> {
-    using B = BwdSweep<NS, NT>;
+template <int NS, int NT, bool DIST, bool LO>
+struct DqSweep : BwdSweep<NS, NT, LO> {
+    using B = BwdSweep<NS, NT, LO>;
     using B::a; using B::lane; using B::tq; using B::h; using B::u; using B::c0; using B::c1; using B::cur; using B::word; using B::bad; using B::mixed;
     using B::RB; using B::SB;
     pair_t acc[NS][2][2], sum[2], nref[NT][2], c[2], e[2], nd[2], S[2], Sd[2];     // Sd: Distance, the sums of dS
@@ -177,7 +177,7 @@ struct DqSweep : BwdSweep<NS, NT> {
     template <int HALF>
     __device__ __forceinline__ void column(uint32_t rb, bool first, bool last) {
         float x[NT][4], y[NT][4];
-        dot_column<NS, NT>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
+        dot_column<NS, NT, LO>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
         if (mixed) {
             scale_tiles<NT>(x, word, cur, 0, 1, HALF);
             scale_tiles<NT>(y, word, cur, 8, 0, HALF);
@@ -212,7 +212,7 @@ struct DqSweep : BwdSweep<NS, NT> {
         for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int r = 0; r < 2; ++r) split2(x[t][2 * r], x[t][2 * r + 1], hi[t][r], lo[t][r]);
-        outer_column<NS, NT, HALF>(hi, lo, tail, rb + HALF * SB + B::outer_off, rb + B::tail_off, S, acc);
+        outer_column<NS, NT, LO, HALF>(hi, lo, tail, rb + HALF * SB + B::outer_off, rb + B::tail_off, S, acc);
     }
 
     __device__ __forceinline__ void step(uint32_t rb, bool first, bool last) {
@@ -267,9 +267,9 @@ struct DqSweep : BwdSweep<NS, NT> {
     }
 };
 
-template <int NS, int NT, bool DIST>
-struct DkdvSweep : BwdSweep<NS, NT> {
-    using B = BwdSweep<NS, NT>;
+template <int NS, int NT, bool DIST, bool LO>
+struct DkdvSweep : BwdSweep<NS, NT, LO> {
+    using B = BwdSweep<NS, NT, LO>;
     using B::a; using B::lane; using B::tq; using B::h; using B::u; using B::c0; using B::c1; using B::cur; using B::word; using B::bad; using B::mixed;
     using B::RB; using B::SB;
     pair_t dk[NS][2][2], dv[NS][2][2], sum[2], mk[NT], bk[2], c[2], e[2], nrm, Sk[2], Sv[2], Sd;      // Sd: Distance, the sums of dS
@@ -303,7 +303,7 @@ struct DkdvSweep : BwdSweep<NS, NT> {
     template <int HALF>
     __device__ __forceinline__ void column(uint32_t rb, bool first, bool last) {
         float x[NT][4], y[NT][4];
-        dot_column<NS, NT>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
+        dot_column<NS, NT, LO>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
         if (mixed) {
             scale_tiles<NT>(x, word, cur, 0, 1, HALF);
             scale_tiles<NT>(y, word, cur, 8, 0, HALF);
@@ -345,12 +345,12 @@ struct DkdvSweep : BwdSweep<NS, NT> {
         for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int r = 0; r < 2; ++r) split2(x[t][2 * r], x[t][2 * r + 1], hi[t][r], lo[t][r]);
-        outer_column<NS, NT, HALF>(hi, lo, tp, rb + HALF * SB + B::outer_off + 64 * NS, rb + B::tail_off + 64 * NS, Sv, dv);
+        outer_column<NS, NT, LO, HALF>(hi, lo, tp, rb + HALF * SB + B::outer_off + 64 * NS, rb + B::tail_off + 64 * NS, Sv, dv);
 #pragma unroll
         for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int r = 0; r < 2; ++r) split2(y[t][2 * r], y[t][2 * r + 1], hi[t][r], lo[t][r]);
-        outer_column<NS, NT, HALF>(hi, lo, td, rb + HALF * SB + B::outer_off, rb + B::tail_off, Sk, dk);
+        outer_column<NS, NT, LO, HALF>(hi, lo, td, rb + HALF * SB + B::outer_off, rb + B::tail_off, Sk, dk);
     }
 
     __device__ __forceinline__ void step(uint32_t rb, bool first, bool last) {
@@ -410,16 +410,16 @@ struct DkdvSweep : BwdSweep<NS, NT> {
     }
 };
 
-template <int NS, int NT, bool DIST>
+template <int NS, int NT, bool DIST, bool LO>
 __global__ void __launch_bounds__(32 * kSplitWarps, 4) split_dq_kernel(const __grid_constant__ SplitArgs a,
                                                                                            const __grid_constant__ CUtensorMap map) {
-    DqSweep<NS, NT, DIST> sweep(a);
+    DqSweep<NS, NT, DIST, LO> sweep(a);
     split_run<NS, NT>(a, &map, sweep);
 }
-template <int NS, int NT, bool DIST>
+template <int NS, int NT, bool DIST, bool LO>
 __global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 ? 4 : 3) split_dkdv_kernel(const __grid_constant__ SplitArgs a,
                                                                                              const __grid_constant__ CUtensorMap map) {
-    DkdvSweep<NS, NT, DIST> sweep(a);
+    DkdvSweep<NS, NT, DIST, LO> sweep(a);
     split_run<NS, NT>(a, &map, sweep);
 }
 
@@ -427,8 +427,13 @@ __global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 ? 4 : 3) split_dkdv_
 
 #define CA_SPLIT_BWD(KERNEL, NSV, NTV)                                                               \
     do {                                                                                             \
-        if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true>), a, L, st);                               \
-        else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false>), a, L, st);                                   \
+        if (g.bf16) {                                                                                \
+            if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true, false>), a, L, st);                    \
+            else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false, false>), a, L, st);                        \
+        } else {                                                                                     \
+            if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true, true>), a, L, st);                     \
+            else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false, true>), a, L, st);                         \
+        }                                                                                            \
     } while (0)
 #define CA_SPLIT_BWD_NT(KERNEL, NSV)                                                                 \
     do {                                                                                             \

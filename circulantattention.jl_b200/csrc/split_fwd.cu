@@ -60,14 +60,14 @@ __device__ __noinline__ void exact_values(const SplitArgs& a, int u, int h, int 
 }
 
 // A warp's eight rows of two columns; a step scores them against two columns of the window.
-template <int NS, int NT, bool DIST>
+template <int NS, int NT, bool DIST, bool LO>
 struct FwdSweep {
     static constexpr int RB = split_row_bytes(NS), SB = split_stage_bytes(NS, NT), T = 2 * NT;
     const SplitArgs& a;
     int lane, tq, h, u;
     uint32_t dot_off, outer_off, tail_off, word_off;
     float sl2;
-    Centre<NS> q;
+    Centre<NS, LO> q;
     pair_t acc[NS][2][2], l[2], nref[NT][2], c[2], S[2];
     float shift[2];                                          // what the references have moved by
     uint32_t cur;                                            // the scales of the step's groups when they are all alike, as they mostly are
@@ -122,7 +122,7 @@ struct FwdSweep {
             for (int r = 0; r < 2; ++r) c[r] = pair(q.scale[r] * exp_scale(ek), q.scale[r] * exp_scale(ek));
         }
         float x[T][4];
-        dot_tiles<NS, NT>(q, rb + dot_off, x);
+        dot_tiles<NS, NT, LO>(q, rb + dot_off, x);
         if (mixed) scale_tiles<NT>(x, word, cur, 0, 1);
         float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -183,7 +183,7 @@ struct FwdSweep {
             split2(x[t][0], x[t][1], hi[t][0], lo[t][0]);
             split2(x[t][2], x[t][3], hi[t][1], lo[t][1]);
         }
-        outer_tiles<NS, NT>(hi, lo, rb + outer_off, rb + tail_off, S, acc);
+        outer_tiles<NS, NT, LO>(hi, lo, rb + outer_off, rb + tail_off, S, acc);
     }
     __device__ __forceinline__ void end(int w0, float poison) {
         const Geo& g = a.g;
@@ -208,23 +208,23 @@ struct FwdSweep {
     }
 };
 
-template <int NS, int NT, bool DIST>
+template <int NS, int NT, bool DIST, bool LO>
 __global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 ? 5 : 4) split_fwd_kernel(const __grid_constant__ SplitArgs a, const __grid_constant__ CUtensorMap map) {
-    FwdSweep<NS, NT, DIST> sweep(a);
+    FwdSweep<NS, NT, DIST, LO> sweep(a);
     split_run<NS, NT>(a, &map, sweep);
 }
 
 // A's values: the scores once more, weighed with the row's log-sum-exp.  The runs of a step's two window columns are put in order in
 // shared memory and leave row by row, 8 ws bytes that are contiguous but for the wrap: stored from the accumulators they
 // were 4-byte pieces 8 bytes apart (128 x 96, 8 units, ws 15: 75 us).
-template <int NS, int NT, bool DIST>
+template <int NS, int NT, bool DIST, bool LO>
 struct EmitSweep {
     static constexpr int RB = split_row_bytes(NS), SB = split_stage_bytes(NS, NT), T = 2 * NT;
     const SplitArgs& a;
     int lane, tq, h, u, w, s, rows;                          // s: the next column of the window; rows of the warp in the image
     uint32_t dot_off, word_off, buf;
     float sl2;
-    Centre<NS> q;
+    Centre<NS, LO> q;
     pair_t nref[2], c[2];
     int at[NT][2];                                           // shared address of a tile's element for the first row and window column, -1: outside
     uint32_t cur;
@@ -284,7 +284,7 @@ struct EmitSweep {
             for (int r = 0; r < 2; ++r) c[r] = pair(q.scale[r] * exp_scale(cur), q.scale[r] * exp_scale(cur));
         }
         float x[T][4];
-        dot_tiles<NS, NT>(q, rb + dot_off, x);
+        dot_tiles<NS, NT, LO>(q, rb + dot_off, x);
         if (mixed) scale_tiles<NT>(x, word, cur, 0, 1);
         __syncwarp();
 #pragma unroll
@@ -333,9 +333,9 @@ struct EmitSweep {
     }
 };
 
-template <int NS, int NT, bool DIST>
+template <int NS, int NT, bool DIST, bool LO>
 __global__ void __launch_bounds__(32 * kSplitWarps, 4) split_emit_kernel(const __grid_constant__ SplitArgs a, const __grid_constant__ CUtensorMap map) {
-    EmitSweep<NS, NT, DIST> sweep(a);
+    EmitSweep<NS, NT, DIST, LO> sweep(a);
     split_run<NS, NT>(a, &map, sweep);
 }
 
@@ -351,8 +351,13 @@ int run_split_fwd(const Geo& g, float scale, int dist, const float* q, const flo
     a.c0 = q; a.o0 = y; a.ostats = stats; a.x0 = k; a.x1 = v;
 #define CA_SPLIT_FWD(KERNEL, NSV, NTV)                                                               \
     do {                                                                                             \
-        if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true>), a, L, st);                               \
-        else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false>), a, L, st);                                   \
+        if (g.bf16) {                                                                                \
+            if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true, false>), a, L, st);                    \
+            else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false, false>), a, L, st);                        \
+        } else {                                                                                     \
+            if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true, true>), a, L, st);                     \
+            else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false, true>), a, L, st);                         \
+        }                                                                                            \
     } while (0)
 #define CA_SPLIT_FWD_NT(KERNEL, NSV)                                                                 \
     do {                                                                                             \
