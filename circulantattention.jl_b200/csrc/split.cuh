@@ -8,10 +8,15 @@
 // tcgen05 is not used: its scores would leave and enter through tensor memory for the mask, the exponential and the
 // split, which costs more than its rate gains at 16 to 64 channels (forward 70.6 us against 62.5 on the FMA pipe).
 //
+// Error against 64 bits (2-norm, standard normal; FMA pipe and here): 64 x 48, 2 units, ws 15: y 5.7e-7 and 2.4e-7, dq 5.8e-7 and
+// 4.1e-7, dk 5.5e-7 and 4.0e-7, dv 5.5e-7 and 4.1e-7; 40 x 37, 4 units, ws 21, Distance: 6.4e-7 and 2.7e-7, 9.0e-7 and 4.9e-7,
+// 7.2e-7 and 4.6e-7, 6.7e-7 and 4.4e-7; 24 x 24, 2 units of 4 channels, ws 3: 2.6e-7 and 1.6e-7, 4.8e-7 and 4.4e-7, 4.6e-7 and
+// 4.3e-7, 4.2e-7 and 4.2e-7.
+//
 // Tiles.  Rows of a product are 16 centre pixels: 8 rows (h) of two neighbouring columns (w), whose windows share all but two
 // columns.  Columns are 8 pixels of the streamed column, so a window column takes NT = ceil((8 + 2p) / 8) tiles and 62 %
 // (window 21) to 44 % (window 7) of the scores are inside the window; 16 rows of one column would leave 52 and 29 %.
-// Scores outside start at -inf in the accumulator, which costs nothing.
+// The mask costs nothing: it rides in the addend of the FMA that scales a score (-inf outside).
 //
 // Streamed rows.  [unit][column][row'][128 NS + 16 bytes] = hi then lo of the first tensor, hi then lo of the second, 16 bytes of
 // scalars; row' = h + p with the circular halo unrolled.  The pitch is an odd number of 16-byte words, so ldmatrix
@@ -19,8 +24,13 @@
 // (a warp's window starts at one), so it is uniform over a tile.  It puts the group's largest magnitude into [2^11, 2^15): an
 // element 2^13 below it keeps all bits, the least step is 2^-36 of the largest.
 //
-// Rows with a NaN or an infinity mark their group; a block that meets one recomputes its pixels from the tensors one
+// Rows with a NaN or an infinity mark their group; a warp that meets one recomputes its pixels from the tensors one
 // by one (exact_*), since a product of a tile would carry them to pixels outside their window.
+//
+// What bounds the sweeps (256 x 256, 8 units, ws 21): the tensor pipe is busy in 47 % (forward) to 54 % (dk/dv) of the cycles, an
+// instruction issues in 48 and 45 %; an mma also takes five issue slots from FMAs and waits behind them, and 12 to 16 warps of
+// 128 to 168 registers do not cover the latencies of the chain score - exponential - split - sum.  Times are beside the rules of
+// the dispatch (split_pack.cu).
 #pragma once
 #include "tile_common.cuh"
 #include <cuda_fp16.h>
