@@ -19,8 +19,8 @@
 // The mask costs nothing: it rides in the addend of the FMA that scales a score (-inf outside).
 //
 // Streamed rows.  [unit][column][row'][128 NS + 16 bytes] = hi then lo of the first tensor, hi then lo of the second, 16 bytes of
-// scalars; row' = h + p with the circular halo unrolled.  The pitch is an odd number of 16-byte words, so ldmatrix
-// reads eight rows without bank conflicts.  The power of two is common to a group of eight rows starting at a multiple of eight
+// scalars; row' = h + p with the circular halo unrolled.  bfloat16 tensors have no lower halves, and their rows no place for
+// them: 64 NS + 16 bytes.  Either pitch is an odd number of 16-byte words, so ldmatrix reads eight rows without bank conflicts.  The power of two is common to a group of eight rows starting at a multiple of eight
 // (a warp's window starts at one), so it is uniform over a tile.  It puts the group's largest magnitude into [2^11, 2^15): an
 // element 2^13 below it keeps all bits, the least step is 2^-36 of the largest.
 //
@@ -88,10 +88,13 @@ int run_split_dkdv(const Geo& g, float scale, int dist, const float* q, const fl
 
 namespace {
 
-__host__ __device__ constexpr int split_row_bytes(int ns) { return 128 * ns + 16; }
+// Where the second tensor of a row begins, where its scalars, and the row's pitch; `lo`: with lower halves.
+__host__ __device__ constexpr int split_second(int ns, bool lo) { return (lo ? 64 : 32) * ns; }
+__host__ __device__ constexpr int split_scalars(int ns, bool lo) { return 2 * split_second(ns, lo); }
+__host__ __device__ constexpr int split_row_bytes(int ns, bool lo) { return split_scalars(ns, lo) + 16; }
 constexpr int kSplitSteps = 3, kSplitWarps = 4;
 __host__ __device__ constexpr int split_rows(int nt) { return 8 * (kSplitWarps - 1) + 8 * nt; }
-__host__ __device__ constexpr int split_stage_bytes(int ns, int nt) { return (split_rows(nt) * split_row_bytes(ns) + 127) & ~127; }
+__host__ __device__ constexpr int split_stage_bytes(int ns, int nt, bool lo) { return (split_rows(nt) * split_row_bytes(ns, lo) + 127) & ~127; }
 __host__ __device__ inline int split_hp(const Geo& g) { return (g.H + 2 * g.p + 3) & ~3; }
 inline int split_tiles(const Geo& g) { return (8 + 2 * g.p + 7) / 8; }
 
@@ -99,6 +102,9 @@ inline int split_tiles(const Geo& g) { return (8 + 2 * g.p + 7) / 8; }
 __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm2(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
 }
 __device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -256,8 +262,10 @@ __device__ __forceinline__ float quad_sum(float x) {
 
 // An A operand: the split vectors of the two pixels of each row of a tile, with each pixel's scale and squared norm.
 // LO: the operands have lower halves.  bfloat16 tensors do not: their 8 bits fit the upper one, which leaves one product of a score
-// and two of a weighted sum (1024 x 1024, 8 units, ws 21: forward
-// 4277 -> 3590 us, dq 5517 -> 4173, dk/dv 7448 -> 6267).
+// and two of a weighted sum (1024 x 1024, 8 units, ws 21: forward 4277 -> 3590 us, dq 5517 -> 4173, dk/dv 7448 -> 6267), rows of 80
+// bytes for 144, one ldmatrix for both tensors' scores in the backward, and registers for one more block per SM (pack and
+// forward together 3930 -> 3815 us, forward and backward 14812 -> 13340; 512 x 512, 8 units: ws 9 1540 -> 1451, ws 13 2328 -> 2111;
+// 200 x 180, 4 units, ws 25: 352 -> 317).
 template <int NS, bool LO>
 struct Centre {
     uint32_t hi[NS][4], lo[NS][4];
@@ -294,9 +302,9 @@ struct Centre {
 };
 
 // Tiles of a step: NT of its first column, then NT of its second; offset of tile f from the step's first row.
-template <int NS, int NT>
+template <int NS, int NT, bool LO>
 __device__ __forceinline__ constexpr int tile_offset(int f) {
-    return (f / NT) * split_stage_bytes(NS, NT) + 8 * (f % NT) * split_row_bytes(NS);
+    return (f / NT) * split_stage_bytes(NS, NT, LO) + 8 * (f % NT) * split_row_bytes(NS, LO);
 }
 
 // x[f] = centre . streamed over the channels for the tiles of a step: `b` is this lane's ldmatrix address inside the first tensor or
@@ -308,7 +316,10 @@ __device__ __forceinline__ void dot_tiles(const Centre<NS, LO>& a, uint32_t b, f
     for (int s = 0; s < NS; ++s) {
         uint32_t f[2 * NT][4];
 #pragma unroll
-        for (int t = 0; t < 2 * NT; ++t) ldsm4(b + tile_offset<NS, NT>(t) + 32 * s, f[t]);      // hi of 8 + 8 channels, lo of 8 + 8
+        for (int t = 0; t < 2 * NT; ++t) {
+            if (LO) ldsm4(b + tile_offset<NS, NT, LO>(t) + 32 * s, f[t]);      // hi of 8 + 8 channels, lo of 8 + 8
+            else ldsm2(b + tile_offset<NS, NT, LO>(t) + 32 * s, f[t]);
+        }
         if (LO) {
 #pragma unroll
             for (int t = 0; t < 2 * NT; ++t) {
@@ -341,7 +352,7 @@ __device__ __forceinline__ void outer_tiles(const uint32_t (&hi)[2 * NT][2], con
         for (int k = 0; k < NT; ++k) {
             const bool tail = (NT & 1) && k == NT - 1;
             const int t = tail ? NT - 1 : (k < NT / 2 ? 2 * k : NT + 2 * (k - NT / 2)), t1 = tail ? 2 * NT - 1 : t + 1;
-            const uint32_t at = (tail ? bt : b) + tile_offset<NS, NT>(t) + 32 * s;
+            const uint32_t at = (tail ? bt : b) + tile_offset<NS, NT, LO>(t) + 32 * s;
             uint32_t x[4], y[4];
             ldsm4t(at, x);                                 // hi: channels 0-7 of 8 + 8 rows, channels 8-15
             if (LO) ldsm4t(at + 32 * NS, y);               // lo
@@ -374,14 +385,19 @@ __device__ __forceinline__ void outer_tiles(const uint32_t (&hi)[2 * NT][2], con
 // column against two centre operands: x from the first tensor (`b`), y from the second.
 template <int NS, int NT, bool LO>
 __device__ __forceinline__ void dot_column(const Centre<NS, LO>& a0, const Centre<NS, LO>& a1, uint32_t b, float (&x)[NT][4], float (&y)[NT][4]) {
-    constexpr int RB = split_row_bytes(NS);
+    constexpr int RB = split_row_bytes(NS, LO);
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
         uint32_t f[NT][4], e[NT][4];
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
             ldsm4(b + 8 * t * RB + 32 * s, f[t]);
-            ldsm4(b + 8 * t * RB + 32 * s + 64 * NS, e[t]);
+            if (LO) {
+                ldsm4(b + 8 * t * RB + 32 * s + split_second(NS, LO), e[t]);
+            } else {                                       // the second tensor's upper halves stand where the first's lower ones would
+                e[t][0] = f[t][2];
+                e[t][1] = f[t][3];
+            }
         }
         if (LO) {
 #pragma unroll
@@ -419,7 +435,7 @@ struct Tail {
 template <int NS, int NT, bool LO, int TAIL>
 __device__ __forceinline__ void outer_column(const uint32_t (&hi)[NT][2], const uint32_t (&lo)[NT][2], Tail& tail, uint32_t b, uint32_t bt,
                                              const pair_t (&S)[2], pair_t (&acc)[NS][2][2]) {
-    constexpr int RB = split_row_bytes(NS), K = NT / 2 + ((NT & 1) && TAIL ? 1 : 0);
+    constexpr int RB = split_row_bytes(NS, LO), K = NT / 2 + ((NT & 1) && TAIL ? 1 : 0);
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
         float c[2][4], d[2][4];
@@ -488,10 +504,10 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // counter, caller's status word), and what it stores is poisoned with NaN.
 // Measured against this cut at 512 x 512, 8 units, ws 21 (forward 1090 us): two pairs of columns per block on the same buffers with
 // half the copies 1100, several pairs of columns one after the other 1100, two buffers instead of three 1170.
-template <int NS, int NT, class Sweep>
+template <int NS, int NT, bool LO, class Sweep>
 __device__ __forceinline__ void split_run(const SplitArgs& a, const CUtensorMap* map, Sweep& sweep) {
-    constexpr int SB = split_stage_bytes(NS, NT);
-    constexpr uint32_t kBytes = 2 * split_rows(NT) * split_row_bytes(NS);
+    constexpr int SB = split_stage_bytes(NS, NT, LO);
+    constexpr uint32_t kBytes = 2 * split_rows(NT) * split_row_bytes(NS, LO);
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * kSplitSteps];
     const Geo& g = a.g;
@@ -519,7 +535,7 @@ __device__ __forceinline__ void split_run(const SplitArgs& a, const CUtensorMap*
     bool lost = false;
     if (live) {
         sweep.begin(w0, stages + 2 * SB * kSplitSteps);
-        uint32_t bar = full, ring = stages + 8 * warp * split_row_bytes(NS), phase = 0;
+        uint32_t bar = full, ring = stages + 8 * warp * split_row_bytes(NS, LO), phase = 0;
 #pragma unroll 1
         for (int step = 0; step < steps; ++step) {
             if (!__all_sync(0xffffffffu, mbar_try(bar, phase))) {
@@ -556,18 +572,18 @@ __device__ __forceinline__ void split_run(const SplitArgs& a, const CUtensorMap*
 }
 
 // This lane's ldmatrix offsets inside a stage, relative to the warp's first row.
-__device__ __forceinline__ uint32_t dot_offset(int lane, int ns) {               // [hi 0-7, hi 8-15, lo 0-7, lo 8-15] of 8 rows
-    return (lane & 7) * split_row_bytes(ns) + ((lane >> 3) & 1) * 16 + (lane >> 4) * 32 * ns;
+__device__ __forceinline__ uint32_t dot_offset(int lane, int ns, bool lo) {      // [hi 0-7, hi 8-15, lo 0-7, lo 8-15] of 8 rows
+    return (lane & 7) * split_row_bytes(ns, lo) + ((lane >> 3) & 1) * 16 + (lane >> 4) * 32 * ns;
 }
-__device__ __forceinline__ uint32_t outer_offset(int lane, int ns, int next) {   // [rows 0-7, those `next` bytes on] x [channels 0-7, 8-15]
-    return (lane & 7) * split_row_bytes(ns) + ((lane >> 3) & 1) * next + (lane >> 4) * 16;
+__device__ __forceinline__ uint32_t outer_offset(int lane, int ns, bool lo, int next) {   // [rows 0-7, those `next` bytes on] x [channels 0-7, 8-15]
+    return (lane & 7) * split_row_bytes(ns, lo) + ((lane >> 3) & 1) * next + (lane >> 4) * 16;
 }
 // Where the word of scales lies that this lane watches: lanes 0-3 the groups of the step's first column, lanes 4-7 those of its
 // second, and so on; groups past the padded rows do not exist.
-template <int NS, int NT>
+template <int NS, int NT, bool LO>
 __device__ __forceinline__ uint32_t word_offset(const Geo& g, int lane, int row0) {
     const int t = min(min(lane & 3, NT - 1), (split_hp(g) - row0 - 1) >> 3);
-    return ((lane >> 2) & 1) * split_stage_bytes(NS, NT) + 8 * t * split_row_bytes(NS) + 128 * NS;
+    return ((lane >> 2) & 1) * split_stage_bytes(NS, NT, LO) + 8 * t * split_row_bytes(NS, LO) + split_scalars(NS, LO);
 }
 // Tiles whose group has another scale than the step's largest (byte `shift` of the words), times the ratio; `least`: the smallest
 // exponent of the ratio (0: it may vanish; groups without a scale hold zeros only).
@@ -597,7 +613,8 @@ __device__ __forceinline__ uint32_t ldsu32(uint32_t addr) {
 // ---------------------------------------------------------------- host
 // Launch geometry, shared memory (`extra` bytes of the sweep's own) and the tensor map of a sweep.
 inline int split_prepare(const Geo& g, float scale, int dist, const float* packed, Launch* L, SplitArgs* a, size_t extra = 0) {
-    const int ns = slabs_of(g), nt = split_tiles(g), rb = split_row_bytes(ns), rf = rb / 4, hp = split_hp(g);
+    const bool lo = !g.bf16;
+    const int ns = slabs_of(g), nt = split_tiles(g), rb = split_row_bytes(ns, lo), rf = rb / 4, hp = split_hp(g);
     a->g = g;
     a->scale = scale;
     a->dist = dist;
@@ -606,7 +623,7 @@ inline int split_prepare(const Geo& g, float scale, int dist, const float* packe
     a->wait_tries = kWaitTries;
     L->grid = dim3((unsigned)((g.W + 1) / 2), (unsigned)((g.H + 8 * kSplitWarps - 1) / (8 * kSplitWarps)), (unsigned)g.units);
     L->threads = 32 * kSplitWarps;
-    L->smem = (size_t)2 * kSplitSteps * split_stage_bytes(ns, nt) + 128 + extra;
+    L->smem = (size_t)2 * kSplitSteps * split_stage_bytes(ns, nt, lo) + 128 + extra;
     if (L->smem > kMaxDynamicSmem || L->grid.y > 65535u) return CA_ERR_UNSUPPORTED;
     const uint64_t dims[4] = {(uint64_t)rf, (uint64_t)hp, (uint64_t)g.Wk, (uint64_t)g.units};
     const uint64_t strides[3] = {(uint64_t)rb, (uint64_t)hp * rb, (uint64_t)hp * rb * g.Wk};

@@ -88,7 +88,7 @@ __device__ __noinline__ void exact_dkdv(const SplitArgs& a, int u, int h, int w)
 // What the two sweeps share: the tiles of a column against two centre operands.
 template <int NS, int NT, bool LO>
 struct BwdSweep {
-    static constexpr int RB = split_row_bytes(NS), SB = split_stage_bytes(NS, NT);
+    static constexpr int RB = split_row_bytes(NS, LO), SB = split_stage_bytes(NS, NT, LO);
     const SplitArgs& a;
     int lane, tq, h, u;
     uint32_t dot_off, outer_off, tail_off, word_off;
@@ -104,10 +104,10 @@ struct BwdSweep {
         h = row0 + (lane >> 2);
         u = blockIdx.z;
         sl2 = a.scale * kLog2e;
-        dot_off = dot_offset(lane, NS);
-        outer_off = outer_offset(lane, NS, 8 * RB);
-        tail_off = outer_offset(lane, NS, SB);
-        word_off = word_offset<NS, NT>(a.g, lane, row0);
+        dot_off = dot_offset(lane, NS, LO);
+        outer_off = outer_offset(lane, NS, LO, 8 * RB);
+        tail_off = outer_offset(lane, NS, LO, SB);
+        word_off = word_offset<NS, NT, LO>(a.g, lane, row0);
     }
     __device__ __forceinline__ void load(int w0) {
         Raw<NS> r0, r1;
@@ -184,7 +184,7 @@ struct DqSweep : BwdSweep<NS, NT, LO> {
         }
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-            const pair_t b = DIST ? lds_pair(rb + HALF * SB + (8 * t + 2 * tq) * RB + 128 * NS + 8) : 0;
+            const pair_t b = DIST ? lds_pair(rb + HALF * SB + (8 * t + 2 * tq) * RB + split_scalars(NS, LO) + 8) : 0;
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const float2 z = unpair(fma_pair(pair(x[t][2 * r], x[t][2 * r + 1]), c[r], DIST ? add_pair(nref[t][r], b) : nref[t][r]));
@@ -308,7 +308,7 @@ struct DkdvSweep : BwdSweep<NS, NT, LO> {
             scale_tiles<NT>(x, word, cur, 0, 1, HALF);
             scale_tiles<NT>(y, word, cur, 8, 0, HALF);
         }
-        const uint32_t sc = rb + HALF * SB + 2 * tq * RB + 128 * NS + 8;
+        const uint32_t sc = rb + HALF * SB + 2 * tq * RB + split_scalars(NS, LO) + 8;
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
             const pair_t A = add_pair(mk[t], lds_pair(sc + 8 * t * RB)), Dn = mul_pair(lds_pair(sc + (8 * t + 1) * RB), nrm);
@@ -345,7 +345,7 @@ struct DkdvSweep : BwdSweep<NS, NT, LO> {
         for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int r = 0; r < 2; ++r) split2(x[t][2 * r], x[t][2 * r + 1], hi[t][r], lo[t][r]);
-        outer_column<NS, NT, LO, HALF>(hi, lo, tp, rb + HALF * SB + B::outer_off + 64 * NS, rb + B::tail_off + 64 * NS, Sv, dv);
+        outer_column<NS, NT, LO, HALF>(hi, lo, tp, rb + HALF * SB + B::outer_off + split_second(NS, LO), rb + B::tail_off + split_second(NS, LO), Sv, dv);
 #pragma unroll
         for (int t = 0; t < NT; ++t)
 #pragma unroll
@@ -410,17 +410,18 @@ struct DkdvSweep : BwdSweep<NS, NT, LO> {
     }
 };
 
+// As many blocks per SM as the registers allow (Distance without lower halves spills 76 to 128 bytes of begin and end).
 template <int NS, int NT, bool DIST, bool LO>
-__global__ void __launch_bounds__(32 * kSplitWarps, 4) split_dq_kernel(const __grid_constant__ SplitArgs a,
+__global__ void __launch_bounds__(32 * kSplitWarps, LO ? 4 : 5) split_dq_kernel(const __grid_constant__ SplitArgs a,
                                                                                            const __grid_constant__ CUtensorMap map) {
     DqSweep<NS, NT, DIST, LO> sweep(a);
-    split_run<NS, NT>(a, &map, sweep);
+    split_run<NS, NT, LO>(a, &map, sweep);
 }
 template <int NS, int NT, bool DIST, bool LO>
-__global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 ? 4 : 3) split_dkdv_kernel(const __grid_constant__ SplitArgs a,
+__global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 || !LO ? 4 : 3) split_dkdv_kernel(const __grid_constant__ SplitArgs a,
                                                                                              const __grid_constant__ CUtensorMap map) {
     DkdvSweep<NS, NT, DIST, LO> sweep(a);
-    split_run<NS, NT>(a, &map, sweep);
+    split_run<NS, NT, LO>(a, &map, sweep);
 }
 
 }  // namespace

@@ -62,7 +62,7 @@ __device__ __noinline__ void exact_values(const SplitArgs& a, int u, int h, int 
 // A warp's eight rows of two columns; a step scores them against two columns of the window.
 template <int NS, int NT, bool DIST, bool LO>
 struct FwdSweep {
-    static constexpr int RB = split_row_bytes(NS), SB = split_stage_bytes(NS, NT), T = 2 * NT;
+    static constexpr int RB = split_row_bytes(NS, LO), SB = split_stage_bytes(NS, NT, LO), T = 2 * NT;
     const SplitArgs& a;
     int lane, tq, h, u;
     uint32_t dot_off, outer_off, tail_off, word_off;
@@ -80,10 +80,10 @@ struct FwdSweep {
         h = row0 + (lane >> 2);
         u = blockIdx.z;
         sl2 = a.scale * kLog2e;
-        dot_off = dot_offset(lane, NS);
-        outer_off = outer_offset(lane, NS, 8 * RB) + 64 * NS;
-        tail_off = outer_offset(lane, NS, SB) + 64 * NS;
-        word_off = word_offset<NS, NT>(a.g, lane, row0);
+        dot_off = dot_offset(lane, NS, LO);
+        outer_off = outer_offset(lane, NS, LO, 8 * RB) + split_second(NS, LO);
+        tail_off = outer_offset(lane, NS, LO, SB) + split_second(NS, LO);
+        word_off = word_offset<NS, NT, LO>(a.g, lane, row0);
     }
 
     __device__ __forceinline__ void begin(int w0, uint32_t) {
@@ -127,7 +127,7 @@ struct FwdSweep {
         float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-            const pair_t b = DIST ? lds_pair(rb + tile_offset<NS, NT>(t) + 2 * tq * RB + 128 * NS + 8) : 0;
+            const pair_t b = DIST ? lds_pair(rb + tile_offset<NS, NT, LO>(t) + 2 * tq * RB + split_scalars(NS, LO) + 8) : 0;
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const float2 y = unpair(fma_pair(pair(x[t][2 * r], x[t][2 * r + 1]), c[r], DIST ? add_pair(nref[t % NT][r], b) : nref[t % NT][r]));
@@ -208,10 +208,11 @@ struct FwdSweep {
     }
 };
 
+// Five blocks per SM where the registers suffice: two tiles a column, or no lower halves (8 to 40 bytes spilled at three and four tiles).
 template <int NS, int NT, bool DIST, bool LO>
-__global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 ? 5 : 4) split_fwd_kernel(const __grid_constant__ SplitArgs a, const __grid_constant__ CUtensorMap map) {
+__global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 || !LO ? 5 : 4) split_fwd_kernel(const __grid_constant__ SplitArgs a, const __grid_constant__ CUtensorMap map) {
     FwdSweep<NS, NT, DIST, LO> sweep(a);
-    split_run<NS, NT>(a, &map, sweep);
+    split_run<NS, NT, LO>(a, &map, sweep);
 }
 
 // A's values: the scores once more, weighed with the row's log-sum-exp.  The runs of a step's two window columns are put in order in
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 ? 5 : 4) split_fwd_k
 // were 4-byte pieces 8 bytes apart (128 x 96, 8 units, ws 15: 75 us).
 template <int NS, int NT, bool DIST, bool LO>
 struct EmitSweep {
-    static constexpr int RB = split_row_bytes(NS), SB = split_stage_bytes(NS, NT), T = 2 * NT;
+    static constexpr int RB = split_row_bytes(NS, LO), SB = split_stage_bytes(NS, NT, LO), T = 2 * NT;
     const SplitArgs& a;
     int lane, tq, h, u, w, s, rows;                          // s: the next column of the window; rows of the warp in the image
     uint32_t dot_off, word_off, buf;
@@ -237,8 +238,8 @@ struct EmitSweep {
         h = row0 + (lane >> 2);
         u = blockIdx.z;
         sl2 = a.scale * kLog2e;
-        dot_off = dot_offset(lane, NS);
-        word_off = word_offset<NS, NT>(a.g, lane, row0);
+        dot_off = dot_offset(lane, NS, LO);
+        word_off = word_offset<NS, NT, LO>(a.g, lane, row0);
     }
 
     __device__ __forceinline__ void begin(int w0, uint32_t own) {
@@ -291,7 +292,7 @@ struct EmitSweep {
         for (int half = 0; half < 2; ++half)
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-                const pair_t b = DIST ? lds_pair(rb + half * SB + (8 * t + 2 * tq) * RB + 128 * NS + 8) : 0;
+                const pair_t b = DIST ? lds_pair(rb + half * SB + (8 * t + 2 * tq) * RB + split_scalars(NS, LO) + 8) : 0;
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     const float2 y = unpair(fma_pair(pair(x[half * NT + t][2 * r], x[half * NT + t][2 * r + 1]), c[r],
@@ -336,7 +337,7 @@ struct EmitSweep {
 template <int NS, int NT, bool DIST, bool LO>
 __global__ void __launch_bounds__(32 * kSplitWarps, 4) split_emit_kernel(const __grid_constant__ SplitArgs a, const __grid_constant__ CUtensorMap map) {
     EmitSweep<NS, NT, DIST, LO> sweep(a);
-    split_run<NS, NT>(a, &map, sweep);
+    split_run<NS, NT, LO>(a, &map, sweep);
 }
 
 }  // namespace

@@ -11,7 +11,8 @@ namespace {
 // contiguous run of 16-byte stores.  Bound: HBM.
 template <int CPE, int NS, bool BF>
 __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
-    constexpr int RB = 128 / NS, RF = split_row_bytes(NS) / 4;
+    constexpr bool LO = !BF;
+    constexpr int RB = 128 / NS, RF = split_row_bytes(NS, LO) / 4;
     __shared__ __align__(16) uint32_t tile[RB * RF];
     __shared__ uint32_t gmax[2][NS][RB / 8];
     __shared__ float sums[2][NS][RB];
@@ -94,12 +95,14 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
         uint32_t hi[8], lo[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) split2(x[t][2 * i] * inv, x[t][2 * i + 1] * inv, hi[i], lo[i]);
-        uint4* d = reinterpret_cast<uint4*>(row + t * 16 * NS + slab * 8);
+        uint4* d = reinterpret_cast<uint4*>(row + t * (split_second(NS, LO) / 4) + slab * 8);
         d[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         d[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
-        d += 2 * NS;
-        d[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        d[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+        if (LO) {
+            d += 2 * NS;
+            d[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            d[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+        }
     }
     if (slab == 0) {
 #pragma unroll
@@ -126,7 +129,7 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
         }
         const float A1 = __shfl_xor_sync(0xffffffffu, A, 1), dot1 = __shfl_xor_sync(0xffffffffu, dot, 1);
         const uint4 odd = make_uint4(exps, 0u, __float_as_uint(-dot1), __float_as_uint(-dot));
-        *reinterpret_cast<uint4*>(row + 32 * NS) = rl & 1 ? odd : make_uint4(exps, 0u, __float_as_uint(A), __float_as_uint(A1));
+        *reinterpret_cast<uint4*>(row + split_scalars(NS, LO) / 4) = rl & 1 ? odd : make_uint4(exps, 0u, __float_as_uint(A), __float_as_uint(A1));
     }
     __syncthreads();
     const int nrows = min(RB, a.Hp - rr0);
@@ -164,18 +167,10 @@ int launch_split_pack(const Geo& g, float scale, int dist, const float* x0, cons
     SplitPackArgs a{};
     a.g = g; a.Hp = split_hp(g); a.x0 = x0; a.x1 = x1; a.stats = stats; a.y = y; a.Din = Din; a.Dout = Dout; a.dst = dst;
     a.norm_mul = dist ? -0.5f * scale * kLog2e : 0.f;
-    const int ns = slabs_of(a.g), rb = 128 / ns;
-    const dim3 grid((a.Hp + rb - 1) / rb, a.g.Wk, a.g.units);
-    if (a.g.bf16) split_pack_kernel<1, 1, true><<<grid, 128, 0, st>>>(a);
-    else if (a.g.cpe == 1) {
-        if (ns == 1) split_pack_kernel<1, 1, false><<<grid, 128, 0, st>>>(a);
-        else if (ns == 2) split_pack_kernel<1, 2, false><<<grid, 128, 0, st>>>(a);
-        else split_pack_kernel<1, 4, false><<<grid, 128, 0, st>>>(a);
-    } else {
-        if (ns == 1) split_pack_kernel<2, 1, false><<<grid, 128, 0, st>>>(a);
-        else if (ns == 2) split_pack_kernel<2, 2, false><<<grid, 128, 0, st>>>(a);
-        else split_pack_kernel<2, 4, false><<<grid, 128, 0, st>>>(a);
-    }
+    const dim3 grid((a.Hp + 127) / 128, g.Wk, g.units);
+    if (g.bf16) split_pack_kernel<1, 1, true><<<grid, 128, 0, st>>>(a);
+    else if (g.cpe == 1) split_pack_kernel<1, 1, false><<<grid, 128, 0, st>>>(a);
+    else split_pack_kernel<2, 1, false><<<grid, 128, 0, st>>>(a);
     CA_CHECK_LAUNCH("split pack kernel");
     return CA_OK;
 }
