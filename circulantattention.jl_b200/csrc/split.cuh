@@ -260,7 +260,15 @@ __device__ __forceinline__ float quad_sum(float x) {
     return x + __shfl_xor_sync(0xffffffffu, x, 2);
 }
 
-// An A operand: the split vectors of the two pixels of each row of a tile, with each pixel's scale and squared norm.
+// Biased exponent of a power of two above |x| (255 for what is no number).
+__device__ __forceinline__ int above(float x) {
+    const uint32_t b = abs_bits(x);
+    return b ? min((int)(b >> 23) + 1, 255) : 0;
+}
+
+// An A operand: the split vectors of the two pixels of each row of a tile, with each pixel's scale, squared norm and `top`, the
+// biased exponent of a power of two above its norm (0: the vector is zero).  `top` comes from the scaled vector, whose squares
+// neither vanish nor overflow: those of cotangents of 1e-19 and below do.
 // LO: the operands have lower halves.  bfloat16 tensors do not: their 8 bits fit the upper one, which leaves one product of a score
 // and two of a weighted sum (1024 x 1024, 8 units, ws 21: forward 4277 -> 3590 us, dq 5517 -> 4173, dk/dv 7448 -> 6267), rows of 80
 // bytes for 144, one ldmatrix for both tensors' scores in the backward, and registers for one more block per SM (pack and
@@ -270,6 +278,7 @@ template <int NS, bool LO>
 struct Centre {
     uint32_t hi[NS][4], lo[NS][4];
     float scale[2], norm2[2];
+    int top[2];
     bool bad;
     __device__ __forceinline__ void form(const Raw<NS>& raw, const Geo& g, int h, int w, int tq, int least) {
         bad = false;
@@ -292,6 +301,13 @@ struct Centre {
             bad |= e == 255;
             scale[r] = exp_scale(e);
             const float inv = exp_inverse(e == 255 ? 0 : e);
+            float ns = 0.f;
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) ns = fmaf(x[s][i] * inv, x[s][i] * inv, ns);
+            ns = quad_sum(ns);
+            top[r] = ns > 0.f ? above(sqrtf(ns)) + e - 127 : 0;
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
                 split2(x[s][0] * inv, x[s][1] * inv, hi[s][r], lo[s][r]);

@@ -10,11 +10,6 @@ namespace {
 
 constexpr float kWeightExp = 14.f;
 
-// Biased exponent of a power of two above |x| (255 for what is no number).
-__device__ __forceinline__ int above(float x) {
-    const uint32_t b = abs_bits(x);
-    return b ? min((int)(b >> 23) + 1, 255) : 0;
-}
 // Biased exponent of the reciprocal of a bound of |dP| + |D|: `norm` above the centre vector's norm, `e` the exponent of the streamed
 // group's scale, whose vectors have norms up to sqrt(16 NS) 2^15, `d` above |D|.
 template <int NS>
@@ -141,7 +136,6 @@ struct DqSweep : BwdSweep<NS, NT, LO> {
     using B::RB; using B::SB;
     pair_t acc[NS][2][2], sum[2], nref[NT][2], c[2], e[2], nd[2], S[2], Sd[2];     // Sd: Distance, the sums of dS
     float D[2];
-    int norm[2];
     Tail tail;
 
     __device__ __forceinline__ DqSweep(const SplitArgs& a_) : B(a_) {}
@@ -165,7 +159,6 @@ struct DqSweep : BwdSweep<NS, NT, LO> {
             const float b = kWeightExp - L - (DIST ? 0.5f * B::sl2 * c0.norm2[r] : 0.f);
 #pragma unroll
             for (int t = 0; t < NT; ++t) nref[t][r] = pair(b + window_mask(lane, g.p, t, 0), b + window_mask(lane, g.p, t, 1));
-            norm[r] = above(sqrtf(c1.norm2[r]));
             sum[r] = c[r] = e[r] = nd[r] = S[r] = Sd[r] = 0;
         }
 #pragma unroll
@@ -225,7 +218,7 @@ struct DqSweep : BwdSweep<NS, NT, LO> {
             mixed = __any_sync(0xffffffffu, word != cur);
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-                const int nb = bound_inverse<NS>(norm[r], ev, above(D[r]));
+                const int nb = bound_inverse<NS>(c1.top[r], ev, above(D[r]));
                 const float nrm = exp_scale(nb), bd = exp_scale(254 - nb) * 0x1p-14f, back = exp_scale(ek) * bd;
                 c[r] = pair(c0.scale[r] * exp_scale(ek), c0.scale[r] * exp_scale(ek));
                 e[r] = pair(c1.scale[r] * nrm * exp_scale(ev), c1.scale[r] * nrm * exp_scale(ev));
@@ -284,8 +277,7 @@ struct DkdvSweep : BwdSweep<NS, NT, LO> {
         B::load(w0);
         most = 0;
         nrm = Sd = 0;
-        norm = above(sqrtf(fmaxf(c1.norm2[0], c1.norm2[1])));
-        norm = __reduce_max_sync(0xffffffffu, norm);
+        norm = __reduce_max_sync(0xffffffffu, max(c1.top[0], c1.top[1]));
 #pragma unroll
         for (int t = 0; t < NT; ++t) mk[t] = pair(kWeightExp + window_mask(lane, g.p, t, 0), kWeightExp + window_mask(lane, g.p, t, 1));
 #pragma unroll

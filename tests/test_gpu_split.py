@@ -83,6 +83,33 @@ def test_magnitudes(ca, what):
         assert_close(got[name], want[name], name, **bars)
 
 
+@pytest.mark.parametrize("simname", ["dot", "distance"])
+@pytest.mark.parametrize("which,mul", [("r", 1e-20), ("r", 1e-30), ("r", 1e20), ("v", 1e-20), ("v", 1e20)])
+def test_norms_whose_squares_are_no_floats(ca, which, mul, simname):
+    """The weights of the gradients are scaled by a bound that follows from the norms of dy and v, whose squares leave the range
+    of Float32 long before the tensors do."""
+    rng = np.random.default_rng(65)
+    shape, ws, heads = (57, 54, 64, 1), 11, 4
+    t = dict(zip("qkvr", (randn(rng, shape) for _ in range(4))))
+    t[which] *= np.float32(mul)
+    got = run(ca, simname, *t.values(), ws, heads)
+    want = oracle(simname, *t.values(), ws, heads)
+    for name in got:
+        assert_close(got[name], want[name], name)
+
+
+def test_pixels_with_small_cotangents(ca):
+    """dq of a pixel is as accurate as its own dy, however small."""
+    rng = np.random.default_rng(66)
+    shape, ws, heads = (57, 54, 64, 1), 11, 4
+    q, k, v, r = (randn(rng, shape) for _ in range(4))
+    small = rng.random(shape[:2]) < 0.1
+    r[small] *= np.float32(1e-20)
+    dq, want = run(ca, "dot", q, k, v, r, ws, heads)["dq"], oracle("dot", q, k, v, r, ws, heads)["dq"]
+    assert_close(dq[small], want[small], "dq of the small")
+    assert_close(dq[~small], want[~small], "dq of the others")
+
+
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 def test_what_is_no_number_stays_in_its_windows(ca, bad):
     rng = np.random.default_rng(63)
