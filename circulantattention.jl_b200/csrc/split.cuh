@@ -18,9 +18,9 @@
 // (window 21) to 44 % (window 7) of the scores are inside the window; 16 rows of one column would leave 52 and 29 %.
 // The mask costs nothing: it rides in the addend of the FMA that scales a score (-inf outside).
 //
-// Streamed rows.  [unit][column][row'][128 NS + 16 bytes] = hi then lo of the first tensor, hi then lo of the second, 16 bytes of
+// Streamed rows.  [unit][column][row'][144 bytes] = hi then lo of the first tensor, hi then lo of the second, 16 bytes of
 // scalars; row' = h + p with the circular halo unrolled.  bfloat16 tensors have no lower halves, and their rows no place for
-// them: 64 NS + 16 bytes.  Either pitch is an odd number of 16-byte words, so ldmatrix reads eight rows without bank conflicts.  The power of two is common to a group of eight rows starting at a multiple of eight
+// them: 80 bytes.  Either pitch is an odd number of 16-byte words, so ldmatrix reads eight rows without bank conflicts.  The power of two is common to a group of eight rows starting at a multiple of eight
 // (a warp's window starts at one), so it is uniform over a tile.  It puts the group's largest magnitude into [2^11, 2^15): an
 // element 2^13 below it keeps all bits, the least step is 2^-36 of the largest.
 //
@@ -89,12 +89,12 @@ int run_split_dkdv(const Geo& g, float scale, int dist, const float* q, const fl
 namespace {
 
 // Where the second tensor of a row begins, where its scalars, and the row's pitch; `lo`: with lower halves.
-__host__ __device__ constexpr int split_second(int ns, bool lo) { return (lo ? 64 : 32) * ns; }
-__host__ __device__ constexpr int split_scalars(int ns, bool lo) { return 2 * split_second(ns, lo); }
-__host__ __device__ constexpr int split_row_bytes(int ns, bool lo) { return split_scalars(ns, lo) + 16; }
+__host__ __device__ constexpr int split_second(bool lo) { return lo ? 64 : 32; }
+__host__ __device__ constexpr int split_scalars(bool lo) { return 2 * split_second(lo); }
+__host__ __device__ constexpr int split_row_bytes(bool lo) { return split_scalars(lo) + 16; }
 constexpr int kSplitSteps = 3, kSplitWarps = 4;
 __host__ __device__ constexpr int split_rows(int nt) { return 8 * (kSplitWarps - 1) + 8 * nt; }
-__host__ __device__ constexpr int split_stage_bytes(int ns, int nt, bool lo) { return (split_rows(nt) * split_row_bytes(ns, lo) + 127) & ~127; }
+__host__ __device__ constexpr int split_stage_bytes(int nt, bool lo) { return (split_rows(nt) * split_row_bytes(lo) + 127) & ~127; }
 __host__ __device__ inline int split_hp(const Geo& g) { return (g.H + 2 * g.p + 3) & ~3; }
 inline int split_tiles(const Geo& g) { return (8 + 2 * g.p + 7) / 8; }
 
@@ -190,57 +190,51 @@ __device__ __forceinline__ void st_channel(float* dst, const Geo& g, int u, int 
     else st_real<false>(dst, goff<1>(u, g.cr, cc, npix, pix), x);
 }
 
-// The channels 2t, 2t+1, 2t+8, 2t+9 of every slab (t = lane % 4) of the two pixels of a lane's row: what a lane holds of a row of an A
+// The channels 2t, 2t+1, 2t+8, 2t+9 (t = lane % 4) of the two pixels of a lane's row: what a lane holds of a row of an A
 // operand and of a result.  Pixels outside the image and channels past the unit's read some other element of the tensor and
 // are zeroed in Centre::form: without conditions all loads of a warp are in flight together.
-template <int NS>
 struct Raw {
-    float x[2][NS][4];
+    float x[2][4];
     __device__ __forceinline__ void load(const float* src, const Geo& g, int u, int h, int w, int tq) {
         const int hc = min(h, g.H - 1);
         const int pix[2] = {hc + g.H * w, hc + g.H * min(w + 1, g.W - 1)};
         if (g.cpe == 2) {
             const float2* s2 = reinterpret_cast<const float2*>(src) + (int64_t)u * g.c * g.Np;
 #pragma unroll
-            for (int s = 0; s < NS; ++s)
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int i = 0; i < 2; ++i)
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        const float2 z = __ldg(s2 + (int64_t)min(8 * s + tq + 4 * i, g.c - 1) * g.Np + pix[r]);
-                        x[r][s][2 * i] = z.x;
-                        x[r][s][2 * i + 1] = z.y;
-                    }
+                for (int r = 0; r < 2; ++r) {
+                    const float2 z = __ldg(s2 + (int64_t)min(tq + 4 * i, g.c - 1) * g.Np + pix[r]);
+                    x[r][2 * i] = z.x;
+                    x[r][2 * i + 1] = z.y;
+                }
             return;
         }
         const int64_t o = (int64_t)u * g.cr * g.Np;
 #pragma unroll
-        for (int s = 0; s < NS; ++s)
+        for (int i = 0; i < 4; ++i) {
+            const int64_t c = o + (int64_t)min(2 * tq + (i & 1) + 8 * (i >> 1), g.cr - 1) * g.Np;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int64_t c = o + (int64_t)min(16 * s + 2 * tq + (i & 1) + 8 * (i >> 1), g.cr - 1) * g.Np;
-#pragma unroll
-                for (int r = 0; r < 2; ++r) x[r][s][i] = g.bf16 ? ld_real<true>(src, c + pix[r]) : ld_real<false>(src, c + pix[r]);
-            }
+            for (int r = 0; r < 2; ++r) x[r][i] = g.bf16 ? ld_real<true>(src, c + pix[r]) : ld_real<false>(src, c + pix[r]);
+        }
     }
 };
-// The channel of element i of slab s.
-__device__ __forceinline__ int lane_channel(const Geo& g, int s, int i, int tq) { return 16 * s + 2 * tq + (i & 1) + 8 * (i >> 1); }
+// The channel of a lane's element i.
+__device__ __forceinline__ int lane_channel(int i, int tq) { return 2 * tq + (i & 1) + 8 * (i >> 1); }
 
-// The four channels of one slab of a pixel: x[0..1] in the result's first eight channels, x[2..3] in its second.
-__device__ __forceinline__ void store_pixel(float* dst, const Geo& g, int u, int slab, int pix, int tq, float x0, float x1, float x2, float x3) {
+// A lane's four channels of a pixel: x[0..1] in the result's first eight channels, x[2..3] in its second.
+__device__ __forceinline__ void store_pixel(float* dst, const Geo& g, int u, int pix, int tq, float x0, float x1, float x2, float x3) {
     if (g.cpe == 2) {
         float2* d2 = reinterpret_cast<float2*>(dst);
-        const int c = 8 * slab + tq;
-        if (c < g.c) d2[((int64_t)u * g.c + c) * g.Np + pix] = make_float2(x0, x1);
-        if (c + 4 < g.c) d2[((int64_t)u * g.c + c + 4) * g.Np + pix] = make_float2(x2, x3);
+        if (tq < g.c) d2[((int64_t)u * g.c + tq) * g.Np + pix] = make_float2(x0, x1);
+        if (tq + 4 < g.c) d2[((int64_t)u * g.c + tq + 4) * g.Np + pix] = make_float2(x2, x3);
         return;
     }
     const float x[4] = {x0, x1, x2, x3};
     const int64_t o = (int64_t)u * g.cr * g.Np + pix;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int c = 16 * slab + 2 * tq + (i & 1) + 8 * (i >> 1);
+        const int c = lane_channel(i, tq);
         if (c >= g.cr) continue;
         if (g.bf16) st_real<true>(dst, o + (int64_t)c * g.Np, x[i]);
         else st_real<false>(dst, o + (int64_t)c * g.Np, x[i]);
@@ -274,28 +268,26 @@ __device__ __forceinline__ int above(float x) {
 // bytes for 144, one ldmatrix for both tensors' scores in the backward, and registers for one more block per SM (pack and
 // forward together 3930 -> 3815 us, forward and backward 14812 -> 13340; 512 x 512, 8 units: ws 9 1540 -> 1451, ws 13 2328 -> 2111;
 // 200 x 180, 4 units, ws 25: 352 -> 317).
-template <int NS, bool LO>
+template <bool LO>
 struct Centre {
-    uint32_t hi[NS][4], lo[NS][4];
+    uint32_t hi[4], lo[4];
     float scale[2], norm2[2];
     int top[2];
     bool bad;
-    __device__ __forceinline__ void form(const Raw<NS>& raw, const Geo& g, int h, int w, int tq, int least) {
+    __device__ __forceinline__ void form(const Raw& raw, const Geo& g, int h, int w, int tq, int least) {
         bad = false;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const bool ok = h < g.H && w + r < g.W;
-            float x[NS][4];
+            float x[4];
             uint32_t m = 0;
             float n = 0.f;
 #pragma unroll
-            for (int s = 0; s < NS; ++s)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    x[s][i] = ok && lane_channel(g, s, i, tq) < g.cr ? raw.x[r][s][i] : 0.f;
-                    m = max(m, abs_bits(x[s][i]));
-                    n = fmaf(x[s][i], x[s][i], n);
-                }
+            for (int i = 0; i < 4; ++i) {
+                x[i] = ok && lane_channel(i, tq) < g.cr ? raw.x[r][i] : 0.f;
+                m = max(m, abs_bits(x[i]));
+                n = fmaf(x[i], x[i], n);
+            }
             const int e = scale_exp(quad_max(m), 1, least);
             norm2[r] = quad_sum(n);
             bad |= e == 255;
@@ -303,53 +295,42 @@ struct Centre {
             const float inv = exp_inverse(e == 255 ? 0 : e);
             float ns = 0.f;
 #pragma unroll
-            for (int s = 0; s < NS; ++s)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) ns = fmaf(x[s][i] * inv, x[s][i] * inv, ns);
+            for (int i = 0; i < 4; ++i) ns = fmaf(x[i] * inv, x[i] * inv, ns);
             ns = quad_sum(ns);
             top[r] = ns > 0.f ? above(sqrtf(ns)) + e - 127 : 0;
-#pragma unroll
-            for (int s = 0; s < NS; ++s) {
-                split2(x[s][0] * inv, x[s][1] * inv, hi[s][r], lo[s][r]);
-                split2(x[s][2] * inv, x[s][3] * inv, hi[s][2 + r], lo[s][2 + r]);
-            }
+            split2(x[0] * inv, x[1] * inv, hi[r], lo[r]);
+            split2(x[2] * inv, x[3] * inv, hi[2 + r], lo[2 + r]);
         }
     }
 };
 
 // Tiles of a step: NT of its first column, then NT of its second; offset of tile f from the step's first row.
-template <int NS, int NT, bool LO>
+template <int NT, bool LO>
 __device__ __forceinline__ constexpr int tile_offset(int f) {
-    return (f / NT) * split_stage_bytes(NS, NT, LO) + 8 * (f % NT) * split_row_bytes(NS, LO);
+    return (f / NT) * split_stage_bytes(NT, LO) + 8 * (f % NT) * split_row_bytes(LO);
 }
 
 // x[f] = centre . streamed over the channels for the tiles of a step: `b` is this lane's ldmatrix address inside the first tensor or
 // the second.  The chains of the tiles advance together (a warp issues in order and a dependent product waits 20 cycles);
 // small products first, since the unit cuts its sums.
-template <int NS, int NT, bool LO>
-__device__ __forceinline__ void dot_tiles(const Centre<NS, LO>& a, uint32_t b, float (&x)[2 * NT][4]) {
+template <int NT, bool LO>
+__device__ __forceinline__ void dot_tiles(const Centre<LO>& a, uint32_t b, float (&x)[2 * NT][4]) {
+    uint32_t f[2 * NT][4];
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-        uint32_t f[2 * NT][4];
+    for (int t = 0; t < 2 * NT; ++t) {
+        if (LO) ldsm4(b + tile_offset<NT, LO>(t), f[t]);       // hi of 8 + 8 channels, lo of 8 + 8
+        else ldsm2(b + tile_offset<NT, LO>(t), f[t]);
+    }
+    if (LO) {
 #pragma unroll
-        for (int t = 0; t < 2 * NT; ++t) {
-            if (LO) ldsm4(b + tile_offset<NS, NT, LO>(t) + 32 * s, f[t]);      // hi of 8 + 8 channels, lo of 8 + 8
-            else ldsm2(b + tile_offset<NS, NT, LO>(t) + 32 * s, f[t]);
-        }
-        if (LO) {
+        for (int t = 0; t < 2 * NT; ++t) mma16(x[t], a.lo, f[t][0], f[t][1]);
 #pragma unroll
-            for (int t = 0; t < 2 * NT; ++t) {
-                if (s == 0) mma16(x[t], a.lo[s], f[t][0], f[t][1]);
-                else mma16(x[t], a.lo[s], f[t][0], f[t][1], x[t]);
-            }
+        for (int t = 0; t < 2 * NT; ++t) mma16(x[t], a.hi, f[t][2], f[t][3], x[t]);
+    }
 #pragma unroll
-            for (int t = 0; t < 2 * NT; ++t) mma16(x[t], a.hi[s], f[t][2], f[t][3], x[t]);
-        }
-#pragma unroll
-        for (int t = 0; t < 2 * NT; ++t) {
-            if (LO || s > 0) mma16(x[t], a.hi[s], f[t][0], f[t][1], x[t]);
-            else mma16(x[t], a.hi[s], f[t][0], f[t][1]);
-        }
+    for (int t = 0; t < 2 * NT; ++t) {
+        if (LO) mma16(x[t], a.hi, f[t][0], f[t][1], x[t]);
+        else mma16(x[t], a.hi, f[t][0], f[t][1]);
     }
 }
 
@@ -358,89 +339,77 @@ __device__ __forceinline__ void dot_tiles(const Centre<NS, LO>& a, uint32_t b, f
 // for 16 rows of a column, `bt` the one for 8 rows of each column.  The unit cuts its sums instead of rounding them, 0.7
 // units of the last place of a partial sum on average; the sums of a step therefore start at zero, the products of the
 // upper halves apart from the small ones, and are added to the running ones in Float32.
-template <int NS, int NT, bool LO>
+template <int NT, bool LO>
 __device__ __forceinline__ void outer_tiles(const uint32_t (&hi)[2 * NT][2], const uint32_t (&lo)[2 * NT][2], uint32_t b, uint32_t bt, const pair_t (&S)[2],
-                                            pair_t (&acc)[NS][2][2]) {
+                                            pair_t (&acc)[2][2]) {
+    float c[2][4], d[2][4];
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-        float c[2][4], d[2][4];
+    for (int k = 0; k < NT; ++k) {
+        const bool tail = (NT & 1) && k == NT - 1;
+        const int t = tail ? NT - 1 : (k < NT / 2 ? 2 * k : NT + 2 * (k - NT / 2)), t1 = tail ? 2 * NT - 1 : t + 1;
+        const uint32_t at = (tail ? bt : b) + tile_offset<NT, LO>(t);
+        uint32_t x[4], y[4];
+        ldsm4t(at, x);                                         // hi: channels 0-7 of 8 + 8 rows, channels 8-15
+        if (LO) ldsm4t(at + 32, y);                            // lo
+        const uint32_t ah[4] = {hi[t][0], hi[t][1], hi[t1][0], hi[t1][1]};
+        const uint32_t al[4] = {lo[t][0], lo[t][1], lo[t1][0], lo[t1][1]};
 #pragma unroll
-        for (int k = 0; k < NT; ++k) {
-            const bool tail = (NT & 1) && k == NT - 1;
-            const int t = tail ? NT - 1 : (k < NT / 2 ? 2 * k : NT + 2 * (k - NT / 2)), t1 = tail ? 2 * NT - 1 : t + 1;
-            const uint32_t at = (tail ? bt : b) + tile_offset<NS, NT, LO>(t) + 32 * s;
-            uint32_t x[4], y[4];
-            ldsm4t(at, x);                                 // hi: channels 0-7 of 8 + 8 rows, channels 8-15
-            if (LO) ldsm4t(at + 32 * NS, y);               // lo
-            const uint32_t ah[4] = {hi[t][0], hi[t][1], hi[t1][0], hi[t1][1]};
-            const uint32_t al[4] = {lo[t][0], lo[t][1], lo[t1][0], lo[t1][1]};
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                if (k == 0) mma16(c[n], ah, x[2 * n], x[2 * n + 1]);
-                else mma16(c[n], ah, x[2 * n], x[2 * n + 1], c[n]);
-            }
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                if (k == 0) mma16(d[n], al, x[2 * n], x[2 * n + 1]);
-                else mma16(d[n], al, x[2 * n], x[2 * n + 1], d[n]);
-            }
-            if (LO) {
-#pragma unroll
-                for (int n = 0; n < 2; ++n) mma16(d[n], ah, y[2 * n], y[2 * n + 1], d[n]);
-            }
+        for (int n = 0; n < 2; ++n) {
+            if (k == 0) mma16(c[n], ah, x[2 * n], x[2 * n + 1]);
+            else mma16(c[n], ah, x[2 * n], x[2 * n + 1], c[n]);
         }
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int n = 0; n < 2; ++n) {
+            if (k == 0) mma16(d[n], al, x[2 * n], x[2 * n + 1]);
+            else mma16(d[n], al, x[2 * n], x[2 * n + 1], d[n]);
+        }
+        if (LO) {
 #pragma unroll
-            for (int i = 0; i < 4; i += 2)
-                acc[s][n][i / 2] = fma_pair(add_pair(pair(c[n][i], c[n][i + 1]), pair(d[n][i], d[n][i + 1])), S[i / 2], acc[s][n][i / 2]);
+            for (int n = 0; n < 2; ++n) mma16(d[n], ah, y[2 * n], y[2 * n + 1], d[n]);
+        }
     }
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; i += 2)
+            acc[n][i / 2] = fma_pair(add_pair(pair(c[n][i], c[n][i + 1]), pair(d[n][i], d[n][i + 1])), S[i / 2], acc[n][i / 2]);
 }
 
 // The same two products a column at a time, for the backward, whose four products need no other independent work.  Scores of one
 // column against two centre operands: x from the first tensor (`b`), y from the second.
-template <int NS, int NT, bool LO>
-__device__ __forceinline__ void dot_column(const Centre<NS, LO>& a0, const Centre<NS, LO>& a1, uint32_t b, float (&x)[NT][4], float (&y)[NT][4]) {
-    constexpr int RB = split_row_bytes(NS, LO);
+template <int NT, bool LO>
+__device__ __forceinline__ void dot_column(const Centre<LO>& a0, const Centre<LO>& a1, uint32_t b, float (&x)[NT][4], float (&y)[NT][4]) {
+    constexpr int RB = split_row_bytes(LO);
+    uint32_t f[NT][4], e[NT][4];
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-        uint32_t f[NT][4], e[NT][4];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            ldsm4(b + 8 * t * RB + 32 * s, f[t]);
-            if (LO) {
-                ldsm4(b + 8 * t * RB + 32 * s + split_second(NS, LO), e[t]);
-            } else {                                       // the second tensor's upper halves stand where the first's lower ones would
-                e[t][0] = f[t][2];
-                e[t][1] = f[t][3];
-            }
-        }
+    for (int t = 0; t < NT; ++t) {
+        ldsm4(b + 8 * t * RB, f[t]);
         if (LO) {
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                if (s == 0) mma16(x[t], a0.lo[s], f[t][0], f[t][1]);
-                else mma16(x[t], a0.lo[s], f[t][0], f[t][1], x[t]);
-            }
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                if (s == 0) mma16(y[t], a1.lo[s], e[t][0], e[t][1]);
-                else mma16(y[t], a1.lo[s], e[t][0], e[t][1], y[t]);
-            }
-#pragma unroll
-            for (int t = 0; t < NT; ++t) mma16(x[t], a0.hi[s], f[t][2], f[t][3], x[t]);
-#pragma unroll
-            for (int t = 0; t < NT; ++t) mma16(y[t], a1.hi[s], e[t][2], e[t][3], y[t]);
+            ldsm4(b + 8 * t * RB + split_second(LO), e[t]);
+        } else {                                               // the second tensor's upper halves stand where the first's lower ones would
+            e[t][0] = f[t][2];
+            e[t][1] = f[t][3];
         }
+    }
+    if (LO) {
 #pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            if (LO || s > 0) mma16(x[t], a0.hi[s], f[t][0], f[t][1], x[t]);
-            else mma16(x[t], a0.hi[s], f[t][0], f[t][1]);
-        }
+        for (int t = 0; t < NT; ++t) mma16(x[t], a0.lo, f[t][0], f[t][1]);
 #pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            if (LO || s > 0) mma16(y[t], a1.hi[s], e[t][0], e[t][1], y[t]);
-            else mma16(y[t], a1.hi[s], e[t][0], e[t][1]);
-        }
+        for (int t = 0; t < NT; ++t) mma16(y[t], a1.lo, e[t][0], e[t][1]);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) mma16(x[t], a0.hi, f[t][2], f[t][3], x[t]);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) mma16(y[t], a1.hi, e[t][2], e[t][3], y[t]);
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        if (LO) mma16(x[t], a0.hi, f[t][0], f[t][1], x[t]);
+        else mma16(x[t], a0.hi, f[t][0], f[t][1]);
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        if (LO) mma16(y[t], a1.hi, e[t][0], e[t][1], y[t]);
+        else mma16(y[t], a1.hi, e[t][0], e[t][1]);
     }
 }
 // acc += S * (weights . streamed) over one column.  An odd last tile of the first column (TAIL 0) waits in `tail` for that of the
@@ -448,44 +417,41 @@ __device__ __forceinline__ void dot_column(const Centre<NS, LO>& a0, const Centr
 struct Tail {
     uint32_t hi[2], lo[2];
 };
-template <int NS, int NT, bool LO, int TAIL>
+template <int NT, bool LO, int TAIL>
 __device__ __forceinline__ void outer_column(const uint32_t (&hi)[NT][2], const uint32_t (&lo)[NT][2], Tail& tail, uint32_t b, uint32_t bt,
-                                             const pair_t (&S)[2], pair_t (&acc)[NS][2][2]) {
-    constexpr int RB = split_row_bytes(NS, LO), K = NT / 2 + ((NT & 1) && TAIL ? 1 : 0);
+                                             const pair_t (&S)[2], pair_t (&acc)[2][2]) {
+    constexpr int RB = split_row_bytes(LO), K = NT / 2 + ((NT & 1) && TAIL ? 1 : 0);
+    float c[2][4], d[2][4];
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
-        float c[2][4], d[2][4];
+    for (int k = 0; k < K; ++k) {
+        const bool last = k == NT / 2;                         // the tails of both columns
+        const uint32_t at = (last ? bt : b) + (last ? 8 * (NT - 1) : 16 * k) * RB;
+        const int t = last ? NT - 1 : 2 * k, t1 = last ? NT - 1 : 2 * k + 1;
+        uint32_t x[4], y[4];
+        ldsm4t(at, x);
+        if (LO) ldsm4t(at + 32, y);
+        const uint32_t ah[4] = {last ? tail.hi[0] : hi[t][0], last ? tail.hi[1] : hi[t][1], hi[t1][0], hi[t1][1]};
+        const uint32_t al[4] = {last ? tail.lo[0] : lo[t][0], last ? tail.lo[1] : lo[t][1], lo[t1][0], lo[t1][1]};
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const bool last = k == NT / 2;                 // the tails of both columns
-            const uint32_t at = (last ? bt : b) + (last ? 8 * (NT - 1) : 16 * k) * RB + 32 * s;
-            const int t = last ? NT - 1 : 2 * k, t1 = last ? NT - 1 : 2 * k + 1;
-            uint32_t x[4], y[4];
-            ldsm4t(at, x);
-            if (LO) ldsm4t(at + 32 * NS, y);
-            const uint32_t ah[4] = {last ? tail.hi[0] : hi[t][0], last ? tail.hi[1] : hi[t][1], hi[t1][0], hi[t1][1]};
-            const uint32_t al[4] = {last ? tail.lo[0] : lo[t][0], last ? tail.lo[1] : lo[t][1], lo[t1][0], lo[t1][1]};
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                if (k == 0) mma16(c[n], ah, x[2 * n], x[2 * n + 1]);
-                else mma16(c[n], ah, x[2 * n], x[2 * n + 1], c[n]);
-            }
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                if (k == 0) mma16(d[n], al, x[2 * n], x[2 * n + 1]);
-                else mma16(d[n], al, x[2 * n], x[2 * n + 1], d[n]);
-            }
-            if (LO) {
-#pragma unroll
-                for (int n = 0; n < 2; ++n) mma16(d[n], ah, y[2 * n], y[2 * n + 1], d[n]);
-            }
+        for (int n = 0; n < 2; ++n) {
+            if (k == 0) mma16(c[n], ah, x[2 * n], x[2 * n + 1]);
+            else mma16(c[n], ah, x[2 * n], x[2 * n + 1], c[n]);
         }
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int n = 0; n < 2; ++n) {
+            if (k == 0) mma16(d[n], al, x[2 * n], x[2 * n + 1]);
+            else mma16(d[n], al, x[2 * n], x[2 * n + 1], d[n]);
+        }
+        if (LO) {
 #pragma unroll
-            for (int i = 0; i < 4; i += 2)
-                acc[s][n][i / 2] = fma_pair(add_pair(pair(c[n][i], c[n][i + 1]), pair(d[n][i], d[n][i + 1])), S[i / 2], acc[s][n][i / 2]);
+            for (int n = 0; n < 2; ++n) mma16(d[n], ah, y[2 * n], y[2 * n + 1], d[n]);
+        }
     }
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; i += 2)
+            acc[n][i / 2] = fma_pair(add_pair(pair(c[n][i], c[n][i + 1]), pair(d[n][i], d[n][i + 1])), S[i / 2], acc[n][i / 2]);
     if ((NT & 1) && !TAIL) {
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -520,10 +486,10 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // counter, caller's status word), and what it stores is poisoned with NaN.
 // Measured against this cut at 512 x 512, 8 units, ws 21 (forward 1090 us): two pairs of columns per block on the same buffers with
 // half the copies 1100, several pairs of columns one after the other 1100, two buffers instead of three 1170.
-template <int NS, int NT, bool LO, class Sweep>
+template <int NT, bool LO, class Sweep>
 __device__ __forceinline__ void split_run(const SplitArgs& a, const CUtensorMap* map, Sweep& sweep) {
-    constexpr int SB = split_stage_bytes(NS, NT, LO);
-    constexpr uint32_t kBytes = 2 * split_rows(NT) * split_row_bytes(NS, LO);
+    constexpr int SB = split_stage_bytes(NT, LO);
+    constexpr uint32_t kBytes = 2 * split_rows(NT) * split_row_bytes(LO);
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * kSplitSteps];
     const Geo& g = a.g;
@@ -551,7 +517,7 @@ __device__ __forceinline__ void split_run(const SplitArgs& a, const CUtensorMap*
     bool lost = false;
     if (live) {
         sweep.begin(w0, stages + 2 * SB * kSplitSteps);
-        uint32_t bar = full, ring = stages + 8 * warp * split_row_bytes(NS, LO), phase = 0;
+        uint32_t bar = full, ring = stages + 8 * warp * split_row_bytes(LO), phase = 0;
 #pragma unroll 1
         for (int step = 0; step < steps; ++step) {
             if (!__all_sync(0xffffffffu, mbar_try(bar, phase))) {
@@ -588,18 +554,18 @@ __device__ __forceinline__ void split_run(const SplitArgs& a, const CUtensorMap*
 }
 
 // This lane's ldmatrix offsets inside a stage, relative to the warp's first row.
-__device__ __forceinline__ uint32_t dot_offset(int lane, int ns, bool lo) {      // [hi 0-7, hi 8-15, lo 0-7, lo 8-15] of 8 rows
-    return (lane & 7) * split_row_bytes(ns, lo) + ((lane >> 3) & 1) * 16 + (lane >> 4) * 32 * ns;
+__device__ __forceinline__ uint32_t dot_offset(int lane, bool lo) {      // [hi 0-7, hi 8-15, lo 0-7, lo 8-15] of 8 rows
+    return (lane & 7) * split_row_bytes(lo) + ((lane >> 3) & 1) * 16 + (lane >> 4) * 32;
 }
-__device__ __forceinline__ uint32_t outer_offset(int lane, int ns, bool lo, int next) {   // [rows 0-7, those `next` bytes on] x [channels 0-7, 8-15]
-    return (lane & 7) * split_row_bytes(ns, lo) + ((lane >> 3) & 1) * next + (lane >> 4) * 16;
+__device__ __forceinline__ uint32_t outer_offset(int lane, bool lo, int next) {   // [rows 0-7, those `next` bytes on] x [channels 0-7, 8-15]
+    return (lane & 7) * split_row_bytes(lo) + ((lane >> 3) & 1) * next + (lane >> 4) * 16;
 }
 // Where the word of scales lies that this lane watches: lanes 0-3 the groups of the step's first column, lanes 4-7 those of its
 // second, and so on; groups past the padded rows do not exist.
-template <int NS, int NT, bool LO>
+template <int NT, bool LO>
 __device__ __forceinline__ uint32_t word_offset(const Geo& g, int lane, int row0) {
     const int t = min(min(lane & 3, NT - 1), (split_hp(g) - row0 - 1) >> 3);
-    return ((lane >> 2) & 1) * split_stage_bytes(NS, NT, LO) + 8 * t * split_row_bytes(NS, LO) + split_scalars(NS, LO);
+    return ((lane >> 2) & 1) * split_stage_bytes(NT, LO) + 8 * t * split_row_bytes(LO) + split_scalars(LO);
 }
 // Tiles whose group has another scale than the step's largest (byte `shift` of the words), times the ratio; `least`: the smallest
 // exponent of the ratio (0: it may vanish; groups without a scale hold zeros only).
@@ -630,7 +596,7 @@ __device__ __forceinline__ uint32_t ldsu32(uint32_t addr) {
 // Launch geometry, shared memory (`extra` bytes of the sweep's own) and the tensor map of a sweep.
 inline int split_prepare(const Geo& g, float scale, int dist, const float* packed, Launch* L, SplitArgs* a, size_t extra = 0) {
     const bool lo = !g.bf16;
-    const int ns = slabs_of(g), nt = split_tiles(g), rb = split_row_bytes(ns, lo), rf = rb / 4, hp = split_hp(g);
+    const int nt = split_tiles(g), rb = split_row_bytes(lo), rf = rb / 4, hp = split_hp(g);
     a->g = g;
     a->scale = scale;
     a->dist = dist;
@@ -639,7 +605,7 @@ inline int split_prepare(const Geo& g, float scale, int dist, const float* packe
     a->wait_tries = kWaitTries;
     L->grid = dim3((unsigned)((g.W + 1) / 2), (unsigned)((g.H + 8 * kSplitWarps - 1) / (8 * kSplitWarps)), (unsigned)g.units);
     L->threads = 32 * kSplitWarps;
-    L->smem = (size_t)2 * kSplitSteps * split_stage_bytes(ns, nt, lo) + 128 + extra;
+    L->smem = (size_t)2 * kSplitSteps * split_stage_bytes(nt, lo) + 128 + extra;
     if (L->smem > kMaxDynamicSmem || L->grid.y > 65535u) return CA_ERR_UNSUPPORTED;
     const uint64_t dims[4] = {(uint64_t)rf, (uint64_t)hp, (uint64_t)g.Wk, (uint64_t)g.units};
     const uint64_t strides[3] = {(uint64_t)rb, (uint64_t)hp * rb, (uint64_t)hp * rb * g.Wk};

@@ -11,10 +11,9 @@ namespace {
 constexpr float kWeightExp = 14.f;
 
 // Biased exponent of the reciprocal of a bound of |dP| + |D|: `norm` above the centre vector's norm, `e` the exponent of the streamed
-// group's scale, whose vectors have norms up to sqrt(16 NS) 2^15, `d` above |D|.
-template <int NS>
+// group's scale, whose vectors have norms up to sqrt(16) 2^15, `d` above |D|.
 __device__ __forceinline__ int bound_inverse(int norm, int e, int d) {
-    const int x = max(norm + e - 127 + 17 + (NS > 1) , d) + 1;
+    const int x = max(norm + e - 127 + 17, d) + 1;
     return min(max(254 - x, 1), 250);
 }
 
@@ -22,7 +21,7 @@ __device__ __forceinline__ int bound_inverse(int norm, int e, int d) {
 __device__ __noinline__ void exact_dq(const SplitArgs& a, int u, int h, int w) {
     const Geo& g = a.g;
     const int j = h + g.H * w;
-    float q[64], dy[64], acc[64];
+    float q[16], dy[16], acc[16];
     for (int c = 0; c < g.cr; ++c) {
         q[c] = ld_channel(a.c0, g, u, c, g.Np, j);
         dy[c] = ld_channel(a.c1, g, u, c, g.Np, j);
@@ -49,7 +48,7 @@ __device__ __noinline__ void exact_dq(const SplitArgs& a, int u, int h, int w) {
 __device__ __noinline__ void exact_dkdv(const SplitArgs& a, int u, int h, int w) {
     const Geo& g = a.g;
     const int i = h + g.H * w;
-    float k[64], v[64], dk[64], dv[64];
+    float k[16], v[16], dk[16], dv[16];
     for (int c = 0; c < g.cr; ++c) {
         k[c] = ld_channel(a.c0, g, u, c, g.Np, i);
         v[c] = ld_channel(a.c1, g, u, c, g.Np, i);
@@ -81,14 +80,14 @@ __device__ __noinline__ void exact_dkdv(const SplitArgs& a, int u, int h, int w)
 }
 
 // What the two sweeps share: the tiles of a column against two centre operands.
-template <int NS, int NT, bool LO>
+template <int NT, bool LO>
 struct BwdSweep {
-    static constexpr int RB = split_row_bytes(NS, LO), SB = split_stage_bytes(NS, NT, LO);
+    static constexpr int RB = split_row_bytes(LO), SB = split_stage_bytes(NT, LO);
     const SplitArgs& a;
     int lane, tq, h, u;
     uint32_t dot_off, outer_off, tail_off, word_off;
     float sl2;
-    Centre<NS, LO> c0, c1;
+    Centre<LO> c0, c1;
     uint32_t cur, word;                                      // the scales of the step's groups when they are all alike; this lane's
     bool bad, mixed;
 
@@ -99,13 +98,13 @@ struct BwdSweep {
         h = row0 + (lane >> 2);
         u = blockIdx.z;
         sl2 = a.scale * kLog2e;
-        dot_off = dot_offset(lane, NS, LO);
-        outer_off = outer_offset(lane, NS, LO, 8 * RB);
-        tail_off = outer_offset(lane, NS, LO, SB);
-        word_off = word_offset<NS, NT, LO>(a.g, lane, row0);
+        dot_off = dot_offset(lane, LO);
+        outer_off = outer_offset(lane, LO, 8 * RB);
+        tail_off = outer_offset(lane, LO, SB);
+        word_off = word_offset<NT, LO>(a.g, lane, row0);
     }
     __device__ __forceinline__ void load(int w0) {
-        Raw<NS> r0, r1;
+        Raw r0, r1;
         r0.load(a.c0, a.g, u, h, w0, tq);
         r1.load(a.c1, a.g, u, h, w0, tq);
         c0.form(r0, a.g, h, w0, tq, kLeastExp);
@@ -129,12 +128,12 @@ struct BwdSweep {
     }
 };
 
-template <int NS, int NT, bool DIST, bool LO>
-struct DqSweep : BwdSweep<NS, NT, LO> {
-    using B = BwdSweep<NS, NT, LO>;
+template <int NT, bool DIST, bool LO>
+struct DqSweep : BwdSweep<NT, LO> {
+    using B = BwdSweep<NT, LO>;
     using B::a; using B::lane; using B::tq; using B::h; using B::u; using B::c0; using B::c1; using B::cur; using B::word; using B::bad; using B::mixed;
     using B::RB; using B::SB;
-    pair_t acc[NS][2][2], sum[2], nref[NT][2], c[2], e[2], nd[2], S[2], Sd[2];     // Sd: Distance, the sums of dS
+    pair_t acc[2][2], sum[2], nref[NT][2], c[2], e[2], nd[2], S[2], Sd[2];     // Sd: Distance, the sums of dS
     float D[2];
     Tail tail;
 
@@ -162,22 +161,20 @@ struct DqSweep : BwdSweep<NS, NT, LO> {
             sum[r] = c[r] = e[r] = nd[r] = S[r] = Sd[r] = 0;
         }
 #pragma unroll
-        for (int s = 0; s < NS; ++s)
-#pragma unroll
-            for (int n = 0; n < 2; ++n) acc[s][n][0] = acc[s][n][1] = 0;
+        for (int n = 0; n < 2; ++n) acc[n][0] = acc[n][1] = 0;
     }
 
     template <int HALF>
     __device__ __forceinline__ void column(uint32_t rb, bool first, bool last) {
         float x[NT][4], y[NT][4];
-        dot_column<NS, NT, LO>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
+        dot_column<NT, LO>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
         if (mixed) {
             scale_tiles<NT>(x, word, cur, 0, 1, HALF);
             scale_tiles<NT>(y, word, cur, 8, 0, HALF);
         }
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-            const pair_t b = DIST ? lds_pair(rb + HALF * SB + (8 * t + 2 * tq) * RB + split_scalars(NS, LO) + 8) : 0;
+            const pair_t b = DIST ? lds_pair(rb + HALF * SB + (8 * t + 2 * tq) * RB + split_scalars(LO) + 8) : 0;
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const float2 z = unpair(fma_pair(pair(x[t][2 * r], x[t][2 * r + 1]), c[r], DIST ? add_pair(nref[t][r], b) : nref[t][r]));
@@ -205,7 +202,7 @@ struct DqSweep : BwdSweep<NS, NT, LO> {
         for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int r = 0; r < 2; ++r) split2(x[t][2 * r], x[t][2 * r + 1], hi[t][r], lo[t][r]);
-        outer_column<NS, NT, LO, HALF>(hi, lo, tail, rb + HALF * SB + B::outer_off, rb + B::tail_off, S, acc);
+        outer_column<NT, LO, HALF>(hi, lo, tail, rb + HALF * SB + B::outer_off, rb + B::tail_off, S, acc);
     }
 
     __device__ __forceinline__ void step(uint32_t rb, bool first, bool last) {
@@ -218,7 +215,7 @@ struct DqSweep : BwdSweep<NS, NT, LO> {
             mixed = __any_sync(0xffffffffu, word != cur);
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-                const int nb = bound_inverse<NS>(c1.top[r], ev, above(D[r]));
+                const int nb = bound_inverse(c1.top[r], ev, above(D[r]));
                 const float nrm = exp_scale(nb), bd = exp_scale(254 - nb) * 0x1p-14f, back = exp_scale(ek) * bd;
                 c[r] = pair(c0.scale[r] * exp_scale(ek), c0.scale[r] * exp_scale(ek));
                 e[r] = pair(c1.scale[r] * nrm * exp_scale(ev), c1.scale[r] * nrm * exp_scale(ev));
@@ -237,7 +234,7 @@ struct DqSweep : BwdSweep<NS, NT, LO> {
             if (tq < 2 && h < g.H && w0 + tq < g.W) exact_dq(a, u, h, w0 + tq);
             return;
         }
-        Raw<NS> raw = {};
+        Raw raw = {};
         if (DIST) raw.load(a.c0, g, u, h, w0, tq);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -249,23 +246,20 @@ struct DqSweep : BwdSweep<NS, NT, LO> {
                 ds = quad_sum(z.x + z.y);
             }
             if (!ok) continue;
-            const float (&qv)[NS][4] = raw.x[r];
-#pragma unroll
-            for (int s = 0; s < NS; ++s) {
-                const float2 y0 = unpair(acc[s][0][r]), y1 = unpair(acc[s][1][r]);
-                store_pixel(a.o0, g, u, s, pix, tq, a.scale * (y0.x - ds * qv[s][0]) + poison, a.scale * (y0.y - ds * qv[s][1]) + poison,
-                            a.scale * (y1.x - ds * qv[s][2]) + poison, a.scale * (y1.y - ds * qv[s][3]) + poison);
-            }
+            const float (&qv)[4] = raw.x[r];
+            const float2 y0 = unpair(acc[0][r]), y1 = unpair(acc[1][r]);
+            store_pixel(a.o0, g, u, pix, tq, a.scale * (y0.x - ds * qv[0]) + poison, a.scale * (y0.y - ds * qv[1]) + poison,
+                        a.scale * (y1.x - ds * qv[2]) + poison, a.scale * (y1.y - ds * qv[3]) + poison);
         }
     }
 };
 
-template <int NS, int NT, bool DIST, bool LO>
-struct DkdvSweep : BwdSweep<NS, NT, LO> {
-    using B = BwdSweep<NS, NT, LO>;
+template <int NT, bool DIST, bool LO>
+struct DkdvSweep : BwdSweep<NT, LO> {
+    using B = BwdSweep<NT, LO>;
     using B::a; using B::lane; using B::tq; using B::h; using B::u; using B::c0; using B::c1; using B::cur; using B::word; using B::bad; using B::mixed;
     using B::RB; using B::SB;
-    pair_t dk[NS][2][2], dv[NS][2][2], sum[2], mk[NT], bk[2], c[2], e[2], nrm, Sk[2], Sv[2], Sd;      // Sd: Distance, the sums of dS
+    pair_t dk[2][2], dv[2][2], sum[2], mk[NT], bk[2], c[2], e[2], nrm, Sk[2], Sv[2], Sd;      // Sd: Distance, the sums of dS
     int norm;
     uint32_t most;                                           // exponent above the |D| met so far
     Tail tp, td;
@@ -287,20 +281,18 @@ struct DkdvSweep : BwdSweep<NS, NT, LO> {
             sum[r] = c[r] = e[r] = Sk[r] = Sv[r] = 0;
         }
 #pragma unroll
-        for (int s = 0; s < NS; ++s)
-#pragma unroll
-            for (int n = 0; n < 2; ++n) dk[s][n][0] = dk[s][n][1] = dv[s][n][0] = dv[s][n][1] = 0;
+        for (int n = 0; n < 2; ++n) dk[n][0] = dk[n][1] = dv[n][0] = dv[n][1] = 0;
     }
 
     template <int HALF>
     __device__ __forceinline__ void column(uint32_t rb, bool first, bool last) {
         float x[NT][4], y[NT][4];
-        dot_column<NS, NT, LO>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
+        dot_column<NT, LO>(c0, c1, rb + HALF * SB + B::dot_off, x, y);
         if (mixed) {
             scale_tiles<NT>(x, word, cur, 0, 1, HALF);
             scale_tiles<NT>(y, word, cur, 8, 0, HALF);
         }
-        const uint32_t sc = rb + HALF * SB + 2 * tq * RB + split_scalars(NS, LO) + 8;
+        const uint32_t sc = rb + HALF * SB + 2 * tq * RB + split_scalars(LO) + 8;
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
             const pair_t A = add_pair(mk[t], lds_pair(sc + 8 * t * RB)), Dn = mul_pair(lds_pair(sc + (8 * t + 1) * RB), nrm);
@@ -337,12 +329,12 @@ struct DkdvSweep : BwdSweep<NS, NT, LO> {
         for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int r = 0; r < 2; ++r) split2(x[t][2 * r], x[t][2 * r + 1], hi[t][r], lo[t][r]);
-        outer_column<NS, NT, LO, HALF>(hi, lo, tp, rb + HALF * SB + B::outer_off + split_second(NS, LO), rb + B::tail_off + split_second(NS, LO), Sv, dv);
+        outer_column<NT, LO, HALF>(hi, lo, tp, rb + HALF * SB + B::outer_off + split_second(LO), rb + B::tail_off + split_second(LO), Sv, dv);
 #pragma unroll
         for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int r = 0; r < 2; ++r) split2(y[t][2 * r], y[t][2 * r + 1], hi[t][r], lo[t][r]);
-        outer_column<NS, NT, LO, HALF>(hi, lo, td, rb + HALF * SB + B::outer_off, rb + B::tail_off, Sk, dk);
+        outer_column<NT, LO, HALF>(hi, lo, td, rb + HALF * SB + B::outer_off, rb + B::tail_off, Sk, dk);
     }
 
     __device__ __forceinline__ void step(uint32_t rb, bool first, bool last) {
@@ -356,7 +348,7 @@ struct DkdvSweep : BwdSweep<NS, NT, LO> {
             most = max(most, __reduce_max_sync(0xffffffffu, top));
             cur = eq | ed << 8;
             mixed = __any_sync(0xffffffffu, word != cur);
-            const int nb = bound_inverse<NS>(norm, ed, most);
+            const int nb = bound_inverse(norm, ed, most);
             const float n = exp_scale(nb), bv = exp_scale(ed) * 0x1p-14f, bd = exp_scale(254 - nb) * 0x1p-14f, back = exp_scale(eq) * bd;
             nrm = pair(n, n);
             Sd = pair(bd, bd);
@@ -378,7 +370,7 @@ struct DkdvSweep : BwdSweep<NS, NT, LO> {
             if (tq < 2 && h < g.H && w0 + tq < g.W) exact_dkdv(a, u, h, w0 + tq);
             return;
         }
-        Raw<NS> raw = {};
+        Raw raw = {};
         if (DIST) raw.load(a.c0, g, u, h, w0, tq);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -390,67 +382,59 @@ struct DkdvSweep : BwdSweep<NS, NT, LO> {
                 ds = quad_sum(z.x + z.y);
             }
             if (!ok) continue;
-            const float (&kv)[NS][4] = raw.x[r];
-#pragma unroll
-            for (int s = 0; s < NS; ++s) {
-                const float2 k0 = unpair(dk[s][0][r]), k1 = unpair(dk[s][1][r]), v0 = unpair(dv[s][0][r]), v1 = unpair(dv[s][1][r]);
-                store_pixel(a.o0, g, u, s, pix, tq, a.scale * (k0.x - ds * kv[s][0]) + poison, a.scale * (k0.y - ds * kv[s][1]) + poison,
-                            a.scale * (k1.x - ds * kv[s][2]) + poison, a.scale * (k1.y - ds * kv[s][3]) + poison);
-                store_pixel(a.o1, g, u, s, pix, tq, v0.x + poison, v0.y + poison, v1.x + poison, v1.y + poison);
-            }
+            const float (&kv)[4] = raw.x[r];
+            const float2 k0 = unpair(dk[0][r]), k1 = unpair(dk[1][r]), v0 = unpair(dv[0][r]), v1 = unpair(dv[1][r]);
+            store_pixel(a.o0, g, u, pix, tq, a.scale * (k0.x - ds * kv[0]) + poison, a.scale * (k0.y - ds * kv[1]) + poison,
+                        a.scale * (k1.x - ds * kv[2]) + poison, a.scale * (k1.y - ds * kv[3]) + poison);
+            store_pixel(a.o1, g, u, pix, tq, v0.x + poison, v0.y + poison, v1.x + poison, v1.y + poison);
         }
     }
 };
 
 // Without lower halves one more block per SM pays for 4 to 128 bytes of spills (forward and backward, 1024 x 1024, 8 units, ws 21, with the same in
 // the forward and dk/dv and rows of 80 bytes: 14812 -> 13340 us, Distance 15857 -> 14770).
-template <int NS, int NT, bool DIST, bool LO>
+template <int NT, bool DIST, bool LO>
 __global__ void __launch_bounds__(32 * kSplitWarps, LO ? 4 : 5) split_dq_kernel(const __grid_constant__ SplitArgs a,
                                                                                            const __grid_constant__ CUtensorMap map) {
-    DqSweep<NS, NT, DIST, LO> sweep(a);
-    split_run<NS, NT, LO>(a, &map, sweep);
+    DqSweep<NT, DIST, LO> sweep(a);
+    split_run<NT, LO>(a, &map, sweep);
 }
-template <int NS, int NT, bool DIST, bool LO>
+template <int NT, bool DIST, bool LO>
 __global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 || !LO ? 4 : 3) split_dkdv_kernel(const __grid_constant__ SplitArgs a,
                                                                                              const __grid_constant__ CUtensorMap map) {
-    DkdvSweep<NS, NT, DIST, LO> sweep(a);
-    split_run<NS, NT, LO>(a, &map, sweep);
+    DkdvSweep<NT, DIST, LO> sweep(a);
+    split_run<NT, LO>(a, &map, sweep);
 }
 
 }  // namespace
 
-#define CA_SPLIT_BWD(KERNEL, NSV, NTV)                                                               \
+#define CA_SPLIT_BWD(KERNEL, NTV)                                                               \
     do {                                                                                             \
         if (g.bf16) {                                                                                \
-            if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true, false>), a, L, st);                    \
-            else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false, false>), a, L, st);                        \
+            if (dist) CA_LAUNCH_SPLIT((KERNEL<NTV, true, false>), a, L, st);                    \
+            else CA_LAUNCH_SPLIT((KERNEL<NTV, false, false>), a, L, st);                        \
         } else {                                                                                     \
-            if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true, true>), a, L, st);                     \
-            else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false, true>), a, L, st);                         \
+            if (dist) CA_LAUNCH_SPLIT((KERNEL<NTV, true, true>), a, L, st);                     \
+            else CA_LAUNCH_SPLIT((KERNEL<NTV, false, true>), a, L, st);                         \
         }                                                                                            \
     } while (0)
-#define CA_SPLIT_BWD_NT(KERNEL, NSV)                                                                 \
+#define CA_SPLIT_BWD_NT(KERNEL)                                                                 \
     do {                                                                                             \
-        if (nt == 2) CA_SPLIT_BWD(KERNEL, NSV, 2);                                                   \
-        else if (nt == 3) CA_SPLIT_BWD(KERNEL, NSV, 3);                                              \
-        else if (nt == 4) CA_SPLIT_BWD(KERNEL, NSV, 4);                                              \
+        if (nt == 2) CA_SPLIT_BWD(KERNEL, 2);                                                   \
+        else if (nt == 3) CA_SPLIT_BWD(KERNEL, 3);                                              \
+        else if (nt == 4) CA_SPLIT_BWD(KERNEL, 4);                                              \
         else return CA_ERR_UNSUPPORTED;                                                              \
-    } while (0)
-#define CA_SPLIT_BWD_NS(KERNEL)                                                                      \
-    do {                                                                                             \
-        if (ns != 1) return CA_ERR_UNSUPPORTED;                                                      \
-        CA_SPLIT_BWD_NT(KERNEL, 1);                                                                  \
     } while (0)
 
 int run_split_dq(const Geo& g, float scale, int dist, const float* q, const float* k, const float* v, const float* dy, const float* stats,
                  const float* D, const float* kv, float* dq, cudaStream_t st) {
     Launch L{};
     SplitArgs a{};
-    const int ns = slabs_of(g), nt = split_tiles(g);
+    const int nt = split_tiles(g);
     const int rc = split_prepare(g, scale, dist, kv, &L, &a);
     if (rc) return rc;
     a.c0 = q; a.c1 = dy; a.stats = stats; a.D = D; a.o0 = dq; a.x0 = k; a.x1 = v;
-    CA_SPLIT_BWD_NS(split_dq_kernel);
+    CA_SPLIT_BWD_NT(split_dq_kernel);
     CA_CHECK_LAUNCH("split dq kernel");
     return CA_OK;
 }
@@ -459,11 +443,11 @@ int run_split_dkdv(const Geo& g, float scale, int dist, const float* q, const fl
                    const float* D, const float* qdy, float* dk, float* dv, cudaStream_t st) {
     Launch L{};
     SplitArgs a{};
-    const int ns = slabs_of(g), nt = split_tiles(g);
+    const int nt = split_tiles(g);
     const int rc = split_prepare(g, scale, dist, qdy, &L, &a);
     if (rc) return rc;
     a.c0 = k; a.c1 = v; a.o0 = dk; a.o1 = dv; a.x0 = q; a.x1 = dy; a.xstats = stats; a.xD = D;
-    CA_SPLIT_BWD_NS(split_dkdv_kernel);
+    CA_SPLIT_BWD_NT(split_dkdv_kernel);
     CA_CHECK_LAUNCH("split dk/dv kernel");
     return CA_OK;
 }

@@ -13,7 +13,7 @@ __device__ __noinline__ void exact_fwd(const SplitArgs& a, int u, int h, int w) 
     const Geo& g = a.g;
     const float sl2 = a.scale * kLog2e;
     const int j = h + g.H * w;
-    float q[64], acc[64];
+    float q[16], acc[16];
     for (int c = 0; c < g.cr; ++c) {
         q[c] = ld_channel(a.c0, g, u, c, g.Np, j);
         acc[c] = 0.f;
@@ -60,15 +60,15 @@ __device__ __noinline__ void exact_values(const SplitArgs& a, int u, int h, int 
 }
 
 // A warp's eight rows of two columns; a step scores them against two columns of the window.
-template <int NS, int NT, bool DIST, bool LO>
+template <int NT, bool DIST, bool LO>
 struct FwdSweep {
-    static constexpr int RB = split_row_bytes(NS, LO), SB = split_stage_bytes(NS, NT, LO), T = 2 * NT;
+    static constexpr int RB = split_row_bytes(LO), SB = split_stage_bytes(NT, LO), T = 2 * NT;
     const SplitArgs& a;
     int lane, tq, h, u;
     uint32_t dot_off, outer_off, tail_off, word_off;
     float sl2;
-    Centre<NS, LO> q;
-    pair_t acc[NS][2][2], l[2], nref[NT][2], c[2], S[2];
+    Centre<LO> q;
+    pair_t acc[2][2], l[2], nref[NT][2], c[2], S[2];
     float shift[2];                                          // what the references have moved by
     uint32_t cur;                                            // the scales of the step's groups when they are all alike, as they mostly are
     bool bad;
@@ -80,15 +80,15 @@ struct FwdSweep {
         h = row0 + (lane >> 2);
         u = blockIdx.z;
         sl2 = a.scale * kLog2e;
-        dot_off = dot_offset(lane, NS, LO);
-        outer_off = outer_offset(lane, NS, LO, 8 * RB) + split_second(NS, LO);
-        tail_off = outer_offset(lane, NS, LO, SB) + split_second(NS, LO);
-        word_off = word_offset<NS, NT, LO>(a.g, lane, row0);
+        dot_off = dot_offset(lane, LO);
+        outer_off = outer_offset(lane, LO, 8 * RB) + split_second(LO);
+        tail_off = outer_offset(lane, LO, SB) + split_second(LO);
+        word_off = word_offset<NT, LO>(a.g, lane, row0);
     }
 
     __device__ __forceinline__ void begin(int w0, uint32_t) {
         const Geo& g = a.g;
-        Raw<NS> raw;
+        Raw raw;
         raw.load(a.c0, g, u, h, w0, tq);
         q.form(raw, g, h, w0, tq, kLeastExp);
         bad = q.bad;
@@ -103,9 +103,7 @@ struct FwdSweep {
             q.scale[r] = fmaxf(q.scale[r] * sl2, 0x1p-70f);
         }
 #pragma unroll
-        for (int s = 0; s < NS; ++s)
-#pragma unroll
-            for (int n = 0; n < 2; ++n) acc[s][n][0] = acc[s][n][1] = 0;
+        for (int n = 0; n < 2; ++n) acc[n][0] = acc[n][1] = 0;
     }
 
     __device__ __forceinline__ void step(uint32_t rb, bool first, bool last) {
@@ -122,12 +120,12 @@ struct FwdSweep {
             for (int r = 0; r < 2; ++r) c[r] = pair(q.scale[r] * exp_scale(ek), q.scale[r] * exp_scale(ek));
         }
         float x[T][4];
-        dot_tiles<NS, NT, LO>(q, rb + dot_off, x);
+        dot_tiles<NT, LO>(q, rb + dot_off, x);
         if (mixed) scale_tiles<NT>(x, word, cur, 0, 1);
         float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-            const pair_t b = DIST ? lds_pair(rb + tile_offset<NS, NT, LO>(t) + 2 * tq * RB + split_scalars(NS, LO) + 8) : 0;
+            const pair_t b = DIST ? lds_pair(rb + tile_offset<NT, LO>(t) + 2 * tq * RB + split_scalars(LO) + 8) : 0;
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const float2 y = unpair(fma_pair(pair(x[t][2 * r], x[t][2 * r + 1]), c[r], DIST ? add_pair(nref[t % NT][r], b) : nref[t % NT][r]));
@@ -159,7 +157,7 @@ struct FwdSweep {
                     shift[r] += d;
                     l[r] = mul_pair(l[r], cc);
 #pragma unroll
-                    for (int i = 0; i < 2 * NS; ++i) acc[i >> 1][i & 1][r] = mul_pair(acc[i >> 1][i & 1][r], cc);
+                    for (int n = 0; n < 2; ++n) acc[n][r] = mul_pair(acc[n][r], cc);
 #pragma unroll
                     for (int t = 0; t < T; ++t) {
                         x[t][2 * r] += d;
@@ -183,7 +181,7 @@ struct FwdSweep {
             split2(x[t][0], x[t][1], hi[t][0], lo[t][0]);
             split2(x[t][2], x[t][3], hi[t][1], lo[t][1]);
         }
-        outer_tiles<NS, NT, LO>(hi, lo, rb + outer_off, rb + tail_off, S, acc);
+        outer_tiles<NT, LO>(hi, lo, rb + outer_off, rb + tail_off, S, acc);
     }
     __device__ __forceinline__ void end(int w0, float poison) {
         const Geo& g = a.g;
@@ -198,34 +196,31 @@ struct FwdSweep {
             if (h >= g.H || w0 + r >= g.W) continue;
             const float inv = 1.f / sum + poison;
             const int pix = h + g.H * (w0 + r);
-#pragma unroll
-            for (int s = 0; s < NS; ++s) {
-                const float2 y0 = unpair(acc[s][0][r]), y1 = unpair(acc[s][1][r]);
-                store_pixel(a.o0, g, u, s, pix, tq, y0.x * inv, y0.y * inv, y1.x * inv, y1.y * inv);
-            }
+            const float2 y0 = unpair(acc[0][r]), y1 = unpair(acc[1][r]);
+            store_pixel(a.o0, g, u, pix, tq, y0.x * inv, y0.y * inv, y1.x * inv, y1.y * inv);
             if (a.ostats && tq == 0) a.ostats[(int64_t)u * g.Np + pix] = (log2f(sum) - shift[r]) * kLn2 + poison;
         }
     }
 };
 
 // Five blocks per SM where the registers suffice: two tiles a column, or no lower halves (8 to 40 bytes spilled at three and four tiles).
-template <int NS, int NT, bool DIST, bool LO>
+template <int NT, bool DIST, bool LO>
 __global__ void __launch_bounds__(32 * kSplitWarps, NT == 2 || !LO ? 5 : 4) split_fwd_kernel(const __grid_constant__ SplitArgs a, const __grid_constant__ CUtensorMap map) {
-    FwdSweep<NS, NT, DIST, LO> sweep(a);
-    split_run<NS, NT, LO>(a, &map, sweep);
+    FwdSweep<NT, DIST, LO> sweep(a);
+    split_run<NT, LO>(a, &map, sweep);
 }
 
 // A's values: the scores once more, weighed with the row's log-sum-exp.  The runs of a step's two window columns are put in order in
 // shared memory and leave row by row, 8 ws bytes that are contiguous but for the wrap: stored from the accumulators they
 // were 4-byte pieces 8 bytes apart (128 x 96, 8 units, ws 15: 75 us).
-template <int NS, int NT, bool DIST, bool LO>
+template <int NT, bool DIST, bool LO>
 struct EmitSweep {
-    static constexpr int RB = split_row_bytes(NS, LO), SB = split_stage_bytes(NS, NT, LO), T = 2 * NT;
+    static constexpr int RB = split_row_bytes(LO), SB = split_stage_bytes(NT, LO), T = 2 * NT;
     const SplitArgs& a;
     int lane, tq, h, u, w, s, rows;                          // s: the next column of the window; rows of the warp in the image
     uint32_t dot_off, word_off, buf;
     float sl2;
-    Centre<NS, LO> q;
+    Centre<LO> q;
     pair_t nref[2], c[2];
     int at[NT][2];                                           // shared address of a tile's element for the first row and window column, -1: outside
     uint32_t cur;
@@ -238,8 +233,8 @@ struct EmitSweep {
         h = row0 + (lane >> 2);
         u = blockIdx.z;
         sl2 = a.scale * kLog2e;
-        dot_off = dot_offset(lane, NS, LO);
-        word_off = word_offset<NS, NT, LO>(a.g, lane, row0);
+        dot_off = dot_offset(lane, LO);
+        word_off = word_offset<NT, LO>(a.g, lane, row0);
     }
 
     __device__ __forceinline__ void begin(int w0, uint32_t own) {
@@ -249,7 +244,7 @@ struct EmitSweep {
         buf = own + (threadIdx.x >> 5) * (16 * 2 * g.ws * 4);
         rows = min(8, g.H - (h - (lane >> 2)));
         cur = 0;
-        Raw<NS> raw;
+        Raw raw;
         float L[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) L[r] = __ldg(a.stats + (int64_t)u * g.Np + min(h, g.H - 1) + g.H * min(w0 + r, g.W - 1));
@@ -285,14 +280,14 @@ struct EmitSweep {
             for (int r = 0; r < 2; ++r) c[r] = pair(q.scale[r] * exp_scale(cur), q.scale[r] * exp_scale(cur));
         }
         float x[T][4];
-        dot_tiles<NS, NT, LO>(q, rb + dot_off, x);
+        dot_tiles<NT, LO>(q, rb + dot_off, x);
         if (mixed) scale_tiles<NT>(x, word, cur, 0, 1);
         __syncwarp();
 #pragma unroll
         for (int half = 0; half < 2; ++half)
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-                const pair_t b = DIST ? lds_pair(rb + half * SB + (8 * t + 2 * tq) * RB + split_scalars(NS, LO) + 8) : 0;
+                const pair_t b = DIST ? lds_pair(rb + half * SB + (8 * t + 2 * tq) * RB + split_scalars(LO) + 8) : 0;
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     const float2 y = unpair(fma_pair(pair(x[half * NT + t][2 * r], x[half * NT + t][2 * r + 1]), c[r],
@@ -334,10 +329,10 @@ struct EmitSweep {
     }
 };
 
-template <int NS, int NT, bool DIST, bool LO>
+template <int NT, bool DIST, bool LO>
 __global__ void __launch_bounds__(32 * kSplitWarps, 4) split_emit_kernel(const __grid_constant__ SplitArgs a, const __grid_constant__ CUtensorMap map) {
-    EmitSweep<NS, NT, DIST, LO> sweep(a);
-    split_run<NS, NT, LO>(a, &map, sweep);
+    EmitSweep<NT, DIST, LO> sweep(a);
+    split_run<NT, LO>(a, &map, sweep);
 }
 
 }  // namespace
@@ -346,29 +341,28 @@ int run_split_fwd(const Geo& g, float scale, int dist, const float* q, const flo
                   cudaStream_t st) {
     Launch L{};
     SplitArgs a{};
-    const int ns = slabs_of(g), nt = split_tiles(g);
+    const int nt = split_tiles(g);
     const int rc = split_prepare(g, scale, dist, kv, &L, &a);
     if (rc) return rc;
     a.c0 = q; a.o0 = y; a.ostats = stats; a.x0 = k; a.x1 = v;
-#define CA_SPLIT_FWD(KERNEL, NSV, NTV)                                                               \
+#define CA_SPLIT_FWD(KERNEL, NTV)                                                               \
     do {                                                                                             \
         if (g.bf16) {                                                                                \
-            if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true, false>), a, L, st);                    \
-            else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false, false>), a, L, st);                        \
+            if (dist) CA_LAUNCH_SPLIT((KERNEL<NTV, true, false>), a, L, st);                    \
+            else CA_LAUNCH_SPLIT((KERNEL<NTV, false, false>), a, L, st);                        \
         } else {                                                                                     \
-            if (dist) CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, true, true>), a, L, st);                     \
-            else CA_LAUNCH_SPLIT((KERNEL<NSV, NTV, false, true>), a, L, st);                         \
+            if (dist) CA_LAUNCH_SPLIT((KERNEL<NTV, true, true>), a, L, st);                     \
+            else CA_LAUNCH_SPLIT((KERNEL<NTV, false, true>), a, L, st);                         \
         }                                                                                            \
     } while (0)
-#define CA_SPLIT_FWD_NT(KERNEL, NSV)                                                                 \
+#define CA_SPLIT_FWD_NT(KERNEL)                                                                 \
     do {                                                                                             \
-        if (nt == 2) CA_SPLIT_FWD(KERNEL, NSV, 2);                                                   \
-        else if (nt == 3) CA_SPLIT_FWD(KERNEL, NSV, 3);                                              \
-        else if (nt == 4) CA_SPLIT_FWD(KERNEL, NSV, 4);                                              \
+        if (nt == 2) CA_SPLIT_FWD(KERNEL, 2);                                                   \
+        else if (nt == 3) CA_SPLIT_FWD(KERNEL, 3);                                              \
+        else if (nt == 4) CA_SPLIT_FWD(KERNEL, 4);                                              \
         else return CA_ERR_UNSUPPORTED;                                                              \
     } while (0)
-    if (ns != 1) return CA_ERR_UNSUPPORTED;
-    CA_SPLIT_FWD_NT(split_fwd_kernel, 1);
+    CA_SPLIT_FWD_NT(split_fwd_kernel);
     CA_CHECK_LAUNCH("split forward kernel");
     return CA_OK;
 }
@@ -377,12 +371,11 @@ int run_split_emit(const Geo& g, float scale, int dist, const float* q, const fl
                    cudaStream_t st) {
     Launch L{};
     SplitArgs a{};
-    const int ns = slabs_of(g), nt = split_tiles(g);
+    const int nt = split_tiles(g);
     const int rc = split_prepare(g, scale, dist, kv, &L, &a, kSplitWarps * 16 * 2 * g.ws * sizeof(float));
     if (rc) return rc;
     a.c0 = q; a.stats = stats; a.o0 = nz; a.x0 = k;
-    if (ns != 1) return CA_ERR_UNSUPPORTED;
-    CA_SPLIT_FWD_NT(split_emit_kernel, 1);
+    CA_SPLIT_FWD_NT(split_emit_kernel);
     CA_CHECK_LAUNCH("split values kernel");
     return CA_OK;
 }

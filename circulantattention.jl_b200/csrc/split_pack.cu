@@ -5,20 +5,16 @@
 namespace ca {
 namespace {
 
-// A block gathers RB = 128 / NS packed rows of one column of one unit: thread (row, slab) reads 16 channels of both tensors
+// A block gathers 128 packed rows of one column of one unit: a thread reads the 16 channels of its row of both tensors
 // (consecutive lanes on consecutive rows: coalesced planar loads, all in flight together), the largest magnitude of each
-// group of eight rows comes from shuffles and, over the slabs, shared memory, and the block writes its rows as one
-// contiguous run of 16-byte stores.  Bound: HBM.
-template <int CPE, int NS, bool BF>
+// group of eight rows comes from shuffles, and the block writes its rows as one contiguous run of 16-byte stores.  Bound: HBM.
+template <int CPE, bool BF>
 __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
     constexpr bool LO = !BF;
-    constexpr int RB = 128 / NS, RF = split_row_bytes(NS, LO) / 4;
+    constexpr int RB = 128, RF = split_row_bytes(LO) / 4;
     __shared__ __align__(16) uint32_t tile[RB * RF];
-    __shared__ uint32_t gmax[2][NS][RB / 8];
-    __shared__ float sums[2][NS][RB];
     const Geo& g = a.g;
-    const int rl = threadIdx.x % RB, slab = threadIdx.x / RB;
-    const int rr0 = blockIdx.x * RB, rr = rr0 + rl, w = blockIdx.y, u = blockIdx.z;
+    const int rl = threadIdx.x, rr0 = blockIdx.x * RB, rr = rr0 + rl, w = blockIdx.y, u = blockIdx.z;
     const bool real_row = rr < g.H + 2 * g.p;
     const int pix = real_row ? (rr - g.p + g.H) % g.H + g.H * w : 0;
     float x[2][16];
@@ -30,7 +26,7 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
         for (int t = 0; t < 2; ++t)
 #pragma unroll
             for (int e = 0; e < 16; e += CPE) {
-                const int64_t o = goff<CPE>(u, g.cr, min(16 * slab + e, g.cr - CPE), g.Npk, pix);
+                const int64_t o = goff<CPE>(u, g.cr, min(e, g.cr - CPE), g.Npk, pix);
                 if (CPE == 2) {
                     const float2 z = __ldg(reinterpret_cast<const float2*>(src[t] + o));
                     x[t][e] = z.x;
@@ -43,12 +39,12 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
         for (int t = 0; t < 2; ++t)
 #pragma unroll
             for (int e = 0; e < 16; ++e)
-                if (!real_row || 16 * slab + e >= g.cr) x[t][e] = 0.f;
+                if (!real_row || e >= g.cr) x[t][e] = 0.f;
         if (a.y) {
             float yv[16];
 #pragma unroll
             for (int e = 0; e < 16; e += CPE) {
-                const int64_t o = goff<CPE>(u, g.cr, min(16 * slab + e, g.cr - CPE), g.Npk, pix);
+                const int64_t o = goff<CPE>(u, g.cr, min(e, g.cr - CPE), g.Npk, pix);
                 if (CPE == 2) {
                     const float2 z = __ldg(reinterpret_cast<const float2*>(a.y + o));
                     yv[e] = z.x;
@@ -59,7 +55,7 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
             }
 #pragma unroll
             for (int e = 0; e < 16; ++e)
-                if (16 * slab + e < g.cr) dot = fmaf(x[1][e], yv[e], dot);
+                if (e < g.cr) dot = fmaf(x[1][e], yv[e], dot);
             if (!real_row) dot = 0.f;
         }
     }
@@ -69,7 +65,9 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
         n2.x = fmaf(x[0][e], x[0][e], n2.x);
         n2.y = fmaf(x[0][e + 1], x[0][e + 1], n2.y);
     }
-    float norm = n2.x + n2.y;
+    const float norm = n2.x + n2.y;
+    uint32_t exps = 0;
+    uint32_t* row = tile + rl * RF;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         uint32_t m = 0;
@@ -77,60 +75,40 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
         for (int e = 0; e < 16; ++e) m = max(m, abs_bits(x[t][e]));
 #pragma unroll
         for (int d = 1; d < 8; d <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-        if ((rl & 7) == 0) gmax[t][slab][rl >> 3] = m;
-    }
-    sums[0][slab][rl] = norm;
-    sums[1][slab][rl] = dot;
-    __syncthreads();
-    uint32_t exps = 0;
-    uint32_t* row = tile + rl * RF;
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        uint32_t m = gmax[t][0][rl >> 3];
-#pragma unroll
-        for (int s = 1; s < NS; ++s) m = max(m, gmax[t][s][rl >> 3]);
         const int e = scale_exp(m, 4, t == 0 ? kLeastExp : 0);
         exps |= (uint32_t)e << (8 * t);
         const float inv = exp_inverse(e == 255 ? 0 : e);
         uint32_t hi[8], lo[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) split2(x[t][2 * i] * inv, x[t][2 * i + 1] * inv, hi[i], lo[i]);
-        uint4* d = reinterpret_cast<uint4*>(row + t * (split_second(NS, LO) / 4) + slab * 8);
+        uint4* d = reinterpret_cast<uint4*>(row + t * (split_second(LO) / 4));
         d[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         d[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
         if (LO) {
-            d += 2 * NS;
-            d[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-            d[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+            d[2] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            d[3] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
         }
     }
-    if (slab == 0) {
-#pragma unroll
-        for (int s = 1; s < NS; ++s) {
-            norm += sums[0][s][rl];
-            dot += sums[1][s][rl];
+    float A = a.norm_mul * norm;
+    if (a.stats) {
+        const int64_t so = (int64_t)u * g.Npk + pix;
+        if (real_row) {
+            A = fmaf(__ldg(a.stats + so), -kLog2e, A);
+            if (a.Din) dot = __ldg(a.Din + so);
+            else if (a.Dout && rr >= g.p && rr < g.p + g.H) a.Dout[so] = dot;
         }
-        float A = a.norm_mul * norm;
-        if (a.stats) {
-            const int64_t so = (int64_t)u * g.Npk + pix;
-            if (real_row) {
-                A = fmaf(__ldg(a.stats + so), -kLog2e, A);
-                if (a.Din) dot = __ldg(a.Din + so);
-                else if (a.Dout && rr >= g.p && rr < g.p + g.H) a.Dout[so] = dot;
-            }
-            uint32_t m = abs_bits(dot);
+        uint32_t m = abs_bits(dot);
 #pragma unroll
-            for (int d = 1; d < 8; d <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-            // a power of two above every |D| of the group; a statistic that is no number marks it, too
-            uint32_t bad = abs_bits(A) >= 0x7f800000u;
-            bad = __ballot_sync(0xffffffffu, bad) >> (rl & 24) & 255u;
-            const uint32_t e = bad || m >= 0x7e800000u ? 255u : (m >> 23) + (m ? 1u : 0u);
-            exps |= e << 16;
-        }
-        const float A1 = __shfl_xor_sync(0xffffffffu, A, 1), dot1 = __shfl_xor_sync(0xffffffffu, dot, 1);
-        const uint4 odd = make_uint4(exps, 0u, __float_as_uint(-dot1), __float_as_uint(-dot));
-        *reinterpret_cast<uint4*>(row + split_scalars(NS, LO) / 4) = rl & 1 ? odd : make_uint4(exps, 0u, __float_as_uint(A), __float_as_uint(A1));
+        for (int d = 1; d < 8; d <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+        // a power of two above every |D| of the group; a statistic that is no number marks it, too
+        uint32_t bad = abs_bits(A) >= 0x7f800000u;
+        bad = __ballot_sync(0xffffffffu, bad) >> (rl & 24) & 255u;
+        const uint32_t e = bad || m >= 0x7e800000u ? 255u : (m >> 23) + (m ? 1u : 0u);
+        exps |= e << 16;
     }
+    const float A1 = __shfl_xor_sync(0xffffffffu, A, 1), dot1 = __shfl_xor_sync(0xffffffffu, dot, 1);
+    const uint4 odd = make_uint4(exps, 0u, __float_as_uint(-dot1), __float_as_uint(-dot));
+    *reinterpret_cast<uint4*>(row + split_scalars(LO) / 4) = rl & 1 ? odd : make_uint4(exps, 0u, __float_as_uint(A), __float_as_uint(A1));
     __syncthreads();
     const int nrows = min(RB, a.Hp - rr0);
     uint4* out = reinterpret_cast<uint4*>(a.dst + (((int64_t)u * g.Wk + w) * a.Hp + rr0) * RF);
@@ -168,9 +146,9 @@ int launch_split_pack(const Geo& g, float scale, int dist, const float* x0, cons
     a.g = g; a.Hp = split_hp(g); a.x0 = x0; a.x1 = x1; a.stats = stats; a.y = y; a.Din = Din; a.Dout = Dout; a.dst = dst;
     a.norm_mul = dist ? -0.5f * scale * kLog2e : 0.f;
     const dim3 grid((a.Hp + 127) / 128, g.Wk, g.units);
-    if (g.bf16) split_pack_kernel<1, 1, true><<<grid, 128, 0, st>>>(a);
-    else if (g.cpe == 1) split_pack_kernel<1, 1, false><<<grid, 128, 0, st>>>(a);
-    else split_pack_kernel<2, 1, false><<<grid, 128, 0, st>>>(a);
+    if (g.bf16) split_pack_kernel<1, true><<<grid, 128, 0, st>>>(a);
+    else if (g.cpe == 1) split_pack_kernel<1, false><<<grid, 128, 0, st>>>(a);
+    else split_pack_kernel<2, false><<<grid, 128, 0, st>>>(a);
     CA_CHECK_LAUNCH("split pack kernel");
     return CA_OK;
 }
