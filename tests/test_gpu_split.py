@@ -83,6 +83,18 @@ def test_magnitudes(ca, what):
         assert_close(got[name], want[name], name, **bars)
 
 
+def test_gradients_of_few_channels_and_a_short_window(ca):
+    """Few terms leave the rounding of the weights itself: of s - L (up to 8: 2.4e-7 at most, ln 2 of that in the weight), of L
+    twice, of the exponential and of the split, 1e-7 rms each, and the cut sums.  A binade more in the exponent shows."""
+    rng = np.random.default_rng(67)
+    shape, ws, heads = (50, 64, 64, 1), 9, 8
+    t = [randn(rng, shape) for _ in range(4)]
+    got, want = run(ca, "dot", *t, ws, heads), oracle("dot", *t, ws, heads)
+    for name in ("dq", "dk", "dv"):
+        err = np.linalg.norm(got[name] - want[name]) / np.linalg.norm(want[name])
+        assert err < 4.2e-7, f"{name}: {err:.3g}"
+
+
 @pytest.mark.parametrize("simname", ["dot", "distance"])
 @pytest.mark.parametrize("which,mul", [("r", 1e-20), ("r", 1e-30), ("r", 1e20), ("v", 1e-20), ("v", 1e20)])
 def test_norms_whose_squares_are_no_floats(ca, which, mul, simname):
