@@ -24,8 +24,15 @@
 // (a warp's window starts at one), so it is uniform over a tile.  It puts the group's largest magnitude into [2^11, 2^15): an
 // element 2^13 below it keeps all bits, the least step is 2^-36 of the largest.
 //
-// Rows with a NaN or an infinity mark their group; a warp that meets one recomputes its pixels from the tensors one
-// by one (exact_*), since a product of a tile would carry them to pixels outside their window.
+// Range.  Half pairs end at a fixed step, so large values would cost pixels whose window does not hold them: their operands when
+// they share a group, their weights when they share a step.  A warp therefore recomputes its pixels from the tensors in Float32
+// (exact_*) when one of its groups is marked (a NaN or an infinity, which a product of a tile would carry to pixels outside their
+// window; a row or a channel too far below the group's largest for its bits, see kLeastValue; magnitudes below 2^-57 in a score's
+// operand) or when the scales of its groups lie further apart than the sweep's weights have bits for (Seen).  Tensors whose
+// magnitudes are alike within a window, or zero, meet neither.  One pixel of k times 1e2, 1e4, 1e6 (57 x 54, 4 units, ws 11), error of
+// dq of the pixels whose windows do not hold it: 8.4e-7, 1.2e-5, 3.1e-3 without this and 4.0e-7, 3.7e-7, 3.7e-7 with it, FMA pipe
+// 5.5e-7.  Where every warp recomputes (512 x 512, 8 units, ws 21, 2 % of v's pixels NaN) the forward takes 5.9 ms for 1.1, dq 7.1 for
+// 1.4, dk/dv 8.9 for 1.9 (310, 379, 707 with a lane per pixel and loads from the tensors); one pixel in 10^4 times 1e6: 1.7, 2.1, 4.1.
 //
 // What bounds the sweeps (256 x 256, 8 units, ws 21): the tensor pipe is busy in 47 % (forward) to 54 % (dk/dv) of the cycles, an
 // instruction issues in 48 and 45 %; an mma also takes five issue slots from FMAs and waits behind them, and 12 to 16 warps of
@@ -34,6 +41,7 @@
 #pragma once
 #include "tile_common.cuh"
 #include <cuda_fp16.h>
+#include <float.h>
 
 namespace ca {
 
@@ -165,9 +173,13 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
-// Biased exponent of the power of two that brings magnitudes up to `bits` below 2^15: a multiple of `step`, 0 for zero,
-// 255 for a NaN or an infinity.
-// `least` is the smallest that is given (also to zeros, where it is not 0).
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// Biased exponent of the power of two that brings magnitudes up to `bits` below 2^15: a multiple of `step`, 255 for a NaN or an
+// infinity.  `least` is the smallest that is given, also to zeros.
 __device__ __forceinline__ int scale_exp(uint32_t bits, int step, int least) {
     const int e = (int)(bits >> 23);
     if (bits == 0) return least;
@@ -176,14 +188,18 @@ __device__ __forceinline__ int scale_exp(uint32_t bits, int step, int least) {
 }
 // Least exponent of a score's operands, 2^-55: the product of two scales is no denormal, so a start of -inf stays -inf.
 constexpr int kLeastExp = 72;
+// The least magnitude of a scaled number of which its halves hold all bits: 22 above the pair's last place of 2^-24, or the 8
+// of a bfloat16 number above the 2^-24 of the upper half.  Groups reach 2^11 at least, so this is 2^-13 of their largest or less.
+__host__ __device__ constexpr float least_value(bool lo) { return lo ? 0x1p-2f : 0x1p-16f; }
+constexpr uint32_t kLeastNormal = 0x00800000u;
+// A factor of scores above this may overflow them (a scaled product is at most 2^34), and a mask of -inf with them.
+constexpr float kMostFactor = 0x1p93f;
+// A factor of scores up to this: the last place of an operand, 2^-25, is no more than 2^-23 in a score.
+constexpr float kFineFactor = 0x1p-14f;
 __device__ __forceinline__ float exp_scale(int e) { return __uint_as_float((uint32_t)e << 23); }
 __device__ __forceinline__ float exp_inverse(int e) { return e ? __uint_as_float((uint32_t)(254 - e) << 23) : 0.f; }
 
 // One real channel of a dense tensor, whatever its storage.
-__device__ __forceinline__ float ld_channel(const float* src, const Geo& g, int u, int cc, int npix, int pix) {
-    if (g.cpe == 2) return __ldg(src + goff<2>(u, g.cr, cc, npix, pix));
-    return g.bf16 ? ld_real<true>(src, goff<1>(u, g.cr, cc, npix, pix)) : ld_real<false>(src, goff<1>(u, g.cr, cc, npix, pix));
-}
 __device__ __forceinline__ void st_channel(float* dst, const Geo& g, int u, int cc, int npix, int pix, float x) {
     if (g.cpe == 2) dst[goff<2>(u, g.cr, cc, npix, pix)] = x;
     else if (g.bf16) st_real<true>(dst, goff<1>(u, g.cr, cc, npix, pix), x);
@@ -221,6 +237,118 @@ struct Raw {
 };
 // The channel of a lane's element i.
 __device__ __forceinline__ int lane_channel(int i, int tq) { return 2 * tq + (i & 1) + 8 * (i >> 1); }
+
+// All channels of one pixel, zeros behind the unit's last.
+__device__ __forceinline__ void load_pixel(const float* src, const Geo& g, int u, int npix, int pix, float (&x)[16]) {
+    if (g.cpe == 2) {
+        const float2* s = reinterpret_cast<const float2*>(src) + (int64_t)u * g.c * npix + pix;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float2 z = i < g.c ? __ldg(s + (int64_t)i * npix) : make_float2(0.f, 0.f);
+            x[2 * i] = z.x;
+            x[2 * i + 1] = z.y;
+        }
+        return;
+    }
+    const int64_t o = (int64_t)u * g.cr * npix + pix;
+    if (g.bf16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = i < g.cr ? ld_real<true>(src, o + (int64_t)i * npix) : 0.f;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = i < g.cr ? __ldg(src + o + (int64_t)i * npix) : 0.f;
+    }
+}
+// Dot products in four short chains, which round less than one of 16.
+__device__ __forceinline__ float dot16(const float (&x)[16], const float (&y)[16]) {
+    pair_t s[2];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const pair_t a = pair(x[2 * i], x[2 * i + 1]), b = pair(y[2 * i], y[2 * i + 1]);
+        s[i & 1] = i < 2 ? mul_pair(a, b) : fma_pair(a, b, s[i & 1]);
+    }
+    const float2 z = unpair(add_pair(s[0], s[1]));
+    return z.x + z.y;
+}
+__device__ __forceinline__ float score(const SplitArgs& a, const float (&x)[16], const float (&y)[16]) {
+    if (!a.dist) return dot16(x, y);
+    float d[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) d[i] = x[i] - y[i];
+    return -0.5f * dot16(d, d);
+}
+// acc += f x
+__device__ __forceinline__ void add_scaled(float (&acc)[16], float f, const float (&x)[16]) {
+    const pair_t ff = pair(f, f);
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+        const float2 z = unpair(fma_pair(pair(x[i], x[i + 1]), ff, pair(acc[i], acc[i + 1])));
+        acc[i] = z.x;
+        acc[i + 1] = z.y;
+    }
+}
+
+// The recomputing paths (see "Range").  A warp puts a column of the two streamed tensors into its share of the step buffers, whose sweep is
+// over, as Float32 rows of kExactPitch numbers: 16 channels of the first, 16 of the second, two scalars.  Lanes l and l + 16 own
+// pixel (row l / 2, column l % 2) of the warp's 16 and take every other row of its window; their sums are added at the end.
+constexpr int kExactPitch = 36, kExactValuesPitch = 20;       // (A's values: the first tensor and the 16 pixels themselves)
+template <int NT, bool LO>
+__device__ __forceinline__ float* exact_rows() {
+    extern __shared__ unsigned char smem_raw[];
+    constexpr int share = 2 * kSplitSteps * split_stage_bytes(NT, LO) / kSplitWarps / 16 * 16;
+    static_assert(share >= 8 * NT * kExactPitch * 4 && share >= (8 * NT + 16) * kExactValuesPitch * 4, "a column of each warp");
+    const uint32_t begin = smem_u32(smem_raw);
+    return reinterpret_cast<float*>(smem_raw + (((begin + 127u) & ~127u) - begin) + (threadIdx.x >> 5) * share);
+}
+struct ExactLane {
+    int lane, half, dh0, r, h, w, pix;                       // dh0: the pixel's first row in the buffer; pix: clamped to the image
+    bool ok;
+    __device__ __forceinline__ ExactLane(const Geo& g, int row0, int w0) {
+        lane = threadIdx.x & 31;
+        half = lane >> 4;
+        dh0 = (lane & 15) >> 1;
+        r = lane & 1;
+        h = row0 + dh0;
+        w = w0 + r;
+        ok = h < g.H && w < g.W;
+        pix = min(h, g.H - 1) + g.H * min(w, g.W - 1);
+    }
+    // Whether the pixel's window holds the s-th column of the warp's.
+    __device__ __forceinline__ bool meets(const Geo& g, int s) const { return s != (r ? 0 : g.ws); }
+    // The pixel of the streamed tensors that this lane copies for the s-th column.
+    __device__ __forceinline__ int streamed(const Geo& g, int row0, int w0, int s) const {
+        return wrap_axis(row0 - g.p + lane, g.H) + g.H * wrap_axis(w0 - g.p + s + g.wk_off, g.Wk);
+    }
+};
+__device__ __forceinline__ void write16(float* to, const float (&x)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(to + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+}
+__device__ __forceinline__ void read16(const float* from, float (&x)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) {
+        const float4 z = *reinterpret_cast<const float4*>(from + i);
+        x[i] = z.x;
+        x[i + 1] = z.y;
+        x[i + 2] = z.z;
+        x[i + 3] = z.w;
+    }
+}
+__device__ __forceinline__ void exact_copy(const SplitArgs& a, int u, int pix, float* row) {
+    float x[16];
+    load_pixel(a.x0, a.g, u, a.g.Npk, pix, x);
+    write16(row, x);
+    load_pixel(a.x1, a.g, u, a.g.Npk, pix, x);
+    write16(row + 16, x);
+}
+// The sums of a pixel's two lanes, times f, into the dense tensor.
+__device__ __forceinline__ void exact_store(float* dst, const Geo& g, int u, const ExactLane& L, const float (&x)[16], float f) {
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+        const float z = (x[c] + __shfl_xor_sync(0xffffffffu, x[c], 16)) * f;
+        if (L.ok && !L.half && c < g.cr) st_channel(dst, g, u, c, g.Np, L.pix, z);
+    }
+}
 
 // A lane's four channels of a pixel: x[0..1] in the result's first eight channels, x[2..3] in its second.
 __device__ __forceinline__ void store_pixel(float* dst, const Geo& g, int u, int pix, int tq, float x0, float x1, float x2, float x3) {
@@ -288,11 +416,13 @@ struct Centre {
                 m = max(m, abs_bits(x[i]));
                 n = fmaf(x[i], x[i], n);
             }
-            const int e = scale_exp(quad_max(m), 1, least);
+            m = quad_max(m);
+            const int e = scale_exp(m, 1, least);
             norm2[r] = quad_sum(n);
             bad |= e == 255;
             scale[r] = exp_scale(e);
             const float inv = exp_inverse(e == 255 ? 0 : e);
+            if (least) bad |= m >= kLeastNormal && __uint_as_float(m) * inv < least_value(LO);
             float ns = 0.f;
 #pragma unroll
             for (int i = 0; i < 4; ++i) ns = fmaf(x[i] * inv, x[i] * inv, ns);
@@ -460,6 +590,32 @@ __device__ __forceinline__ void outer_column(const uint32_t (&hi)[NT][2], const 
         }
     }
 }
+
+// What a warp has met: the largest scale of both tensors, then the smallest but for zeros, in a byte each; 0 once its pixels have to be
+// recomputed.  The word waits in shared memory, since it changes rarely and the sweeps have no register to spare; all lanes hold
+// and write the same one.
+struct Seen {
+    static __device__ __forceinline__ volatile uint32_t* slot() {
+        __shared__ uint32_t slots[kSplitWarps];
+        return &slots[threadIdx.x >> 5];
+    }
+    static __device__ __forceinline__ void clear(bool bad) { *slot() = __any_sync(0xffffffffu, bad) ? 0u : 0xffff0000u; }
+    static __device__ __forceinline__ bool bad() { return *slot() == 0; }
+    // The largest scales of a step.
+    static __device__ __forceinline__ void tops(uint32_t word, uint32_t& e0, uint32_t& e1) {
+        e0 = __reduce_max_sync(0xffffffffu, word & 255u);
+        e1 = __reduce_max_sync(0xffffffffu, word >> 8 & 255u);
+    }
+    // Takes them in; the pixels are recomputed from a mark on, when the extremes lie further apart than the limits (binary orders), or
+    // when a lane says so.
+    static __device__ __forceinline__ void add(uint32_t word, uint32_t e0, uint32_t e1, int limit0, int limit1, bool bad) {
+        const uint32_t bytes = *slot(), b0 = word & 255u, b1 = word >> 8 & 255u;
+        const uint32_t hi0 = max(bytes & 255u, e0), lo0 = min(bytes >> 16 & 255u, __reduce_min_sync(0xffffffffu, b0 ? b0 : 255u));
+        const uint32_t hi1 = max(bytes >> 8 & 255u, e1), lo1 = min(bytes >> 24, __reduce_min_sync(0xffffffffu, b1 ? b1 : 255u));
+        bad |= bytes == 0 || hi0 == 255u || hi1 == 255u || (int)hi0 > (int)lo0 + limit0 || (int)hi1 > (int)lo1 + limit1;
+        *slot() = __any_sync(0xffffffffu, bad) ? 0u : hi0 | hi1 << 8 | lo0 << 16 | lo1 << 24;
+    }
+};
 
 // 0 for a score inside the window of the lane's row, -inf outside (tile t, element i of the lane's four).
 __device__ __forceinline__ float window_mask(int lane, int p, int t, int i) {

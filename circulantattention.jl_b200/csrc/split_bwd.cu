@@ -19,66 +19,77 @@ __device__ __forceinline__ int bound_inverse(int norm, int e, int d) {
     return min(max(254 - x, 1), 236);
 }
 
-// One pixel from the tensors themselves (a warp that met a NaN or an infinity).
-__device__ __noinline__ void exact_dq(const SplitArgs& a, int u, int h, int w) {
+__device__ __noinline__ void exact_dq(const SplitArgs& a, int u, int row0, int w0, float* buf) {
     const Geo& g = a.g;
-    const int j = h + g.H * w;
+    const float sl2 = a.scale * kLog2e;
+    const ExactLane L(g, row0, w0);
     float q[16], dy[16], acc[16];
-    for (int c = 0; c < g.cr; ++c) {
-        q[c] = ld_channel(a.c0, g, u, c, g.Np, j);
-        dy[c] = ld_channel(a.c1, g, u, c, g.Np, j);
-        acc[c] = 0.f;
-    }
-    const float L = a.stats[(int64_t)u * g.Np + j] * kLog2e, D = a.D[(int64_t)u * g.Np + j], sl2 = a.scale * kLog2e;
-    for (int dw = -g.p; dw <= g.p; ++dw) {
-        const int kw = wrap_axis(w + dw + g.wk_off, g.Wk);
-        for (int dh = -g.p; dh <= g.p; ++dh) {
-            const int pix = wrap_axis(h + dh, g.H) + g.H * kw;
-            float s = 0.f, dp = 0.f;
-            for (int c = 0; c < g.cr; ++c) {
-                const float kc = ld_channel(a.x0, g, u, c, g.Npk, pix);
-                s = a.dist ? fmaf(-0.5f * (q[c] - kc), q[c] - kc, s) : fmaf(q[c], kc, s);
-                dp = fmaf(dy[c], ld_channel(a.x1, g, u, c, g.Npk, pix), dp);
+    load_pixel(a.c0, g, u, g.Np, L.pix, q);
+    load_pixel(a.c1, g, u, g.Np, L.pix, dy);
+    const float stat = a.stats[(int64_t)u * g.Np + L.pix] * kLog2e, D = a.D[(int64_t)u * g.Np + L.pix];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) acc[c] = 0.f;
+#pragma unroll 1
+    for (int s = 0; s <= g.ws; ++s) {
+        __syncwarp();
+        if (L.lane < 8 + 2 * g.p) exact_copy(a, u, L.streamed(g, row0, w0, s), buf + L.lane * kExactPitch);
+        __syncwarp();
+        if (!L.meets(g, s)) continue;
+#pragma unroll 1
+        for (int dh = L.half; dh < g.ws; dh += 2) {
+            const float* row = buf + (L.dh0 + dh) * kExactPitch;
+            float k[16], v[16];
+            read16(row, k);
+            read16(row + 16, v);
+            const float ds = fast_exp2(score(a, q, k) * sl2 - stat) * (dot16(dy, v) - D);
+            if (a.dist) {
+#pragma unroll
+                for (int c = 0; c < 16; ++c) k[c] -= q[c];
             }
-            const float ds = fast_exp2(s * sl2 - L) * (dp - D);
-            for (int c = 0; c < g.cr; ++c) acc[c] = fmaf(ds, ld_channel(a.x0, g, u, c, g.Npk, pix) - (a.dist ? q[c] : 0.f), acc[c]);
+            add_scaled(acc, ds, k);
         }
     }
-    for (int c = 0; c < g.cr; ++c) st_channel(a.o0, g, u, c, g.Np, j, a.scale * acc[c]);
+    exact_store(a.o0, g, u, L, acc, a.scale);
 }
 
-__device__ __noinline__ void exact_dkdv(const SplitArgs& a, int u, int h, int w) {
+__device__ __noinline__ void exact_dkdv(const SplitArgs& a, int u, int row0, int w0, float* buf) {
     const Geo& g = a.g;
-    const int i = h + g.H * w;
-    float k[16], v[16], dk[16], dv[16];
-    for (int c = 0; c < g.cr; ++c) {
-        k[c] = ld_channel(a.c0, g, u, c, g.Np, i);
-        v[c] = ld_channel(a.c1, g, u, c, g.Np, i);
-        dk[c] = dv[c] = 0.f;
-    }
     const float sl2 = a.scale * kLog2e;
-    for (int dw = -g.p; dw <= g.p; ++dw) {
-        const int jw = wrap_axis(w + dw + g.wk_off, g.Wk);
-        for (int dh = -g.p; dh <= g.p; ++dh) {
-            const int pix = wrap_axis(h + dh, g.H) + g.H * jw;
-            const int64_t row = (int64_t)u * g.Npk + pix;
-            float s = 0.f, dp = 0.f;
-            for (int c = 0; c < g.cr; ++c) {
-                const float qc = ld_channel(a.x0, g, u, c, g.Npk, pix);
-                s = a.dist ? fmaf(-0.5f * (qc - k[c]), qc - k[c], s) : fmaf(qc, k[c], s);
-                dp = fmaf(ld_channel(a.x1, g, u, c, g.Npk, pix), v[c], dp);
+    const ExactLane L(g, row0, w0);
+    float k[16], v[16], dk[16], dv[16];
+    load_pixel(a.c0, g, u, g.Np, L.pix, k);
+    load_pixel(a.c1, g, u, g.Np, L.pix, v);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) dk[c] = dv[c] = 0.f;
+#pragma unroll 1
+    for (int s = 0; s <= g.ws; ++s) {
+        __syncwarp();
+        if (L.lane < 8 + 2 * g.p) {
+            const int pix = L.streamed(g, row0, w0, s);
+            float* row = buf + L.lane * kExactPitch;
+            exact_copy(a, u, pix, row);
+            row[32] = a.xstats[(int64_t)u * g.Npk + pix] * kLog2e;
+            row[33] = a.xD[(int64_t)u * g.Npk + pix];
+        }
+        __syncwarp();
+        if (!L.meets(g, s)) continue;
+#pragma unroll 1
+        for (int dh = L.half; dh < g.ws; dh += 2) {
+            const float* row = buf + (L.dh0 + dh) * kExactPitch;
+            float q[16], dy[16];
+            read16(row, q);
+            read16(row + 16, dy);
+            const float p = fast_exp2(score(a, q, k) * sl2 - row[32]), ds = p * (dot16(dy, v) - row[33]);
+            if (a.dist) {
+#pragma unroll
+                for (int c = 0; c < 16; ++c) q[c] -= k[c];
             }
-            const float p = fast_exp2(s * sl2 - a.xstats[row] * kLog2e), ds = p * (dp - a.xD[row]);
-            for (int c = 0; c < g.cr; ++c) {
-                dk[c] = fmaf(ds, ld_channel(a.x0, g, u, c, g.Npk, pix) - (a.dist ? k[c] : 0.f), dk[c]);
-                dv[c] = fmaf(p, ld_channel(a.x1, g, u, c, g.Npk, pix), dv[c]);
-            }
+            add_scaled(dk, ds, q);
+            add_scaled(dv, p, dy);
         }
     }
-    for (int c = 0; c < g.cr; ++c) {
-        st_channel(a.o0, g, u, c, g.Np, i, a.scale * dk[c]);
-        st_channel(a.o1, g, u, c, g.Np, i, dv[c]);
-    }
+    exact_store(a.o0, g, u, L, dk, a.scale);
+    exact_store(a.o1, g, u, L, dv, 1.f);
 }
 
 // What the two sweeps share: the tiles of a column against two centre operands.
@@ -91,7 +102,7 @@ struct BwdSweep {
     float sl2;
     Centre<LO> c0, c1;
     uint32_t cur, word;                                      // the scales of the step's groups when they are all alike; this lane's
-    bool bad, mixed;
+    bool bad, mixed;                                         // bad: a centre operand cannot be split
 
     __device__ __forceinline__ BwdSweep(const SplitArgs& a_) : a(a_) {
         const int row0 = blockIdx.y * 8 * kSplitWarps + 8 * (threadIdx.x >> 5);
@@ -162,6 +173,7 @@ struct DqSweep : BwdSweep<NT, LO> {
             for (int t = 0; t < NT; ++t) nref[t][r] = pair(b + window_mask(lane, g.p, t, 0), b + window_mask(lane, g.p, t, 1));
             sum[r] = c[r] = e[r] = nd[r] = S[r] = Sd[r] = 0;
         }
+        Seen::clear(bad);
 #pragma unroll
         for (int n = 0; n < 2; ++n) acc[n][0] = acc[n][1] = 0;
     }
@@ -211,8 +223,10 @@ struct DqSweep : BwdSweep<NT, LO> {
         word = ldsu32(rb + B::word_off) & 0xffffu;
         mixed = false;
         if (__any_sync(0xffffffffu, word != cur)) {
-            bad |= (word & 255u) == 255u || (word >> 8) == 255u;
-            const uint32_t ek = __reduce_max_sync(0xffffffffu, word & 255u), ev = __reduce_max_sync(0xffffffffu, word >> 8);
+            // weights are mostly 2^-7 to 2^2 of 2^-24 steps: a scale further than 2^4 below the step's largest would show
+            uint32_t ek, ev;
+            Seen::tops(word, ek, ev);
+            Seen::add(word, ek, ev, 4, 4, !(fmaxf(c0.scale[0], c0.scale[1]) * exp_scale(ek) < kMostFactor));
             cur = ek | ev << 8;
             mixed = __any_sync(0xffffffffu, word != cur);
 #pragma unroll
@@ -232,8 +246,8 @@ struct DqSweep : BwdSweep<NT, LO> {
 
     __device__ __forceinline__ void end(int w0, float poison) {
         const Geo& g = a.g;
-        if (__any_sync(0xffffffffu, bad)) {
-            if (tq < 2 && h < g.H && w0 + tq < g.W) exact_dq(a, u, h, w0 + tq);
+        if (Seen::bad() && poison == 0.f) {
+            exact_dq(a, u, h - (lane >> 2), w0, exact_rows<NT, LO>());
             return;
         }
         Raw raw = {};
@@ -273,7 +287,11 @@ struct DkdvSweep : BwdSweep<NT, LO> {
         B::load(w0);
         most = 0;
         nrm = Sd = 0;
-        norm = __reduce_max_sync(0xffffffffu, max(c1.top[0], c1.top[1]));
+        // The largest norm bounds the weights of all 16 pixels.  Those four rows from a pixel meet queries that it does not.
+        const int top = max(c1.top[0], c1.top[1]);
+        const int upper = __reduce_max_sync(0xffffffffu, lane < 16 ? top : 0), lower = __reduce_max_sync(0xffffffffu, lane < 16 ? 0 : top);
+        norm = max(upper, lower);
+        Seen::clear(bad || (min(upper, lower) && abs(upper - lower) > 4));
 #pragma unroll
         for (int t = 0; t < NT; ++t) mk[t] = pair(window_mask(lane, g.p, t, 0), window_mask(lane, g.p, t, 1));
 #pragma unroll
@@ -347,9 +365,13 @@ struct DkdvSweep : BwdSweep<NT, LO> {
         word &= 0xffffu;
         mixed = false;
         if (__any_sync(0xffffffffu, word != cur || top > most)) {
-            bad |= (word & 255u) == 255u || (word >> 8) == 255u || top == 255u;
-            const uint32_t eq = __reduce_max_sync(0xffffffffu, word & 255u), ed = __reduce_max_sync(0xffffffffu, word >> 8);
+            uint32_t eq, ed;
+            Seen::tops(word, eq, ed);
             most = max(most, __reduce_max_sync(0xffffffffu, top));
+            // the largest |D| rules the weights, also of groups whose own is far below it
+            Seen::add(word, eq, ed, 4, 4,
+                      most == 255u || (top && most > top + 6u && (int)most > norm + (int)ed - 127 + 17) ||
+                          !(fmaxf(c0.scale[0], c0.scale[1]) * exp_scale(eq) < kMostFactor));
             cur = eq | ed << 8;
             mixed = __any_sync(0xffffffffu, word != cur);
             const int nb = bound_inverse(norm, ed, most);
@@ -370,8 +392,8 @@ struct DkdvSweep : BwdSweep<NT, LO> {
 
     __device__ __forceinline__ void end(int w0, float poison) {
         const Geo& g = a.g;
-        if (__any_sync(0xffffffffu, bad)) {
-            if (tq < 2 && h < g.H && w0 + tq < g.W) exact_dkdv(a, u, h, w0 + tq);
+        if (Seen::bad() && poison == 0.f) {
+            exact_dkdv(a, u, h - (lane >> 2), w0, exact_rows<NT, LO>());
             return;
         }
         Raw raw = {};

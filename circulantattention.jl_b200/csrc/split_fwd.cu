@@ -8,53 +8,80 @@ namespace {
 // largest score of its first window column, which gets weight 2^kStart, and moves when a score passes the bound.
 constexpr float kTop = 15.f, kStart = 7.f;
 
-// One pixel from the tensors themselves (blocks that met a NaN or an infinity).
-__device__ __noinline__ void exact_fwd(const SplitArgs& a, int u, int h, int w) {
+__device__ __noinline__ void exact_fwd(const SplitArgs& a, int u, int row0, int w0, float* buf) {
     const Geo& g = a.g;
     const float sl2 = a.scale * kLog2e;
-    const int j = h + g.H * w;
-    float q[16], acc[16];
-    for (int c = 0; c < g.cr; ++c) {
-        q[c] = ld_channel(a.c0, g, u, c, g.Np, j);
-        acc[c] = 0.f;
-    }
-    float m = -INFINITY, l = 0.f;
-    for (int dw = -g.p; dw <= g.p; ++dw) {
-        const int kw = wrap_axis(w + dw + g.wk_off, g.Wk);
-        for (int dh = -g.p; dh <= g.p; ++dh) {
-            const int pix = wrap_axis(h + dh, g.H) + g.H * kw;
-            float s = 0.f;
-            for (int c = 0; c < g.cr; ++c) {
-                const float kc = ld_channel(a.x0, g, u, c, g.Npk, pix);
-                s = a.dist ? fmaf(-0.5f * (q[c] - kc), q[c] - kc, s) : fmaf(q[c], kc, s);
+    const ExactLane L(g, row0, w0);
+    float q[16], acc[16], m = -FLT_MAX, l = 0.f;
+    load_pixel(a.c0, g, u, g.Np, L.pix, q);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) acc[c] = 0.f;
+#pragma unroll 1
+    for (int s = 0; s <= g.ws; ++s) {
+        __syncwarp();
+        if (L.lane < 8 + 2 * g.p) exact_copy(a, u, L.streamed(g, row0, w0, s), buf + L.lane * kExactPitch);
+        __syncwarp();
+        if (!L.meets(g, s)) continue;
+#pragma unroll 1
+        for (int dh = L.half; dh < g.ws; dh += 2) {
+            const float* row = buf + (L.dh0 + dh) * kExactPitch;
+            float k[16], v[16];
+            read16(row, k);
+            const float z = score(a, q, k) * sl2, mn = fmaxf(m, z), p = fast_exp2(z - mn);
+            read16(row + 16, v);
+            if (mn != m) {
+                const float corr = fast_exp2(m - mn);
+                l *= corr;
+#pragma unroll
+                for (int c = 0; c < 16; ++c) acc[c] *= corr;
+                m = mn;
             }
-            s *= sl2;
-            const float mn = fmaxf(m, s), corr = fast_exp2(m - mn), p = fast_exp2(s - mn);
-            l = l * corr + p;
-            for (int c = 0; c < g.cr; ++c) acc[c] = acc[c] * corr + p * ld_channel(a.x1, g, u, c, g.Npk, pix);
-            m = mn;
+            l += p;
+            add_scaled(acc, p, v);
         }
     }
-    for (int c = 0; c < g.cr; ++c) st_channel(a.o0, g, u, c, g.Np, j, acc[c] / l);
-    if (a.ostats) a.ostats[(int64_t)u * g.Np + j] = (m + log2f(l)) * kLn2;
+    const float top = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16)), f = fast_exp2(m - top);
+    l *= f;
+    const float sum = l + __shfl_xor_sync(0xffffffffu, l, 16);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) acc[c] *= f;
+    exact_store(a.o0, g, u, L, acc, 1.f / sum);
+    if (a.ostats && L.ok && !L.half) a.ostats[(int64_t)u * g.Np + L.pix] = (top + log2f(sum)) * kLn2;
 }
 
-// The values of one pixel's row.
-__device__ __noinline__ void exact_values(const SplitArgs& a, int u, int h, int w) {
+// The values of the warp's rows of A: here a lane owns a row of the windows, whose values are neighbours, and the centre vectors lie
+// behind the column.
+__device__ __noinline__ void exact_values(const SplitArgs& a, int u, int row0, int w0, float* buf) {
     const Geo& g = a.g;
-    const int j = h + g.H * w;
-    const float sl2 = a.scale * kLog2e, L = a.stats[(int64_t)u * g.Np + j] * kLog2e;
-    for (int dw = -g.p; dw <= g.p; ++dw) {
-        const int kw = wrap_axis(w + dw + g.wk_off, g.Wk);
-        for (int dh = -g.p; dh <= g.p; ++dh) {
-            const int pix = wrap_axis(h + dh, g.H) + g.H * kw;
-            float s = 0.f;
-            for (int c = 0; c < g.cr; ++c) {
-                const float qc = ld_channel(a.c0, g, u, c, g.Np, j), kc = ld_channel(a.x0, g, u, c, g.Npk, pix);
-                s = a.dist ? fmaf(-0.5f * (qc - kc), qc - kc, s) : fmaf(qc, kc, s);
-            }
-            a.o0[((int64_t)u * g.Np + j) * g.K + axis_pos(dw, w, g.W, g.p, g.ws) * g.ws + axis_pos(dh, h, g.H, g.p, g.ws)] =
-                fast_exp2(s * sl2 - L);
+    const float sl2 = a.scale * kLog2e;
+    const ExactLane L(g, row0, w0);
+    constexpr int kPitch = kExactValuesPitch;
+    float* centre = buf + (8 + 2 * g.p) * kPitch;
+    float x[16];
+    __syncwarp();
+    if (!L.half) {
+        load_pixel(a.c0, g, u, g.Np, L.pix, x);
+        write16(centre + L.lane * kPitch, x);
+        centre[L.lane * kPitch + 16] = a.stats[(int64_t)u * g.Np + L.pix] * kLog2e;
+    }
+#pragma unroll 1
+    for (int s = 0; s <= g.ws; ++s) {
+        __syncwarp();
+        if (L.lane < 8 + 2 * g.p) {
+            load_pixel(a.x0, g, u, g.Npk, L.streamed(g, row0, w0, s), x);
+            write16(buf + L.lane * kPitch, x);
+        }
+        __syncwarp();
+        if (L.lane >= g.ws) continue;
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i) {
+            const int h = row0 + (i >> 1), r = i & 1, w = w0 + r;
+            if (s == (r ? 0 : g.ws) || h >= g.H || w >= g.W) continue;
+            float q[16];
+            read16(centre + i * kPitch, q);
+            read16(buf + ((i >> 1) + L.lane) * kPitch, x);
+            a.o0[((int64_t)u * g.Np + h + g.H * w) * g.K + axis_pos(s - g.p - r, w, g.W, g.p, g.ws) * g.ws +
+                 axis_pos(L.lane - g.p, h, g.H, g.p, g.ws)] = fast_exp2(score(a, q, x) * sl2 - centre[i * kPitch + 16]);
         }
     }
 }
@@ -71,7 +98,6 @@ struct FwdSweep {
     pair_t acc[2][2], l[2], nref[NT][2], c[2], S[2];
     float shift[2];                                          // what the references have moved by
     uint32_t cur;                                            // the scales of the step's groups when they are all alike, as they mostly are
-    bool bad;
 
     __device__ __forceinline__ FwdSweep(const SplitArgs& a_) : a(a_) {
         const int warp = threadIdx.x >> 5, row0 = blockIdx.y * 8 * kSplitWarps + 8 * (warp % kSplitWarps);
@@ -91,7 +117,7 @@ struct FwdSweep {
         Raw raw;
         raw.load(a.c0, g, u, h, w0, tq);
         q.form(raw, g, h, w0, tq, kLeastExp);
-        bad = q.bad;
+        Seen::clear(q.bad);
         cur = 0;
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -110,9 +136,12 @@ struct FwdSweep {
         const uint32_t word = ldsu32(rb + word_off);
         bool mixed = false;
         if (__any_sync(0xffffffffu, word != cur)) {
-            bad |= (word & 255u) == 255u || (word >> 8 & 255u) == 255u;
-            const uint32_t ek = __reduce_max_sync(0xffffffffu, word & 255u);
-            const uint32_t ev = __reduce_max_sync(0xffffffffu, word >> 8 & 255u);
+            // Weights start at 2^7 for a row's largest and end at 2^-24: scales of v that are 2^8 apart leave them 23 bits.  A score
+            // loses to other rows of its group what lies below 2^-36 of their largest.
+            uint32_t ek, ev;
+            Seen::tops(word, ek, ev);
+            const float most = fmaxf(q.scale[0], q.scale[1]) * exp_scale(ek);
+            Seen::add(word, ek, ev, __any_sync(0xffffffffu, most > kFineFactor) ? 8 : 255, 8, !(most < kMostFactor));
             cur = ek | ev << 8;
             mixed = __any_sync(0xffffffffu, word != cur);
             S[0] = S[1] = pair(exp_scale(ev), exp_scale(ev));
@@ -185,8 +214,8 @@ struct FwdSweep {
     }
     __device__ __forceinline__ void end(int w0, float poison) {
         const Geo& g = a.g;
-        if (__any_sync(0xffffffffu, bad)) {
-            if (tq < 2 && h < g.H && w0 + tq < g.W) exact_fwd(a, u, h, w0 + tq);
+        if (Seen::bad() && poison == 0.f) {
+            exact_fwd(a, u, h - (lane >> 2), w0, exact_rows<NT, LO>());
             return;
         }
 #pragma unroll
@@ -224,7 +253,6 @@ struct EmitSweep {
     pair_t nref[2], c[2];
     int at[NT][2];                                           // shared address of a tile's element for the first row and window column, -1: outside
     uint32_t cur;
-    bool bad;
 
     __device__ __forceinline__ EmitSweep(const SplitArgs& a_) : a(a_) {
         const int row0 = blockIdx.y * 8 * kSplitWarps + 8 * (threadIdx.x >> 5);
@@ -250,7 +278,7 @@ struct EmitSweep {
         for (int r = 0; r < 2; ++r) L[r] = __ldg(a.stats + (int64_t)u * g.Np + min(h, g.H - 1) + g.H * min(w0 + r, g.W - 1));
         raw.load(a.c0, g, u, h, w0, tq);
         q.form(raw, g, h, w0, tq, kLeastExp);
-        bad = q.bad;
+        Seen::clear(q.bad);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const float b = (DIST ? -0.5f * sl2 * q.norm2[r] : 0.f) - L[r] * kLog2e;
@@ -273,8 +301,10 @@ struct EmitSweep {
         const uint32_t word = ldsu32(rb + word_off) & 255u;
         bool mixed = false;
         if (__any_sync(0xffffffffu, word != cur)) {
-            bad |= word == 255u;
-            cur = __reduce_max_sync(0xffffffffu, word);
+            uint32_t none;
+            Seen::tops(word, cur, none);
+            const float most = fmaxf(q.scale[0], q.scale[1]) * exp_scale(cur);
+            Seen::add(word, cur, none, __any_sync(0xffffffffu, most > kFineFactor) ? 8 : 255, 8, !(most < kMostFactor));
             mixed = __any_sync(0xffffffffu, word != cur);
 #pragma unroll
             for (int r = 0; r < 2; ++r) c[r] = pair(q.scale[r] * exp_scale(cur), q.scale[r] * exp_scale(cur));
@@ -317,14 +347,10 @@ struct EmitSweep {
 
     __device__ __forceinline__ void end(int w0, float poison) {
         const Geo& g = a.g;
-        const bool exact = __any_sync(0xffffffffu, bad);
-        if (!exact && poison == 0.f) return;
-        if (tq < 2 && h < g.H && w0 + tq < g.W) {
-            if (exact) {
-                exact_values(a, u, h, w0 + tq);
-            } else {
-                for (int i = 0; i < g.K; ++i) a.o0[((int64_t)u * g.Np + h + g.H * (w0 + tq)) * g.K + i] = poison;
-            }
+        if (poison == 0.f) {
+            if (Seen::bad()) exact_values(a, u, h - (lane >> 2), w0, exact_rows<NT, LO>());
+        } else if (tq < 2 && h < g.H && w0 + tq < g.W) {
+            for (int i = 0; i < g.K; ++i) a.o0[((int64_t)u * g.Np + h + g.H * (w0 + tq)) * g.K + i] = poison;
         }
     }
 };

@@ -5,6 +5,19 @@
 namespace ca {
 namespace {
 
+// Whether the halves would lose bits of a whole row of the lane's group of eight (`small`; with one channel a row is a single number, which
+// may be any) or of a whole channel of it.
+__device__ __forceinline__ bool marked(const float (&x)[16], bool small, float inv, float least) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        uint32_t c = abs_bits(x[e]);
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1) c = max(c, __shfl_xor_sync(0xffffffffu, c, d));
+        small |= c >= kLeastNormal && __uint_as_float(c) * inv < least;
+    }
+    return __ballot_sync(0xffffffffu, small) >> (threadIdx.x & 24) & 255u;
+}
+
 // A block gathers 128 packed rows of one column of one unit: a thread reads the 16 channels of its row of both tensors
 // (consecutive lanes on consecutive rows: coalesced planar loads, all in flight together), the largest magnitude of each
 // group of eight rows comes from shuffles, and the block writes its rows as one contiguous run of 16-byte stores.  Bound: HBM.
@@ -68,19 +81,39 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
     const float norm = n2.x + n2.y;
     uint32_t exps = 0;
     uint32_t* row = tile + rl * RF;
+    int ex[2];
+    float inv[2];
+    bool small[2], look = false;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         uint32_t m = 0;
+        float low = INFINITY;
 #pragma unroll
         for (int e = 0; e < 16; ++e) m = max(m, abs_bits(x[t][e]));
 #pragma unroll
+        for (int e = 0; e < 16; e += 2)
+            if (e < g.cr) low = min3(low, fabsf(x[t][e]), e + 1 < g.cr ? fabsf(x[t][e + 1]) : INFINITY);
+        const uint32_t mine = m;
+#pragma unroll
         for (int d = 1; d < 8; d <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
-        const int e = scale_exp(m, 4, t == 0 ? kLeastExp : 0);
-        exps |= (uint32_t)e << (8 * t);
-        const float inv = exp_inverse(e == 255 ? 0 : e);
+        ex[t] = m ? scale_exp(m, 4, t == 0 ? kLeastExp : 0) : 0;
+        inv[t] = exp_inverse(ex[t] == 255 ? 0 : ex[t]);
+        small[t] = g.cr > 1 && mine >= kLeastNormal && __uint_as_float(mine) * inv[t] < least_value(LO);
+        // a channel of small numbers has one in all eight rows, which is rare
+        const uint32_t rows = __ballot_sync(0xffffffffu, low * inv[t] < least_value(LO)) >> (rl & 24) & 255u;
+        look |= small[t] || (m && rows == 255u);
+    }
+    if (__any_sync(0xffffffffu, look)) {
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+            if (marked(x[t], small[t], inv[t], least_value(LO))) ex[t] = 255;
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        exps |= (uint32_t)ex[t] << (8 * t);
         uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) split2(x[t][2 * i] * inv, x[t][2 * i + 1] * inv, hi[i], lo[i]);
+        for (int i = 0; i < 8; ++i) split2(x[t][2 * i] * inv[t], x[t][2 * i + 1] * inv[t], hi[i], lo[i]);
         uint4* d = reinterpret_cast<uint4*>(row + t * (split_second(LO) / 4));
         d[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         d[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
