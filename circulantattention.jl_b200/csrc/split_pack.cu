@@ -6,14 +6,15 @@ namespace ca {
 namespace {
 
 // Whether the halves would lose bits of a whole row of the lane's group of eight (`small`; with one channel a row is a single number, which
-// may be any) or of a whole channel of it.
-__device__ __forceinline__ bool marked(const float (&x)[16], bool small, float inv, float least) {
+// may be any) or of a whole channel of it (`channels`: of few rows that are not zero, as at the end of a column, a channel may be
+// any small numbers, too).
+__device__ __forceinline__ bool marked(const float (&x)[16], bool small, bool channels, float inv, float least) {
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
         uint32_t c = abs_bits(x[e]);
 #pragma unroll
         for (int d = 1; d < 8; d <<= 1) c = max(c, __shfl_xor_sync(0xffffffffu, c, d));
-        small |= c >= kLeastNormal && __uint_as_float(c) * inv < least;
+        small |= channels && c >= kLeastNormal && __uint_as_float(c) * inv < least;
     }
     return __ballot_sync(0xffffffffu, small) >> (threadIdx.x & 24) & 255u;
 }
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
     uint32_t* row = tile + rl * RF;
     int ex[2];
     float inv[2];
-    bool small[2], look = false;
+    bool small[2], channels[2], look = false;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         uint32_t m = 0;
@@ -101,12 +102,14 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
         small[t] = g.cr > 1 && mine >= kLeastNormal && __uint_as_float(mine) * inv[t] < least_value(LO);
         // a channel of small numbers has one in all eight rows, which is rare
         const uint32_t rows = __ballot_sync(0xffffffffu, low * inv[t] < least_value(LO)) >> (rl & 24) & 255u;
-        look |= small[t] || (m && rows == 255u);
+        const uint32_t filled = __ballot_sync(0xffffffffu, mine) >> (rl & 24) & 255u;
+        channels[t] = rows == 255u && __popc(filled) >= 4;
+        look |= small[t] || channels[t];
     }
     if (__any_sync(0xffffffffu, look)) {
 #pragma unroll
         for (int t = 0; t < 2; ++t)
-            if (marked(x[t], small[t], inv[t], least_value(LO))) ex[t] = 255;
+            if (marked(x[t], small[t], channels[t], inv[t], least_value(LO))) ex[t] = 255;
     }
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
