@@ -277,7 +277,7 @@ struct DkdvSweep : BwdSweep<NT, LO> {
     using B::RB; using B::SB;
     pair_t dk[2][2], dv[2][2], sum[2], mk[NT], bk[2], c[2], e[2], nrm, Sk[2], Sv[2], Sd;      // Sd: Distance, the sums of dS
     int norm;
-    uint32_t most;                                           // exponent above the |D| met so far
+    int bound;                                               // exponent above the |dP| and the |D| of the step
     Tail tp, td;
 
     __device__ __forceinline__ DkdvSweep(const SplitArgs& a_) : B(a_) {}
@@ -285,7 +285,7 @@ struct DkdvSweep : BwdSweep<NT, LO> {
     __device__ __forceinline__ void begin(int w0, uint32_t) {
         const Geo& g = a.g;
         B::load(w0);
-        most = 0;
+        bound = 0;
         nrm = Sd = 0;
         // The largest norm bounds the weights of all 16 pixels.  Those four rows from a pixel meet queries that it does not.
         const int top = max(c1.top[0], c1.top[1]);
@@ -364,16 +364,17 @@ struct DkdvSweep : BwdSweep<NT, LO> {
         const uint32_t top = word >> 16;
         word &= 0xffffu;
         mixed = false;
-        if (__any_sync(0xffffffffu, word != cur || top > most)) {
+        if (__any_sync(0xffffffffu, word != cur || (int)top > bound)) {
             uint32_t eq, ed;
             Seen::tops(word, eq, ed);
-            most = max(most, __reduce_max_sync(0xffffffffu, top));
-            // the largest |D| rules the weights, also of groups whose own is far below it
+            // Where a |D| rules the weights, groups with smaller ones lose bits to it; such a step's bound is not kept for the next.
+            const int dp = norm + (int)ed - 127 + 17, most = __reduce_max_sync(0xffffffffu, top);
+            bound = min(max(dp, most), 254);
             Seen::add(word, eq, ed, 4, 4,
-                      most == 255u || (top && most > top + 6u && (int)most > norm + (int)ed - 127 + 17) ||
-                          !(fmaxf(c0.scale[0], c0.scale[1]) * exp_scale(eq) < kMostFactor));
+                      most == 255 || (top && most > dp && most > (int)top + 6) || !(fmaxf(c0.scale[0], c0.scale[1]) * exp_scale(eq) < kMostFactor));
             cur = eq | ed << 8;
             mixed = __any_sync(0xffffffffu, word != cur);
+            if (most > dp) cur |= 1u << 16;
             const int nb = bound_inverse(norm, ed, most);
             const float n = exp_scale(nb) * kWeight, bv = exp_scale(ed) / kWeight, bd = exp_scale(254 - nb) / kWeight, back = exp_scale(eq) * bd;
             nrm = pair(n, n);
