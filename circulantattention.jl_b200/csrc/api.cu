@@ -18,6 +18,8 @@ static std::atomic<int64_t> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 static std::atomic<int64_t> g_tiled_launches{0};
 void count_tiled_launch() { g_tiled_launches.fetch_add(1, std::memory_order_relaxed); }
+static std::atomic<int64_t> g_tensor_launches{0};
+void count_tensor_launch() { g_tensor_launches.fetch_add(1, std::memory_order_relaxed); }
 
 // FP32 FMA peak probe: 16 independent packed-FMA chains per thread, registers only.
 __global__ void __launch_bounds__(256) ffma_probe_kernel(int iters, float* __restrict__ sink) {
@@ -198,6 +200,8 @@ int ca_version(void) { return 100; }
 int64_t ca_probe_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
 int64_t ca_probe_tiled_launch_count(void) { return g_tiled_launches.load(std::memory_order_relaxed); }
+
+int64_t ca_probe_tensor_launch_count(void) { return g_tensor_launches.load(std::memory_order_relaxed); }
 
 int ca_probe_ffma(int32_t blocks, int32_t iters, float* sink, void* stream) {
     if (blocks < 1 || iters < 1) { set_error("blocks and iters must be positive"); return CA_ERR_BAD_DESC; }

@@ -19,6 +19,7 @@ int* status_word();
 
 void count_launch();
 void count_tiled_launch();     // launches of the TMA-tiled kernels only (tests use it to see which path ran)
+void count_tensor_launch();    // of those, the sweeps on the tensor cores
 
 #define CA_CHECK_LAUNCH(what)                                        \
     do {                                                             \

@@ -776,6 +776,7 @@ inline int split_prepare(const Geo& g, float scale, int dist, const float* packe
         if (rc__) return rc__;                                                        \
         KERNEL<<<(L).grid, (L).threads, (L).smem, st>>>(a, (L).mv);                   \
         count_tiled_launch();                                                         \
+        count_tensor_launch();                                                        \
     } while (0)
 
 }  // namespace

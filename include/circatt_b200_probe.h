@@ -19,6 +19,9 @@ int64_t ca_probe_launch_count(void);
  * on the generic kernels). */
 int64_t ca_probe_tiled_launch_count(void);
 
+/* Of those, the sweeps on the tensor cores. */
+int64_t ca_probe_tensor_launch_count(void);
+
 /* Launches one kernel of `blocks` x 256 threads; each thread runs `iters`
  * rounds of 16 independent packed FP32 FMAs (fma.rn.f32x2) on registers and
  * stores one value to `sink` (blocks*256 floats).  The kernel executes
