@@ -154,26 +154,30 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
 
 }  // namespace
 
+// Whether the tiles of 32 rows of the FMA kernels leave a sixteenth of their lanes idle on this image.
+static bool idle_rows(const Geo& g) { return 16 * ((32 - g.H % 32) % 32) >= g.H; }
+
 // Units of one slab (more channels would need their results in registers for 32 or 64 channels), windows up to 25 (four tiles a
-// column), and enough pixels to fill the chip: a few are done sooner in the smaller tiles of the FMA kernels (train, 100 x 90,
-// 1 unit, ws 11: under 89 and 109 us; 64 x 64, 3 units: 89 and 87).
-// dk/dv from window 9 on, and at 7 on grids of up to 2^18 pixels: what a warp spends outside its steps, and the scores outside the
-// window, weigh more the shorter it is.  FMA pipe and tensor cores: 500 x 400, 8 units: ws 5 289 and 358 us, 7: 431 and 418,
-// 9: 588 and 480, 13: 1022 and 817; 512 x 512, 8 units: ws 7 555 and 540, ws 21 2966 and 1720; 200 x 180, 4 units: ws 5 40 and
-// 43, 7: 59 and 50, 9: 90 and 56.
+// column), and enough pixels to fill the chip: 12000 is on the safe side (forward and backward on the FMA pipe and here, us: 64 x 64, 2
+// units, ws 9: 33 and 31, ws 21: 65 and 52).
+// dk/dv from window 9 on, in bfloat16 from 7; in Float32 at 7 where the FMA kernels have idle rows and up to 2^18 pixels.  What a warp
+// spends outside its steps, and the scores outside the window, weigh more the shorter it is.  Backward with the FMA pipe's dk/dv and
+// with this one (dq on the FMA pipe), us: ws 7: 200 x 180, 4 units 104 and 99, 97 x 400, 4 units 119 and 114, 256 x 256, 4 units 152 and 158,
+// 500 x 400, 8 units 814 and 837; bfloat16: 256 x 256, 4 units 158 and 143, 512 x 512, 8 units 1092 and 1011; ws 9: 256 x 256, 4 units 200
+// and 186, 512 x 512, 8 units 1379 and 1307; ws 11: 260 and 248, 1808 and 1803; ws 13: 346 and 297, 2317 and 2127.
 bool split_dkdv_ok(const Geo& g, float scale) {
     const int64_t pixels = (int64_t)g.Np * g.units;
     return tiled_shape_ok(g) && g.wsw == g.ws && slabs_of(g) == 1 && split_tiles(g) <= 4 && scale > 0.f && g.Wk <= 65535 && pixels > 12000 &&
-           (g.ws >= 9 || (g.ws == 7 && pixels <= (1 << 18)));
+           (g.ws >= 9 || (g.ws == 7 && (g.bf16 || (idle_rows(g) && pixels <= (1 << 18)))));
 }
 
-// Forward, A's values and dq, which share the packed (k|v): window 9, whose 16 keys are two tiles exactly, and from 13 on; at 11 (18
-// keys of three tiles) where the FMA kernels' warps of 32 rows do not divide the image either.  Evaluation without and
-// with A, start and here: 200 x 180, 4 units: ws 7 43, 61 and 41, 73 us, 9: 55, 92 and 45, 92, 11: 70, 144 and 60, 121, 13:
-// 86, 172 and 66, 134; 256 x 256, 4 units: ws 7 57, 104 and 66, 116, 9: 73, 168 and 72, 145, 11: 91, 201 and 95, 189, 13:
-// 112, 252 and 104, 211.
+// Forward, A's values and dq, which share the packed (k|v): from window 13 on, in bfloat16 from 9; in Float32 at 9 and 11 where the FMA
+// kernels have idle rows.  Forward on the FMA pipe and here, us: ws 9: 256 x 256, 4 units (no idle rows) 73 and 76, 500 x 400, 8 units
+// (2 %) 361 and 378, 1001 x 300, 4 units (2 %) 277 and 288, 240 x 240, 4 units (7 %) 73 and 68, 257 x 255, 4 units (12 %) 84 and 81,
+// 200 x 180, 4 units (12 %) 55 and 46; ws 11: 93 and 97, 467 and 509, 357 and 387, -, 109 and 104, 72 and 62; ws 13: 113 and 107, 578 and
+// 561, 441 and 427, -, 134 and 113, 87 and 67; bfloat16, ws 9: 71 and 63, 363 and 326, 280 and 249, -, 82 and 67, 54 and 40.
 bool split_shape_ok(const Geo& g, float scale) {
-    return split_dkdv_ok(g, scale) && g.ws >= 9 && (g.ws != 11 || g.H % 32 != 0);
+    return split_dkdv_ok(g, scale) && (g.ws >= 13 || (g.ws >= 9 && (g.bf16 || idle_rows(g))));
 }
 
 int launch_split_pack(const Geo& g, float scale, int dist, const float* x0, const float* x1, const float* stats, const float* y, const float* Din,
