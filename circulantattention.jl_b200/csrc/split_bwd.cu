@@ -291,7 +291,7 @@ struct DkdvSweep : BwdSweep<NT, LO> {
         const int top = max(c1.top[0], c1.top[1]);
         const int upper = __reduce_max_sync(0xffffffffu, lane < 16 ? top : 0), lower = __reduce_max_sync(0xffffffffu, lane < 16 ? 0 : top);
         norm = max(upper, lower);
-        Seen::clear(bad || (min(upper, lower) && abs(upper - lower) > 4));
+        Seen::clear(bad || (min(upper, lower) && abs(upper - lower) > 2));
 #pragma unroll
         for (int t = 0; t < NT; ++t) mk[t] = pair(window_mask(lane, g.p, t, 0), window_mask(lane, g.p, t, 1));
 #pragma unroll

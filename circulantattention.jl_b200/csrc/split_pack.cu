@@ -5,9 +5,8 @@
 namespace ca {
 namespace {
 
-// Whether the halves would lose bits of a whole row of the lane's group of eight (`small`; with one channel a row is a single number, which
-// may be any) or of a whole channel of it (`channels`: of few rows that are not zero, as at the end of a column, a channel may be
-// any small numbers, too).
+// Whether the halves would lose bits of a whole row of the lane's group of eight (`small`) or of a whole channel of it (`channels`: of few
+// rows that are not zero, as at the end of a column, a channel may be any small numbers).
 __device__ __forceinline__ bool marked(const float (&x)[16], bool small, bool channels, float inv, float least) {
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
@@ -18,6 +17,12 @@ __device__ __forceinline__ bool marked(const float (&x)[16], bool small, bool ch
     }
     return __ballot_sync(0xffffffffu, small) >> (threadIdx.x & 24) & 255u;
 }
+
+// How far the rows of a group may be apart, in the bits of a float: 2^6, since the bound of the gradients' weights is the group's and
+// windows of 9 rows fit between lines that leave no group without a large row (57 x 54, 4 units, ws 9, every 12th row of dy and v times 3000:
+// dq between them 3.1e-5 off without this, 3.4e-7 with it, FMA pipe 4.9e-7).  Rows of two and three channels may be any small numbers
+// more often, and give only what the halves need; those of one channel nothing.
+__device__ __forceinline__ uint32_t row_span(int channels) { return channels >= 4 ? 6u << 23 : channels > 1 ? 13u << 23 : 0x7f000000u; }
 
 // A block gathers 128 packed rows of one column of one unit: a thread reads the 16 channels of its row of both tensors
 // (consecutive lanes on consecutive rows: coalesced planar loads, all in flight together), the largest magnitude of each
@@ -85,6 +90,7 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
     int ex[2];
     float inv[2];
     bool small[2], channels[2], look = false;
+    const uint32_t span = row_span(g.cr);
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         uint32_t m = 0;
@@ -99,7 +105,8 @@ __global__ void __launch_bounds__(128, 6) split_pack_kernel(SplitPackArgs a) {
         for (int d = 1; d < 8; d <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
         ex[t] = m ? scale_exp(m, 4, t == 0 ? kLeastExp : 0) : 0;
         inv[t] = exp_inverse(ex[t] == 255 ? 0 : ex[t]);
-        small[t] = g.cr > 1 && mine >= kLeastNormal && __uint_as_float(mine) * inv[t] < least_value(LO);
+        // a row far below the group's largest, or a group below the least scale
+        small[t] = mine >= kLeastNormal && (mine + span < m || __uint_as_float(m) * inv[t] < 64.f * least_value(LO));
         // a channel of small numbers has one in all eight rows, which is rare
         const uint32_t rows = __ballot_sync(0xffffffffu, low * inv[t] < least_value(LO)) >> (rl & 24) & 255u;
         const uint32_t filled = __ballot_sync(0xffffffffu, mine) >> (rl & 24) & 255u;

@@ -54,6 +54,25 @@ def test_a_small_channel(ca, which, simname):
         assert_close(got[name][:, :, 3::16], want[name][:, :, 3::16], name)
 
 
+@pytest.mark.parametrize("simname", ["dot", "distance"])
+@pytest.mark.parametrize("mul", [20, 3000])
+@pytest.mark.parametrize("each", [10, 13])
+def test_between_large_lines(ca, each, mul, simname):
+    """Every group of eight rows that a warp meets may hold a large row, and the windows between the lines none.  A Float32 sum of 81
+    terms of mixed signs, of weights with some 2^-22 of error each, is within 1e-6 of its norm."""
+    t, ws = tensors(77), 9
+    for name in "vr":
+        t[name][::each] *= np.float32(mul)
+    got, want = run(ca, simname, *t.values(), ws, HEADS), oracle(simname, *t.values(), ws, HEADS)
+    lines = np.zeros(SHAPE[0], bool)
+    lines[::each] = True
+    between = ~np.any([np.roll(lines, d) for d in range(-(ws // 2), ws // 2 + 1)], axis=0)
+    assert between.any()
+    for name in got:
+        err = np.linalg.norm(got[name][between] - want[name][between]) / np.linalg.norm(want[name][between])
+        assert err < 1e-6, f"{name}: {err:.3g}"
+
+
 @pytest.mark.parametrize("which", ["k", "v", "r"])
 def test_a_large_half(ca, which):
     t = tensors(73)
