@@ -8,34 +8,35 @@
 // tcgen05 is not used: its scores would leave and enter through tensor memory for the mask, the exponential and the
 // split, which costs more than its rate gains at 16 to 64 channels (forward 70.6 us against 62.5 on the FMA pipe).
 //
-// Error against 64 bits (2-norm, standard normal; FMA pipe and here): 64 x 48, 2 units, ws 15: y 5.7e-7 and 2.4e-7, dq 5.8e-7 and
-// 4.1e-7, dk 5.5e-7 and 4.0e-7, dv 5.5e-7 and 4.1e-7; 40 x 37, 4 units, ws 21, Distance: 6.4e-7 and 2.7e-7, 9.0e-7 and 4.9e-7,
-// 7.2e-7 and 4.6e-7, 6.7e-7 and 4.4e-7; 24 x 24, 2 units of 4 channels, ws 3: 2.6e-7 and 1.6e-7, 4.8e-7 and 4.4e-7, 4.6e-7 and
-// 4.3e-7, 4.2e-7 and 4.2e-7.
+// Error against 64 bits (2-norm, standard normal, 57 x 54; y, dq, dk, dv in 1e-7, FMA pipe with 3 units and here with 4): ws 9, 8 channels
+// 4.2, 4.6, 4.0, 3.7 and 2.2, 3.9, 3.7, 3.8, Distance 4.8, 6.6, 4.3, 3.9 and 2.2, 4.3, 3.9, 3.8; ws 11, 16 channels 5.6, 5.1, 4.7, 4.4 and
+// 2.3, 3.8, 3.7, 3.7, Distance 6.1, 8.2, 5.1, 4.7 and 2.5, 4.5, 4.1, 4.0; ws 21, 16 channels 6.0, 6.3, 6.1, 6.1 and 2.7, 3.9, 3.8, 3.6,
+// Distance 6.5, 8.7, 6.6, 6.2 and 2.7, 5.4, 4.6, 4.2.
 //
 // Tiles.  Rows of a product are 16 centre pixels: 8 rows (h) of two neighbouring columns (w), whose windows share all but two
 // columns.  Columns are 8 pixels of the streamed column, so a window column takes NT = ceil((8 + 2p) / 8) tiles and 62 %
-// (window 21) to 44 % (window 7) of the scores are inside the window; 16 rows of one column would leave 52 and 29 %.
+// (window 21) to 38 % (window 7) of the scores are inside the window; 16 rows of one column would leave 52 and 29 %.
 // The mask costs nothing: it rides in the addend of the FMA that scales a score (-inf outside).
 //
 // Streamed rows.  [unit][column][row'][144 bytes] = hi then lo of the first tensor, hi then lo of the second, 16 bytes of
 // scalars; row' = h + p with the circular halo unrolled.  bfloat16 tensors have no lower halves, and their rows no place for
-// them: 80 bytes.  Either pitch is an odd number of 16-byte words, so ldmatrix reads eight rows without bank conflicts.  The power of two is common to a group of eight rows starting at a multiple of eight
-// (a warp's window starts at one), so it is uniform over a tile.  It puts the group's largest magnitude into [2^11, 2^15): an
-// element 2^13 below it keeps all bits, the least step is 2^-36 of the largest.
+// them: 80 bytes.  Either pitch is an odd number of 16-byte words, so ldmatrix reads eight rows without bank conflicts.  The power of
+// two is common to a group of eight rows starting at a multiple of eight (a warp's window starts at one), so it is uniform over a
+// tile.  It puts the group's largest magnitude into [2^11, 2^15): an element 2^13 below it keeps all bits, the least step is 2^-36 of
+// the largest.
 //
 // Range.  Half pairs end at a fixed step, so large values would cost pixels whose window does not hold them: their operands when
 // they share a group, their weights when they share a step.  A warp therefore recomputes its pixels from the tensors in Float32
 // (exact_*) when one of its groups is marked (a NaN or an infinity, which a product of a tile would carry to pixels outside their
-// window; a row or a channel too far below the group's largest for its bits, see kLeastValue; magnitudes below 2^-57 in a score's
-// operand) or when the scales of its groups lie further apart than the sweep's weights have bits for (Seen).  Tensors whose
+// window; a row or a channel too far below the group's largest; magnitudes below 2^-51 in a score's operand; split_pack.cu has the
+// limits) or when the scales of its groups lie further apart than the sweep's weights have bits for (Seen).  Tensors whose
 // magnitudes are alike within a window, or zero, meet neither.  One pixel of k times 1e2, 1e4, 1e6 (57 x 54, 4 units, ws 11), error of
 // dq of the pixels whose windows do not hold it: 8.4e-7, 1.2e-5, 3.1e-3 without this and 4.0e-7, 3.7e-7, 3.7e-7 with it, FMA pipe
 // 5.5e-7.  Where every warp recomputes (512 x 512, 8 units, ws 21, 2 % of v's pixels NaN) the forward takes 5.9 ms for 1.1, dq 7.1 for
 // 1.4, dk/dv 8.9 for 1.9 (310, 379, 707 with a lane per pixel and loads from the tensors); one pixel in 10^4 times 1e6: 1.7, 2.1, 4.1.
 //
-// What bounds the sweeps (256 x 256, 8 units, ws 21): the tensor pipe is busy in 47 % (forward) to 54 % (dk/dv) of the cycles, an
-// instruction issues in 48 and 45 %; an mma also takes five issue slots from FMAs and waits behind them, and 12 to 16 warps of
+// What bounds the sweeps (512 x 512, 8 units, ws 21): the tensor pipe is busy in 47 % (forward) to 54 % (dq, dk/dv) of the cycles, an
+// instruction issues in 48 and 45 % (bfloat16: 29 to 37 %, 58 %); an mma also takes five issue slots from FMAs and waits behind them, and 12 to 16 warps of
 // 128 to 168 registers do not cover the latencies of the chain score - exponential - split - sum.  Times are beside the rules of
 // the dispatch (split_pack.cu).
 #pragma once

@@ -34,8 +34,9 @@
 // chain, and the forward only touches the maximum when the sign bits of a chunk
 // of relative scores say that one of them is positive.
 //
-// Softmax on 2-D windows from 9 to 25 at up to 16 real channels per unit runs on the tensor cores instead (split.cuh; split_shape_ok
-// and split_dkdv_ok have the rules).
+// Softmax at up to 16 real channels per unit on more than 12000 pixels x units runs on the tensor cores instead (split.cuh) where they are
+// faster: windows 13 to 25, 9 and 11 in bfloat16 or where tiles of 32 rows would leave lanes idle, dk/dv also at all of 9 to 25 and at some
+// of 7 (split_shape_ok and split_dkdv_ok have the rules and what they rest on).
 //
 // Small grids.  Where it pays, the column stages of a tile are split between up to four groups of warps of the same CTA
 // (each with its own copy pipeline) whose partial results are merged through shared memory.

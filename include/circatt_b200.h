@@ -136,7 +136,9 @@ int ca_apply(const ca_desc* d, const float* nz, const void* v, void* out,
  * ca_attention_fwd_workspace() bytes (may be NULL when that is 0); the tiled
  * sm_100a kernels keep their packed copies of k and v there.  A NULL workspace
  * where one is needed selects the slower untiled kernels (softmax) or is an
- * error (entmax without nz). */
+ * error (entmax without nz).  Accuracy is that of Float32 sums.  Larger softmax
+ * problems run on the tensor cores; pixels whose windows hold magnitudes too
+ * far apart for that are recomputed in Float32 by a slower path. */
 size_t ca_attention_fwd_workspace(const ca_desc* d, int32_t want_nz);
 int ca_attention_fwd(const ca_desc* d, const void* q, const void* k, const void* v,
                      void* y, float* nz, float* stats, void* workspace, void* stream);
